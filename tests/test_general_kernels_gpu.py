@@ -1,0 +1,54 @@
+"""The kernels of the 32-bit form and the general attention at the edges of their tiles, splits and load widths."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("aligned", [True, False])
+@pytest.mark.parametrize("M,N,K", [(1, 4, 4), (2, 7, 513), (3, 130, 2049), (4, 33, 512), (5, 4, 1030), (8, 200, 511), (9, 128, 256), (63, 129, 2048),
+                                   (64, 127, 260), (65, 256, 1027), (129, 5, 4096), (400, 300, 777)])
+def test_f32_linear_at_tile_and_split_edges(M, N, K, aligned):
+    """Rows of the streaming kernel (up to 2, 4, 8), 64 x 128 tiles, K split over a cluster; 16-byte and 4-byte loads.  A sum of K
+    products of random signs carries at most about sqrt(K) / 2 roundings of 6e-8 relative to its own size: 2e-6 at K = 4,096."""
+    from mojo_linuxperiments_b200.ops import dense as D
+    g = torch.Generator(device=DEV).manual_seed(M * 7919 + N)
+    pad = 0 if aligned else 1
+    ld = (K + 3) // 4 * 4 + pad
+    x = torch.full((M, ld + pad), float("nan"), device=DEV)[:, pad:]           # what lies beyond K must not matter
+    x[:, :K] = torch.randn((M, K), generator=g, device=DEV)
+    w = torch.full((N, ld + pad), float("nan"), device=DEV)[:, pad:]
+    w[:, :K] = torch.randn((N, K), generator=g, device=DEV) * K ** -0.5
+    y = D.linear(x, D.DenseW(w, N, K))[:, :N]
+    want = x[:, :K].double() @ w[:, :K].double().t()
+    assert (y.double() - want).norm() <= 2e-6 * want.norm()
+    assert (y.double() - want).abs().max() <= 2e-5 * want.abs().max().clamp_min(1.0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dk,dv,chunk", [(10, 6, None), (8, 8, 40), (130, 516, None), (36, 644, 100)])
+def test_general_attention_with_uneven_head_sizes(dk, dv, chunk, dtype):
+    """Head sizes that are no multiple of four, several parts of value dimensions, one to several blocks of keys per warp."""
+    from mojo_linuxperiments_b200.ops import attention as A
+    H, G, n, ps = 4, 2, 300, 16
+    g = torch.Generator(device=DEV).manual_seed(dk)
+    cache = A.PagedKVCache(32, G, ps, DEV, dk=dk, dv=dv, dtype=dtype)
+    cache.data.normal_(generator=g)
+    table = torch.randperm(32, generator=torch.Generator().manual_seed(1))[:20].to(torch.int32).view(1, 20).to(DEV)
+    where = [0, 1, 31, 32, 33, 127, 128, 129, 255, n - 1]
+    pos = torch.tensor(where, dtype=torch.int32, device=DEV)
+    q = torch.randn((len(where), H * dk), generator=g, device=DEV).to(dtype)
+    sink = torch.randn(H, generator=g, device=DEV)
+    out = torch.full((len(where), H * dv), float("nan"), dtype=dtype, device=DEV)
+    A.attn_paged(q, H, pos, torch.zeros_like(pos), cache, table, A.attn_spec(dk ** -0.5, chunk=chunk, sink=sink), out)
+    page, row = table[0].long()[torch.arange(n, device=DEV) // ps], torch.arange(n, device=DEV) % ps
+    k, v = cache.keys()[page, :, row].double(), cache.values()[page, :, row].double()
+    for i, p in enumerate(where):
+        lo = p // chunk * chunk if chunk else 0
+        kk, vv = (t[lo:p + 1].repeat_interleave(H // G, 1) for t in (k, v))
+        s = torch.einsum("hd,jhd->hj", q[i].double().view(H, dk), kk) * dk ** -0.5
+        s = torch.cat([s, sink.double()[:, None]], 1).softmax(-1)[:, :-1]
+        want = torch.einsum("hj,jhd->hd", s, vv).reshape(-1)
+        # fp32 sums of up to 300 terms of size one; a bf16 result is rounded once (2^-9 of values up to 5)
+        assert (out[i].double() - want).abs().max().item() < (1e-5 if dtype == torch.float32 else 1.2e-2), p
