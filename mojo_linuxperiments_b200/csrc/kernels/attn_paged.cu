@@ -1,9 +1,11 @@
-// General attention over a paged cache, bf16 or fp32, any head size: one warp per (query token, query head).
+// General attention over a paged cache, bf16 or fp32, any head size: one CTA of four warps per (query token, query head).
 //
-// The 32-bit form of a model and head sizes beyond the tensor-core kernels run here.  Keys are taken 32 at a time (lane <->
-// key, exact dot product in fp32), online softmax per block of 32, then the lanes share out the value dimensions (512 at a
-// time; blockIdx.z picks the part).  The latent form reads the query in two parts and takes the first dimensions of a
-// cached key as its value.
+// The 32-bit form of a model and head sizes beyond the tensor-core kernels run here.  Blocks of 32 keys go to the warps in turn.
+// Scores: eight lanes per key, four elements each at a time, so that a load of the warp covers whole lines of four keys (a
+// lane per key touched 32 lines for four bytes each); fp32 sums, added across the eight lanes.  Then an online softmax per
+// block, the lanes share out the value dimensions (512 at a time; blockIdx.y picks the part), and the warps' sums are merged
+// through shared memory.  The latent form reads the query in two parts and takes the first dimensions of a cached key as its
+// value.  Bound by latency in decoding (few CTAs), by the cache lines of keys and values in prefill.
 #include "ptx.cuh"
 #include "api.h"
 #include "launch.cuh"
@@ -13,9 +15,22 @@ namespace b200 {
 template <typename T> __device__ __forceinline__ float ap_f(T v);
 template <> __device__ __forceinline__ float ap_f<float>(float v) { return v; }
 template <> __device__ __forceinline__ float ap_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
+// up to four neighbouring elements of a row that has n left; VEC: rows start on 16 bytes (fp32) or 8 (bf16) and n >= 4
+template <bool VEC, typename T>
+__device__ __forceinline__ float4 ap_f4(const T* p, int n) {
+  if constexpr (VEC && sizeof(T) == 4) return *reinterpret_cast<const float4*>(p);
+  if constexpr (VEC && sizeof(T) == 2) {
+    const uint2 r = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+  }
+  return make_float4(ap_f(p[0]), n > 1 ? ap_f(p[1]) : 0.f, n > 2 ? ap_f(p[2]) : 0.f, n > 3 ? ap_f(p[3]) : 0.f);
+}
 
 constexpr int APG_WARPS = 4;
 constexpr int APG_MAX_DV = 512;
+constexpr int APG_DV4 = APG_MAX_DV / 128;      // groups of four value dimensions a lane may hold
 
 struct AttnPagedParams {
   const void* q; long long ldq;
@@ -30,49 +45,66 @@ struct AttnPagedParams {
   int* status;
 };
 
-template <typename T>
+template <typename T, bool VEC>
 __global__ void __launch_bounds__(32 * APG_WARPS) attn_paged_kernel(const __grid_constant__ AttnPagedParams p) {
+  extern __shared__ __align__(16) float apg_q[];        // the query in fp32, [dk rounded up to four], zeros at the end
+  __shared__ float part_ml[APG_WARPS][2];
+  __shared__ __align__(16) float part_acc[APG_WARPS][APG_MAX_DV];
   pdl_launch_dependents();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.y * APG_WARPS + warp, tok = blockIdx.x;
-  if (h >= p.hq) return;
-  const int dk = p.c.dk, dv = p.dv, ps = p.c.page_size, d0 = blockIdx.z * APG_MAX_DV;
+  const int tok = blockIdx.x / p.hq, h = blockIdx.x % p.hq;
+  const int dk = p.c.dk, dv = p.dv, ps = p.c.page_size, d0 = blockIdx.y * APG_MAX_DV, dn = min(dv - d0, APG_MAX_DV);
   const int seq = p.seq_ids ? p.seq_ids[tok] : tok;
-  T* o = static_cast<T*>(p.out) + static_cast<size_t>(tok) * p.ldo + static_cast<size_t>(h) * dv;
+  T* o = static_cast<T*>(p.out) + static_cast<size_t>(tok) * p.ldo + static_cast<size_t>(h) * dv + d0;
   const int pos = p.positions[tok];
   const bool empty = p.seq_lens && p.seq_lens[tok] <= 0;            // decode over a slot without a sequence
   const bool bad = pos < 0 || seq < 0 || seq >= p.c.num_seqs || pos / ps >= p.c.max_pages;
   if (bad || empty) {
-    if (bad && lane == 0 && p.status) atomicCAS(p.status, 0, static_cast<int>(ST_BAD_ARGUMENT) | (14 << 8));
-    for (int d = d0 + lane; d < min(dv, d0 + APG_MAX_DV); d += 32) o[d] = T(0.f);
+    if (bad && threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, static_cast<int>(ST_BAD_ARGUMENT) | (14 << 8));
+    for (int d = threadIdx.x; d < dn; d += 32 * APG_WARPS) o[d] = T(0.f);
     return;
   }
   const int kvh = h / (p.hq / p.c.kv_heads);
   const T* q = static_cast<const T*>(p.q) + static_cast<size_t>(tok) * p.ldq + static_cast<size_t>(h) * p.q_head;
   const T* q2 = static_cast<const T*>(p.q2) + static_cast<size_t>(tok) * p.ldq2 + static_cast<size_t>(h) * p.q2_head;
+  for (int d = threadIdx.x; d < ((dk + 3) & ~3); d += 32 * APG_WARPS) apg_q[d] = d < p.q_len ? ap_f(q[d]) : d < dk ? ap_f(q2[d - p.q_len]) : 0.f;
+  __syncthreads();
   const int* pt = p.c.page_table + static_cast<size_t>(seq) * p.c.max_pages;
   const size_t rec = static_cast<size_t>(p.c.kv_heads) * ps * (dk + (p.latent ? 0 : dv));
   const int vp = p.latent ? dk : dv;                                 // pitch of the value rows
   const T* cache = static_cast<const T*>(p.c.data);
   const int first = p.s.chunk > 0 ? pos - pos % p.s.chunk : 0;
-  // the sink opens the softmax: a term of the denominator without a value
-  float m = p.s.sink ? p.s.sink[h] : -INFINITY, l = p.s.sink ? 1.f : 0.f;
-  float acc[APG_MAX_DV / 32];
+  // the sink opens the softmax: a term of the denominator without a value (one warp counts it)
+  float m = p.s.sink && warp == 0 ? p.s.sink[h] : -INFINITY, l = p.s.sink && warp == 0 ? 1.f : 0.f;
+  float4 acc[APG_DV4];
 #pragma unroll
-  for (int i = 0; i < APG_MAX_DV / 32; ++i) acc[i] = 0.f;
-  for (int k0 = first; k0 <= pos; k0 += 32) {
+  for (int i = 0; i < APG_DV4; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int sub = lane >> 3, at = (lane & 7) * 4;                    // key of a group of four, first element of this lane
+  for (int k0 = first + 32 * warp; k0 <= pos; k0 += 32 * APG_WARPS) {
     const int key = k0 + lane;
+    const int page = key <= pos ? pt[key / ps] : -1;
+    // this lane's key: its row among all rows of its kind, or -1
+    const bool there = page >= 0 && page < p.c.num_pages;
+    const long long row = there ? static_cast<long long>(kvh) * ps + key % ps : 0;
+    const long long koff = there ? static_cast<long long>(page) * rec + row * dk : -1;
+    const long long voff = there ? static_cast<long long>(page) * rec + (p.latent ? 0 : static_cast<long long>(p.c.kv_heads) * ps * dk) + row * vp + d0 : -1;
     float s = -INFINITY;
-    if (key <= pos) {
-      const int page = pt[key / ps];
-      if (page >= 0 && page < p.c.num_pages) {
-        const T* kr = cache + static_cast<size_t>(page) * rec + (static_cast<size_t>(kvh) * ps + key % ps) * dk;
-        float d = 0.f;
-        for (int i = 0; i < p.q_len; ++i) d = fmaf(ap_f(q[i]), ap_f(kr[i]), d);
-        for (int i = p.q_len; i < dk; ++i) d = fmaf(ap_f(q2[i - p.q_len]), ap_f(kr[i]), d);
-        s = d * p.s.scale;
-      }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const long long ko = __shfl_sync(0xffffffffu, koff, 4 * j + sub);
+      float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (ko >= 0)
+        for (int i = at; i < dk; i += 32) {
+          const float4 kv = ap_f4<VEC>(cache + ko + i, dk - i), qv = *reinterpret_cast<const float4*>(apg_q + i);
+          d.x = fmaf(qv.x, kv.x, d.x); d.y = fmaf(qv.y, kv.y, d.y); d.z = fmaf(qv.z, kv.z, d.z); d.w = fmaf(qv.w, kv.w, d.w);
+        }
+      float t = (d.x + d.y) + (d.z + d.w);
+      t += __shfl_xor_sync(0xffffffffu, t, 1);
+      t += __shfl_xor_sync(0xffffffffu, t, 2);
+      t += __shfl_xor_sync(0xffffffffu, t, 4);
+      t = __shfl_sync(0xffffffffu, t, (lane & 3) * 8);               // key 4 j + (lane & 3)
+      if ((lane >> 2) == j && there) s = t * p.s.scale;
     }
     float mx = s;
 #pragma unroll
@@ -87,36 +119,69 @@ __global__ void __launch_bounds__(32 * APG_WARPS) attn_paged_kernel(const __grid
     l = l * a + sum;
     m = m_new;
 #pragma unroll
-    for (int i = 0; i < APG_MAX_DV / 32; ++i) acc[i] *= a;
+    for (int i = 0; i < APG_DV4; ++i) { acc[i].x *= a; acc[i].y *= a; acc[i].z *= a; acc[i].w *= a; }
     const int n = min(32, pos - k0 + 1);
+#pragma unroll 4
     for (int j = 0; j < n; ++j) {
       const float w = __shfl_sync(0xffffffffu, e, j);
-      const int kj = k0 + j, page = pt[kj / ps];
-      if (page < 0 || page >= p.c.num_pages) continue;
-      const T* vr = cache + static_cast<size_t>(page) * rec + (p.latent ? 0 : static_cast<size_t>(p.c.kv_heads) * ps * dk) +
-                    (static_cast<size_t>(kvh) * ps + kj % ps) * vp + d0;
+      const long long vo = __shfl_sync(0xffffffffu, voff, j);
+      if (vo < 0) continue;
 #pragma unroll
-      for (int i = 0; i < APG_MAX_DV / 32; ++i)
-        if (d0 + i * 32 + lane < dv) acc[i] = fmaf(w, ap_f(vr[i * 32 + lane]), acc[i]);
+      for (int i = 0; i < APG_DV4; ++i)
+        if (i * 128 + lane * 4 < dn) {
+          const float4 v = ap_f4<VEC>(cache + vo + i * 128 + lane * 4, dn - i * 128 - lane * 4);
+          acc[i].x = fmaf(w, v.x, acc[i].x); acc[i].y = fmaf(w, v.y, acc[i].y);
+          acc[i].z = fmaf(w, v.z, acc[i].z); acc[i].w = fmaf(w, v.w, acc[i].w);
+        }
     }
   }
-  float f = l > 0.f ? 1.f / l : 0.f;
-  if (p.s.gate) f *= 1.f / (1.f + expf(-ap_f(static_cast<const T*>(p.s.gate)[static_cast<size_t>(tok) * p.s.ldg + h])));
+  if (lane == 0) { part_ml[warp][0] = m; part_ml[warp][1] = l; }
 #pragma unroll
-  for (int i = 0; i < APG_MAX_DV / 32; ++i)
-    if (d0 + i * 32 + lane < dv) o[d0 + i * 32 + lane] = T(acc[i] * f);
+  for (int i = 0; i < APG_DV4; ++i)
+    if (i * 128 + lane * 4 < dn) *reinterpret_cast<float4*>(&part_acc[warp][i * 128 + lane * 4]) = acc[i];
+  __syncthreads();
+  float top = part_ml[0][0];
+#pragma unroll
+  for (int i = 1; i < APG_WARPS; ++i) top = fmaxf(top, part_ml[i][0]);
+  float share[APG_WARPS], total = 0.f;
+#pragma unroll
+  for (int i = 0; i < APG_WARPS; ++i) {
+    share[i] = part_ml[i][0] == -INFINITY ? 0.f : expf(part_ml[i][0] - top);
+    total += share[i] * part_ml[i][1];
+  }
+  float f = total > 0.f ? 1.f / total : 0.f;
+  if (p.s.gate) f *= 1.f / (1.f + expf(-ap_f(static_cast<const T*>(p.s.gate)[static_cast<size_t>(tok) * p.s.ldg + h])));
+  for (int d = threadIdx.x; d < dn; d += 32 * APG_WARPS) {
+    float v = 0.f;
+#pragma unroll
+    for (int i = 0; i < APG_WARPS; ++i) v += share[i] * part_acc[i][d];
+    o[d] = T(v * f);
+  }
 }
 
 }  // namespace b200
 
 using namespace b200;
 
-static int launch_attn_paged(const AttnPagedParams& p, cudaStream_t stream) {
-  const dim3 grid(p.M, (p.hq + APG_WARPS - 1) / APG_WARPS, (p.dv + APG_MAX_DV - 1) / APG_MAX_DV);
-  if (p.c.f32) launch_ex(attn_paged_kernel<float>, grid, dim3(32 * APG_WARPS), 0, stream, 0, p);
-  else launch_ex(attn_paged_kernel<__nv_bfloat16>, grid, dim3(32 * APG_WARPS), 0, stream, 0, p);
+template <typename T, bool VEC>
+static int launch_attn_paged_as(const AttnPagedParams& p, cudaStream_t stream) {
+  const size_t smem = static_cast<size_t>((p.c.dk + 3) & ~3) * sizeof(float);
+  if (smem > (32u << 10)) {            // with the static part this passes what a kernel may use unasked
+    cudaError_t e = cudaFuncSetAttribute(attn_paged_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return -1000 - static_cast<int>(e);
+  }
+  launch_ex(attn_paged_kernel<T, VEC>, dim3(static_cast<unsigned>(p.M) * p.hq, (p.dv + APG_MAX_DV - 1) / APG_MAX_DV), dim3(32 * APG_WARPS), smem,
+            stream, 0, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
+}
+
+static int launch_attn_paged(const AttnPagedParams& p, cudaStream_t stream) {
+  if (static_cast<long long>(p.M) * p.hq > 0x7fffffffll) return -3;
+  const int elem = p.c.f32 ? 4 : 2;
+  const bool vec = p.c.dk % 4 == 0 && p.dv % 4 == 0 && reinterpret_cast<uintptr_t>(p.c.data) % (4 * elem) == 0;
+  if (p.c.f32) return vec ? launch_attn_paged_as<float, true>(p, stream) : launch_attn_paged_as<float, false>(p, stream);
+  return vec ? launch_attn_paged_as<__nv_bfloat16, true>(p, stream) : launch_attn_paged_as<__nv_bfloat16, false>(p, stream);
 }
 
 extern "C" int b200_attn_paged(const void* q, long long ldq, void* out, long long ldo, int hq, int M, const int* positions,
