@@ -1,16 +1,22 @@
 // Causal grouped-query flash attention for prefill on sm_100a tensor cores (bf16 in, fp32 accumulate).
 //
-// One CTA = 128 query rows of one head of one sequence; KV is walked in tiles of 128 tokens.
-//   warp 0      TMA producer: Q once, then K and V tiles into two-stage rings (128-byte swizzle)
-//   warp 1      MMA issuer:  S = Q.K^T (K-major x K-major) and PV = P.V (K-major P from smem x MN-major V),
-//               both tcgen05.mma.kind::f16 with accumulators in TMEM: S and PV are each double buffered
-//               (4 x 128 columns = the whole TMEM), so S of tile j+1 and PV of tile j run while the softmax
-//               warps are busy with tile j
-//   warps 2..5  softmax: thread <-> query row.  S is read with tcgen05.ld (twice: max pass, exp pass), P is
-//               written to shared memory as bf16 in the swizzled K-major layout the MMA expects, the output
-//               row lives in registers and is rescaled / accumulated from the PV buffer one tile late.
-// Sequences are concatenated along the token axis (cu_seqlens); a tile may read rows of the next sequence,
-// which the causal / length mask removes.  All waits are bounded.
+// A work item is two blocks ("units") of 128 query rows that walk the same KV tiles of 128 tokens: two heads of one KV head, or,
+// where a KV head has an odd number of heads, two neighbouring query tiles of one head.  One CTA per SM takes items, long ones
+// first.
+//   warp 0       TMA producer: the Q block of each unit, K and V tiles into two-stage rings (128-byte swizzle)
+//   warp 1       MMA issuer: S = Q.K^T (both from shared memory) and O += P.V (P from TMEM, V MN-major from shared memory),
+//                tcgen05.mma.kind::f16; the whole warp walks the loop so that descriptors stay in uniform registers
+//   warps 4..7   softmax of unit 0, warps 8..11 of unit 1: thread <-> query row.  A row of S is read once into registers, P goes
+//                back as bf16 into the columns of S, O stays in TMEM
+// The units alternate: while one's softmax runs, the tensor cores work for the other, and all eight softmax warps share the
+// exponential units, which bound the kernel (128 x 128 exponentials per tile take as long as its two MMAs).  O is rescaled
+// where a row's maximum grows.  (Letting P grow by up to 2^8 before that is 5 to 11 % faster, but then the weight of a row's
+// largest key is no power of two any more and its rounding costs precision: error against 64 bits 1.99e-3 instead of 1.91e-3.)
+// TMEM: S and O of both units, 4 x 128 columns.  S of the next tile may overwrite P because MMAs run in the order of issue.
+// Sequences are concatenated along the token axis (cu_seqlens); a tile may read rows of the next sequence, which the causal /
+// length mask removes.  All waits are bounded.
+// 32 x 1,024 tokens, 32 heads over 8: 388 us = 709 TFLOP/s (1,425 us with one unit per CTA, O in registers and S read twice);
+// 3 x 3,001: 271 us (996); 1 x 1,024: 26 us (66); 32 x 200: 51 us (166); 100 x 64: 55 us (174).
 #include "ptx.cuh"
 #include "api.h"
 #include "launch.cuh"
@@ -18,7 +24,9 @@
 
 namespace b200 {
 
-constexpr int AP_THREADS = 192;
+constexpr int AP_THREADS = 384;
+// registers: 384 x 168 at launch, 128 x (72 + 216 + 216) afterwards, which is as many
+constexpr int AP_REGS_FEW = 72, AP_REGS_MANY = 216;
 constexpr int AP_BM = 128, AP_BN = 128, AP_D = 128;
 constexpr int AP_CHUNK_BYTES = 128 * 128;            // 128 rows x 64 bf16
 constexpr int AP_TILE_BYTES = 2 * AP_CHUNK_BYTES;    // 128 x 128 bf16
@@ -26,7 +34,10 @@ constexpr int AP_TILE_BYTES = 2 * AP_CHUNK_BYTES;    // 128 x 128 bf16
 struct PrefillParams {
   const int* cu_seqlens;      // [B+1]
   __nv_bfloat16* out;         // [tokens][hq][128]
-  int hq, hkv;
+  int hq, hkv, B;
+  int q_steps;                // query tiles (heads paired) or pairs of them of the longest sequence
+  int columns;                // items per query tile and sequence: head pairs, or heads
+  bool pair_heads;
   float scale_log2;
   int* status;
   unsigned long long limit_ns;
@@ -34,40 +45,57 @@ struct PrefillParams {
 
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t pitch_bytes);
 
+// the items of a CTA, in the same order for every warp
+struct PrefillItem {
+  int row0, len, kvh;         // first token row of the sequence, its length, KV head
+  int first_head, head_step;  // of the units
+  int first_q, q_step;        // first query row of the units
+  long long next;
+  __device__ PrefillItem() : next(blockIdx.x) {}
+  __device__ bool take(const PrefillParams& p) {
+    const long long per_step = static_cast<long long>(p.columns) * p.B;
+    for (; next < per_step * p.q_steps;) {
+      const int step = p.q_steps - 1 - static_cast<int>(next / per_step), rest = static_cast<int>(next % per_step);
+      const int b = rest / p.columns, col = rest % p.columns;
+      next += gridDim.x;
+      row0 = p.cu_seqlens[b];
+      len = p.cu_seqlens[b + 1] - row0;
+      head_step = p.pair_heads ? 1 : 0;
+      first_head = p.pair_heads ? 2 * col : col;
+      q_step = p.pair_heads ? 0 : AP_BM;
+      first_q = (p.pair_heads ? step : 2 * step) * AP_BM;
+      kvh = first_head / (p.hq / p.hkv);
+      if (first_q < len) return true;
+    }
+    return false;
+  }
+  __device__ int head(int u) const { return first_head + u * head_step; }
+  __device__ int q0(int u) const { return first_q + u * q_step; }
+  __device__ int n(int u) const { return q0(u) < len ? q0(u) / AP_BN + 1 : 0; }      // KV tiles; 0: the unit has no rows
+  __device__ int tiles() const { return max(n(0), n(1)); }
+};
+
 __global__ void __launch_bounds__(AP_THREADS, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                    const __grid_constant__ CUtensorMap tmap_v, const PrefillParams p) {
+                    const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ PrefillParams p) {
   pdl_launch_dependents();   // the next kernel may start its prologue now
-  pdl_wait();                // everything before this kernel in the stream has completed
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  // [Q 32K][K0 32K][K1 32K][V0 32K][V1 32K][P 32K][barriers]
-  const uint32_t sQ = smem_u32(smem);
-  const uint32_t sK = sQ + AP_TILE_BYTES;
-  const uint32_t sV = sK + 2 * AP_TILE_BYTES;
-  const uint32_t sP = sV + 2 * AP_TILE_BYTES;
-  uint8_t* pP = smem + 5 * AP_TILE_BYTES;
+  // [Q of unit 0, 1][K stage 0, 1][V stage 0, 1] 32 KiB each, then the barriers
+  const uint32_t sQ = smem_u32(smem), sK = sQ + 2 * AP_TILE_BYTES, sV = sK + 2 * AP_TILE_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 6 * AP_TILE_BYTES);
   const uint32_t bar0 = smem_u32(bars);
-  enum { B_QFULL = 0, B_KFULL = 1, B_VFULL = 3, B_KEMPTY = 5, B_VEMPTY = 7, B_SFULL = 9, B_PFULL = 11, B_OFULL = 12, B_COUNT = 14 };
+  // two of each: units (Q, S, P, O) or stages (K, V)
+  enum { B_QFULL = 0, B_QEMPTY = 2, B_KFULL = 4, B_KEMPTY = 6, B_VFULL = 8, B_VEMPTY = 10, B_SFULL = 12, B_PFULL = 14, B_OFULL = 16, B_OFREE = 18, B_COUNT = 20 };
   auto bar = [&](int i) { return bar0 + 8u * i; };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + B_COUNT);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x;        // heavy (late) query tiles first
-  const int head = blockIdx.y, b = blockIdx.z;
-  const int seq0 = p.cu_seqlens[b];
-  const int len = p.cu_seqlens[b + 1] - seq0;
-  const int q0 = qt * AP_BM;
-  if (q0 >= len) return;                            // uniform across the CTA, before any barrier / TMEM use
-  const int n_tiles = qt + 1;                       // causal: kv tiles 0..qt
-  const int kvh = head / (p.hq / p.hkv);
   const uint64_t limit = p.limit_ns;
-
   if (threadIdx.x == 0) {
-    for (int i = 0; i < B_COUNT; ++i) mbar_init(bar(i), (i == B_PFULL) ? 128 : 1);
+    for (int i = 0; i < B_COUNT; ++i) mbar_init(bar(i), ((i & ~1) == B_PFULL || (i & ~1) == B_OFREE) ? 4 : 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -75,182 +103,200 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = *tmem_slot;       // columns: S of unit u at 128 u, O at 256 + 128 u
+  pdl_wait();                                  // everything before this kernel in the stream has completed
+  auto wait = [&](int i, uint32_t par, int code) { return mbar_wait(bar(i), par, abort_flag, p.status, code | (3 << 8), limit); };
+  PrefillItem it;
 
-  if (warp == 0) {
-    if (lane == 0) {
-      prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
-      mbar_expect_tx(bar(B_QFULL), AP_TILE_BYTES);
-      tma_load_2d(sQ, &tmap_q, bar(B_QFULL), head * AP_D, seq0 + q0);
-      tma_load_2d(sQ + AP_CHUNK_BYTES, &tmap_q, bar(B_QFULL), head * AP_D + 64, seq0 + q0);
-      bool ok = true;
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        const int st = j & 1;
-        const uint32_t ph = (j >> 1) & 1u;
-        const int row = seq0 + j * AP_BN;
-        if (!mbar_wait(bar(B_KEMPTY + st), ph ^ 1u, abort_flag, p.status, (ST_TIMEOUT_SMEM_EMPTY | (3 << 8)), limit)) { ok = false; break; }
-        mbar_expect_tx(bar(B_KFULL + st), AP_TILE_BYTES);
-        tma_load_2d(sK + st * AP_TILE_BYTES, &tmap_k, bar(B_KFULL + st), kvh * AP_D, row);
-        tma_load_2d(sK + st * AP_TILE_BYTES + AP_CHUNK_BYTES, &tmap_k, bar(B_KFULL + st), kvh * AP_D + 64, row);
-        if (!mbar_wait(bar(B_VEMPTY + st), ph ^ 1u, abort_flag, p.status, (ST_TIMEOUT_SMEM_EMPTY | (3 << 8)), limit)) { ok = false; break; }
-        mbar_expect_tx(bar(B_VFULL + st), AP_TILE_BYTES);
-        tma_load_2d(sV + st * AP_TILE_BYTES, &tmap_v, bar(B_VFULL + st), kvh * AP_D, row);
-        tma_load_2d(sV + st * AP_TILE_BYTES + AP_CHUNK_BYTES, &tmap_v, bar(B_VFULL + st), kvh * AP_D + 64, row);
+  if (warp < 4) {
+    warpgroup_regs_dec<AP_REGS_FEW>();
+    if (warp == 0) {
+      if (lane == 0) {
+        prefetch_tmap(&tmap_q); prefetch_tmap(&tmap_k); prefetch_tmap(&tmap_v);
+        uint32_t kv = 0, items = 0;              // tiles loaded so far; bit u: parity of unit u's items
+        bool ok = true;
+        auto load = [&](uint32_t dst, const CUtensorMap* m, int b, int col, int row) {
+          mbar_expect_tx(bar(b), AP_TILE_BYTES);
+          tma_load_2d(dst, m, bar(b), col, row);
+          tma_load_2d(dst + AP_CHUNK_BYTES, m, bar(b), col + 64, row);
+        };
+        while (ok && it.take(p)) {
+#pragma unroll 1
+          for (int u = 0; u < 2 && ok; ++u) {
+            if (it.n(u) == 0) continue;
+            ok = wait(B_QEMPTY + u, ((items >> u) & 1u) ^ 1u, ST_TIMEOUT_SMEM_EMPTY);
+            items ^= 1u << u;
+            if (ok) load(sQ + u * AP_TILE_BYTES, &tmap_q, B_QFULL + u, it.head(u) * AP_D, it.row0 + it.q0(u));
+          }
+          for (int j = 0; j < it.tiles() && ok; ++j, ++kv) {
+            const int st = kv & 1, row = it.row0 + j * AP_BN;
+            const uint32_t ph = ((kv >> 1) & 1u) ^ 1u;
+            ok = wait(B_KEMPTY + st, ph, ST_TIMEOUT_SMEM_EMPTY);
+            if (!ok) break;
+            load(sK + st * AP_TILE_BYTES, &tmap_k, B_KFULL + st, it.kvh * AP_D, row);
+            ok = wait(B_VEMPTY + st, ph, ST_TIMEOUT_SMEM_EMPTY);
+            if (!ok) break;
+            load(sV + st * AP_TILE_BYTES, &tmap_v, B_VFULL + st, it.kvh * AP_D, row);
+          }
+        }
+        if (!ok) { const uint64_t t0 = globaltimer_ns(); while (globaltimer_ns() - t0 < 2000000ull) { } }   // copies in flight land
       }
-      if (!ok) { const uint64_t t0 = globaltimer_ns(); while (globaltimer_ns() - t0 < 2000000ull) { } }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    if (lane == 0) {
+      __syncwarp();
+    } else if (warp == 1) {
+      const bool one = elect_one();
       constexpr uint32_t IDESC_S = umma_idesc_bf16(128, 128, 0, 0);
       constexpr uint32_t IDESC_PV = umma_idesc_bf16(128, 128, 0, 1);     // B (= V) is MN-major
-      auto issue_s = [&](int j) {
-        const int st = j & 1;
-        const uint32_t d = tmem_base + (j & 1) * 128;
+      const uint64_t q_desc = umma_desc_k_sw128(sQ), k_desc = umma_desc_k_sw128(sK), v_desc = umma_desc_mn_sw128(sV, AP_CHUNK_BYTES, 1024);
+      uint32_t kv = 0, items = 0, tiles = 0;    // KV tiles so far; bit u: parity of unit u's items and P tiles
+      bool ok = true;
+      auto issue_s = [&](int u, uint32_t st, bool last) {
+        const uint64_t a = q_desc + static_cast<uint32_t>(u * (AP_TILE_BYTES >> 4)), bd = k_desc + st * (AP_TILE_BYTES >> 4);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t off = (kk >> 2) * AP_CHUNK_BYTES;
-          const uint64_t a = umma_desc_k_sw128(sQ + off) + 2ull * (kk & 3);
-          const uint64_t bd = umma_desc_k_sw128(sK + st * AP_TILE_BYTES + off) + 2ull * (kk & 3);
-          umma_f16_ss(d, a, bd, IDESC_S, kk > 0 ? 1u : 0u);
+          const uint32_t off = (kk >> 2) * (AP_CHUNK_BYTES >> 4) + 2 * (kk & 3);
+          if (one) umma_f16_ss(tmem_base + u * 128, a + off, bd + off, IDESC_S, kk > 0 ? 1u : 0u);
         }
-        umma_commit(bar(B_KEMPTY + st));
-        umma_commit(bar(B_SFULL + (j & 1)));
+        if (one) { umma_commit(bar(B_SFULL + u)); if (last) umma_commit(bar(B_QEMPTY + u)); }
       };
-      bool ok = mbar_wait(bar(B_QFULL), 0, abort_flag, p.status, (ST_TIMEOUT_SMEM_FULL | (3 << 8)), limit) &&
-                mbar_wait(bar(B_KFULL + 0), 0, abort_flag, p.status, (ST_TIMEOUT_SMEM_FULL | (3 << 8)), limit);
-      if (ok) { tc_fence_after(); issue_s(0); }
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        const int st = j & 1;
-        const uint32_t ph = (j >> 1) & 1u;
-        if (j + 1 < n_tiles) {
-          if (!mbar_wait(bar(B_KFULL + ((j + 1) & 1)), ((j + 1) >> 1) & 1u, abort_flag, p.status, (ST_TIMEOUT_SMEM_FULL | (3 << 8)), limit)) { ok = false; break; }
-          tc_fence_after();
-          issue_s(j + 1);
-        }
-        if (!mbar_wait(bar(B_PFULL), j & 1u, abort_flag, p.status, (ST_TIMEOUT_PEER_FLAG | (3 << 8)), limit)) { ok = false; break; }
-        if (!mbar_wait(bar(B_VFULL + st), ph, abort_flag, p.status, (ST_TIMEOUT_SMEM_FULL | (3 << 8)), limit)) { ok = false; break; }
+      auto issue_pv = [&](int u, uint32_t st, bool first, bool last) {
+        if (!wait(B_PFULL + u, (tiles >> u) & 1u, ST_TIMEOUT_PEER_FLAG)) return false;
+        tiles ^= 1u << u;
+        if (first && !wait(B_OFREE + u, ((items >> u) & 1u) ^ 1u, ST_TIMEOUT_TMEM_EMPTY)) return false;
         tc_fence_after();
-        const uint32_t d = tmem_base + 256 + (j & 1) * 128;
+        const uint64_t bd = v_desc + st * (AP_TILE_BYTES >> 4);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint64_t a = umma_desc_k_sw128(sP + (kk >> 2) * AP_CHUNK_BYTES) + 2ull * (kk & 3);
-          const uint64_t bd = umma_desc_mn_sw128(sV + st * AP_TILE_BYTES + kk * 2048, AP_CHUNK_BYTES, 1024);
-          umma_f16_ss(d, a, bd, IDESC_PV, kk > 0 ? 1u : 0u);
-        }
-        umma_commit(bar(B_VEMPTY + st));
-        umma_commit(bar(B_OFULL + (j & 1)));
-      }
-    }
-    __syncwarp();
-  } else {
-    const int qd = warp & 3;
-    const int r = qd * 32 + lane;                    // row inside the tile == TMEM lane
-    const int q_idx = q0 + r;
-    const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(qd * 32) << 16);
-    float o[AP_D];
-#pragma unroll
-    for (int i = 0; i < AP_D; ++i) o[i] = 0.f;
-    float m_run = -INFINITY, l_run = 0.f, alpha_prev = 1.f;
-    bool ok = true;
-    uint8_t* p_row = pP + (r >> 3) * 1024 + (r & 7) * 128;
-    const int sw = r & 7;
-
-    auto o_update = [&](int j, float alpha) -> bool {
-      if (!mbar_wait(bar(B_OFULL + (j & 1)), (j >> 1) & 1u, abort_flag, p.status, (ST_TIMEOUT_TMEM_FULL | (3 << 8)), limit)) return false;
-      tc_fence_after();
-      const uint32_t t_pv = t_lane + 256 + (j & 1) * 128;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t v[32];
-        tmem_ld_x32(t_pv + c * 32, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[c * 32 + i] = o[c * 32 + i] * alpha + __uint_as_float(v[i]);
-      }
-      tc_fence_before();
-      return true;
-    };
-
-    for (int j = 0; j < n_tiles; ++j) {
-      if (!mbar_wait(bar(B_SFULL + (j & 1)), (j >> 1) & 1u, abort_flag, p.status, (ST_TIMEOUT_TMEM_FULL | (3 << 8)), limit)) { ok = false; break; }
-      tc_fence_after();
-      const uint32_t t_s = t_lane + (j & 1) * 128;
-      const int kv0 = j * AP_BN;
-      const bool need_mask = (kv0 + AP_BN > q0) || (kv0 + AP_BN > len);
-      // pass 1: row max
-      float mx = -INFINITY;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t v[32];
-        tmem_ld_x32(t_s + c * 32, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          float s = __uint_as_float(v[i]);
-          if (need_mask) { const int kv = kv0 + c * 32 + i; if (kv > q_idx || kv >= len) s = -INFINITY; }
-          mx = fmaxf(mx, s);
-        }
-      }
-      const float m_new = fmaxf(m_run, mx * p.scale_log2);
-      const float alpha = (m_run == -INFINITY) ? 0.f : exp2f(m_run - m_new);
-      const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-      // the P buffer is free once the PV MMA of the previous tile has completed
-      if (j > 0) {
-        if (!mbar_wait(bar(B_OFULL + ((j - 1) & 1)), ((j - 1) >> 1) & 1u, abort_flag, p.status, (ST_TIMEOUT_TMEM_FULL | (3 << 8)), limit)) { ok = false; break; }
-      }
-      // pass 2: probabilities -> bf16 -> swizzled shared memory
-      float sum = 0.f;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t v[32];
-        tmem_ld_x32(t_s + c * 32, v);
-        tmem_ld_wait();
-        uint32_t pk[16];
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float s0 = __uint_as_float(v[i]), s1 = __uint_as_float(v[i + 1]);
-          if (need_mask) {
-            const int kv = kv0 + c * 32 + i;
-            if (kv > q_idx || kv >= len) s0 = -INFINITY;
-            if (kv + 1 > q_idx || kv + 1 >= len) s1 = -INFINITY;
+        for (int kk = 0; kk < 8; ++kk)
+          if (one) umma_f16_ts(tmem_base + 256 + u * 128, tmem_base + u * 128 + kk * 8, bd + kk * (2048 >> 4), IDESC_PV, kk > 0 ? 1u : (first ? 0u : 1u));
+        if (last && one) umma_commit(bar(B_OFULL + u));
+        return true;
+      };
+      while (ok && it.take(p)) {
+        const int n = it.tiles();
+        for (int j = 0; j <= n && ok; ++j) {                             // S of tile j, PV of tile j - 1
+          const uint32_t ks = (kv + j) & 1, vs = (kv + j + 1) & 1;
+          if (j < n) ok = wait(B_KFULL + ks, ((kv + j) >> 1) & 1u, ST_TIMEOUT_SMEM_FULL);
+          if (ok && j > 0) ok = wait(B_VFULL + vs, ((kv + j - 1) >> 1) & 1u, ST_TIMEOUT_SMEM_FULL);
+#pragma unroll 1
+          for (int u = 0; u < 2 && ok; ++u) {
+            if (j > 0 && j <= it.n(u)) ok = issue_pv(u, vs, j == 1, j == it.n(u));
+            if (ok && j < it.n(u)) {
+              if (j == 0) ok = wait(B_QFULL + u, (items >> u) & 1u, ST_TIMEOUT_SMEM_FULL);
+              if (!ok) break;
+              tc_fence_after();
+              issue_s(u, ks, j + 1 == it.n(u));
+            }
           }
-          const float e0 = exp2f(s0 * p.scale_log2 - m_use), e1 = exp2f(s1 * p.scale_log2 - m_use);
-          const __nv_bfloat162 pb = __floats2bfloat162_rn(e0, e1);
-          // sum what the MMA will actually see
-          sum += __low2float(pb) + __high2float(pb);
-          pk[i >> 1] = *reinterpret_cast<const uint32_t*>(&pb);
+          if (ok && one) {
+            if (j < n) umma_commit(bar(B_KEMPTY + ks));
+            if (j > 0) umma_commit(bar(B_VEMPTY + vs));
+          }
         }
-        // 32 columns = 4 sixteen-byte units; unit u of 128-byte row chunk lands at (u ^ (row & 7))
-        uint8_t* chunk = p_row + (c >> 1) * AP_CHUNK_BYTES;
-#pragma unroll
-        for (int u4 = 0; u4 < 4; ++u4) {
-          const int u = (c & 1) * 4 + u4;
-          *reinterpret_cast<uint4*>(chunk + ((u ^ sw) << 4)) = make_uint4(pk[4 * u4], pk[4 * u4 + 1], pk[4 * u4 + 2], pk[4 * u4 + 3]);
-        }
+        kv += n;
+        items ^= 1u | (it.n(1) > 0 ? 2u : 0u);
       }
-      l_run = l_run * alpha + sum;
-      m_run = m_new;
-      tc_fence_before();
-      fence_proxy_async_smem();
-      mbar_arrive(bar(B_PFULL));
-      // while the tensor core works on PV of this tile, fold in PV of the previous one
-      if (j > 0) { if (!o_update(j - 1, alpha_prev)) { ok = false; break; } }
-      alpha_prev = alpha;
+      __syncwarp();
     }
-    if (ok) ok = o_update(n_tiles - 1, alpha_prev);
-    if (ok && q_idx < len) {
-      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-      uint4* dst = reinterpret_cast<uint4*>(p.out + (static_cast<size_t>(seq0 + q_idx) * p.hq + head) * AP_D);
+  } else {
+    warpgroup_regs_inc<AP_REGS_MANY>();
+    const int u = (warp - 4) >> 2, qd = warp & 3;    // unit; TMEM lane quarter this warp may read
+    const int r = qd * 32 + lane;                    // row inside the tile == TMEM lane
+    const uint32_t t_s = tmem_base + (static_cast<uint32_t>(qd * 32) << 16) + u * 128, t_o = t_s + 256;
+    uint32_t tiles = 0, items = 0;
+    bool ok = true;
+    // one verdict per warp: the TMEM accesses need all lanes
+    auto wait_all = [&](int i, uint32_t par) { return __all_sync(0xffffffffu, wait(i, par, ST_TIMEOUT_TMEM_FULL)) != 0; };
+    while (ok && it.take(p)) {
+      const int n = it.n(u);
+      if (n == 0) continue;
+      const int q_idx = it.q0(u) + r;
+      float m_ref = -INFINITY, l = 0.f;
+      for (int j = 0; j < n; ++j) {
+        ok = wait_all(B_SFULL + u, tiles++ & 1u);
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t v[4][32];
 #pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        uint32_t w[4];
+        for (int c = 0; c < 4; ++c) tmem_ld_x32(t_s + c * 32, v[c]);
+        tmem_ld_wait();
+        const int visible = min(q_idx, it.len - 1) - j * AP_BN + 1;    // columns of this tile that the row sees
+        if (__any_sync(0xffffffffu, visible < AP_BN)) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const __nv_bfloat162 pb = __floats2bfloat162_rn(o[u * 8 + 2 * k] * inv, o[u * 8 + 2 * k + 1] * inv);
-          w[k] = *reinterpret_cast<const uint32_t*>(&pb);
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int i = 0; i < 32; ++i) if (c * 32 + i >= visible) v[c][i] = 0xff800000u;      // -inf
         }
-        dst[u] = make_uint4(w[0], w[1], w[2], w[3]);
+        float mx[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          mx[c] = __uint_as_float(v[c][0]);
+#pragma unroll
+          for (int i = 1; i < 32; ++i) mx[c] = fmaxf(mx[c], __uint_as_float(v[c][i]));
+        }
+        const float m_new = fmaxf(m_ref, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2);
+        if (__any_sync(0xffffffffu, m_new > m_ref)) {
+          const float alpha = m_ref == -INFINITY ? 0.f : exp2f(m_ref - m_new);
+          l *= alpha;
+          m_ref = m_new;
+          if (j > 0) {       // PV of the tiles before has completed: S of this one was issued after it
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              uint32_t o[32];
+              tmem_ld_x32(t_o + c * 32, o);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+              tmem_st_x32(t_o + c * 32, o);
+            }
+          }
+        }
+        const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float e0 = exp2f(__uint_as_float(v[c][2 * i]) * p.scale_log2 - m_use), e1 = exp2f(__uint_as_float(v[c][2 * i + 1]) * p.scale_log2 - m_use);
+            const __nv_bfloat162 pb = __floats2bfloat162_rn(e0, e1);
+            pk[i] = *reinterpret_cast<const uint32_t*>(&pb);
+            sum[c] += __uint_as_float(pk[i] << 16) + __uint_as_float(pk[i] & 0xffff0000u);     // what the MMA will actually see
+          }
+          tmem_st_x16(t_s + c * 16, pk);
+        }
+        l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(B_PFULL + u));
+      }
+      if (ok) ok = wait_all(B_OFULL + u, items & 1u);
+      if (!ok) break;
+      ++items;
+      tc_fence_after();
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      uint4* dst = reinterpret_cast<uint4*>(p.out + (static_cast<size_t>(it.row0 + q_idx) * p.hq + it.head(u)) * AP_D);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint32_t o[32];
+        tmem_ld_x32(t_o + c * 32, o);
+        tmem_ld_wait();
+        if (c == 3) {                                // the row is in registers: the next item's PV may overwrite it
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(B_OFREE + u));
+        }
+        if (q_idx < it.len) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            uint32_t w[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const __nv_bfloat162 pb = __floats2bfloat162_rn(__uint_as_float(o[g * 8 + 2 * k]) * inv, __uint_as_float(o[g * 8 + 2 * k + 1]) * inv);
+              w[k] = *reinterpret_cast<const uint32_t*>(&pb);
+            }
+            dst[c * 4 + g] = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
       }
     }
   }
@@ -302,20 +348,21 @@ extern "C" int b200_attn_prefill(const void* q, long long ld_q, const void* k, l
   if (make_tmap_2d_bf16(&tk, k, static_cast<uint64_t>(hkv) * AP_D, total_tokens, static_cast<uint64_t>(ld_k) * 2)) return -12;
   if (make_tmap_2d_bf16(&tv, v, static_cast<uint64_t>(hkv) * AP_D, total_tokens, static_cast<uint64_t>(ld_v) * 2)) return -13;
   PrefillParams p;
-  p.cu_seqlens = cu_seqlens; p.out = static_cast<__nv_bfloat16*>(out); p.hq = hq; p.hkv = hkv;
+  p.cu_seqlens = cu_seqlens; p.out = static_cast<__nv_bfloat16*>(out); p.hq = hq; p.hkv = hkv; p.B = B;
+  const int q_tiles = (max_len + AP_BM - 1) / AP_BM;
+  p.pair_heads = (hq / hkv) % 2 == 0;
+  p.q_steps = p.pair_heads ? q_tiles : (q_tiles + 1) / 2;
+  p.columns = p.pair_heads ? hq / 2 : hq;
   p.scale_log2 = scale * 1.4426950408889634f; p.status = status; p.limit_ns = 2000000000ull;
   constexpr int SMEM = 6 * AP_TILE_BYTES + 1024 + 256;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    // ask for the largest shared-memory carveout: with the default preference the occupancy calculator (and the
-    // launch) may settle for a split of the L1 / shared array that holds fewer CTAs per SM than the kernel was sized for
-    cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return -1000 - static_cast<int>(e);
     configured = true;
   }
-  dim3 grid((max_len + AP_BM - 1) / AP_BM, hq, B);
-  launch_ex(attn_prefill_kernel, dim3(grid), dim3(AP_THREADS), SMEM, stream, 0, tq, tk, tv, p);
+  const long long items = static_cast<long long>(p.q_steps) * p.columns * B;
+  launch_ex(attn_prefill_kernel, dim3(static_cast<unsigned>(items < 148 ? items : 148)), dim3(AP_THREADS), SMEM, stream, 0, tq, tk, tv, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }

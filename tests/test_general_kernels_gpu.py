@@ -52,3 +52,26 @@ def test_general_attention_with_uneven_head_sizes(dk, dv, chunk, dtype):
         want = torch.einsum("hj,jhd->hd", s, vv).reshape(-1)
         # fp32 sums of up to 300 terms of size one; a bf16 result is rounded once (2^-9 of values up to 5)
         assert (out[i].double() - want).abs().max().item() < (1e-5 if dtype == torch.float32 else 1.2e-2), p
+
+
+def _ok():
+    from mojo_linuxperiments_b200.ops.workspace import default_workspace
+    default_workspace(torch.device(DEV)).check_status()
+
+
+@pytest.mark.parametrize("lens,hq,hkv", [([127, 128, 129], 8, 2), ([255, 256, 257, 1], 6, 2), ([130, 300], 3, 3), ([513, 64], 5, 1), ([200] * 40, 16, 4),
+                                         ([1, 2, 700], 4, 4)])
+def test_prefill_attention_pairs_heads_or_query_tiles(lens, hq, hkv):
+    """Two heads of a KV head share a CTA; an odd number of them: two query tiles.  Tile edges, more items than CTAs, short
+    sequences among long ones.  bf16 weights and outputs: 2^-8 of values up to 4."""
+    from mojo_linuxperiments_b200.ops import attention as A
+    g = torch.Generator(device=DEV).manual_seed(sum(lens))
+    x = torch.randn((sum(lens), hq + 2 * hkv, 128), generator=g, device=DEV).to(torch.bfloat16)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32).to(DEV)
+    out = A.attn_prefill(x[:, :hq].contiguous(), x[:, hq:hq + hkv], x[:, hq + hkv:], cu, max(lens), kv_chunk=0)
+    _ok()
+    for part, o in zip(x.split(lens), out.split(lens)):
+        q, k, v = (t.double() for t in (part[:, :hq], part[:, hq:hq + hkv].repeat_interleave(hq // hkv, 1), part[:, hq + hkv:].repeat_interleave(hq // hkv, 1)))
+        s = torch.einsum("ihd,jhd->hij", q, k) * 128 ** -0.5
+        s = s.masked_fill(torch.ones(s.shape[1:], dtype=torch.bool, device=DEV).triu(1), float("-inf")).softmax(-1)
+        assert (o.double() - torch.einsum("hij,jhd->ihd", s, v)).abs().max().item() < 1.6e-2
