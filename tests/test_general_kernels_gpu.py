@@ -75,3 +75,34 @@ def test_prefill_attention_pairs_heads_or_query_tiles(lens, hq, hkv):
         s = torch.einsum("ihd,jhd->hij", q, k) * 128 ** -0.5
         s = s.masked_fill(torch.ones(s.shape[1:], dtype=torch.bool, device=DEV).triu(1), float("-inf")).softmax(-1)
         assert (o.double() - torch.einsum("hij,jhd->ihd", s, v)).abs().max().item() < 1.6e-2
+
+
+@pytest.mark.parametrize("tokens", [1, 1100])
+@pytest.mark.parametrize("norm", [False, True])
+def test_rotary_writes_the_same_with_narrow_accesses(tokens, norm):
+    from mojo_linuxperiments_b200.ops import attention as A
+    hq, hkv = 6, 2
+    g = torch.Generator(device=DEV).manual_seed(tokens)
+    W = (hq + 2 * hkv) * 128
+    raw = torch.randn((tokens, W + 1), generator=g, device=DEV).to(torch.bfloat16)
+    pos = (torch.arange(tokens, device=DEV) % 550).to(torch.int32)
+    seq = (torch.arange(tokens, device=DEV) // 550).to(torch.int32)
+    cos, sin = A.rope_tables(550, 1e4, DEV)
+    w = (1 + 0.1 * torch.randn(128, generator=g, device=DEV)).to(torch.bfloat16) if norm else None
+    got = []
+    for x in (raw[:, 1:], raw[:, 1:].contiguous()):                  # odd pitch and start, then aligned rows
+        cache = A.PagedKVCache(70, hkv, 16, DEV)
+        k = torch.empty((tokens, hkv, 128), dtype=torch.bfloat16, device=DEV)
+        q = A.rope_kv_write(x, pos, cos, sin, hq, hkv, k_out=k, cache=cache, page_table=torch.arange(70, dtype=torch.int32, device=DEV).view(2, 35),
+                            seq_ids=seq, q_norm_w=w, k_norm_w=w)
+        got.append((q, k, cache.data))
+    _ok()
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    x = raw[:, 1:].double().view(tokens, -1, 128)[:, :hq + hkv]
+    if norm:
+        x = x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    c, s = cos[pos.long()].double()[:, None], sin[pos.long()].double()[:, None]
+    a, b = x[..., :64], x[..., 64:]
+    want = torch.cat([a * c - b * s, b * c + a * s], -1)
+    assert (torch.cat([got[0][0], got[0][1]], 1).double() - want).abs().max() < 2.5e-2      # one bf16 rounding of values up to 6
