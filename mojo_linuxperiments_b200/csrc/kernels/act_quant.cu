@@ -1,10 +1,9 @@
 // Activation prologue for every W8A8 linear: (residual add) -> (RMSNorm) | (SwiGLU) -> block-Hadamard
 // rotation (block 128, Sylvester order, scaled 1/sqrt(128)) -> per-token symmetric int8 quantisation.
 //
-//   one CTA per token row, 8 warps; warp w owns 128-blocks w, w+8, ...; inside a block lane l holds the four
-//   consecutive elements 4l..4l+3, so the seven butterfly stages are two in-register stages plus five
-//   warp-shuffle stages.  Rotated values stay in registers between the abs-max pass and the quantise pass,
-//   so the row is read from HBM exactly once and written once (int8 + one fp32 scale).
+// Two kernels: one CTA per token row (more than 64 rows, long rows, normalised copy wanted), and for decode-sized calls a
+// cluster of CTAs per row.  Rotated values stay in registers between the abs-max pass and the quantise pass, so the row is
+// read from HBM exactly once and written once (int8 + one fp32 scale).
 #include "ptx.cuh"
 #include "api.h"
 #include "launch.cuh"
@@ -15,15 +14,10 @@ namespace b200 {
 
 constexpr int AQ_THREADS = 256;
 constexpr int AQ_WARPS = AQ_THREADS / 32;
+constexpr int AQ_ROW_WARPS = 16;          // most warps of the one-CTA form
 
 enum ActQuantMode : int { AQ_PLAIN = 0, AQ_NORM = 1, AQ_ADD_NORM = 2, AQ_SWIGLU = 3 };
 
-__device__ __forceinline__ void load4_bf16(const __nv_bfloat16* p, float (&v)[4]) {
-  const uint2 raw = *reinterpret_cast<const uint2*>(p);
-  const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&raw.x);
-  const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
-  v[0] = __low2float(lo); v[1] = __high2float(lo); v[2] = __low2float(hi); v[3] = __high2float(hi);
-}
 __device__ __forceinline__ void store4_bf16(__nv_bfloat16* p, const float (&v)[4]) {
   __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]);
   __nv_bfloat162 hi = __floats2bfloat162_rn(v[2], v[3]);
@@ -33,8 +27,13 @@ __device__ __forceinline__ void store4_bf16(__nv_bfloat16* p, const float (&v)[4
   *reinterpret_cast<uint2*>(p) = raw;
 }
 
-template <int MAXB, int MODE>
-__global__ void __launch_bounds__(AQ_THREADS)
+// One CTA per token row.  A warp takes up to MAXC chunks of four 128-blocks: eight lanes per block, 16 consecutive elements per
+// lane (pair i of a lane: elements i and i + 8), so that a lane's loads are 16 bytes wide (WIDE; 8 bytes where alignment
+// does not allow it) and the rotation needs three lane-crossing stages instead of five, on pairs.  Instructions per element
+// bound this kernel, not its bytes: 32,768 x 14,336 SwiGLU 591 us = 4.0 TB/s (896 with a block per warp and four elements per
+// lane), 32,768 x 4,096 with residual and norm 199 (229), 32,768 x 4,096 plain 112 (152), 32,768 x 768 SwiGLU 37 (83).
+template <int MAXC, int MODE, bool WIDE>
+__global__ void __launch_bounds__(AQ_ROW_WARPS * 32, 2)
 act_quant_kernel(const __nv_bfloat16* x, long long ldx, __nv_bfloat16* residual,
                  long long ldr, const __nv_bfloat16* gamma, float eps, int8_t* q,
                  long long ldq, float* scale, __nv_bfloat16* xn_out, long long ldn,
@@ -45,136 +44,134 @@ act_quant_kernel(const __nv_bfloat16* x, long long ldx, __nv_bfloat16* residual,
   pdl_wait();                // everything before this kernel in the stream has completed
   if (threadIdx.x == 0) B200_TRACE(TK_ACT_QUANT, TP_DEPS);
 
-  __shared__ float red[AQ_WARPS];
-  __shared__ float bcast;
-  const int row = blockIdx.x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ float red[2][AQ_ROW_WARPS];
+  const long long row = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int nblocks = K >> 7;
-  const __nv_bfloat16* xr = x + static_cast<size_t>(row) * ldx;
-
-  float v[MAXB][4];
-  float ss = 0.f;
-  // All global loads of the row are issued first, with no arithmetic in between, so their latencies overlap;
-  // the element-wise math (which contains slow-path divisions / exponentials) runs afterwards.
-  uint2 raw_a[MAXB], raw_b[MAXB];
+  constexpr bool NORM = MODE == AQ_NORM || MODE == AQ_ADD_NORM;
+  auto at = [&](int i) { return ((warp + i * warps) * 4 + (lane >> 3)) * 128 + (lane & 7) * 16; };   // first element of this lane
+  auto have = [&](int i) { return (warp + i * warps) * 4 + (lane >> 3) < nblocks; };
+  auto load16 = [](const __nv_bfloat16* p, uint32_t (&r)[8]) {
+    if constexpr (WIDE) {
 #pragma unroll
-  for (int i = 0; i < MAXB; ++i) {
-    const int b = warp + i * AQ_WARPS;
-    raw_a[i] = make_uint2(0u, 0u);
-    raw_b[i] = make_uint2(0u, 0u);
-    if (b < nblocks) {
-      const int k = b * 128 + lane * 4;
-      raw_a[i] = *reinterpret_cast<const uint2*>(xr + k);
-      if constexpr (MODE == AQ_SWIGLU) raw_b[i] = *reinterpret_cast<const uint2*>(xr + K + k);
-      if constexpr (MODE == AQ_ADD_NORM) raw_b[i] = *reinterpret_cast<const uint2*>(residual + static_cast<size_t>(row) * ldr + k);
-    }
-  }
-  auto unpack4 = [](const uint2& r, float (&o)[4]) {
-    o[0] = __uint_as_float(r.x << 16); o[1] = __uint_as_float(r.x & 0xffff0000u);
-    o[2] = __uint_as_float(r.y << 16); o[3] = __uint_as_float(r.y & 0xffff0000u);
-  };
-#pragma unroll
-  for (int i = 0; i < MAXB; ++i) {
-    const int b = warp + i * AQ_WARPS;
-    if (b < nblocks) {
-      const int k = b * 128 + lane * 4;
-      if constexpr (MODE == AQ_SWIGLU) {
-        float g[4], u[4];
-        unpack4(raw_a[i], g);
-        unpack4(raw_b[i], u);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[i][j] = __fdividef(g[j], 1.f + __expf(-g[j])) * u[j];
-      } else {
-        unpack4(raw_a[i], v[i]);
-        if constexpr (MODE == AQ_ADD_NORM) {
-          float r[4];
-          unpack4(raw_b[i], r);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            // the residual stream is kept in bf16: round the sum once, and normalise what was stored
-            v[i][j] = __bfloat162float(__float2bfloat16(v[i][j] + r[j]));
-          }
-          store4_bf16(residual + static_cast<size_t>(row) * ldr + k, v[i]);
-        }
-        if constexpr (MODE == AQ_NORM || MODE == AQ_ADD_NORM) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) ss += v[i][j] * v[i][j];
-        }
+      for (int g = 0; g < 2; ++g) {
+        const uint4 t = reinterpret_cast<const uint4*>(p)[g];
+        r[4 * g] = t.x; r[4 * g + 1] = t.y; r[4 * g + 2] = t.z; r[4 * g + 3] = t.w;
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) v[i][j] = 0.f;
-    }
-  }
-
-  uint2 raw_g[MAXB];
-  if constexpr (MODE == AQ_NORM || MODE == AQ_ADD_NORM) {
-#pragma unroll
-    for (int i = 0; i < MAXB; ++i) {
-      const int b = warp + i * AQ_WARPS;
-      raw_g[i] = make_uint2(0u, 0u);
-      if (b < nblocks) raw_g[i] = __ldg(reinterpret_cast<const uint2*>(gamma + b * 128 + lane * 4));
-    }
-  }
-  if constexpr (MODE == AQ_NORM || MODE == AQ_ADD_NORM) {
-    ss = warp_sum(ss);
-    if (lane == 0) red[warp] = ss;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      float t = 0.f;
-#pragma unroll
-      for (int w = 0; w < AQ_WARPS; ++w) t += red[w];
-      bcast = rsqrtf(t / static_cast<float>(K) + eps);
-    }
-    __syncthreads();
-    const float rstd = bcast;
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < MAXB; ++i) {
-      const int b = warp + i * AQ_WARPS;
-      if (b < nblocks) {
-        const int k = b * 128 + lane * 4;
-        float g[4];
-        unpack4(raw_g[i], g);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[i][j] = v[i][j] * rstd * g[j];
-        if (xn_out) store4_bf16(xn_out + static_cast<size_t>(row) * ldn + k, v[i]);
+      for (int g = 0; g < 4; ++g) {
+        const uint2 t = reinterpret_cast<const uint2*>(p)[g];
+        r[2 * g] = t.x; r[2 * g + 1] = t.y;
       }
     }
-  }
+  };
+  auto store16 = [](__nv_bfloat16* p, const float2 (&v)[8]) {
+    uint32_t r[8];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(v[2 * g].x, v[2 * g + 1].x), hi = __floats2bfloat162_rn(v[2 * g].y, v[2 * g + 1].y);
+      r[g] = *reinterpret_cast<const uint32_t*>(&lo);
+      r[g + 4] = *reinterpret_cast<const uint32_t*>(&hi);
+    }
+    if constexpr (WIDE) {
+#pragma unroll
+      for (int g = 0; g < 2; ++g) reinterpret_cast<uint4*>(p)[g] = make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+    } else {
+#pragma unroll
+      for (int g = 0; g < 4; ++g) reinterpret_cast<uint2*>(p)[g] = make_uint2(r[2 * g], r[2 * g + 1]);
+    }
+  };
+  // element pair i of the 16 in r: (i, i + 8)
+  auto pair = [](const uint32_t (&r)[8], int i) {
+    return i & 1 ? make_float2(__uint_as_float(r[i >> 1] & 0xffff0000u), __uint_as_float(r[4 + (i >> 1)] & 0xffff0000u))
+                 : make_float2(__uint_as_float(r[i >> 1] << 16), __uint_as_float(r[4 + (i >> 1)] << 16));
+  };
 
+  const __nv_bfloat16* xr = x + row * ldx;
+  float2 v[MAXC][8];
+  float2 ss = make_float2(0.f, 0.f);
   float amax = 0.f;
 #pragma unroll
-  for (int i = 0; i < MAXB; ++i) {
-    const int b = warp + i * AQ_WARPS;
-    if (b < nblocks) {
-      fwht128_lane4(v[i], lane);
+  for (int i = 0; i < MAXC; ++i) {
+    if (!have(i)) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) amax = fmaxf(amax, fabsf(v[i][j]));
+      for (int j = 0; j < 8; ++j) v[i][j] = make_float2(0.f, 0.f);
+      continue;
     }
+    uint32_t a[8], b[8];
+    load16(xr + at(i), a);
+    if constexpr (MODE == AQ_SWIGLU) load16(xr + K + at(i), b);
+    if constexpr (MODE == AQ_ADD_NORM) load16(residual + row * ldr + at(i), b);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[i][j] = pair(a, j);
+      if constexpr (MODE == AQ_SWIGLU) {
+        const float2 u = pair(b, j);
+        v[i][j].x = __fdividef(v[i][j].x, 1.f + __expf(-v[i][j].x)) * u.x;
+        v[i][j].y = __fdividef(v[i][j].y, 1.f + __expf(-v[i][j].y)) * u.y;
+      }
+      if constexpr (MODE == AQ_ADD_NORM) {
+        // the residual stream is kept in bf16: round the sum once, and normalise what was stored
+        const float2 t = add2(v[i][j], pair(b, j));
+        v[i][j].x = __bfloat162float(__float2bfloat16(t.x));
+        v[i][j].y = __bfloat162float(__float2bfloat16(t.y));
+      }
+      if constexpr (NORM) ss = fma2(v[i][j], v[i][j], ss);
+    }
+    if constexpr (MODE == AQ_ADD_NORM) store16(residual + row * ldr + at(i), v[i]);
+  }
+  if constexpr (NORM) {
+    const float sum = warp_sum(ss.x + ss.y);
+    if (lane == 0) red[0][warp] = sum;
+    __syncthreads();
+    float t = 0.f;
+    for (int w = 0; w < warps; ++w) t += red[0][w];
+    const float rstd = rsqrtf(t / static_cast<float>(K) + eps);
+#pragma unroll
+    for (int i = 0; i < MAXC; ++i) {
+      if (!have(i)) continue;
+      uint32_t g[8];
+      load16(gamma + at(i), g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[i][j] = mul2(mul2(v[i][j], make_float2(rstd, rstd)), pair(g, j));
+      if (xn_out) store16(xn_out + row * ldn + at(i), v[i]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < MAXC; ++i) {
+    if ((warp + i * warps) * 4 >= nblocks) break;            // the same for the whole warp; blocks beyond the row are zeros
+    fwht128_lane16(v[i], lane);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fmaxf(fabsf(v[i][j].x), fabsf(v[i][j].y)));
   }
   if (threadIdx.x == 0) B200_TRACE(TK_ACT_QUANT, 2);
   amax = warp_max(amax);
-  if (lane == 0) red[warp] = amax;
+  if (lane == 0) red[1][warp] = amax;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.f;
-#pragma unroll
-    for (int w = 0; w < AQ_WARPS; ++w) t = fmaxf(t, red[w]);
-    const float s = quant_scale_from_amax(t);
-    bcast = s;
-    scale[row] = s;
-  }
-  __syncthreads();
-  const float s = bcast;
+  float t = 0.f;
+  for (int w = 0; w < warps; ++w) t = fmaxf(t, red[1][w]);
+  const float s = quant_scale_from_amax(t);
   const float inv_s = quant_inv_scale(s);
-  int8_t* qr = q + static_cast<size_t>(row) * ldq;
+  if (threadIdx.x == 0) scale[row] = s;
+  int8_t* qr = q + row * ldq;
 #pragma unroll
-  for (int i = 0; i < MAXB; ++i) {
-    const int b = warp + i * AQ_WARPS;
-    if (b < nblocks) {
-      *reinterpret_cast<uint32_t*>(qr + b * 128 + lane * 4) = quant_pack4(v[i], inv_s);
+  for (int i = 0; i < MAXC; ++i) {
+    if (!have(i)) continue;
+    int n[16];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float2 t2 = mul2(v[i][j], make_float2(inv_s, inv_s));
+      n[j] = __float2int_rn(t2.x);
+      n[j + 8] = __float2int_rn(t2.y);
     }
+    uint32_t r[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) r[g] = quant_bytes4(n[4 * g], n[4 * g + 1], n[4 * g + 2], n[4 * g + 3]);
+    if constexpr (WIDE) *reinterpret_cast<uint4*>(qr + at(i)) = make_uint4(r[0], r[1], r[2], r[3]);
+    else
+#pragma unroll
+      for (int g = 0; g < 4; ++g) reinterpret_cast<uint32_t*>(qr + at(i))[g] = r[g];
   }
   if (threadIdx.x == 0) B200_TRACE(TK_ACT_QUANT, TP_EXIT);
   B200_TRACE_FLUSH(TK_ACT_QUANT);
@@ -318,16 +315,27 @@ static int aq_cluster_size(int M, int K, bool want_normed) {
   return c;
 }
 
-template <int MAXB>
+template <int MAXC, bool WIDE>
 static void launch_aq(int mode, const __nv_bfloat16* x, long long ldx, __nv_bfloat16* residual, long long ldr,
                       const __nv_bfloat16* gamma, float eps, int8_t* q, long long ldq, float* scale,
-                      __nv_bfloat16* xn, long long ldn, int M, int K, cudaStream_t st) {
+                      __nv_bfloat16* xn, long long ldn, int M, int K, int warps, cudaStream_t st) {
+  const dim3 grid(M), block(32 * warps);
   switch (mode) {
-    case AQ_PLAIN: launch_ex(act_quant_kernel<MAXB, AQ_PLAIN>, dim3(M), dim3(AQ_THREADS), 0, st, 0, x, ldx, residual, ldr, gamma, eps, q, ldq, scale, xn, ldn, K); break;
-    case AQ_NORM: launch_ex(act_quant_kernel<MAXB, AQ_NORM>, dim3(M), dim3(AQ_THREADS), 0, st, 0, x, ldx, residual, ldr, gamma, eps, q, ldq, scale, xn, ldn, K); break;
-    case AQ_ADD_NORM: launch_ex(act_quant_kernel<MAXB, AQ_ADD_NORM>, dim3(M), dim3(AQ_THREADS), 0, st, 0, x, ldx, residual, ldr, gamma, eps, q, ldq, scale, xn, ldn, K); break;
-    default: launch_ex(act_quant_kernel<MAXB, AQ_SWIGLU>, dim3(M), dim3(AQ_THREADS), 0, st, 0, x, ldx, residual, ldr, gamma, eps, q, ldq, scale, xn, ldn, K); break;
+    case AQ_PLAIN: launch_ex(act_quant_kernel<MAXC, AQ_PLAIN, WIDE>, grid, block, 0, st, 0, x, ldx, residual, ldr, gamma, eps, q, ldq, scale, xn, ldn, K); break;
+    case AQ_NORM: launch_ex(act_quant_kernel<MAXC, AQ_NORM, WIDE>, grid, block, 0, st, 0, x, ldx, residual, ldr, gamma, eps, q, ldq, scale, xn, ldn, K); break;
+    case AQ_ADD_NORM: launch_ex(act_quant_kernel<MAXC, AQ_ADD_NORM, WIDE>, grid, block, 0, st, 0, x, ldx, residual, ldr, gamma, eps, q, ldq, scale, xn, ldn, K); break;
+    default: launch_ex(act_quant_kernel<MAXC, AQ_SWIGLU, WIDE>, grid, block, 0, st, 0, x, ldx, residual, ldr, gamma, eps, q, ldq, scale, xn, ldn, K); break;
   }
+}
+
+// a chunk of four blocks per warp up to sixteen warps, then two (14,336: fourteen warps of two)
+template <bool WIDE>
+static void launch_aq_rows(int mode, const __nv_bfloat16* x, long long ldx, __nv_bfloat16* residual, long long ldr,
+                           const __nv_bfloat16* gamma, float eps, int8_t* q, long long ldq, float* scale,
+                           __nv_bfloat16* xn, long long ldn, int M, int K, cudaStream_t st) {
+  const int chunks = (K + 511) / 512;
+  if (chunks <= AQ_ROW_WARPS) launch_aq<1, WIDE>(mode, x, ldx, residual, ldr, gamma, eps, q, ldq, scale, xn, ldn, M, K, chunks, st);
+  else launch_aq<2, WIDE>(mode, x, ldx, residual, ldr, gamma, eps, q, ldq, scale, xn, ldn, M, K, (chunks + 1) / 2, st);
 }
 
 }  // namespace b200
@@ -358,8 +366,10 @@ extern "C" int b200_act_quant(const void* x, long long ldx, void* residual, long
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
   }
-  if (nb <= 4 * AQ_WARPS) launch_aq<4>(mode, X, ldx, R, ldr, G, eps, Q, ldq, scale, XN, ldn, M, K, stream);
-  else launch_aq<16>(mode, X, ldx, R, ldr, G, eps, Q, ldq, scale, XN, ldn, M, K, stream);
+  auto al16 = [](const void* p, long long ld, int elem) { return !p || (!(reinterpret_cast<uintptr_t>(p) & 15) && ld * elem % 16 == 0); };
+  const bool wide = al16(x, ldx, 2) && al16(residual, ldr, 2) && al16(gamma, 0, 2) && al16(q, ldq, 1) && al16(xn_out, ldn, 2);
+  if (wide) launch_aq_rows<true>(mode, X, ldx, R, ldr, G, eps, Q, ldq, scale, XN, ldn, M, K, stream);
+  else launch_aq_rows<false>(mode, X, ldx, R, ldr, G, eps, Q, ldq, scale, XN, ldn, M, K, stream);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }

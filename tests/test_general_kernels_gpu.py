@@ -77,6 +77,41 @@ def test_prefill_attention_pairs_heads_or_query_tiles(lens, hq, hkv):
         assert (o.double() - torch.einsum("hij,jhd->ihd", s, v)).abs().max().item() < 1.6e-2
 
 
+@pytest.mark.parametrize("shift", [0, 4])
+@pytest.mark.parametrize("K", [128, 384, 512, 640, 2048, 4096, 8192, 8320, 14336, 16384])
+@pytest.mark.parametrize("mode", [0, 1, 2, 3])
+def test_activation_rows_of_the_one_cta_form(mode, K, shift):
+    """Chunks of four blocks, a last one that is partly filled, one and two chunks per warp; 16-byte and 8-byte accesses.  The whole
+    numbers are those of the definition except where fp32 rounding moves a value across an edge (at most one step)."""
+    from mojo_linuxperiments_b200.oracle import quant as Q
+    from mojo_linuxperiments_b200.ops import linear as L
+    M = 70
+    g = torch.Generator(device=DEV).manual_seed(K + mode)
+    W = K * (2 if mode == 3 else 1)
+    x = torch.randn((M, W + 8), generator=g, device=DEV).to(torch.bfloat16)[:, shift:shift + W]
+    x[3] = 0
+    gamma = (1 + 0.1 * torch.randn(K, generator=g, device=DEV)).to(torch.bfloat16)
+    res = torch.randn((M, K), generator=g, device=DEV).to(torch.bfloat16) if mode == 2 else None
+    if res is not None:
+        res[3] = 0
+    base = None
+    f = x.float()
+    if mode == 3:
+        f = Q.swiglu(x)
+    elif mode == 2:
+        base = (f + res.float()).to(torch.bfloat16)
+        f = Q.rmsnorm(base, gamma, 1e-5)
+    elif mode == 1:
+        f = Q.rmsnorm(x, gamma, 1e-5)
+    q, s = L.act_quant(x, mode=mode, gamma=gamma if mode in (1, 2) else None, residual=res)
+    if base is not None:
+        assert torch.equal(res, base)
+    wq, ws = Q.rotate_quantize(f)
+    assert (s - ws).abs().max() <= 3e-6 * ws.abs().max() and s[3] == 1.0
+    d = (q.int() - wq.int()).abs()
+    assert d.max() <= 1 and (d > 0).float().mean() < 2e-3
+
+
 @pytest.mark.parametrize("tokens", [1, 1100])
 @pytest.mark.parametrize("norm", [False, True])
 def test_rotary_writes_the_same_with_narrow_accesses(tokens, norm):
