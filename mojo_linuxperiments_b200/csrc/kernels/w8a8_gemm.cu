@@ -436,6 +436,10 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmP
 }
 
 
+// two CTAs per 256 x bn tile (w8a8_gemm_pair.cu)
+int w8a8_gemm_pair(const void* xq, const float* sx, const void* wq, const float* sw, void* y, int M, int N, int K, int ldy, int bn,
+                   int* status, int num_sms, cudaStream_t stream);
+
 // token-tile width (swapped) or channel-tile width (normal)
 int gemm_pick_bn(int M, int N, int num_sms) {
   if (M <= 16) return 16;
@@ -484,6 +488,23 @@ extern "C" int b200_w8a8_gemm(const void* xq, const float* sx, const void* wq, c
                               int num_sms, int force_mode, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0 || (K % 16) != 0) return -1;
   if ((reinterpret_cast<uintptr_t>(xq) & 15) || (reinterpret_cast<uintptr_t>(wq) & 15)) return -2;
+  const bool pair_ok = !out_fp32 && !residual && N % 8 == 0 && ldy % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0 &&
+                       (reinterpret_cast<uintptr_t>(sw) & 15) == 0;
+  if (pair_ok && (force_mode >= 64 || (force_mode < 0 && M > 128))) {
+    // Rounds of the pairs times the cost of a tile (main loop ~ its channels, plus a fixed part).  Above 128 tokens a pair
+    // is never slower than a CTA alone: 200 x 28,672 x 4,096 30 us (40), 1,024 x 6,144 x 4,096 23 (37), 32,768 x 28,672 x
+    // 4,096 2,351 (2,989), 32,768 x 4,096 x 14,336 1,150 (1,341).
+    int bn = force_mode;
+    if (bn < 0) {
+      long long best = -1;
+      for (int cand : {256, 224, 192, 160, 128}) {
+        const long long tiles = static_cast<long long>((M + 255) / 256) * ((N + cand - 1) / cand), pairs = num_sms / 2;
+        const long long cost = (tiles + pairs - 1) / pairs * (cand + 32);
+        if (best < 0 || cost < best) { best = cost; bn = cand; }
+      }
+    }
+    return w8a8_gemm_pair(xq, sx, wq, sw, y, M, N, K, ldy, bn, status, num_sms, stream);
+  }
   const bool swap = M <= SWAP_MAX_M;
   const int bn = gemm_pick_bn(M, N, num_sms);
   GemmParams p;

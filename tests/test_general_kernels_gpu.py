@@ -141,3 +141,19 @@ def test_rotary_writes_the_same_with_narrow_accesses(tokens, norm):
     a, b = x[..., :64], x[..., 64:]
     want = torch.cat([a * c - b * s, b * c + a * s], -1)
     assert (torch.cat([got[0][0], got[0][1]], 1).double() - want).abs().max() < 2.5e-2      # one bf16 rounding of values up to 6
+
+
+@pytest.mark.parametrize("bn", [-1, 256, 224, 192, 160, 128])
+@pytest.mark.parametrize("M,N,K", [(129, 8, 16), (256, 264, 128), (257, 512, 272), (300, 1000, 1040), (1000, 2048, 896), (5000, 1288, 256)])
+def test_int8_linear_of_two_ctas_per_tile(M, N, K, bn):
+    """Edges of the 256-row tiles, channels that end inside a tile, K that ends inside a block, more tiles than pairs.  Whole
+    sums, scaled in fp32 (two roundings of 2^-24) and rounded once to bf16, whose eight bits of significand leave 2^-8: 2^-7.99."""
+    from mojo_linuxperiments_b200.ops import linear as L
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    x = torch.randint(-127, 128, (M, K), generator=g, device=DEV, dtype=torch.int8)
+    w = torch.randint(-127, 128, (N, K), generator=g, device=DEV, dtype=torch.int8)
+    sx, sw = torch.rand(M, generator=g, device=DEV) + 0.1, torch.rand(N, generator=g, device=DEV) + 0.1
+    y = L.w8a8_gemm(x, sx, w, sw, force_mode=bn)
+    _ok()
+    want = (x.double() @ w.double().t()) * sx.double()[:, None] * sw.double()
+    assert ((y.double() - want).abs() <= 2 ** -7.99 * want.abs()).all()
