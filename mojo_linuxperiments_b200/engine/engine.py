@@ -93,6 +93,7 @@ class Engine:
         self._admitted = max_total_len
         self._active_host = [0] * batch     # what ``active`` holds
         self._lens = [0] * batch            # tokens per slot already in the cache (host mirror of ``positions``); 0: empty
+        self._pages_at = [0] * batch        # tokens per slot from which on its pages have to be looked at again (0: at the next step)
         self._host_len = 0                  # longest of them
 
     def _place_buffers(self, batch: int) -> None:
@@ -158,7 +159,7 @@ class Engine:
         self.active[:B].fill_(1)
         self._active_host[:B] = [1] * B
         for b in range(B):
-            self._lens[b] = S
+            self._set_len(b, S)
         self._host_len = max(self._lens)
         return self.tokens.clone()
 
@@ -232,7 +233,7 @@ class Engine:
         self.active[:B].fill_(1)
         self._active_host[:B] = [1] * B
         for b in range(B):
-            self._lens[b] = lens[b]
+            self._set_len(b, lens[b])
         self._host_len = max(self._lens)
         return self.tokens.clone()
 
@@ -247,7 +248,11 @@ class Engine:
 
     def _reset_slot(self, slot: int) -> None:
         self.kv.release(slot)
-        self._lens[slot] = 0
+        self._set_len(slot, 0)
+
+    def _set_len(self, slot: int, n: int) -> None:
+        self._lens[slot] = n
+        self._pages_at[slot] = 0
 
     # ---- explicit steps: given tokens in, logits out --------------------------------------------------------------
     def step(self, entries, use_graph: bool = True) -> list[torch.Tensor]:
@@ -287,8 +292,8 @@ class Engine:
             oi = torch.tensor(others, dtype=torch.int64).to(self.device, non_blocking=True)
             self.tokens.index_copy_(0, oi, keep.index_select(0, oi))
         logits = self._graph_logits[self.batch] if use_graph else self.model.last_logits
-        return [logits[s:s + 1][:len(w)].float().repeat(len(w), 1) if w else logits.new_empty((0, logits.shape[1]), dtype=torch.float32)
-                for s, _, w in entries]
+        rows = torch.tensor([s for s, _, w in entries for _ in w], dtype=torch.int64).to(self.device, non_blocking=True)
+        return list(logits.index_select(0, rows).float().split([len(w) for _, _, w in entries]))
 
     def _extend(self, entries) -> list[torch.Tensor]:
         """Portions of any length for any set of slots; long ones are cut so that a call carries at most
@@ -297,7 +302,13 @@ class Engine:
         if not self.model.supports_portions and any(self._lens[s] > 0 or t.numel() > cap for s, t, _ in entries):
             raise ValueError("this model's prefill takes whole prompts only")
         dev = self.device
-        out = [torch.empty((len(w), self.cfg.vocab), dtype=torch.float32, device=dev) for _, _, w in entries]
+        counts = [len(w) for _, _, w in entries]
+        first = [sum(counts[:i]) for i in range(len(counts))]
+        out = torch.empty((sum(counts), self.cfg.vocab), dtype=torch.float32, device=dev)
+
+        def index(values):
+            return torch.tensor(values, dtype=torch.int64).to(dev, non_blocking=True)
+
         done = [0] * len(entries)
         while True:
             room, part = cap, []                    # (entry, first token, tokens)
@@ -323,7 +334,7 @@ class Engine:
                     got.append((i, here, len(rows), next((len(rows) + j for j, k in enumerate(here) if want[k] == toks.numel() - 1), None)))
                     rows += [cu[-1] + want[k] - a for k in here]
                 cu.append(cu[-1] + n)
-                self._lens[slot] = start + n
+                self._set_len(slot, start + n)
                 done[i] = a + n
             self.kv.flush()
             last = torch.tensor(rows if rows or self.model.supports_portions else [0], dtype=torch.int64)
@@ -333,19 +344,20 @@ class Engine:
                                      last_idx=last.to(dev, non_blocking=True),
                                      portions=[(a, n) for a, (_, _, n) in zip(starts, part)])
             default_workspace(dev).next_step()
-            for i, ks, r0, final in got:
-                out[i].index_copy_(0, torch.tensor(ks, dtype=torch.int64).to(dev, non_blocking=True),
-                                   self.model.last_logits[r0:r0 + len(ks)].float())
-                if final is not None:                    # the portion's last token was asked for: its greedy continuation
-                    self.tokens[entries[i][0]:entries[i][0] + 1].copy_(nxt[final:final + 1])
-        for slot, _, _ in entries:
-            n = self._lens[slot]
-            self.positions[slot:slot + 1].fill_(n)
-            self.kv.seq_lens[slot:slot + 1].fill_(n + 1)
-            self.active[slot:slot + 1].fill_(1)
-            self._active_host[slot] = 1
+            if got:
+                out.index_copy_(0, index([first[i] + k for i, ks, _, _ in got for k in ks]), self.model.last_logits[:len(rows)].float())
+            ends = [(entries[i][0], final) for i, _, _, final in got if final is not None]
+            if ends:                                     # the portions' last tokens that were asked for: their greedy continuations
+                self.tokens.index_copy_(0, index([s for s, _ in ends]), nxt.index_select(0, index([r for _, r in ends])).to(self.tokens.dtype))
+        at = index([s for s, _, _ in entries])
+        lens = torch.tensor([self._lens[s] for s, _, _ in entries], dtype=torch.int32).to(dev, non_blocking=True)
+        self.positions.index_copy_(0, at, lens)
+        self.kv.seq_lens.index_copy_(0, at, lens + 1)
+        self.active.index_fill_(0, at, 1)
+        for s, _, _ in entries:
+            self._active_host[s] = 1
         self._host_len = max(self._lens)
-        return out
+        return list(out.split(counts))
 
     def admit_sequence(self, slot: int, prompt: torch.Tensor, use_graph: bool = True) -> torch.Tensor:
         """Between two decode steps: put a new sequence into slot ``slot`` (empty, or whose sequence is finished) of the
@@ -368,7 +380,7 @@ class Engine:
         self.kv.seq_lens[slot:slot + 1].fill_(S + 1)
         self.active[slot:slot + 1].fill_(1)
         self._active_host[slot] = 1
-        self._lens[slot] = S
+        self._set_len(slot, S)
         self._host_len = max(self._lens)
         return self.tokens[slot:slot + 1].clone()
 
@@ -382,7 +394,7 @@ class Engine:
         self.active[slot:slot + 1].zero_()
         self._active_host[slot] = 0
         self.tokens[slot:slot + 1].zero_()
-        self._lens[slot] = 0
+        self._set_len(slot, 0)
         self._host_len = max(self._lens)
 
     def _prefill_consts(self, b0: int, b1: int, S: int):
@@ -426,13 +438,16 @@ class Engine:
         # this step writes token number len + 1 of every running sequence: take the page it lands on if the sequence
         # does not own it yet (once per page_size steps and sequence), give back what no layer can see any more, and
         # push the page table if a row changed
+        # (looked at only where that can have changed: the GPU waits while the host goes through the slots)
         for b in run:
             n = self._lens[b]
-            self.kv.retire(b, n)
-            self.kv.admit(b, n + 1)
-            self._lens[b] = n + 1
+            if n >= self._pages_at[b]:
+                self.kv.retire(b, n)
+                self.kv.admit(b, n + 1)
+                self._pages_at[b] = self.kv.next_change(n)
         want = [0] * self.batch
         for b in run:
+            self._lens[b] += 1
             want[b] = 1
         if want != self._active_host:
             self.active.copy_(torch.tensor(want, dtype=torch.int32), non_blocking=True)

@@ -89,10 +89,12 @@ class KVState:
         self.seq_lens = alloc((num_seqs,), torch.int32)
         self.free_pages = list(range(self.num_pages - 2, -1, -1))
         self.owned: dict[int, list[int]] = {}       # page ids of a slot in token order; -1: given back by ``retire``
+        self._periods = {self.page_size, *(s.chunk for s in self.layout if s is not None and s.chunk)}
         self._retired: dict[int, int] = {}          # leading entries of ``owned`` that are -1
         # host mirror of the page table: rows are edited here; ``flush`` sends a snapshot (a ring of pinned buffers, so
         # that a copy still queued on the stream never sees an edit that belongs to a later step)
         self.table_host = torch.full((num_seqs, self.max_pages), self.scratch_page, dtype=torch.int32)
+        self._table = self.table_host.numpy()       # the same memory
         self._cuda = torch.cuda.is_available() and torch.device(device).type == "cuda"
         self._ring = [(self.table_host.clone().pin_memory(), torch.cuda.Event()) for _ in range(4)] if self._cuda else []
         self._turn = 0
@@ -107,15 +109,22 @@ class KVState:
         have = self.owned.setdefault(seq, [])
         if need - len(have) > len(self.free_pages):
             raise RuntimeError("KV cache exhausted")
-        while len(have) < need:
-            self.table_host[seq, len(have)] = self.free_pages[-1]
-            have.append(self.free_pages.pop())
+        if len(have) < need:
+            # one slice per call: an element of a tensor costs microseconds to set, and a batch of prompts takes thousands of pages
+            new = self.free_pages[len(have) - need:][::-1]
+            del self.free_pages[len(have) - need:]
+            self._table[seq, len(have):need] = new
+            have += new
             self._dirty = True
         self.pages_high_water = max(self.pages_high_water, self.num_pages - 1 - len(self.free_pages))
 
     def first_visible(self, pos: int) -> int:
         """Oldest position that some layer of a token at ``pos`` (or any later one) can still see."""
         return min(((pos - pos % s.chunk) if s.chunk else 0 for s in self.layout if s is not None), default=pos)
+
+    def next_change(self, pos: int) -> int:
+        """First position after ``pos`` at which a growing sequence needs another page or stops seeing one."""
+        return min((pos // n + 1) * n for n in self._periods)
 
     def retire(self, seq: int, pos: int) -> None:
         """The next token of slot ``seq`` goes to position ``pos``: pages that lie wholly before everything it can see
@@ -128,7 +137,7 @@ class KVState:
             self.free_pages.append(pages[i])
             pages[i] = -1
         if n1 > n0:
-            self.table_host[seq, n0:n1] = self.scratch_page
+            self._table[seq, n0:n1] = self.scratch_page
             self._retired[seq] = n1
             self._dirty = True
 
@@ -138,7 +147,7 @@ class KVState:
         self._retired.pop(seq, None)
         if pages:
             self.free_pages.extend(p for p in reversed(pages) if p >= 0)
-            self.table_host[seq].fill_(self.scratch_page)
+            self._table[seq] = self.scratch_page
             self._dirty = True
 
     def flush(self) -> None:

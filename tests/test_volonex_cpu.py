@@ -176,6 +176,26 @@ def test_cache_gives_back_pages_no_layer_can_see():
         kv.admit(1, 100)
 
 
+@pytest.mark.parametrize("start", [1, 15, 16, 17, 40, 77])
+def test_cache_changes_only_where_it_says(start):
+    """A sequence that grows token by token: looked at only at the positions ``next_change`` names, the cache takes and gives back the
+    same pages at the same positions as when every position is looked at."""
+    cfg = LC.tiny_volonex()
+    every, named = (KVState(cfg, RuntimeConfig(max_prefill_tokens=32), "cpu", 2, 512) for _ in range(2))
+    for kv in (every, named):
+        kv.admit(0, start + 1)
+    due = 0
+    for pos in range(start, 400):
+        every.retire(0, pos)
+        every.admit(0, pos + 1)
+        if pos >= due:
+            named.retire(0, pos)
+            named.admit(0, pos + 1)
+            due = named.next_change(pos)
+            assert due > pos
+        assert every.owned == named.owned and every.free_pages == named.free_pages and (every.table_host == named.table_host).all()
+
+
 def test_command_line_refuses_what_a_family_cannot_do(tmp_path, capsys):
     from mojo_linuxperiments_b200 import cli
     assert cli.main(["models"]) == 0
