@@ -1,4 +1,4 @@
-// W8A8 GEMM for decode (M <= 64 tokens): weight streaming with a split-K thread-block cluster.
+// W8A8 GEMM for decode (M <= 128 tokens): weight streaming with a split-K thread-block cluster.
 //
 //   Y[m,n] = (sum_k Xq[m,k] * Wq[n,k]) * sx[m] * sw[n]  (+ residual[m,n])
 //
@@ -10,7 +10,7 @@
 //     memory (tcgen05.alloc), whatever its other resources; in-kernel time stamps show two CTAs per SM running, so
 //     the host doubles the calculator's cluster counts for the two-CTA forms;
 //   * each CTA runs the usual TMA -> tcgen05.mma.kind::i8 -> TMEM pipeline (weights are the 128-row A operand, the
-//     token tile of BN in {16,32,64} rows is the B operand);
+//     token tile of BN in {16,32,64,128} rows is the B operand);
 //   * the S partial accumulators are combined through distributed shared memory: every CTA sends, for each of
 //     the S row slices of the tile, its int32 partial to the CTA that owns the slice (16-byte st.shared::cluster
 //     into an exchange buffer of its own, so nobody waits for a pipeline to drain), the cluster synchronises once,
@@ -115,6 +115,12 @@ __device__ __forceinline__ void emit2(const OutSink& k, int m, int n, float v0, 
   *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(k.y) + o) = __floats2bfloat162_rn(v0, v1);
 }
 
+// The 128-token form takes calls that the persistent kernel would also serve: it multiplies the scales in that kernel's order.
+template <int BN>
+__device__ __forceinline__ float scaled(int32_t acc, float w, float x) {
+  return BN > 64 ? static_cast<float>(acc) * (w * x) : static_cast<float>(acc) * w * x;
+}
+
 // u / m for the handful of values the inline prologue meets (u < 8 unrolled, m = 1..4)
 __device__ __forceinline__ int inl_div(int u, int m) {
   return m == 1 ? u : (m == 2 ? (u >> 1) : (m == 3 ? ((u * 11) >> 5) : (u >> 2)));
@@ -126,12 +132,18 @@ constexpr int INL_MAX_ROWS = 4;       // token rows the inline prologue handles
 constexpr int INL_UNITS = 8;          // (k-block, row) pairs per quantising warp: their rotated values stay in registers
 
 // dynamic shared memory: pipeline stages, split-K exchange buffer, channel / token scales, barriers, alignment slack
-constexpr int decode_smem_bytes(int bn, int stages) {
-  return stages * (TILE_N * BLOCK_K + bn * BLOCK_K) + (TILE_N + 16) * (bn + 4) * 4 + (TILE_N + 64) * 4 + STAT_BYTES + 1024 + 256;
+constexpr int decode_smem_bytes(int bn, int stages, bool xch = true) {
+  return stages * (TILE_N * BLOCK_K + bn * BLOCK_K) + (xch ? (TILE_N + 16) * (bn + 4) * 4 : 0) + (TILE_N + (bn > 64 ? bn : 64)) * 4 +
+         STAT_BYTES + 1024 + 256;
 }
 
-template <int BN, int STAGES>
-__global__ void __launch_bounds__(GEMM_THREADS, (BN == 64 ? 1 : 2))
+// XCH = false: no split along K (S == 1) and no exchange buffer, whose 74 KB are what keeps two CTAs of the 128-token form
+// from sharing an SM.
+// 65 to 128 tokens: the persistent kernel's tiles of 128 tokens x 64 to 256 channels left most SMs idle or ran in two rounds.
+// 100 tokens x 28,672 x 4,096 36 -> 25 us, x 4,096 x 14,336 36 -> 20, x 32,000 x 4,096 29 -> 26, x 6,144 x 4,096 14 -> 16 (the
+// exchange of 64 KB per CTA): a decode step of four layers spends 319 us in its linears, 388 before.
+template <int BN, int STAGES, bool XCH = true>
+__global__ void __launch_bounds__(GEMM_THREADS, ((BN >= 64 && XCH) ? 1 : 2))
 w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                         const DecodeGemmParams p) {
   constexpr int A_BYTES = TILE_N * BLOCK_K;
@@ -141,7 +153,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   constexpr uint32_t IDESC = umma_idesc_i8(TILE_N, BN);
   constexpr int XS = BN + 4;                      // words per channel row of the exchange buffer (16-byte aligned rows)
   constexpr int EX_ROWS = TILE_N + 16;            // S senders x (slice of at most 2 * ceil(64 / S) channels) <= 128 + 2 S
-  constexpr int EX_BYTES = EX_ROWS * XS * 4;      // [sender][channel of the slice][token]
+  constexpr int EX_BYTES = XCH ? EX_ROWS * XS * 4 : 0;      // [sender][channel of the slice][token]
   static_assert(STAGES * STAGE_BYTES >= BN * TILE_N * 4, "the staging buffer of the all-reduce tail aliases the pipeline stages");
 
   pdl_launch_dependents();     // the next kernel may be scheduled: it only reads our output after its own pdl_wait
@@ -150,7 +162,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   int32_t* ex = reinterpret_cast<int32_t*>(smem + STAGES * STAGE_BYTES);          // split-K exchange buffer
   float* sw_s = reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES + EX_BYTES);  // [128] channel scales of this tile
   float* sx_s = sw_s + TILE_N;                                                     // [BN] token scales
-  float* stat_s = sx_s + 64;                                                       // inline prologue: row statistics
+  float* stat_s = sx_s + (BN > 64 ? BN : 64);                                                       // inline prologue: row statistics
   uint64_t* bars = reinterpret_cast<uint64_t*>(stat_s + STAT_BYTES / 4);           // full[S], empty[S], tfull
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -163,7 +175,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   const uint32_t tfull_bar = bar_base + 8u * (2 * STAGES);
   const uint32_t xch_bar = bar_base + 8u * (2 * STAGES + 1);     // split-K exchange: bytes the other CTAs send to this one
 
-  const int S = p.splits;
+  const int S = XCH ? p.splits : 1;
   const int rank = static_cast<int>(cluster_ctarank());          // == blockIdx.x: position along K
   const bool prolog = p.qp.mode != QR_NONE;
   const bool inl = BN == 16 && prolog && p.qp.rows == 0;     // a few tokens: this CTA quantises its own operand (below)
@@ -538,7 +550,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < CH; ++j)
-          tile_f[(c * CH + j) * TP + row] = static_cast<float>(static_cast<int32_t>(r[j])) * swn * sx_s[c * CH + j];
+          tile_f[(c * CH + j) * TP + row] = scaled<BN>(static_cast<int32_t>(r[j]), swn, sx_s[c * CH + j]);
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");
       const size_t col0 = static_cast<size_t>(n_tile) * TILE_N;
@@ -577,7 +589,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         if (!n_ok || jm <= 0) continue;
 #pragma unroll
         for (int j = 0; j < CH; ++j)
-          if (j < jm) emit1(sink, mc + j, n, static_cast<float>(static_cast<int32_t>(r[j])) * swn * sx_s[c * CH + j]);
+          if (j < jm) emit1(sink, mc + j, n, scaled<BN>(static_cast<int32_t>(r[j]), swn, sx_s[c * CH + j]));
       }
     }
   } else {
@@ -665,8 +677,8 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
           if (!on[u]) continue;
           const int n = n_base + rr[u];
           const float sxj = sx_s[jj[u]];
-          const float v0 = static_cast<float>(a[u][0]) * sw_s[sw_off + rr[u]] * sxj;
-          const float v1 = static_cast<float>(a[u][1]) * sw_s[sw_off + rr[u] + 1] * sxj;
+          const float v0 = scaled<BN>(a[u][0], sw_s[sw_off + rr[u]], sxj);
+          const float v1 = scaled<BN>(a[u][1], sw_s[sw_off + rr[u] + 1], sxj);
           if (n + 1 < p.N) emit2(sink, m0 + jj[u], n, v0, v1);
           else if (n < p.N) emit1(sink, m0 + jj[u], n, v0);
         }
@@ -829,35 +841,35 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   B200_TRACE_FLUSH(TK_GEMM_DECODE);
 }
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, bool XCH = true>
 static int launch_decode(const CUtensorMap& tw, const CUtensorMap& tx, const DecodeGemmParams& p, dim3 grid, cudaStream_t stream) {
-  constexpr int SMEM = decode_smem_bytes(BN, STAGES);
+  constexpr int SMEM = decode_smem_bytes(BN, STAGES, XCH);
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(w8a8_gemm_decode_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    cudaError_t e = cudaFuncSetAttribute(w8a8_gemm_decode_kernel<BN, STAGES, XCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     // ask for the largest shared-memory carveout: with the default preference the occupancy calculator (and the
     // launch) may settle for a split of the L1 / shared array that holds fewer CTAs per SM than the kernel was sized for
-    cudaFuncSetAttribute(w8a8_gemm_decode_kernel<BN, STAGES>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute(w8a8_gemm_decode_kernel<BN, STAGES, XCH>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return -1000 - static_cast<int>(e);
     configured = true;
   }
-  cudaError_t e = launch_ex(w8a8_gemm_decode_kernel<BN, STAGES>, grid, dim3(GEMM_THREADS), SMEM, stream, static_cast<int>(grid.x), tw, tx, p);
+  cudaError_t e = launch_ex(w8a8_gemm_decode_kernel<BN, STAGES, XCH>, grid, dim3(GEMM_THREADS), SMEM, stream, static_cast<int>(grid.x), tw, tx, p);
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }
 
 // How many clusters of `s` CTAs of this kernel the GPU can hold at once (cached per instantiation and cluster size).
 static int resident_clusters_reported(int bn, int s);
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, bool XCH = true>
 static int max_resident_clusters(int s) {
   static int cache[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   if (s < 1 || s > 8) return 0;
   if (cache[s] > 0) return cache[s];
-  constexpr int SMEM = decode_smem_bytes(BN, STAGES);
-  cudaFuncSetAttribute(w8a8_gemm_decode_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+  constexpr int SMEM = decode_smem_bytes(BN, STAGES, XCH);
+  cudaFuncSetAttribute(w8a8_gemm_decode_kernel<BN, STAGES, XCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   // ask for the largest shared-memory carveout: with the default preference the occupancy calculator (and the
   // launch) may settle for a split of the L1 / shared array that holds fewer CTAs per SM than the kernel was sized for
-  cudaFuncSetAttribute(w8a8_gemm_decode_kernel<BN, STAGES>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  cudaFuncSetAttribute(w8a8_gemm_decode_kernel<BN, STAGES, XCH>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(s, 64, 1);
   cfg.blockDim = dim3(GEMM_THREADS);
@@ -867,14 +879,14 @@ static int max_resident_clusters(int s) {
   attr[0].val.clusterDim.x = s; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, w8a8_gemm_decode_kernel<BN, STAGES>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+  if (cudaOccupancyMaxActiveClusters(&n, w8a8_gemm_decode_kernel<BN, STAGES, XCH>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
   cache[s] = n > 0 ? n : -1;
   return cache[s];
 }
 
 // CTAs of the decode GEMM one SM really holds: two when twice the shared memory (plus the per-CTA reservation) fits
 static int ctas_per_sm(int bn) {
-  const int smem = bn <= 16 ? decode_smem_bytes(16, 5) : (bn <= 32 ? decode_smem_bytes(32, 4) : decode_smem_bytes(64, 7));
+  const int smem = bn <= 16 ? decode_smem_bytes(16, 5) : (bn <= 32 ? decode_smem_bytes(32, 4) : (bn <= 64 ? decode_smem_bytes(64, 7) : decode_smem_bytes(128, 4)));
   return 2 * (smem + 1024) <= 228 * 1024 ? 2 : 1;
 }
 
@@ -886,7 +898,8 @@ static int resident_clusters_reported(int bn, int s) {
   switch (bn) {
     case 16: return max_resident_clusters<16, 5>(s);
     case 32: return max_resident_clusters<32, 4>(s);
-    default: return max_resident_clusters<64, 7>(s);
+    case 64: return max_resident_clusters<64, 7>(s);
+    default: return max_resident_clusters<128, 4>(s);
   }
 }
 
@@ -918,8 +931,9 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
                             int num_sms, int force_splits, const ArTail* ar, cudaStream_t stream,
                             int groups = 0, const int* grp_offsets = nullptr, const int* grp_counts = nullptr,
                             int x_rows = 0, const QuantProlog* qp = nullptr) {
-  // Plain calls may bring several token tiles of 64 (one grid layer each; every layer streams the weights again, so this
-  // is for narrow outputs such as a router); the grouped, fused-prologue and all-reduce forms take one tile.
+  // Plain calls may bring several token tiles (one grid layer each; every layer streams the weights again, so this
+  // is for narrow outputs such as a router, whose tiles stay at 64 tokens so that more CTAs share the work); the grouped,
+  // fused-prologue and all-reduce forms take one tile.
   constexpr int MULTI_TILE_MAX_M = 4 * SWAP_MAX_M;
   if (M <= 0 || N <= 0 || K <= 0 || (K % 16) != 0) return -1;
   if (M > ((groups > 0 || qp || ar) ? SWAP_MAX_M : MULTI_TILE_MAX_M)) return -1;
@@ -935,7 +949,7 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
   }
   if (groups > 0 && ((N % TILE_N) || !grp_offsets || !grp_counts || ar)) return -1;
   if ((reinterpret_cast<uintptr_t>(xq) & 15) || (reinterpret_cast<uintptr_t>(wq) & 15)) return -2;
-  const int bn = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
+  const int bn = M <= 16 ? 16 : (M <= 32 ? 32 : ((M <= SWAP_MAX_M || N <= TILE_N) ? 64 : 128));
   DecodeGemmParams p;
   p.M = M; p.N = N; p.K = K;
   p.kblocks = (K + BLOCK_K - 1) / BLOCK_K;
@@ -1009,7 +1023,8 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
   switch (bn) {
     case 16: return launch_decode<16, 5>(tw, tx, p, grid, stream);
     case 32: return launch_decode<32, 4>(tw, tx, p, grid, stream);
-    default: return launch_decode<64, 7>(tw, tx, p, grid, stream);
+    case 64: return launch_decode<64, 7>(tw, tx, p, grid, stream);
+    default: return s > 1 ? launch_decode<128, 4>(tw, tx, p, grid, stream) : launch_decode<128, 3, false>(tw, tx, p, grid, stream);
   }
 }
 

@@ -37,6 +37,7 @@ def act_quant(x: torch.Tensor, *, mode: int = AQ_PLAIN, gamma: torch.Tensor | No
 
 
 DECODE_MAX_M = 64
+CLUSTER_MAX_M = 128     # the 128-token form of the cluster kernel: plain calls of more than one channel tile
 
 
 def w8a8_gemm(xq: torch.Tensor, sx: torch.Tensor, wq: torch.Tensor, sw: torch.Tensor, *,
@@ -45,7 +46,7 @@ def w8a8_gemm(xq: torch.Tensor, sx: torch.Tensor, wq: torch.Tensor, sw: torch.Te
               force_mode: int = -1, force_splits: int = 0, narrow: bool = False) -> torch.Tensor:
     """y[m,n] = (sum_k xq[m,k] wq[n,k]) * sx[m] * sw[n] (+ residual); int8 operands, int32 accumulate in TMEM.
 
-    Up to 64 tokens the cluster split-K weight-streaming kernel runs (``force_mode`` -1) unless the problem has
+    Up to 128 tokens the cluster split-K weight-streaming kernel runs (``force_mode`` -1) unless the problem has
     enough tiles for the persistent kernel; ``force_mode`` 0 / 1 select the persistent kernel's whole-tile / stream-K
     schedules, ``force_mode`` 2 the cluster kernel with ``force_splits`` CTAs per cluster, 128 to 256 the two-CTA kernel with that
     many channels per tile (its default above 128 tokens: what fills the rounds of the 74 pairs best)."""
@@ -61,7 +62,7 @@ def w8a8_gemm(xq: torch.Tensor, sx: torch.Tensor, wq: torch.Tensor, sw: torch.Te
         assert residual.dtype == torch.bfloat16 and residual.stride(0) == out.stride(0) and residual.stride(1) == 1
     w = workspace or default_workspace(xq.device)
     n_tiles = (N + 127) // 128
-    use_cluster = M <= DECODE_MAX_M and (force_mode == 2 or (force_mode == -1 and n_tiles < _DECODE_TILE_WAVES * _lib.num_sms(xq.device.index)))
+    use_cluster = (M <= DECODE_MAX_M or (M <= CLUSTER_MAX_M and n_tiles > 1)) and (force_mode == 2 or (force_mode == -1 and n_tiles < _DECODE_TILE_WAVES * _lib.num_sms(xq.device.index)))
     # a narrow output (a router: one channel tile) for up to 256 tokens is still a weight stream: the persistent
     # kernel would walk its whole K loop on one or two CTAs, the cluster kernel splits K and takes 64 tokens per grid layer
     # (one channel tile only: wider outputs stay on the persistent kernel, whose results the token-sharded paths are

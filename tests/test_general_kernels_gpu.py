@@ -157,3 +157,22 @@ def test_int8_linear_of_two_ctas_per_tile(M, N, K, bn):
     _ok()
     want = (x.double() @ w.double().t()) * sx.double()[:, None] * sw.double()
     assert ((y.double() - want).abs() <= 2 ** -7.99 * want.abs()).all()
+
+
+@pytest.mark.parametrize("splits", [0, 1, 2, 3, 5, 8])
+@pytest.mark.parametrize("M,N,K", [(65, 129, 1024), (96, 1000, 1040), (97, 384, 1792), (100, 4096, 1152), (128, 640, 2048), (128, 28672, 1024)])
+def test_int8_linear_of_65_to_128_tokens(M, N, K, splits):
+    """The 128-token form of the cluster kernel: ragged rows and channels, K that ends inside a block, every way to split.  Whole sums,
+    scaled in fp32 (two roundings of 2^-24); bf16 rounds once more: 2^-7.99 of the value as above, 2^-22 for an fp32 result."""
+    from mojo_linuxperiments_b200.ops import linear as L
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    x = torch.randint(-127, 128, (M, K), generator=g, device=DEV, dtype=torch.int8)
+    w = torch.randint(-127, 128, (N, K), generator=g, device=DEV, dtype=torch.int8)
+    sx, sw = torch.rand(M, generator=g, device=DEV) + 0.1, torch.rand(N, generator=g, device=DEV) + 0.1
+    y = L.w8a8_gemm(x, sx, w, sw, force_mode=2, force_splits=splits)
+    yf = L.w8a8_gemm(x, sx, w, sw, force_mode=2, force_splits=splits, out_dtype=torch.float32)
+    _ok()
+    want = (x.double() @ w.double().t()) * sx.double()[:, None] * sw.double()
+    assert ((y.double() - want).abs() <= 2 ** -7.99 * want.abs()).all() and ((yf.double() - want).abs() <= 2 ** -22 * want.abs()).all()
+    if splits == 0:
+        assert torch.equal(L.w8a8_gemm(x, sx, w, sw), y)
