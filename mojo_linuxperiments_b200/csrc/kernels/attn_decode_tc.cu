@@ -78,15 +78,18 @@ struct DecodeTcParams {
   int* status;
   unsigned long long limit_ns;
   // 1: the splits of a (sequence, kv head) are one thread-block cluster (cluster dims 1 x 1 x splits) and their partials
-  // meet in the shared memory of the cluster's first CTA, which merges them: no global scratch, no counter, no fence
+  // meet in the shared memory of the cluster's CTA of split 0, which merges them: no global scratch, no counter, no fence
   int cluster_merge;
+  // fused form: 1 = all CTAs of a sequence are one cluster (cluster dims hkv x 1 x splits, at most eight CTAs) that agrees on the
+  // row's scale; several splits merge as with cluster_merge first
+  int head_cluster;
   int early_tiles;     // fused form: request the first two K / V tiles before the dependency wait
   DecodeFuse f;
 };
 
 constexpr int ADC_ZONE_ROW = ADC_D + 2;            // one partial row in the merge zone: 128 values, max, sum
 constexpr int ADC_ZONE_MAX_SPLITS = 8;             // portable cluster size
-constexpr int ADC_ZONE_MAX_G = 4;                  // the zone is sized for groups of up to four query heads
+constexpr int ADC_ZONE_ROWS = 32;                  // the zone holds this many partial rows: splits x query heads of the group
 
 __device__ __forceinline__ void unpack8_bf16(const uint4& raw, float (&o)[8]) {
   const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
@@ -105,11 +108,11 @@ __device__ __forceinline__ uint4 pack8_bf16(const float (&v)[8]) {
 __device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16(v)); }
 
 // One head (128 values) handled by 8 consecutive lanes: lane c holds elements 8c..8c+7 (lo) and 64+8c..64+8c+7 (hi).
-// Optional RMSNorm over the head, then the rotate-half rotary embedding with the pairs (i, i + 64).  All 32 lanes of the
-// warp must call this together (the reduction shuffles inside groups of 8 lanes).
-__device__ __forceinline__ void head_norm_rope(float (&lo)[8], float (&hi)[8], const __nv_bfloat16* nw, float eps, int c,
+// Optional RMSNorm over the head (its weights wl, wh), then the rotate-half rotary embedding with the pairs (i, i + 64).  All 32
+// lanes of the warp must call this together (the reduction shuffles inside groups of 8 lanes).
+__device__ __forceinline__ void head_norm_rope(float (&lo)[8], float (&hi)[8], bool norm, const uint4& wl_raw, const uint4& wh_raw, float eps,
                                                const float (&cs)[8], const float (&sn)[8]) {
-  if (nw) {
+  if (norm) {
     float ss = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) ss += lo[j] * lo[j] + hi[j] * hi[j];
@@ -118,8 +121,8 @@ __device__ __forceinline__ void head_norm_rope(float (&lo)[8], float (&hi)[8], c
     ss += __shfl_xor_sync(0xffffffffu, ss, 4);
     const float r = rsqrtf(ss * (1.f / 128.f) + eps);
     float wl[8], wh[8];
-    unpack8_bf16(*reinterpret_cast<const uint4*>(nw + 8 * c), wl);
-    unpack8_bf16(*reinterpret_cast<const uint4*>(nw + 64 + 8 * c), wh);
+    unpack8_bf16(wl_raw, wl);
+    unpack8_bf16(wh_raw, wh);
 #pragma unroll
     for (int j = 0; j < 8; ++j) { lo[j] *= r * wl[j]; hi[j] *= r * wh[j]; }
   }
@@ -156,7 +159,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const DecodeT
   float* xch = reinterpret_cast<float*>(pQ + ADC_Q_TILE);          // [2][4 warps][16]: per-warp max, then sum
   float* ml_s = xch + 128;                                         // [16][2]: final (m, l) per head
   uint64_t* bars = reinterpret_cast<uint64_t*>(ml_s + 32);
-  enum { B_FULL = 0, B_EMPTY = 2, B_SFULL = 4, B_PFULL = 4 + NB, B_OFULL = 4 + 2 * NB, B_XCH = 5 + 2 * NB, B_COUNT = 6 + 2 * NB };
+  enum { B_FULL = 0, B_EMPTY = 2, B_SFULL = 4, B_PFULL = 4 + NB, B_OFULL = 4 + 2 * NB, B_XCH = 5 + 2 * NB, B_ROW = 6 + 2 * NB, B_COUNT = 7 + 2 * NB };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + B_COUNT);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* last_flag = const_cast<int*>(abort_flag) + 1;
@@ -166,7 +169,8 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const DecodeT
   float* vnew_s = row_s + G * ADC_D;               // [128]
   float* snew_s = vnew_s + ADC_D;                  // [16]
   float* amax_s = snew_s + 16;                     // [8]
-  float* zone = amax_s + 8;                        // cluster merge: [splits][G][ADC_ZONE_ROW] (G <= 4 only)
+  float* stat_s = amax_s + 8;                      // [8][4]: head cluster, the largest rotated value of each of its CTAs
+  float* zone = stat_s + 32;                       // cluster merge: [splits][G][ADC_ZONE_ROW]
   const uint32_t sRing = smem_u32(smem);
   const uint32_t sP = smem_u32(pP), sQ = smem_u32(pQ);
   const uint32_t bar0 = smem_u32(bars);
@@ -247,9 +251,9 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const DecodeT
         if (n) bulk_prefetch_l2(p.f.next_w + lo, static_cast<uint32_t>(n));
       }
     }
-    pdl_wait();
-    if (tid == 0) B200_TRACE(TK_ATTN_DECODE, TP_DEPS);
     // ---- rotate q (every CTA), and in the CTA that owns the new token: rotate k, append k and v to the cache, score ----
+    // Everything but the projections is read before the dependency wait, so that one round trip is left behind it
+    // (position -> tables and page -> projections were three: 3.0 -> 1.4 us at one sequence).
     const int pos = p.f.positions[b];
     const bool pos_ok = pos >= 0 && pos < p.f.max_pos;
     const __nv_bfloat16* row = p.f.qkv + static_cast<size_t>(b) * p.f.ld_qkv;
@@ -262,10 +266,12 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const DecodeT
       cache_row = (static_cast<size_t>(page) * 2 * p.hkv + kvh) * 16 + (pos & 15);      // K row; the V row is hkv * 16 rows further
     }
     if (has_new && !store_ok && tid == 0 && p.status) atomicCAS(p.status, 0, (int)ST_BAD_ARGUMENT | (5 << 8));
-    if (warp < (G * 8 + 31) / 32) {
-      const bool act = tid < G * 8;
-      const int g = act ? (tid >> 3) : 0, c = tid & 7;
-      float cs[8], sn[8];
+    const bool rotates = warp < (G * 8 + 31) / 32;
+    const bool act = tid < G * 8;
+    const int g = act ? (tid >> 3) : 0, c = tid & 7;
+    float cs[8], sn[8];
+    uint4 nw[4];                                       // norm weights of this lane: q lo, q hi, k lo, k hi
+    if (rotates) {
       if (pos_ok) {
         const float4 c0 = *reinterpret_cast<const float4*>(p.f.cos_tab + static_cast<size_t>(pos) * 64 + 8 * c);
         const float4 c1 = *reinterpret_cast<const float4*>(p.f.cos_tab + static_cast<size_t>(pos) * 64 + 8 * c + 4);
@@ -277,11 +283,23 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const DecodeT
 #pragma unroll
         for (int j = 0; j < 8; ++j) { cs[j] = 1.f; sn[j] = 0.f; }
       }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const __nv_bfloat16* w = i < 2 ? p.f.q_norm_w : p.f.k_norm_w;
+        nw[i] = w ? *reinterpret_cast<const uint4*>(w + 64 * (i & 1) + 8 * c) : make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
+    pdl_wait();
+    if (tid == 0) B200_TRACE(TK_ATTN_DECODE, TP_DEPS);
+    if (rotates) {
       const __nv_bfloat16* qh = row + static_cast<size_t>(kvh * G + g) * ADC_D;
+      const __nv_bfloat16* kh = row + static_cast<size_t>(p.hq + kvh) * ADC_D;
+      const uint4 q0 = *reinterpret_cast<const uint4*>(qh + 8 * c), q1 = *reinterpret_cast<const uint4*>(qh + 64 + 8 * c);
+      const uint4 k0 = *reinterpret_cast<const uint4*>(kh + 8 * c), k1 = *reinterpret_cast<const uint4*>(kh + 64 + 8 * c);
       float qlo[8], qhi[8];
-      unpack8_bf16(*reinterpret_cast<const uint4*>(qh + 8 * c), qlo);
-      unpack8_bf16(*reinterpret_cast<const uint4*>(qh + 64 + 8 * c), qhi);
-      head_norm_rope(qlo, qhi, p.f.q_norm_w, p.f.eps, c, cs, sn);
+      unpack8_bf16(q0, qlo);
+      unpack8_bf16(q1, qhi);
+      head_norm_rope(qlo, qhi, p.f.q_norm_w != nullptr, nw[0], nw[1], p.f.eps, cs, sn);
       const uint4 qa = pack8_bf16(qlo), qb = pack8_bf16(qhi);
       if (act) {
         *reinterpret_cast<uint4*>(pQ + (g >> 3) * 1024 + (g & 7) * 128 + ((c ^ (g & 7)) << 4)) = qa;            // chunk c
@@ -289,11 +307,10 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const DecodeT
       }
       if (has_new) {
         // every group of 8 lanes rotates the same k head; group 0 stores it
-        const __nv_bfloat16* kh = row + static_cast<size_t>(p.hq + kvh) * ADC_D;
         float klo[8], khi[8];
-        unpack8_bf16(*reinterpret_cast<const uint4*>(kh + 8 * c), klo);
-        unpack8_bf16(*reinterpret_cast<const uint4*>(kh + 64 + 8 * c), khi);
-        head_norm_rope(klo, khi, p.f.k_norm_w, p.f.eps, c, cs, sn);
+        unpack8_bf16(k0, klo);
+        unpack8_bf16(k1, khi);
+        head_norm_rope(klo, khi, p.f.k_norm_w != nullptr, nw[2], nw[3], p.f.eps, cs, sn);
         const uint4 ka = pack8_bf16(klo), kb = pack8_bf16(khi);
         if (act && g == 0 && store_ok) {
           __nv_bfloat16* dst = p.f.cache + cache_row * ADC_D;
@@ -326,9 +343,12 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const DecodeT
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (tid == 0) B200_TRACE(TK_ATTN_DECODE, 10);             // queries rotated, new token scored
   const uint32_t tmem_base = *tmem_slot;
   const bool cmerge = p.cluster_merge != 0;
-  if (cmerge) cluster_arrive_relaxed();          // "this CTA runs": waited for before the first store into a peer's zone
+  const bool hcl = FUSED && p.head_cluster != 0;
+  if (hcl && tid == 0) mbar_expect_tx(bar(B_ROW), static_cast<uint32_t>(p.hkv) * 16);       // one message of each CTA, this one included
+  if (cmerge || hcl) cluster_arrive_release();   // "this CTA runs": waited for before the first store into a peer's shared memory
 
   if (warp == 0) {
     if (lane == 0 && nb > 0) {
@@ -520,9 +540,9 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const DecodeT
       }
     }
     if (cmerge && p.splits > 1) {
-      // partial rows go straight into the shared memory of the cluster's first CTA
+      // partial rows go straight into the shared memory of the CTA of split 0
       cluster_wait_acquire();
-      const uint32_t z0 = mapa_shared(smem_u32(zone), 0u);
+      const uint32_t z0 = mapa_shared(smem_u32(zone), hcl ? static_cast<uint32_t>(kvh) : 0u);
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         const uint32_t zr = z0 + 4u * static_cast<uint32_t>((split * G + g) * ADC_ZONE_ROW);
@@ -635,6 +655,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const DecodeT
     }
     am = warp_max(am);
     if (lane == 0) amax_s[warp] = am;
+    if (tid == 0) B200_TRACE(TK_ATTN_DECODE, 8);            // rotated
     if (p.hkv == 1) {
       __syncthreads();
       float row_amax = 0.f;
@@ -647,6 +668,35 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const DecodeT
         if (g < G) *reinterpret_cast<uint32_t*>(p.f.xq + static_cast<size_t>(b) * p.f.ldq + g * ADC_D + 4 * lane) = quant_pack4(v[i], inv);
       }
       if (tid == 0) p.f.sx[b] = scale;
+    } else if (hcl) {
+      // The token's heads are spread over the cluster: every CTA tells the others its largest value (16 bytes counted on an
+      // mbarrier of the receiver) and quantises its own heads from registers.  Against the form below (rows parked in global
+      // memory, fence, counter, the last CTA reads them back): 1.4 us of 10 at one sequence instead of 2.3.
+      __syncthreads();
+      if (!cmerge) cluster_wait_acquire();             // every CTA of the cluster runs (the merge has waited for that already)
+      if (tid < p.hkv) {
+        float blk = 0.f;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) blk = fmaxf(blk, amax_s[w]);
+        const uint32_t bits = __float_as_uint(blk);
+        st_async_cluster_v4(mapa_shared(smem_u32(stat_s + 4 * kvh), static_cast<uint32_t>(tid)), bits, bits, bits, bits,
+                            mapa_shared(bar(B_ROW), static_cast<uint32_t>(tid)));
+      }
+      __syncwarp();
+      cluster_arrive_relaxed();                        // "my message is out": waited for below, so that no CTA leaves before
+      if (mbar_wait(bar(B_ROW), 0, abort_flag, p.status, (ST_TIMEOUT_PEER_FLAG | (5 << 8)), limit)) {
+        float row_amax = 0.f;
+        for (int k = 0; k < p.hkv; ++k) row_amax = fmaxf(row_amax, stat_s[4 * k]);
+        const float scale = quant_scale_from_amax(row_amax), inv = quant_inv_scale(scale);
+#pragma unroll
+        for (int i = 0; i < (GI < 2 ? 2 : GI); ++i) {
+          const int g = warp + i * NW;
+          if (g < G) *reinterpret_cast<uint32_t*>(p.f.xq + static_cast<size_t>(b) * p.f.ldq + (kvh * G + g) * ADC_D + 4 * lane) = quant_pack4(v[i], inv);
+        }
+        if (kvh == 0 && tid == 0) p.f.sx[b] = scale;
+      }
+      __syncwarp();
+      cluster_wait_acquire();
     } else {
       // the token's heads are spread over hkv CTAs: park the rotated rows, the last CTA to arrive quantises the token
 #pragma unroll
@@ -670,14 +720,29 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const DecodeT
       }
       __syncthreads();
       if (!*last_flag) { B200_TRACE_FLUSH(TK_ATTN_DECODE); return; }
+      if (tid == 0) B200_TRACE(TK_ATTN_DECODE, 9);          // the token's last CTA
       __threadfence();
-      float row_amax = 0.f;
-      for (int k = 0; k < p.hkv; ++k) row_amax = fmaxf(row_amax, __ldcg(p.f.blk_amax + static_cast<size_t>(b) * p.hkv + k));
-      const float scale = quant_scale_from_amax(row_amax), inv = quant_inv_scale(scale);
-      for (int h = warp; h < p.hq; h += NW) {
-        const float4 x = __ldcg(reinterpret_cast<const float4*>(p.f.rot_scratch + (static_cast<size_t>(b) * p.hq + h) * ADC_D + 4 * lane));
-        const float xv[4] = {x.x, x.y, x.z, x.w};
-        *reinterpret_cast<uint32_t*>(p.f.xq + static_cast<size_t>(b) * p.f.ldq + h * ADC_D + 4 * lane) = quant_pack4(xv, inv);
+      // up to HB heads of a warp and the maxima are requested together: one round trip to L2 instead of one per head
+      // (2.9 -> 1 us of a CTA's 12)
+      constexpr int HB = 6;
+      float row_amax = 0.f, scale = 0.f, inv = 0.f;
+      for (int h0 = warp; h0 < p.hq; h0 += HB * NW) {
+        float4 x[HB];
+#pragma unroll
+        for (int i = 0; i < HB; ++i)
+          if (h0 + i * NW < p.hq)
+            x[i] = __ldcg(reinterpret_cast<const float4*>(p.f.rot_scratch + (static_cast<size_t>(b) * p.hq + h0 + i * NW) * ADC_D + 4 * lane));
+        if (h0 == warp) {
+          for (int k = lane; k < p.hkv; k += 32) row_amax = fmaxf(row_amax, __ldcg(p.f.blk_amax + static_cast<size_t>(b) * p.hkv + k));
+          row_amax = warp_max(row_amax);
+          scale = quant_scale_from_amax(row_amax); inv = quant_inv_scale(scale);
+        }
+#pragma unroll
+        for (int i = 0; i < HB; ++i) {
+          if (h0 + i * NW >= p.hq) break;
+          const float xv[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+          *reinterpret_cast<uint32_t*>(p.f.xq + static_cast<size_t>(b) * p.f.ldq + (h0 + i * NW) * ADC_D + 4 * lane) = quant_pack4(xv, inv);
+        }
       }
       if (tid == 0) p.f.sx[b] = scale;
     }
@@ -1075,9 +1140,9 @@ typedef CUresult (*EncodeTiledFn3)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
 template <int G, bool FUSED, int NB>
 static int launch_adc(const CUtensorMap& tm, const DecodeTcParams& p, dim3 grid, cudaStream_t stream) {
   // rows of the CTA's heads, the new token's value row, a few scalars, and (groups of up to four heads) the merge zone
-  constexpr int SMEM = 2 * ADC_TILE + NB * ADC_P_TILE + ADC_Q_TILE + (128 + 32) * 4 + (6 + 2 * NB) * 8 + 64 + NB * 8 * 4 + 1024 +
+  constexpr int SMEM = 2 * ADC_TILE + NB * ADC_P_TILE + ADC_Q_TILE + (128 + 32) * 4 + (7 + 2 * NB) * 8 + 64 + NB * 8 * 4 + 1024 +
                        (G * ADC_D + ADC_D + 32) * 4 + 16 +
-                       ((G <= ADC_ZONE_MAX_G && NB <= ADC_NB) ? ADC_ZONE_MAX_SPLITS * G * ADC_ZONE_ROW * 4 : 0);
+                       (NB <= ADC_NB ? ADC_ZONE_ROWS * ADC_ZONE_ROW * 4 : 0);
   static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two CTAs per SM");
   static bool configured = false;
   if (!configured) {
@@ -1088,7 +1153,8 @@ static int launch_adc(const CUtensorMap& tm, const DecodeTcParams& p, dim3 grid,
     if (e != cudaSuccess) return -1000 - static_cast<int>(e);
     configured = true;
   }
-  if (p.cluster_merge) launch_ex_cluster(attn_decode_tc_kernel<G, FUSED, NB>, dim3(grid), dim3(ADC_THREADS), SMEM, stream, dim3(1, 1, grid.z), tm, p);
+  if (p.head_cluster) launch_ex_cluster(attn_decode_tc_kernel<G, FUSED, NB>, dim3(grid), dim3(ADC_THREADS), SMEM, stream, dim3(grid.x, 1, grid.z), tm, p);
+  else if (p.cluster_merge) launch_ex_cluster(attn_decode_tc_kernel<G, FUSED, NB>, dim3(grid), dim3(ADC_THREADS), SMEM, stream, dim3(1, 1, grid.z), tm, p);
   else launch_ex(attn_decode_tc_kernel<G, FUSED, NB>, dim3(grid), dim3(ADC_THREADS), SMEM, stream, 0, tm, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
@@ -1185,8 +1251,12 @@ static int attn_decode_tc_common(const void* q, const void* cache, int num_pages
   const int blocks_max = (max_pages * 16 + 127) / 128, per_max = (blocks_max + splits - 1) / splits;
   const bool long_form = fuse && !persistent && per_max > ADC_NB && G <= 8;   // (sixteen heads: the scores of nine blocks would not fit the registers)        // whole (or half) sequences per CTA: no merge zone
   if (per_max > (long_form ? ADC_NB_LONG : ADC_NB)) return -1;
-  p.cluster_merge = (!persistent && !long_form && cluster_env && G <= ADC_ZONE_MAX_G && splits >= 2 && splits <= ADC_ZONE_MAX_SPLITS &&
+  p.cluster_merge = (!persistent && !long_form && cluster_env && G * splits <= ADC_ZONE_ROWS && splits >= 2 && splits <= ADC_ZONE_MAX_SPLITS &&
                      static_cast<long long>(B) * hkv * splits <= 2ll * sm_count) ? 1 : 0;
+  // All CTAs of a sequence as one cluster, in a grid that is resident in one go as above: a decode step of four layers 271.8 ->
+  // 268.3 us at one sequence and 327.5 -> 324.3 at 32; at 100 sequences (800 CTAs in three waves) 496 -> 514.
+  p.head_cluster = fuse && fuse->xq && hkv > 1 && hkv * splits <= 8 && (splits == 1 || p.cluster_merge) &&
+                   static_cast<long long>(B) * hkv * splits <= 2ll * sm_count;
   if (splits > 1 && !p.cluster_merge && (!scratch || !counters)) return -1;
   if (persistent) {
     const int items = B * hkv * splits;
@@ -1253,7 +1323,7 @@ extern "C" int b200_attn_decode_fused(const void* qkv, long long ld_qkv, const i
 
 // CTAs of the tensor-core decode attention (group size 4, plain form) one SM holds at once.
 extern "C" int b200_attn_decode_tc_ctas_per_sm() {
-  constexpr int SMEM = 2 * ADC_TILE + ADC_NB * ADC_P_TILE + ADC_Q_TILE + (128 + 32) * 4 + (6 + 2 * ADC_NB) * 8 + 64 + ADC_NB * 8 * 4 + 1024;
+  constexpr int SMEM = 2 * ADC_TILE + ADC_NB * ADC_P_TILE + ADC_Q_TILE + (128 + 32) * 4 + (7 + 2 * ADC_NB) * 8 + 64 + ADC_NB * 8 * 4 + 1024;
   cudaFuncSetAttribute(attn_decode_tc_kernel<4, false, ADC_NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   cudaFuncSetAttribute(attn_decode_tc_kernel<4, false, ADC_NB>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   int blocks = 0;

@@ -174,7 +174,9 @@ def decode_impl(page_size: int, group: int) -> str:
 def pick_decode_splits_tc(B: int, hkv: int, max_len: int, num_sms: int = 148, fused: bool = False) -> int:
     """KV splits for the tensor-core decode kernel.  Measured on B200 its time is close to
     waves x (128-token blocks per CTA + 1.6) x 2.7 us with two CTAs per SM (the 1.6 is the per-CTA set-up, softmax
-    exchange and partial write), plus a little per split for the merge: few, long CTAs win once the grid fills the GPU."""
+    exchange and partial write), plus a merge (one unit and a little per split): few, long CTAs win once the grid fills the
+    GPU, and two blocks are not worth a merge (16 sequences x 4 KV heads x 256 tokens, four layers: 502 us a step in one
+    CTA each, 514 in two; 7 blocks in four CTAs 303, in one 316)."""
     blocks = max(1, (max_len + 127) // 128)
     smin = tc_min_splits(max_len, fused)     # fused: a CTA may take a whole sequence (one wave of long CTAs beats three
                                              # of short ones: every CTA pays ~1.6 blocks' worth of set-up and epilogue)
@@ -183,7 +185,7 @@ def pick_decode_splits_tc(B: int, hkv: int, max_len: int, num_sms: int = 148, fu
     # up to eight splits are one thread-block cluster that merges in shared memory: stay there when that is possible
     cap = 8 if smin <= 8 else 32
     for s in range(smin, max(smin, min(cap, blocks)) + 1):
-        cost = -(-(max(1, B * hkv) * s) // slots) * (-(-blocks // s) + 1.6) + 0.15 * s
+        cost = -(-(max(1, B * hkv) * s) // slots) * (-(-blocks // s) + 1.6) + 0.15 * s + (s > 1)
         if best_cost is None or cost < best_cost - 1e-9:
             best, best_cost = s, cost
     return best

@@ -279,3 +279,11 @@ def test_attn_decode_fused_refuses_a_position_outside_the_pages():
     assert code & 255 == 6, code
     assert cache.data[1, :, :, 15].abs().sum().item() > 0             # sequence 0 appended token 31
     assert cache.data[2:].abs().sum().item() == 0                      # nothing was written for sequence 1
+
+
+@pytest.mark.parametrize("hq,hkv,qk_norm,splits,longest", [(32, 4, True, 2, 300), (16, 2, False, 4, 1500), (8, 2, True, 3, 1400),
+                                                           (16, 1, True, 2, 300), (8, 1, False, 4, 1500), (14, 7, False, 1, 300)])
+def test_attn_decode_fused_with_one_cluster_per_sequence(hq, hkv, qk_norm, splits, longest):
+    """Up to eight CTAs of a sequence (KV heads x splits) as one cluster that merges and agrees on the row's scale, and the largest
+    merge zones: the bounds of the test above."""
+    test_attn_decode_fused_matches_the_three_kernels_it_replaces(hq, hkv, qk_norm, splits, longest)
