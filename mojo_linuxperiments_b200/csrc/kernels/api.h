@@ -104,6 +104,8 @@ int b200_argmax_rows_f32(const float* logits, long long ld, int rows, int n, int
                          long long* out_idx, cudaStream_t stream);
 int b200_argmax_merge(const float* cand_val, const long long* cand_idx, int world, int rows, long long* out_idx,
                       cudaStream_t stream);
+int b200_decode_advance(const long long* next, const int* active, int rows, long long* tokens, int* positions, int* seq_lens,
+                        int* step, int step_words, cudaStream_t stream);
 size_t b200_attn_decode_scratch_floats(int B, int hq, int splits);
 // seq_lens[b] > max_pages * page_size is clamped to that and ST_BAD_ARGUMENT is recorded in *status (optional).
 int b200_attn_decode(const void* q, const void* cache, const int* page_table, const int* seq_lens, void* out,

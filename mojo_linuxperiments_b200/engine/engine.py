@@ -15,6 +15,7 @@ import torch
 from ..models.config import RuntimeConfig
 from ..models.kvcache import KVState
 from ..models.registry import family_of
+from ..ops.attention import decode_advance
 from ..ops.workspace import Workspace, default_workspace, has_default_workspace, install_default_workspace
 from ..parallel.comm import Comm
 from ..utils.trace import op_range
@@ -414,10 +415,8 @@ class Engine:
 
     def _decode_body(self) -> None:
         nxt = self.model.forward(self.tokens, self.positions, self.kv, mode="decode", max_len=self.rt.max_seq_len)
-        self.tokens.copy_(nxt)
-        self.positions.add_(self.active)        # empty slots stay at position 0, length 0
-        self.kv.seq_lens.add_(self.active)
-        default_workspace(self.device).next_step()      # a launch replayed next step must not match this step's row flags
+        # empty slots stay at position 0, length 0; the step words: a launch replayed next step must not match this step's row flags
+        decode_advance(nxt, self.tokens, self.positions, self.kv.seq_lens, self.active, default_workspace(self.device).step)
 
     def decode_step(self, use_graph: bool = True) -> torch.Tensor:
         """One greedy token for every sequence of the batch; returns the device tensor of new ids [B].

@@ -123,6 +123,7 @@ class _Sig:
     b200_attn_prefill_paged = (I, [P, LL, P, LL, I, I, I, I, P, P, P, P, P, P, P])
     b200_attn_decode_paged = (I, [P, LL, P, LL, I, I, P, P, P, P, I, I, I, P, P, I, P, P])
     b200_argmax_merge = (I, [P, P, I, I, P, P])
+    b200_decode_advance = (I, [P, P, I, P, P, P, P, I, P])
     b200_attn_decode_scratch_floats = (c_size_t, [I, I, I])
     b200_attn_decode = (I, [P, P, P, P, P, P, P, I, I, I, I, I, I, F, P, P])
     b200_attn_decode_noalloc = (I, [P, P, P, P, P, I, I, I, I, I, I, F, P])

@@ -325,6 +325,16 @@ def argmax_merge(cand_val: torch.Tensor, cand_idx: torch.Tensor, out_idx: torch.
     return out_idx
 
 
+def decode_advance(nxt: torch.Tensor, tokens: torch.Tensor, positions: torch.Tensor, seq_lens: torch.Tensor, active: torch.Tensor,
+                   step: torch.Tensor) -> None:
+    """End of a decode step: ``tokens`` = ``nxt`` (int64), ``positions`` and ``seq_lens`` += ``active`` (int32), the step words += 1."""
+    rows = tokens.numel()
+    assert nxt.dtype == tokens.dtype == torch.int64 and nxt.numel() == rows and all(t.is_contiguous() for t in (nxt, tokens, step))
+    assert all(t.dtype == torch.int32 and t.is_contiguous() and t.numel() == rows for t in (positions, seq_lens, active)) and step.dtype == torch.int32
+    _lib.check(_lib.lib().b200_decode_advance(nxt.data_ptr(), active.data_ptr(), rows, tokens.data_ptr(), positions.data_ptr(), seq_lens.data_ptr(),
+                                              step.data_ptr(), step.numel(), _lib.stream()), "decode_advance")
+
+
 # ---------------------------------------------------------------------------------------------------------
 # attention over the paged cache with free head sizes (bf16 or fp32), optional chunk mask, sink and output gate
 # ---------------------------------------------------------------------------------------------------------

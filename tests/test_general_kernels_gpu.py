@@ -176,3 +176,20 @@ def test_int8_linear_of_65_to_128_tokens(M, N, K, splits):
     assert ((y.double() - want).abs() <= 2 ** -7.99 * want.abs()).all() and ((yf.double() - want).abs() <= 2 ** -22 * want.abs()).all()
     if splits == 0:
         assert torch.equal(L.w8a8_gemm(x, sx, w, sw), y)
+
+
+@pytest.mark.parametrize("rows", [1, 127, 128, 129, 300])
+def test_end_of_a_decode_step(rows):
+    """Whole numbers: exact."""
+    from mojo_linuxperiments_b200.ops import attention as A
+    g = torch.Generator(device=DEV).manual_seed(rows)
+
+    def ints(n, dtype=torch.int32):
+        return torch.randint(0, 9999, (n,), generator=g, device=DEV, dtype=dtype)
+
+    nxt, tokens, pos, lens, step = ints(rows, torch.int64), ints(rows, torch.int64), ints(rows), ints(rows), ints(4)
+    active = ints(rows) % 2
+    want = (pos + active, lens + active, step + 1)
+    A.decode_advance(nxt, tokens, pos, lens, active, step)
+    torch.cuda.synchronize()
+    assert torch.equal(tokens, nxt) and all(torch.equal(a, b) for a, b in zip((pos, lens, step), want))
