@@ -1,4 +1,4 @@
-// bf16 linear for prefill-sized calls on sm_100a:  v[m,n] = sum_k X[m,k] W[n,k], then a fused epilogue (dense_epilogue.cuh).
+// bf16 linear for calls of 65 to 128 tokens and for row lists on sm_100a (larger plain calls: bf16_gemm_pair.cu):  v[m,n] = sum_k X[m,k] W[n,k], then a fused epilogue (dense_epilogue.cuh).
 //
 //   X bf16 [M,K] (row pitch ldx), W bf16 [N,K] (row pitch ldw), fp32 accumulation in TMEM.
 //
@@ -7,9 +7,7 @@
 //     maps end at K and fill with zeros.
 //   * Persistent grid over whole tiles; the accumulator is double buffered in TMEM, so the epilogue of one tile runs
 //     under the main loop of the next.
-//   * Warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 epilogue.  An epilogue warp turns its 32 x 32 piece through
-//     shared memory, so that eight lanes share one token row and every global access is a run of 128 bytes: the residual
-//     form reads and writes fp32 rows.
+//   * Warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 epilogue (dense_tile.cuh).
 //   * Grouped form (experts): a table of row tiles names each tile's rows and its group, whose weights are rows
 //     group * N .. of one stacked matrix; a column tile that reaches into the next group's rows is cut in the epilogue.
 //   * Every wait is bounded; a CTA that gives up records a status code, drains and exits.
@@ -17,13 +15,12 @@
 #include "api.h"
 #include "launch.cuh"
 #include "gemm_common.cuh"
-#include "dense_epilogue.cuh"
+#include "dense_tile.cuh"
 
 namespace b200 {
 
 constexpr int BG_BK = 64;              // bf16 per k-block: one 128-byte swizzle row
 constexpr int BG_GROUP_M = 8;          // token tiles per rasterisation group
-constexpr int BG_SP = 36;              // floats per row of an epilogue warp's staging piece (conflict-free 16-byte accesses)
 
 struct BfGemmParams {
   int M, N, m_tiles, n_tiles, kblocks, num_tiles;
@@ -54,7 +51,7 @@ __device__ __forceinline__ BfTile bg_tile_at(const BfGemmParams& p, int m_tiles,
 }
 
 template <int BN, int STAGES>
-constexpr int bg_smem_bytes() { return STAGES * (128 + BN) * 128 + 4 * 32 * BG_SP * 4 + 1024 + 256; }
+constexpr int bg_smem_bytes() { return STAGES * (128 + BN) * 128 + 4 * 32 * DT_SP * 4 + 1024 + 256; }
 
 template <int BN, int STAGES>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
@@ -67,8 +64,8 @@ bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
   pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  float* stage_f = reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES);                  // [4 warps][32][BG_SP]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(stage_f + 4 * 32 * BG_SP);                  // full, empty, tfull[2], tempty[2]
+  float* stage_f = reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES);                  // [4 warps][32][DT_SP]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(stage_f + 4 * 32 * DT_SP);                  // full, empty, tfull[2], tempty[2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -143,107 +140,20 @@ bf16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     __syncwarp();
   } else {
     const int q = warp & 3;                 // TMEM lane quarter this warp may read
-    float* piece = stage_f + (warp - 2) * 32 * BG_SP;
+    float* piece = stage_f + (warp - 2) * 32 * DT_SP;
     int idx = 0;
-    const bool residual = p.epi.mode == B200_EPI_RESIDUAL, plain = p.epi.mode == B200_EPI_STORE && !p.epi.gate;
-    const bool plain16 = plain && !p.epi.out_f32, relu2 = p.epi.act == B200_ACT_RELU2;
-    const int r8 = lane >> 2, c8 = (lane & 3) * 8;           // the same with eight columns per lane
-    const int rr0 = lane >> 3, c4 = (lane & 7) * 4;          // row group and column quad of this lane in a 32 x 32 piece
+    DenseTileRows rows(p.epi, p.N, lane, piece);
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++idx) {
       const int a = idx & 1;
       const BfTile t = bg_tile_at(p, m_tiles, tile);
       const int m0 = t.m0 + q * 32, n0 = t.n_tile * BN;
-      // The residual rows of a piece are requested one piece ahead (the first even before the accumulator is complete):
-      // the epilogue is four warps, so what it needs is loads in flight.
-      float4 xn[8];
-      auto load_x = [&](int c) {
-        const int n = n0 + c * 32 + c4;
-#pragma unroll
-        for (int it = 0; it < 8; ++it) {
-          const int m = m0 + it * 4 + rr0;
-          if (m < t.m_end && n < p.N) xn[it] = *reinterpret_cast<const float4*>(p.epi.x + static_cast<long long>(m) * p.epi.ldx + n);
-        }
-      };
-      if (residual) load_x(0);
+      rows.begin(m0, t.m_end, n0);
       // one verdict per warp: the lanes stay together at the TMEM loads
       const bool ok = __all_sync(0xffffffffu, mbar_wait(tfull_bar(a), (idx >> 1) & 1u, abort_flag, p.status, (ST_TIMEOUT_TMEM_FULL | (9 << 8)), limit));
       if (!ok) break;
       tc_fence_after();
       const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + a * BN;
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        if (n0 + c * 32 >= p.N) break;
-        uint32_t r[32];
-        tmem_ld_x32(t_addr + c * 32, r);
-        float4 xc[8];
-        if (residual) {
-#pragma unroll
-          for (int it = 0; it < 8; ++it) xc[it] = xn[it];
-          if (c + 1 < BN / 32) load_x(c + 1);
-        }
-        tmem_ld_wait();
-        float* mine = piece + lane * BG_SP;
-#pragma unroll
-        for (int g = 0; g < 8; ++g)
-          *reinterpret_cast<float4*>(mine + 4 * g) = make_float4(__uint_as_float(r[4 * g]), __uint_as_float(r[4 * g + 1]),
-                                                                 __uint_as_float(r[4 * g + 2]), __uint_as_float(r[4 * g + 3]));
-        __syncwarp();
-        const int n = n0 + c * 32 + c4;
-        if (plain16) {
-          const int n8 = n0 + c * 32 + c8;
-          if (n8 < p.N) {
-            __nv_bfloat16* y = static_cast<__nv_bfloat16*>(p.epi.y) + static_cast<long long>(m0 + r8) * p.epi.ldy + n8;
-#pragma unroll
-            for (int it = 0; it < 4; ++it) {
-              const float* src = piece + (it * 8 + r8) * BG_SP + c8;
-              float v[8];
-              *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(src);
-              *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(src + 4);
-              if (relu2) {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) { v[k] = fmaxf(v[k], 0.f); v[k] *= v[k]; }
-              }
-              uint4 o;
-              uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const __nv_bfloat162 pb = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
-                ow[k] = *reinterpret_cast<const uint32_t*>(&pb);
-              }
-              if (m0 + it * 8 + r8 < t.m_end) *reinterpret_cast<uint4*>(y + static_cast<long long>(it * 8) * p.epi.ldy) = o;
-            }
-          }
-        } else if (plain) {
-          if (n < p.N) {
-            float* y = static_cast<float*>(p.epi.y) + static_cast<long long>(m0 + rr0) * p.epi.ldy + n;
-#pragma unroll
-            for (int it = 0; it < 8; ++it) {
-              float4 v = *reinterpret_cast<const float4*>(piece + (it * 4 + rr0) * BG_SP + c4);
-              if (relu2) {
-                v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f); v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f);
-                v.x *= v.x; v.y *= v.y; v.z *= v.z; v.w *= v.w;
-              }
-              if (m0 + it * 4 + rr0 < t.m_end) *reinterpret_cast<float4*>(y + static_cast<long long>(it * 4) * p.epi.ldy) = v;
-            }
-          }
-        } else if (n < p.N) {
-          if (residual) {
-            const EpiNorm nw = epi_norm_columns(p.epi, n);
-#pragma unroll
-            for (int it = 0; it < 8; ++it) {
-              const int rr = it * 4 + rr0, m = m0 + rr;
-              if (m < t.m_end) epi_residual4(p.epi, nw, m, n, *reinterpret_cast<const float4*>(piece + rr * BG_SP + c4), xc[it]);
-            }
-          } else {
-#pragma unroll
-            for (int it = 0; it < 8; ++it) {
-              const int rr = it * 4 + rr0, m = m0 + rr;
-              if (m < t.m_end) epi_apply4(p.epi, m, n, *reinterpret_cast<const float4*>(piece + rr * BG_SP + c4), t.group);
-            }
-          }
-        }
-        __syncwarp();
-      }
+      rows.template finish<BN / 32>(t_addr, t.group);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(tempty_bar(a));
@@ -268,6 +178,9 @@ static int launch_bf16_gemm(const CUtensorMap& tx, const CUtensorMap& tw, const 
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }
+
+int bf16_gemm_pair(const void* x, long long ldx, const void* w, long long ldw, int M, int N, int K, const b200_dense_epilogue* epi, int bn,
+                   int* status, int num_sms, cudaStream_t stream);
 
 // shared with the decode form: everything epi_apply4 relies on
 int dense_epilogue_check(const b200_dense_epilogue* e, int N) {
@@ -294,6 +207,21 @@ static int bf16_gemm_any(const void* x, long long ldx, const void* w, long long 
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w) & 15)) return -2;
   if (int rc = dense_epilogue_check(epi, N)) return rc;
   if (g && (g->groups <= 0 || !g->tiles || !g->num_tiles || g->max_tiles <= 0 || epi->mode != B200_EPI_STORE)) return -3;
+  if (!g && (force_bn < 0 || (force_bn == 0 && M > 128))) {
+    // As for int8 (w8a8_gemm.cu): rounds of the pairs times the cost of a tile; -force_bn names the channels.  From 130 tokens on a
+    // pair beats the best tile of a CTA alone: 130 x 16,384 x 2,048 22 -> 19 us, 200 x 2,048 x 8,192 43 -> 34, 1,000 x 576 x 2,048
+    // 17.6 -> 16.3, 4,200 x 16,384 x 2,048 226 -> 198 (1,425 TFLOP/s), 4,200 x 2,048 x 8,192 146 -> 100, 4,000 x 64 x 2,048 15 -> 13.
+    int bn = -force_bn;
+    if (bn != 256 && bn != 224 && bn != 192 && bn != 160 && bn != 128) {
+      long long best = -1;
+      for (int cand : {256, 224, 192, 160, 128}) {
+        const long long tiles = static_cast<long long>((M + 255) / 256) * ((N + cand - 1) / cand), pairs = num_sms / 2;
+        const long long cost = (tiles + pairs - 1) / pairs * (cand + 32);
+        if (best < 0 || cost < best) { best = cost; bn = cand; }
+      }
+    }
+    return bf16_gemm_pair(x, ldx, w, ldw, M, N, K, epi, bn, status, num_sms, stream);
+  }
   BfGemmParams p;
   p.M = M; p.N = N;
   p.m_tiles = g ? g->max_tiles : (M + 127) / 128;

@@ -193,3 +193,30 @@ def test_end_of_a_decode_step(rows):
     A.decode_advance(nxt, tokens, pos, lens, active, step)
     torch.cuda.synchronize()
     assert torch.equal(tokens, nxt) and all(torch.equal(a, b) for a, b in zip((pos, lens, step), want))
+
+
+@pytest.mark.parametrize("bn", [0, 256, 224, 192, 160, 128])
+@pytest.mark.parametrize("M,N,K", [(129, 4, 8), (256, 264, 136), (257, 518, 130), (300, 1000, 1040), (1000, 2048, 896), (5000, 1288, 256)])
+def test_bf16_linear_of_two_ctas_per_tile(M, N, K, bn):
+    """Edges of the 256-row tiles, channels that end inside a tile or a piece, K that ends inside a block, more tiles than pairs, all
+    three epilogues.  K products of bf16 are summed in fp32: K 2^-24 of the sum of their magnitudes at most; a bf16 result
+    rounds once more (2^-9 of the value, 2-norm below 4e-3)."""
+    from mojo_linuxperiments_b200.ops import dense as D
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    x = D.rows(M, K, torch.bfloat16, DEV)
+    x[:, :K].normal_(generator=g)
+    W = torch.randn((N, K), generator=g, device=DEV).to(torch.bfloat16)
+    w, xd, wd = D.DenseW.of(W, torch.bfloat16, DEV), x[:, :K].double(), W.double()
+    want, bound = xd @ wd.t(), K * 2 ** -24 * (xd.abs() @ wd.abs().t())
+    y, y16 = D.linear(x, w, out_dtype=torch.float32, force=-bn)[:, :N], D.linear(x, w, force=-bn)[:, :N]
+    s = D.rows(M, N, torch.float32, DEV)
+    s.normal_(generator=g)
+    base = s[:, :N].double()
+    D.linear_residual(x, w, s, 1.0, None, None, force=-bn)
+    glu = D.linear_glu(x, w, 7.0, force=-bn)[:, :N // 2].double()
+    _ok()
+    assert ((y.double() - want).abs() <= bound).all()
+    assert ((s[:, :N].double() - base - want).abs() <= bound + 2 ** -23 * (base.abs() + want.abs())).all()
+    a, u = want[:, 0::2].clamp(max=7.0), want[:, 1::2].clamp(-7.0, 7.0)
+    for got, ref in ((y16.double(), want), (glu, a * torch.sigmoid(1.702 * a) * (u + 1))):
+        assert (got - ref).norm() <= 4e-3 * ref.norm()
