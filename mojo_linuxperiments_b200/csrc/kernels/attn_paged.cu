@@ -1,11 +1,11 @@
-// General attention over a paged cache, bf16 or fp32, any head size: one CTA of four warps per (query token, query head).
+// General attention over a paged cache, bf16 or fp32, any head size: one CTA of four or eight warps per (query token, query head).
 //
 // The 32-bit form of a model and head sizes beyond the tensor-core kernels run here.  Blocks of 32 keys go to the warps in turn.
 // Scores: eight lanes per key, four elements each at a time, so that a load of the warp covers whole lines of four keys (a
 // lane per key touched 32 lines for four bytes each); fp32 sums, added across the eight lanes.  Then an online softmax per
 // block, the lanes share out the value dimensions (512 at a time; blockIdx.y picks the part), and the warps' sums are merged
 // through shared memory.  The latent form reads the query in two parts and takes the first dimensions of a cached key as its
-// value.  Bound by latency in decoding (few CTAs), by the cache lines of keys and values in prefill.
+// value.  Bound by latency in decoding and by the cache lines of keys and values in prefill.
 #include "ptx.cuh"
 #include "api.h"
 #include "launch.cuh"
@@ -28,7 +28,6 @@ __device__ __forceinline__ float4 ap_f4(const T* p, int n) {
   return make_float4(ap_f(p[0]), n > 1 ? ap_f(p[1]) : 0.f, n > 2 ? ap_f(p[2]) : 0.f, n > 3 ? ap_f(p[3]) : 0.f);
 }
 
-constexpr int APG_WARPS = 4;
 constexpr int APG_MAX_DV = 512;
 constexpr int APG_DV4 = APG_MAX_DV / 128;      // groups of four value dimensions a lane may hold
 
@@ -45,8 +44,9 @@ struct AttnPagedParams {
   int* status;
 };
 
-template <typename T, bool VEC>
+template <typename T, bool VEC, int APG_WARPS>
 __global__ void __launch_bounds__(32 * APG_WARPS) attn_paged_kernel(const __grid_constant__ AttnPagedParams p) {
+  constexpr bool FEW = APG_WARPS == 8;                  // few CTAs: loads in batches
   extern __shared__ __align__(16) float apg_q[];        // the query in fp32, [dk rounded up to four], zeros at the end
   __shared__ float part_ml[APG_WARPS][2];
   __shared__ __align__(16) float part_acc[APG_WARPS][APG_MAX_DV];
@@ -90,21 +90,63 @@ __global__ void __launch_bounds__(32 * APG_WARPS) attn_paged_kernel(const __grid
     const long long koff = there ? static_cast<long long>(page) * rec + row * dk : -1;
     const long long voff = there ? static_cast<long long>(page) * rec + (p.latent ? 0 : static_cast<long long>(p.c.kv_heads) * ps * dk) + row * vp + d0 : -1;
     float s = -INFINITY;
+    if constexpr (FEW) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const long long ko = __shfl_sync(0xffffffffu, koff, 4 * j + sub);
-      float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (ko >= 0)
-        for (int i = at; i < dk; i += 32) {
-          const float4 kv = ap_f4<VEC>(cache + ko + i, dk - i), qv = *reinterpret_cast<const float4*>(apg_q + i);
-          d.x = fmaf(qv.x, kv.x, d.x); d.y = fmaf(qv.y, kv.y, d.y); d.z = fmaf(qv.z, kv.z, d.z); d.w = fmaf(qv.w, kv.w, d.w);
+      for (int j0 = 0; j0 < 8; j0 += 4) {
+        long long ko[4];
+        float4 d[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          ko[j] = __shfl_sync(0xffffffffu, koff, 4 * (j0 + j) + sub);
+          d[j] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-      float t = (d.x + d.y) + (d.z + d.w);
-      t += __shfl_xor_sync(0xffffffffu, t, 1);
-      t += __shfl_xor_sync(0xffffffffu, t, 2);
-      t += __shfl_xor_sync(0xffffffffu, t, 4);
-      t = __shfl_sync(0xffffffffu, t, (lane & 3) * 8);               // key 4 j + (lane & 3)
-      if ((lane >> 2) == j && there) s = t * p.s.scale;
+        for (int i0 = at; i0 < dk; i0 += 128) {
+          float4 kv[4][4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              kv[j][u] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (ko[j] >= 0 && i0 + 32 * u < dk) kv[j][u] = ap_f4<VEC>(cache + ko[j] + i0 + 32 * u, dk - i0 - 32 * u);
+            }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (i0 + 32 * u >= dk) break;
+            const float4 qv = *reinterpret_cast<const float4*>(apg_q + i0 + 32 * u);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              d[j].x = fmaf(qv.x, kv[j][u].x, d[j].x); d[j].y = fmaf(qv.y, kv[j][u].y, d[j].y);
+              d[j].z = fmaf(qv.z, kv[j][u].z, d[j].z); d[j].w = fmaf(qv.w, kv[j][u].w, d[j].w);
+            }
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float t = (d[j].x + d[j].y) + (d[j].z + d[j].w);
+          t += __shfl_xor_sync(0xffffffffu, t, 1);
+          t += __shfl_xor_sync(0xffffffffu, t, 2);
+          t += __shfl_xor_sync(0xffffffffu, t, 4);
+          t = __shfl_sync(0xffffffffu, t, (lane & 3) * 8);             // key 4 (j0 + j) + (lane & 3)
+          if ((lane >> 2) == j0 + j && there) s = t * p.s.scale;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const long long ko = __shfl_sync(0xffffffffu, koff, 4 * j + sub);
+        float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ko >= 0)
+          for (int i = at; i < dk; i += 32) {
+            const float4 kv = ap_f4<VEC>(cache + ko + i, dk - i), qv = *reinterpret_cast<const float4*>(apg_q + i);
+            d.x = fmaf(qv.x, kv.x, d.x); d.y = fmaf(qv.y, kv.y, d.y); d.z = fmaf(qv.z, kv.z, d.z); d.w = fmaf(qv.w, kv.w, d.w);
+          }
+        float t = (d.x + d.y) + (d.z + d.w);
+        t += __shfl_xor_sync(0xffffffffu, t, 1);
+        t += __shfl_xor_sync(0xffffffffu, t, 2);
+        t += __shfl_xor_sync(0xffffffffu, t, 4);
+        t = __shfl_sync(0xffffffffu, t, (lane & 3) * 8);               // key 4 j + (lane & 3)
+        if ((lane >> 2) == j && there) s = t * p.s.scale;
+      }
     }
     float mx = s;
 #pragma unroll
@@ -121,18 +163,42 @@ __global__ void __launch_bounds__(32 * APG_WARPS) attn_paged_kernel(const __grid
 #pragma unroll
     for (int i = 0; i < APG_DV4; ++i) { acc[i].x *= a; acc[i].y *= a; acc[i].z *= a; acc[i].w *= a; }
     const int n = min(32, pos - k0 + 1);
-#pragma unroll 4
-    for (int j = 0; j < n; ++j) {
-      const float w = __shfl_sync(0xffffffffu, e, j);
-      const long long vo = __shfl_sync(0xffffffffu, voff, j);
-      if (vo < 0) continue;
+    if constexpr (FEW) {
 #pragma unroll
-      for (int i = 0; i < APG_DV4; ++i)
-        if (i * 128 + lane * 4 < dn) {
-          const float4 v = ap_f4<VEC>(cache + vo + i * 128 + lane * 4, dn - i * 128 - lane * 4);
-          acc[i].x = fmaf(w, v.x, acc[i].x); acc[i].y = fmaf(w, v.y, acc[i].y);
-          acc[i].z = fmaf(w, v.z, acc[i].z); acc[i].w = fmaf(w, v.w, acc[i].w);
+      for (int i = 0; i < APG_DV4; ++i) {
+        if (i * 128 >= dn) break;
+        const int d = i * 128 + lane * 4;
+        for (int j0 = 0; j0 < n; j0 += 8) {
+          float4 v[8];
+          float w[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            w[j] = __shfl_sync(0xffffffffu, e, j0 + j);                  // 0 where there is no key
+            const long long vo = __shfl_sync(0xffffffffu, voff, j0 + j);
+            v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (vo >= 0 && d < dn) v[j] = ap_f4<VEC>(cache + vo + d, dn - d);
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            acc[i].x = fmaf(w[j], v[j].x, acc[i].x); acc[i].y = fmaf(w[j], v[j].y, acc[i].y);
+            acc[i].z = fmaf(w[j], v[j].z, acc[i].z); acc[i].w = fmaf(w[j], v[j].w, acc[i].w);
+          }
         }
+      }
+    } else {
+#pragma unroll 4
+      for (int j = 0; j < n; ++j) {
+        const float w = __shfl_sync(0xffffffffu, e, j);
+        const long long vo = __shfl_sync(0xffffffffu, voff, j);
+        if (vo < 0) continue;
+#pragma unroll
+        for (int i = 0; i < APG_DV4; ++i)
+          if (i * 128 + lane * 4 < dn) {
+            const float4 v = ap_f4<VEC>(cache + vo + i * 128 + lane * 4, dn - i * 128 - lane * 4);
+            acc[i].x = fmaf(w, v.x, acc[i].x); acc[i].y = fmaf(w, v.y, acc[i].y);
+            acc[i].z = fmaf(w, v.z, acc[i].z); acc[i].w = fmaf(w, v.w, acc[i].w);
+          }
+      }
     }
   }
   if (lane == 0) { part_ml[warp][0] = m; part_ml[warp][1] = l; }
@@ -163,17 +229,25 @@ __global__ void __launch_bounds__(32 * APG_WARPS) attn_paged_kernel(const __grid
 
 using namespace b200;
 
-template <typename T, bool VEC>
-static int launch_attn_paged_as(const AttnPagedParams& p, cudaStream_t stream) {
+template <typename T, bool VEC, int WARPS>
+static int launch_attn_paged_warps(const AttnPagedParams& p, cudaStream_t stream) {
   const size_t smem = static_cast<size_t>((p.c.dk + 3) & ~3) * sizeof(float);
-  if (smem > (32u << 10)) {            // with the static part this passes what a kernel may use unasked
-    cudaError_t e = cudaFuncSetAttribute(attn_paged_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  if (smem > (30u << 10)) {            // with the static part this passes what a kernel may use unasked
+    cudaError_t e = cudaFuncSetAttribute(attn_paged_kernel<T, VEC, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return -1000 - static_cast<int>(e);
   }
-  launch_ex(attn_paged_kernel<T, VEC>, dim3(static_cast<unsigned>(p.M) * p.hq, (p.dv + APG_MAX_DV - 1) / APG_MAX_DV), dim3(32 * APG_WARPS), smem,
+  launch_ex(attn_paged_kernel<T, VEC, WARPS>, dim3(static_cast<unsigned>(p.M) * p.hq, (p.dv + APG_MAX_DV - 1) / APG_MAX_DV), dim3(32 * WARPS), smem,
             stream, 0, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
+}
+// Up to one CTA per SM (decoding a few sequences) the latency of the loads counts: eight warps, and the parts of four keys (eight
+// values) are on their way before the first is used: 2 sequences of 190 keys, 16 heads of 128 in fp32, 14.6 us (25.9 with four warps
+// and a key at a time), 1 of 1,000 23 (92).  With more CTAs than that the registers of the batches cost more than they give: 32
+// sequences of 500 keys, 32 heads, 97 us as it is, 105 in batches; 300 tokens, heads of 512, 217 and 316.
+template <typename T, bool VEC>
+static int launch_attn_paged_as(const AttnPagedParams& p, cudaStream_t stream) {
+  return static_cast<long long>(p.M) * p.hq <= 148 ? launch_attn_paged_warps<T, VEC, 8>(p, stream) : launch_attn_paged_warps<T, VEC, 4>(p, stream);
 }
 
 static int launch_attn_paged(const AttnPagedParams& p, cudaStream_t stream) {

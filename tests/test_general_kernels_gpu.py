@@ -27,16 +27,18 @@ def test_f32_linear_at_tile_and_split_edges(M, N, K, aligned):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("repeat", [1, 4])
 @pytest.mark.parametrize("dk,dv,chunk", [(10, 6, None), (8, 8, 40), (130, 516, None), (36, 644, 100)])
-def test_general_attention_with_uneven_head_sizes(dk, dv, chunk, dtype):
-    """Head sizes that are no multiple of four, several parts of value dimensions, one to several blocks of keys per warp."""
+def test_general_attention_with_uneven_head_sizes(dk, dv, chunk, repeat, dtype):
+    """Head sizes that are no multiple of four, several parts of value dimensions, one to several blocks of keys per warp; few CTAs
+    (eight warps) and many."""
     from mojo_linuxperiments_b200.ops import attention as A
     H, G, n, ps = 4, 2, 300, 16
     g = torch.Generator(device=DEV).manual_seed(dk)
     cache = A.PagedKVCache(32, G, ps, DEV, dk=dk, dv=dv, dtype=dtype)
     cache.data.normal_(generator=g)
     table = torch.randperm(32, generator=torch.Generator().manual_seed(1))[:20].to(torch.int32).view(1, 20).to(DEV)
-    where = [0, 1, 31, 32, 33, 127, 128, 129, 255, n - 1]
+    where = [0, 1, 31, 32, 33, 127, 128, 129, 255, n - 1] * repeat
     pos = torch.tensor(where, dtype=torch.int32, device=DEV)
     q = torch.randn((len(where), H * dk), generator=g, device=DEV).to(dtype)
     sink = torch.randn(H, generator=g, device=DEV)
