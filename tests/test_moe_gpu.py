@@ -96,3 +96,38 @@ def test_tiny_moe_model_matches_oracle():
             assert (top2[0] - top2[1]).item() < 0.08 * logs[t].abs().max().item()
             break
     assert agree >= B * NEW // 2
+
+
+@pytest.mark.parametrize("M,k,E,e0,n_local,d", [(511, 8, 128, 0, 128, 2048), (512, 8, 128, 0, 128, 2048), (1366, 3, 16, 0, 16, 272), (4097, 1, 8, 2, 5, 4112),
+                                                (2000, 10, 64, 32, 32, 512), (900, 6, 1024, 0, 1024, 16)])
+def test_work_list_of_many_pairs(M, k, E, e0, n_local, d):
+    """Around and above the 4,096 pairs from which on a cluster builds the list and warps walk the rows: whole numbers, exact; the
+    weighted sum in fp32 (k terms, each rounded twice by 2^-24) rounded once to bf16, whose eight bits of significand leave 2^-8."""
+    from mojo_linuxperiments_b200.ops import moe as MO
+    g = torch.Generator().manual_seed(M)
+    ids = torch.stack([torch.randperm(E, generator=g)[:k] for _ in range(M)]).to(torch.int32).cuda()
+    w = MO.moe_align(ids, e0, n_local)
+    local = (ids >= e0) & (ids < e0 + n_local)
+    counts = torch.bincount((ids[local] - e0).long(), minlength=n_local)
+    total = int(counts.sum())
+    first = torch.cat([counts.new_zeros(1), counts.cumsum(0)])
+    assert torch.equal(w.counts.long(), counts) and torch.equal(w.offsets.long(), first) and w.meta[0] == total
+    assert torch.equal(w.inv >= 0, local) and torch.equal(w.inv[local].long().sort().values, torch.arange(total, device="cuda"))
+    slot, expert = w.inv[local].long(), (ids[local] - e0).long()
+    assert ((slot >= first[expert]) & (slot < first[expert + 1])).all()
+    token = torch.arange(M, device="cuda")[:, None].expand(M, k)[local]
+    assert torch.equal(w.slot_token[slot].long(), token)
+    tiles = [[e, f + j, min(128, c - j), 0] for e, (c, f) in enumerate(zip(counts.tolist(), first.tolist())) for j in range(0, c, 128)]
+    assert w.meta[1] == len(tiles) and w.tiles[:len(tiles)].tolist() == tiles
+    xq = torch.randint(-127, 128, (M, d), generator=g, dtype=torch.int8).cuda()
+    sx, wts = torch.rand(M, generator=g).cuda(), torch.rand((M, k), generator=g).cuda()
+    xp, sp = MO.moe_gather(xq, sx, w)
+    x16 = xq.to(torch.bfloat16)
+    rows = MO.gather_rows(x16, w)
+    at = w.slot_token[:total].long()
+    assert torch.equal(xp[:total], xq[at]) and torch.equal(sp[:total], sx[at]) and torch.equal(rows[:total], x16[at])
+    y = torch.randn((w.max_slots, d), generator=g).to(torch.bfloat16).cuda()
+    out = MO.moe_combine(y, w, wts)
+    want = (y[w.inv.clamp(min=0).long()].double() * (wts.double() * local)[:, :, None]).sum(1)
+    bound = 2 ** -7.99 * want.abs() + k * 2 ** -23 * (y[w.inv.clamp(min=0).long()].double().abs() * wts.double()[:, :, None]).sum(1)
+    assert ((out.double() - want).abs() <= bound).all()
