@@ -48,8 +48,9 @@ def w8a8_gemm(xq: torch.Tensor, sx: torch.Tensor, wq: torch.Tensor, sw: torch.Te
 
     Up to 128 tokens the cluster split-K weight-streaming kernel runs (``force_mode`` -1) unless the problem has
     enough tiles for the persistent kernel; ``force_mode`` 0 / 1 select the persistent kernel's whole-tile / stream-K
-    schedules, ``force_mode`` 2 the cluster kernel with ``force_splits`` CTAs per cluster, 128 to 256 the two-CTA kernel with that
-    many channels per tile (its default above 128 tokens: what fills the rounds of the 74 pairs best)."""
+    schedules, ``force_mode`` 2 the cluster kernel with ``force_splits`` CTAs per cluster, 128, 160, 192, 224 or 256 the two-CTA
+    kernel with that many channels per tile (its default above 128 tokens: what fills the rounds of the 74 pairs best).
+    Any other number is -1, and a width has no effect where the two-CTA kernel cannot take the call."""
     assert xq.is_cuda and xq.dtype == torch.int8 and wq.dtype == torch.int8
     assert xq.is_contiguous() and wq.is_contiguous()
     M, K = xq.shape

@@ -161,6 +161,21 @@ def test_int8_linear_of_two_ctas_per_tile(M, N, K, bn):
     assert ((y.double() - want).abs() <= 2 ** -7.99 * want.abs()).all()
 
 
+@pytest.mark.parametrize("force", [3, 64, 100, 127, 129, 200, 512])
+@pytest.mark.parametrize("M", [100, 300])
+def test_int8_linear_takes_a_number_that_names_no_tile_width_as_none(M, force):
+    """Same kernel as without it above 128 tokens, the one-CTA kernel as with 0 below: the same bits either way."""
+    from mojo_linuxperiments_b200.ops import linear as L
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x = torch.randint(-127, 128, (M, 512), generator=g, device=DEV, dtype=torch.int8)
+    w = torch.randint(-127, 128, (520, 512), generator=g, device=DEV, dtype=torch.int8)
+    sx, sw = torch.rand(M, generator=g, device=DEV), torch.rand(520, generator=g, device=DEV)
+    want = L.w8a8_gemm(x, sx, w, sw, force_mode=-1 if M > 128 else 0)
+    got = L.w8a8_gemm(x, sx, w, sw, force_mode=force)
+    _ok()
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("splits", [0, 1, 2, 3, 5, 8])
 @pytest.mark.parametrize("M,N,K", [(65, 129, 1024), (96, 1000, 1040), (97, 384, 1792), (100, 4096, 1152), (128, 640, 2048), (128, 28672, 1024)])
 def test_int8_linear_of_65_to_128_tokens(M, N, K, splits):
