@@ -93,6 +93,7 @@ struct OutSink {
   float* vals; int cw, m0, n_base;
   __nv_bfloat16* part; int N;
   void* y; const __nv_bfloat16* residual; int ldy, out_fp32;
+  bool pairs;                   // bf16 pairs at even offsets of y and residual lie on four bytes
 };
 __device__ __forceinline__ void emit1(const OutSink& k, int m, int n, float v) {
   if (k.mode == 1) { k.vals[(m - k.m0) * k.cw + (n - k.n_base)] = v; return; }
@@ -107,7 +108,7 @@ __device__ __forceinline__ void emit2(const OutSink& k, int m, int n, float v0, 
   if (k.mode == 1) { *reinterpret_cast<float2*>(k.vals + (m - k.m0) * k.cw + (n - k.n_base)) = make_float2(v0, v1); return; }
   if (k.mode == 2) { *reinterpret_cast<__nv_bfloat162*>(k.part + static_cast<size_t>(m) * k.N + n) = __floats2bfloat162_rn(v0, v1); return; }
   const size_t o = static_cast<size_t>(m) * k.ldy + n;
-  if (k.out_fp32 || (o & 1)) { emit1(k, m, n, v0); emit1(k, m, n + 1, v1); return; }
+  if (k.out_fp32 || !k.pairs || (o & 1)) { emit1(k, m, n, v0); emit1(k, m, n + 1, v1); return; }
   if (k.residual) {
     const __nv_bfloat162 rb = *reinterpret_cast<const __nv_bfloat162*>(k.residual + o);
     v0 += __low2float(rb); v1 += __high2float(rb);
@@ -519,6 +520,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   sink.mode = ll ? 1 : (fuse_ar ? 2 : 0);
   sink.vals = vals; sink.cw = cw; sink.m0 = m0; sink.n_base = n_base; sink.part = part; sink.N = p.N;
   sink.y = p.y; sink.residual = p.residual; sink.ldy = p.ldy; sink.out_fp32 = p.out_fp32;
+  sink.pairs = ((reinterpret_cast<uintptr_t>(p.y) | reinterpret_cast<uintptr_t>(p.residual)) & 3) == 0;
 
   if (S == 1) {
     if (epi) asm volatile("bar.sync 1, 128;" ::: "memory");          // sx_s is complete (epilogue warps only)

@@ -195,6 +195,30 @@ def test_int8_linear_of_65_to_128_tokens(M, N, K, splits):
         assert torch.equal(L.w8a8_gemm(x, sx, w, sw), y)
 
 
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("M,N,ld", [(20, 256, 258), (100, 256, 258), (100, 257, 259), (200, 256, 258), (100, 256, 257)])
+def test_int8_linear_writes_rows_that_start_anywhere(M, N, ld, residual):
+    """Results and residual rows whose first element lies on two bytes only, even and odd pitches, in every kernel of the range: the
+    values of an aligned call (the scales may be multiplied in another order: one bf16 step), and nothing beside the rows."""
+    from mojo_linuxperiments_b200.ops import linear as L
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    x = torch.randint(-127, 128, (M, 2048), generator=g, device=DEV, dtype=torch.int8)
+    w = torch.randint(-127, 128, (N, 2048), generator=g, device=DEV, dtype=torch.int8)
+    sx, sw = torch.rand(M, generator=g, device=DEV) + 0.1, torch.rand(N, generator=g, device=DEV) + 0.1
+    buf, rbuf = (torch.full((M * ld + 1,), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    y, r = (b[1:].view(M, ld)[:, :N] for b in (buf, rbuf))
+    r.copy_(1e5 * torch.randn((M, N), generator=g, device=DEV))
+    L.w8a8_gemm(x, sx, w, sw, out=y, residual=r if residual else None)
+    _ok()
+    want = (x.double() @ w.double().t()) * sx.double()[:, None] * sw.double()
+    bound = 2 ** -7.99 * want.abs()                      # one rounding to bf16, before or after the residual joins
+    if residual:
+        want = want + r.double()
+        bound = bound + 2 ** -7.99 * want.abs()
+    assert ((y.double() - want).abs() <= bound).all()
+    assert buf[0] == 7.0 and (buf[1:].view(M, ld)[:, N:] == 7.0).all()
+
+
 @pytest.mark.parametrize("rows", [1, 127, 128, 129, 300])
 def test_end_of_a_decode_step(rows):
     """Whole numbers: exact."""
