@@ -116,6 +116,7 @@ int b200_attn_decode_tma(const void* q, const void* cache, int num_pages, const 
                          int max_pages, int splits, float scale, int* status, cudaStream_t stream);
 // Tensor-core form of the same (tcgen05 MMAs, scores in TMEM); needs splits >= b200_attn_decode_tc_min_splits(longest sequence).
 int b200_attn_decode_tc_min_splits(int max_len);
+int b200_attn_decode_tc_smem(int group, int long_form);
 int b200_attn_decode_tc(const void* q, const void* cache, int num_pages, const int* page_table, const int* seq_lens,
                         void* out, float* scratch, unsigned* counters, int B, int hq, int hkv, int page_size,
                         int max_pages, int splits, float scale, int* status, cudaStream_t stream);

@@ -91,6 +91,30 @@ constexpr int ADC_ZONE_ROW = ADC_D + 2;            // one partial row in the mer
 constexpr int ADC_ZONE_MAX_SPLITS = 8;             // portable cluster size
 constexpr int ADC_ZONE_ROWS = 32;                  // the zone holds this many partial rows: splits x query heads of the group
 
+// Shared memory of a CTA, in bytes from its 1,024-byte aligned start: what the kernel addresses and what a launch asks for.
+template <int G, int NB>
+struct AdcShared {
+  static constexpr int align16(int n) { return (n + 15) & ~15; }
+  static constexpr int BARRIERS = 7 + 2 * NB;
+  static constexpr int P = 2 * ADC_TILE;                       // [NB] behind the ring of two tiles
+  static constexpr int Q = P + NB * ADC_P_TILE;
+  static constexpr int XCH = Q + ADC_Q_TILE;                   // [2][4 warps][16] floats: per-warp max, then sum
+  static constexpr int BARS = XCH + 128 * 4;
+  static constexpr int WORDS = BARS + BARRIERS * 8;            // tensor-memory address, abort flag, last-CTA flag
+  static constexpr int PAGES = WORDS + 3 * 4;                  // [NB * 8] page ids of this CTA's blocks
+  // fused form: the finished (bf16-rounded) output rows of this CTA's heads, v and the scores of the new token, ...
+  static constexpr int ROW = align16(PAGES + NB * 8 * 4);      // [G][128] floats
+  static constexpr int VNEW = ROW + G * ADC_D * 4;             // [128]
+  static constexpr int SNEW = VNEW + ADC_D * 4;                // [16]
+  static constexpr int AMAX = SNEW + 16 * 4;                   // [8]: largest rotated value of each warp
+  static constexpr int STAT = AMAX + 8 * 4;                    // [8][4]: head cluster, the same of each of its CTAs
+  static constexpr int ZONE = STAT + 32 * 4;                   // [splits][G][ADC_ZONE_ROW] where splits merge as a cluster
+  static constexpr int END = ZONE + (NB <= ADC_NB ? ADC_ZONE_ROWS * ADC_ZONE_ROW * 4 : 0);
+  static constexpr int BYTES = END + 1024;                     // the start is rounded up
+  static_assert(BARS % 8 == 0 && STAT % 16 == 0, "barriers on 8 bytes, messages of 16");
+  static_assert(2 * (BYTES + 1024) <= 228 * 1024, "two CTAs per SM");
+};
+
 __device__ __forceinline__ void unpack8_bf16(const uint4& raw, float (&o)[8]) {
   const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
@@ -153,24 +177,23 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_kv, const DecodeT
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  // [ring 2 x 32K][P NB x 4K][Q 4K][exchange floats][barriers]
-  uint8_t* pP = smem + 2 * ADC_TILE;
-  uint8_t* pQ = pP + NB * ADC_P_TILE;
-  float* xch = reinterpret_cast<float*>(pQ + ADC_Q_TILE);          // [2][4 warps][16]: per-warp max, then sum
-  float* ml_s = xch + 128;                                         // [16][2]: final (m, l) per head
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ml_s + 32);
+  using Sh = AdcShared<G, NB>;
+  uint8_t* pP = smem + Sh::P;
+  uint8_t* pQ = smem + Sh::Q;
+  float* xch = reinterpret_cast<float*>(smem + Sh::XCH);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Sh::BARS);
   enum { B_FULL = 0, B_EMPTY = 2, B_SFULL = 4, B_PFULL = 4 + NB, B_OFULL = 4 + 2 * NB, B_XCH = 5 + 2 * NB, B_ROW = 6 + 2 * NB, B_COUNT = 7 + 2 * NB };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + B_COUNT);
+  static_assert(B_COUNT == Sh::BARRIERS, "barriers");
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Sh::WORDS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* last_flag = const_cast<int*>(abort_flag) + 1;
-  int* page_s = last_flag + 1;                     // [NB * 8] page ids of this CTA's blocks
-  // fused form only: the finished (bf16-rounded) output rows of this CTA's heads, v and the scores of the new token
-  float* row_s = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(page_s + NB * 8) + 15) & ~uintptr_t(15));   // [G][128]
-  float* vnew_s = row_s + G * ADC_D;               // [128]
-  float* snew_s = vnew_s + ADC_D;                  // [16]
-  float* amax_s = snew_s + 16;                     // [8]
-  float* stat_s = amax_s + 8;                      // [8][4]: head cluster, the largest rotated value of each of its CTAs
-  float* zone = stat_s + 32;                       // cluster merge: [splits][G][ADC_ZONE_ROW]
+  int* page_s = reinterpret_cast<int*>(smem + Sh::PAGES);
+  float* row_s = reinterpret_cast<float*>(smem + Sh::ROW);
+  float* vnew_s = reinterpret_cast<float*>(smem + Sh::VNEW);
+  float* snew_s = reinterpret_cast<float*>(smem + Sh::SNEW);
+  float* amax_s = reinterpret_cast<float*>(smem + Sh::AMAX);
+  float* stat_s = reinterpret_cast<float*>(smem + Sh::STAT);
+  float* zone = reinterpret_cast<float*>(smem + Sh::ZONE);
   const uint32_t sRing = smem_u32(smem);
   const uint32_t sP = smem_u32(pP), sQ = smem_u32(pQ);
   const uint32_t bar0 = smem_u32(bars);
@@ -1139,11 +1162,7 @@ typedef CUresult (*EncodeTiledFn3)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
 // whole sequence of up to 1,152 tokens - both sized for two CTAs per SM.
 template <int G, bool FUSED, int NB>
 static int launch_adc(const CUtensorMap& tm, const DecodeTcParams& p, dim3 grid, cudaStream_t stream) {
-  // rows of the CTA's heads, the new token's value row, a few scalars, and (groups of up to four heads) the merge zone
-  constexpr int SMEM = 2 * ADC_TILE + NB * ADC_P_TILE + ADC_Q_TILE + (128 + 32) * 4 + (7 + 2 * NB) * 8 + 64 + NB * 8 * 4 + 1024 +
-                       (G * ADC_D + ADC_D + 32) * 4 + 16 +
-                       (NB <= ADC_NB ? ADC_ZONE_ROWS * ADC_ZONE_ROW * 4 : 0);
-  static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two CTAs per SM");
+  constexpr int SMEM = AdcShared<G, NB>::BYTES;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(attn_decode_tc_kernel<G, FUSED, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
@@ -1321,9 +1340,21 @@ extern "C" int b200_attn_decode_fused(const void* qkv, long long ld_qkv, const i
                                max_pages, splits, scale, status, 0, 0, stream, &f);
 }
 
+// Dynamic shared memory of a CTA with `group` query heads per KV head; long_form: of the fused form for up to nine blocks.
+extern "C" int b200_attn_decode_tc_smem(int group, int long_form) {
+  switch (group) {
+    case 1: return long_form ? AdcShared<1, ADC_NB_LONG>::BYTES : AdcShared<1, ADC_NB>::BYTES;
+    case 2: return long_form ? AdcShared<2, ADC_NB_LONG>::BYTES : AdcShared<2, ADC_NB>::BYTES;
+    case 4: return long_form ? AdcShared<4, ADC_NB_LONG>::BYTES : AdcShared<4, ADC_NB>::BYTES;
+    case 8: return long_form ? AdcShared<8, ADC_NB_LONG>::BYTES : AdcShared<8, ADC_NB>::BYTES;
+    case 16: return long_form ? -1 : AdcShared<16, ADC_NB>::BYTES;
+    default: return -1;
+  }
+}
+
 // CTAs of the tensor-core decode attention (group size 4, plain form) one SM holds at once.
 extern "C" int b200_attn_decode_tc_ctas_per_sm() {
-  constexpr int SMEM = 2 * ADC_TILE + ADC_NB * ADC_P_TILE + ADC_Q_TILE + (128 + 32) * 4 + (7 + 2 * ADC_NB) * 8 + 64 + ADC_NB * 8 * 4 + 1024;
+  constexpr int SMEM = AdcShared<4, ADC_NB>::BYTES;
   cudaFuncSetAttribute(attn_decode_tc_kernel<4, false, ADC_NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   cudaFuncSetAttribute(attn_decode_tc_kernel<4, false, ADC_NB>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   int blocks = 0;

@@ -1,0 +1,28 @@
+"""What the kernel library's host side decides, and rules its sources keep: no GPU needed."""
+import pytest
+
+from mojo_linuxperiments_b200.ops import _lib
+
+
+@pytest.fixture(scope="module")
+def lib():
+    if not _lib._lib_path().exists():
+        pytest.skip("kernel library not built")
+    return _lib.lib()
+
+
+@pytest.mark.parametrize("long_form", [0, 1])
+@pytest.mark.parametrize("group", [1, 2, 4, 8, 16])
+def test_decode_attention_asks_for_all_the_shared_memory_it_addresses(lib, group, long_form):
+    """The parts of a CTA, one by one: ring, weights, queries, exchange, barriers, three words, page ids, rows of the heads, value and
+    scores of the new token, largest values of the warps and of the cluster's CTAs, merge zone."""
+    if group == 16 and long_form:
+        assert lib.b200_attn_decode_tc_smem(group, long_form) < 0
+        return
+    nb = 9 if long_form else 4
+    parts = 2 * 32768 + nb * 4096 + 4096 + 128 * 4 + (7 + 2 * nb) * 8
+    parts = (parts + 3 * 4 + nb * 8 * 4 + 15) // 16 * 16
+    parts += (group * 128 + 128 + 16 + 8 + 8 * 4) * 4 + (0 if long_form else 32 * 130 * 4)
+    got = lib.b200_attn_decode_tc_smem(group, long_form)
+    assert got >= parts + 1023                          # the start is moved to a multiple of 1,024
+    assert 2 * (got + 1024) <= 228 * 1024               # two CTAs per SM
