@@ -1,6 +1,7 @@
 """What the kernel library's host side decides, and rules its sources keep: no GPU needed."""
 import pytest
 
+from mojo_linuxperiments_b200 import _build
 from mojo_linuxperiments_b200.ops import _lib
 
 
@@ -26,3 +27,15 @@ def test_decode_attention_asks_for_all_the_shared_memory_it_addresses(lib, group
     got = lib.b200_attn_decode_tc_smem(group, long_form)
     assert got >= parts + 1023                          # the start is moved to a multiple of 1,024
     assert 2 * (got + 1024) <= 228 * 1024               # two CTAs per SM
+
+
+def test_cluster_barriers_are_reached_by_whole_warps():
+    """``barrier.cluster`` with ``.aligned`` is defined for converged warps only: every one of them stands behind a ``__syncwarp``."""
+    found = 0
+    for path in sorted((_build.CSRC / "kernels").glob("*.cu*")):
+        lines = path.read_text().splitlines()
+        for i, line in enumerate(lines):
+            if "barrier.cluster." in line and ".aligned" in line and "asm" in line:
+                found += 1
+                assert "__syncwarp();" in lines[i - 1], f"{path.name}:{i + 1}"
+    assert found >= 3
