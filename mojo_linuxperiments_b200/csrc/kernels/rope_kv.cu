@@ -239,8 +239,8 @@ __global__ void argmax_merge_kernel(const float* cand_val, const long long* cand
 }
 
 // End of a decode step: the sampled ids become the next step's tokens, the sequences that run move on by one.  One launch for
-// what were a copy and three additions, each a kernel of 1.3 to 1.8 us behind the last (a step of 268.3 us: 265.8).  The next
-// kernel must not start before this one is through: kernels read lengths and positions before their dependency wait.
+// what were a copy and three additions, each a kernel of 1.3 to 1.8 us behind the last (a step of 268.3 us: 265.8).  Kernels of the
+// next step read lengths and positions before their dependency wait: that step's first kernel is launched behind all of this one.
 __global__ void decode_advance_kernel(const long long* next, const int* active, int rows, long long* tokens, int* positions, int* seq_lens,
                                       int* step, int step_words) {
   pdl_wait();
@@ -287,7 +287,7 @@ extern "C" int b200_embed_gather(const long long* ids, const void* table, void* 
                                  cudaStream_t stream) {
   if (M <= 0) return 0;
   if (d % 8) return -1;
-  launch_ex(embed_gather_kernel, dim3(M), dim3(128), 0, stream, 0, ids, static_cast<const __nv_bfloat16*>(table), static_cast<__nv_bfloat16*>(out), d, vocab);
+  launch_first(embed_gather_kernel, dim3(M), dim3(128), 0, stream, ids, static_cast<const __nv_bfloat16*>(table), static_cast<__nv_bfloat16*>(out), d, vocab);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }

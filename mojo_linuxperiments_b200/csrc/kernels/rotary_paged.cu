@@ -127,8 +127,8 @@ extern "C" int b200_embed_norm(const long long* ids, const void* table, long lon
   const int d4 = (d + 3) & ~3;
   if (!ids || !table || !x || !norm || vocab <= 0 || d <= 0 || ldt < d4 || norm->ldx < d4 || norm->ldx % 4) return -1;
   if (norm->y && (norm->ldy < d4 || norm->ldy % 8)) return -2;
-  if (table_f32) launch_ex(embed_norm_kernel<float>, dim3(M), dim3(256), 0, stream, 0, ids, static_cast<const float*>(table), ldt, vocab, scale, d4, x, copy, *norm);
-  else launch_ex(embed_norm_kernel<__nv_bfloat16>, dim3(M), dim3(256), 0, stream, 0, ids, static_cast<const __nv_bfloat16*>(table), ldt, vocab, scale, d4, x, copy, *norm);
+  if (table_f32) launch_first(embed_norm_kernel<float>, dim3(M), dim3(256), 0, stream, ids, static_cast<const float*>(table), ldt, vocab, scale, d4, x, copy, *norm);
+  else launch_first(embed_norm_kernel<__nv_bfloat16>, dim3(M), dim3(256), 0, stream, ids, static_cast<const __nv_bfloat16*>(table), ldt, vocab, scale, d4, x, copy, *norm);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }

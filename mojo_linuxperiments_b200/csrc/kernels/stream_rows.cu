@@ -168,12 +168,14 @@ __global__ void __launch_bounds__(THREADS) stream_rows_kernel(const __grid_const
 template <typename T>
 static void launch_stream_rows(const StreamRowsParams& p, dim3 grid, cudaStream_t stream) {
   const int d4 = (p.d + 3) / 4;
-  if (d4 <= 64) launch_ex(stream_rows_kernel<T, 1, 64>, grid, dim3(64), 0, stream, 0, p);
-  else if (d4 <= 256) launch_ex(stream_rows_kernel<T, 1, 256>, grid, dim3(256), 0, stream, 0, p);
-  else if (d4 <= 512) launch_ex(stream_rows_kernel<T, 2, 256>, grid, dim3(256), 0, stream, 0, p);
-  else if (d4 <= 1024) launch_ex(stream_rows_kernel<T, 4, 256>, grid, dim3(256), 0, stream, 0, p);
-  else if (d4 <= 2048) launch_ex(stream_rows_kernel<T, 4, 512>, grid, dim3(512), 0, stream, 0, p);
-  else launch_ex(stream_rows_kernel<T, 8, 1024>, grid, dim3(1024), 0, stream, 0, p);
+  // embedding rows open a step (launch_first)
+  auto launch = [&](auto kernel, int threads) { launch_with(p.r.ids == nullptr, dim3(0, 1, 1), kernel, grid, dim3(threads), 0, stream, p); };
+  if (d4 <= 64) launch(stream_rows_kernel<T, 1, 64>, 64);
+  else if (d4 <= 256) launch(stream_rows_kernel<T, 1, 256>, 256);
+  else if (d4 <= 512) launch(stream_rows_kernel<T, 2, 256>, 256);
+  else if (d4 <= 1024) launch(stream_rows_kernel<T, 4, 256>, 256);
+  else if (d4 <= 2048) launch(stream_rows_kernel<T, 4, 512>, 512);
+  else launch(stream_rows_kernel<T, 8, 1024>, 1024);
 }
 
 }  // namespace b200

@@ -39,3 +39,13 @@ def test_cluster_barriers_are_reached_by_whole_warps():
                 found += 1
                 assert "__syncwarp();" in lines[i - 1], f"{path.name}:{i + 1}"
     assert found >= 3
+
+
+def test_the_kernels_that_open_a_step_wait_for_all_of_the_step_before():
+    """Kernels of a step read lengths, positions and page tables before their dependency wait; what orders them behind the writers is
+    that the first kernel (embedding rows, in each of its three forms) does not start early."""
+    for name, kernel, starts in (("rope_kv.cu", "embed_gather_kernel", ("launch_first(",)), ("rotary_paged.cu", "embed_norm_kernel", ("launch_first(",)),
+                                 ("stream_rows.cu", "launch_with(", ("launch_with(p.r.ids == nullptr,",))):
+        text = (_build.CSRC / "kernels" / name).read_text()
+        lines = [ln for ln in text.splitlines() if kernel in ln and "launch" in ln]
+        assert lines and all(any(s in ln for s in starts) for ln in lines), name

@@ -65,6 +65,30 @@ def test_graph_and_eager_decode_agree():
     assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("hkv", [2, 1])
+def test_eager_steps_of_a_tiny_model_follow_each_other(hkv):
+    """One sequence, one layer: kernels of a few microseconds whose prologues reach into the step before.  70 eager steps over
+    several pages give the tokens and the cache of the captured step."""
+    from dataclasses import replace
+    from mojo_linuxperiments_b200.engine.engine import Engine
+    cfg = replace(C.tiny_dense(), n_layers=1, n_kv_heads=hkv)
+    ck, _ = _setup(cfg, 5)
+    eng = Engine(cfg, C.RuntimeConfig(max_seq_len=128), weights=Wt.shard_from_checkpoint(cfg, ck, 1, 0, "cuda"))
+    prompt = torch.randint(0, cfg.vocab, (1, 11), generator=torch.Generator().manual_seed(4))
+    got = []
+    for graph in (True, False, False):
+        eng.start_batch(1, 128)
+        toks = [eng.prefill(prompt, use_graph=graph)]
+        for _ in range(70):
+            toks.append(eng.decode_step(use_graph=graph).clone())
+        eng.check_status()
+        page, row = eng.kv.page_table[0].long()[torch.arange(81, device="cuda") // 16], torch.arange(81, device="cuda") % 16
+        c = eng.kv.layers[0]
+        got.append((torch.cat(toks), c.keys()[page, :, row].clone(), c.values()[page, :, row].clone(), eng.positions.clone()))
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], other))
+
+
 def test_decode_past_the_admitted_length_is_refused_on_the_host():
     from mojo_linuxperiments_b200.engine.engine import Engine
     cfg = C.tiny_dense()
