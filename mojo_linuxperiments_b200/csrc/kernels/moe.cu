@@ -188,10 +188,10 @@ __global__ void __launch_bounds__(128) moe_gather_kernel(const int8_t* xq, const
 
 // many slots: a warp per slot at a time
 __global__ void __launch_bounds__(32 * MOE_WALK_WARPS) moe_gather_walk_kernel(const int8_t* xq, const float* sx, int d, const int* slot_token,
-                                                                              const int* meta, int8_t* xq_perm, float* sx_perm) {
+                                                                              const int* meta, int max_slots, int8_t* xq_perm, float* sx_perm) {
   pdl_launch_dependents();
   pdl_wait();
-  const int lane = threadIdx.x & 31, used = meta[0];
+  const int lane = threadIdx.x & 31, used = min(meta[0], max_slots);
   for (int s = blockIdx.x * MOE_WALK_WARPS + (threadIdx.x >> 5); s < used; s += gridDim.x * MOE_WALK_WARPS) {
     const int t = slot_token[s];
     moe_copy_row(reinterpret_cast<const uint4*>(xq + static_cast<size_t>(t) * d), reinterpret_cast<uint4*>(xq_perm + static_cast<size_t>(s) * d), d / 16, lane);
@@ -277,7 +277,7 @@ extern "C" int b200_moe_gather(const void* xq, const float* sx, int d, const int
   if (d % 16) return -1;
   if (max_slots >= MOE_MANY_SLOTS)
     launch_ex(moe_gather_walk_kernel, dim3(MOE_WALK_CTAS), dim3(32 * MOE_WALK_WARPS), 0, stream, 0, static_cast<const int8_t*>(xq), sx, d, slot_token, meta,
-              static_cast<int8_t*>(xq_perm), sx_perm);
+              max_slots, static_cast<int8_t*>(xq_perm), sx_perm);
   else launch_ex(moe_gather_kernel, dim3(max_slots), dim3(128), 0, stream, 0, static_cast<const int8_t*>(xq), sx, d, slot_token, meta,
                                                    static_cast<int8_t*>(xq_perm), sx_perm);
   cudaError_t e = cudaGetLastError();

@@ -117,10 +117,10 @@ __global__ void __launch_bounds__(128) moe_gather_rows_kernel(const uint8_t* x, 
 }
 
 // many slots: a warp per slot at a time
-__global__ void __launch_bounds__(32 * MOE_WALK_WARPS) moe_gather_rows_walk_kernel(const uint8_t* x, long long row_bytes, const int* slot_token, const int* meta, uint8_t* out) {
+__global__ void __launch_bounds__(32 * MOE_WALK_WARPS) moe_gather_rows_walk_kernel(const uint8_t* x, long long row_bytes, const int* slot_token, const int* meta, int max_slots, uint8_t* out) {
   pdl_launch_dependents();
   pdl_wait();
-  const int lane = threadIdx.x & 31, used = meta[0];
+  const int lane = threadIdx.x & 31, used = min(meta[0], max_slots);
   for (int s = blockIdx.x * MOE_WALK_WARPS + (threadIdx.x >> 5); s < used; s += gridDim.x * MOE_WALK_WARPS)
     moe_copy_row(reinterpret_cast<const uint4*>(x + slot_token[s] * row_bytes), reinterpret_cast<uint4*>(out + s * row_bytes), static_cast<int>(row_bytes / 16), lane);
 }
@@ -151,7 +151,7 @@ extern "C" int b200_moe_gather_rows(const void* x, long long row_bytes, const in
   if (!x || !slot_token || !meta || !out || row_bytes <= 0 || row_bytes % 16 || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return -1;
   if (max_slots >= MOE_MANY_SLOTS)
     launch_ex(moe_gather_rows_walk_kernel, dim3(MOE_WALK_CTAS), dim3(32 * MOE_WALK_WARPS), 0, stream, 0, static_cast<const uint8_t*>(x), row_bytes, slot_token, meta,
-              static_cast<uint8_t*>(out));
+              max_slots, static_cast<uint8_t*>(out));
   else launch_ex(moe_gather_rows_kernel, dim3(max_slots), dim3(128), 0, stream, 0, static_cast<const uint8_t*>(x), row_bytes, slot_token, meta, static_cast<uint8_t*>(out));
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);

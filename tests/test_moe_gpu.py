@@ -131,3 +131,23 @@ def test_work_list_of_many_pairs(M, k, E, e0, n_local, d):
     want = (y[w.inv.clamp(min=0).long()].double() * (wts.double() * local)[:, :, None]).sum(1)
     bound = 2 ** -7.99 * want.abs() + k * 2 ** -23 * (y[w.inv.clamp(min=0).long()].double().abs() * wts.double()[:, :, None]).sum(1)
     assert ((out.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("max_slots", [100, 4095, 4096, 5000])
+def test_gathering_stops_at_the_bound_of_the_buffer(max_slots):
+    """Fewer rows of room than the work list has slots, below and above the number from which on warps walk the rows."""
+    from mojo_linuxperiments_b200.ops import _lib
+    from mojo_linuxperiments_b200.ops import moe as MO
+    g = torch.Generator().manual_seed(max_slots)
+    M, d = 6000, 64
+    w = MO.moe_align(torch.randint(0, 4, (M, 1), generator=g, dtype=torch.int32).cuda(), 0, 4)
+    xq, sx = torch.randint(-100, 100, (M, d), generator=g, dtype=torch.int8).cuda(), torch.rand(M, generator=g).cuda()
+    at = w.slot_token[:max_slots].long()
+    xp, sp, rows = torch.full((M, d), 111, dtype=torch.int8, device="cuda"), torch.full((M,), 7.0, device="cuda"), torch.full((M, d), 111, dtype=torch.int8, device="cuda")
+    L = _lib.lib()
+    _lib.check(L.b200_moe_gather(xq.data_ptr(), sx.data_ptr(), d, w.slot_token.data_ptr(), w.meta.data_ptr(), max_slots, xp.data_ptr(), sp.data_ptr(), _lib.stream()), "moe_gather")
+    _lib.check(L.b200_moe_gather_rows(xq.data_ptr(), d, w.slot_token.data_ptr(), w.meta.data_ptr(), max_slots, rows.data_ptr(), _lib.stream()), "moe_gather_rows")
+    torch.cuda.synchronize()
+    for got in (xp, rows):
+        assert torch.equal(got[:max_slots], xq[at]) and (got[max_slots:] == 111).all()
+    assert torch.equal(sp[:max_slots], sx[at]) and (sp[max_slots:] == 7.0).all()
