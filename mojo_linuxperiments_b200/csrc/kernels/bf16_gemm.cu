@@ -15,6 +15,7 @@
 #include "api.h"
 #include "launch.cuh"
 #include "gemm_common.cuh"
+#include "gemm_pair.cuh"
 #include "dense_tile.cuh"
 
 namespace b200 {
@@ -208,18 +209,10 @@ static int bf16_gemm_any(const void* x, long long ldx, const void* w, long long 
   if (int rc = dense_epilogue_check(epi, N)) return rc;
   if (g && (g->groups <= 0 || !g->tiles || !g->num_tiles || g->max_tiles <= 0 || epi->mode != B200_EPI_STORE)) return -3;
   if (!g && (force_bn < 0 || (force_bn == 0 && M > 128))) {
-    // As for int8 (w8a8_gemm.cu): rounds of the pairs times the cost of a tile; -force_bn names the channels.  From 130 tokens on a
+    // -force_bn names the channels.  From 130 tokens on a
     // pair beats the best tile of a CTA alone: 130 x 16,384 x 2,048 22 -> 19 us, 200 x 2,048 x 8,192 43 -> 34, 1,000 x 576 x 2,048
     // 17.6 -> 16.3, 4,200 x 16,384 x 2,048 226 -> 198 (1,425 TFLOP/s), 4,200 x 2,048 x 8,192 146 -> 100, 4,000 x 64 x 2,048 15 -> 13.
-    int bn = -force_bn;
-    if (bn != 256 && bn != 224 && bn != 192 && bn != 160 && bn != 128) {
-      long long best = -1;
-      for (int cand : {256, 224, 192, 160, 128}) {
-        const long long tiles = static_cast<long long>((M + 255) / 256) * ((N + cand - 1) / cand), pairs = num_sms / 2;
-        const long long cost = (tiles + pairs - 1) / pairs * (cand + 32);
-        if (best < 0 || cost < best) { best = cost; bn = cand; }
-      }
-    }
+    const int bn = pair_width(-force_bn) ? -force_bn : pair_pick_width(M, N, num_sms);
     return bf16_gemm_pair(x, ldx, w, ldw, M, N, K, epi, bn, status, num_sms, stream);
   }
   BfGemmParams p;

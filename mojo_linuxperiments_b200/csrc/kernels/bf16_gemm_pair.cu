@@ -69,8 +69,7 @@ int bf16_gemm_pair(const void* x, long long ldx, const void* w, long long ldw, i
   CUtensorMap tx, tw;
   if (make_tmap_2d_u8(&tx, x, static_cast<uint64_t>(K) * 2, M, static_cast<uint64_t>(ldx) * 2, 128)) return -11;
   if (make_tmap_2d_u8(&tw, w, static_cast<uint64_t>(K) * 2, static_cast<uint64_t>(N), static_cast<uint64_t>(ldw) * 2, bn / 2)) return -12;
-  const long long all = static_cast<long long>(p.m_tiles) * p.n_tiles;
-  const int pairs = static_cast<int>(all < num_sms / 2 ? all : num_sms / 2);
+  const int pairs = pair_count(static_cast<long long>(p.m_tiles) * p.n_tiles, num_sms);
   switch (bn) {
     case 256: return launch_bf16_pair<256, 6>(tx, tw, p, pairs, stream);
     case 224: return launch_bf16_pair<224, 6>(tx, tw, p, pairs, stream);

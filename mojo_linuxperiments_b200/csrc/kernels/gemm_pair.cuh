@@ -20,6 +20,25 @@ constexpr int PAIR_M = 256;               // token rows of a tile
 constexpr int PAIR_GROUP_M = 8;           // token tiles per rasterisation group
 constexpr int PAIR_PIECE = 32 * 144;      // staging bytes of an epilogue warp: 32 rows of up to 144 bytes
 
+// channels per tile that the kernels exist for
+inline bool pair_width(int bn) { return bn == 256 || bn == 224 || bn == 192 || bn == 160 || bn == 128; }
+// pairs that work on `tiles` tiles
+inline int pair_count(long long tiles, int num_sms) {
+  const int pairs = num_sms < 4 ? 1 : num_sms / 2;
+  return static_cast<int>(tiles < pairs ? tiles : pairs);
+}
+// the width with the fewest rounds of the pairs times the cost of a tile (main loop ~ its channels, plus a fixed part)
+inline int pair_pick_width(int M, int N, int num_sms) {
+  long long best = -1;
+  int bn = 0;
+  for (int cand : {256, 224, 192, 160, 128}) {
+    const long long tiles = static_cast<long long>((M + PAIR_M - 1) / PAIR_M) * ((N + cand - 1) / cand), pairs = pair_count(tiles, num_sms);
+    const long long cost = (tiles + pairs - 1) / pairs * (cand + 32);
+    if (best < 0 || cost < best) { best = cost; bn = cand; }
+  }
+  return bn;
+}
+
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols) : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");

@@ -28,6 +28,7 @@
 #include "launch.cuh"
 #include "w8_tile.cuh"
 #include "gemm_common.cuh"
+#include "gemm_pair.cuh"
 
 namespace b200 {
 
@@ -500,20 +501,11 @@ extern "C" int b200_w8a8_gemm(const void* xq, const float* sx, const void* wq, c
   const bool pair_ok = !out_fp32 && !residual && N % 8 == 0 && ldy % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0 &&
                        (reinterpret_cast<uintptr_t>(sw) & 15) == 0;
   // a number that names no tile width (0 and 1: the schedules of the one-CTA kernel) leaves the choice to the rule
-  const bool width = force_mode == 256 || force_mode == 224 || force_mode == 192 || force_mode == 160 || force_mode == 128;
+  const bool width = pair_width(force_mode);
   if (pair_ok && (width || (force_mode != 0 && force_mode != 1 && M > 128))) {
-    // Rounds of the pairs times the cost of a tile (main loop ~ its channels, plus a fixed part).  Above 128 tokens a pair
-    // is never slower than a CTA alone: 200 x 28,672 x 4,096 30 us (40), 1,024 x 6,144 x 4,096 23 (37), 32,768 x 28,672 x
+    // Above 128 tokens a pair is never slower than a CTA alone: 200 x 28,672 x 4,096 30 us (40), 1,024 x 6,144 x 4,096 23 (37), 32,768 x 28,672 x
     // 4,096 2,351 (2,989), 32,768 x 4,096 x 14,336 1,150 (1,341).
-    int bn = force_mode;
-    if (!width) {
-      long long best = -1;
-      for (int cand : {256, 224, 192, 160, 128}) {
-        const long long tiles = static_cast<long long>((M + 255) / 256) * ((N + cand - 1) / cand), pairs = num_sms / 2;
-        const long long cost = (tiles + pairs - 1) / pairs * (cand + 32);
-        if (best < 0 || cost < best) { best = cost; bn = cand; }
-      }
-    }
+    const int bn = width ? force_mode : pair_pick_width(M, N, num_sms);
     return w8a8_gemm_pair(xq, sx, wq, sw, y, M, N, K, ldy, bn, status, num_sms, stream);
   }
   const bool swap = M <= SWAP_MAX_M;

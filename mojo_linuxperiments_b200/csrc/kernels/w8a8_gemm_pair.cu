@@ -109,8 +109,7 @@ int w8a8_gemm_pair(const void* xq, const float* sx, const void* wq, const float*
   CUtensorMap tw, tx;
   if (make_tmap_2d_u8(&tw, wq, static_cast<uint64_t>(K), static_cast<uint64_t>(N), static_cast<uint64_t>(K), bn / 2)) return -11;
   if (make_tmap_2d_u8(&tx, xq, static_cast<uint64_t>(K), static_cast<uint64_t>(M), static_cast<uint64_t>(K), 128)) return -12;
-  const long long all = static_cast<long long>(p.m_tiles) * p.n_tiles;
-  const int pairs = static_cast<int>(all < num_sms / 2 ? all : num_sms / 2);
+  const int pairs = pair_count(static_cast<long long>(p.m_tiles) * p.n_tiles, num_sms);
   switch (bn) {
     case 256: return launch_w8_pair<256, 6>(tx, tw, p, pairs, stream);
     case 224: return launch_w8_pair<224, 6>(tx, tw, p, pairs, stream);

@@ -1,4 +1,8 @@
 """What the kernel library's host side decides, and rules its sources keep: no GPU needed."""
+import os
+import subprocess
+import sys
+
 import pytest
 
 from mojo_linuxperiments_b200 import _build
@@ -49,3 +53,21 @@ def test_the_kernels_that_open_a_step_wait_for_all_of_the_step_before():
         text = (_build.CSRC / "kernels" / name).read_text()
         lines = [ln for ln in text.splitlines() if kernel in ln and "launch" in ln]
         assert lines and all(any(s in ln for s in starts) for ln in lines), name
+
+
+@pytest.mark.parametrize("sms", [1, 3])
+@pytest.mark.parametrize("name", ["w8a8_gemm", "bf16_gemm"])
+def test_a_linear_told_of_a_single_multiprocessor_returns(lib, name, sms):
+    """The linears of two CTAs per tile share tiles out to half the multiprocessors: one is a pair's worth, not none (which was a
+    division by zero).  Without a driver the call ends at its first tensor map; in a process of its own, since it ended there."""
+    code = f"""
+import ctypes
+from mojo_linuxperiments_b200.ops import _lib
+a, L = 1 << 20, _lib.lib()
+e = _lib.DenseEpilogue(mode=0, y=a, ldy=512)
+rc = (L.b200_w8a8_gemm(a, a, a, a, a, None, 300, 512, 512, 512, 0, None, 0, None, 0, a, {sms}, -1, None) if "{name}" == "w8a8_gemm" else
+      L.b200_bf16_gemm(a, 512, a, 512, 300, 512, 512, ctypes.byref(e), a, {sms}, 0, None))
+print("rc", rc)
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=_build.PKG.parent, env={**os.environ, "CUDA_VISIBLE_DEVICES": ""})
+    assert r.returncode == 0 and "rc -" in r.stdout, (r.returncode, r.stdout, r.stderr[-500:])
