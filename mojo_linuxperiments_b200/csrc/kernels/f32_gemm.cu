@@ -4,7 +4,7 @@
 // Two kernels, chosen by the number of rows (f32_gemm_any):
 //   * up to 8 rows a linear is a stream of weights.  A CTA owns four output columns; its warps share out K, every lane takes
 //     16 bytes of each column's row at a time, and the first block of weights is on its way before the kernel waits for
-//     its input.  Bound by HBM: 2 rows x 16,384 x 2,048 in 25 us = 5.4 TB/s (260 us with the 64 x 64 tiles of one
+//     its input (row lists: once the group is known to have rows).  Bound by HBM: 2 rows x 16,384 x 2,048 in 25 us = 5.4 TB/s (260 us with the 64 x 64 tiles of one
 //     CTA per tile that served all sizes before), 2 rows x 2,048 x 8,192 in 18 us (594 us).
 //   * above that, 64 x 128 tiles through a three-stage cp.async ring, 4 x 8 outputs per thread.  Two fused multiply-adds
 //     are one instruction (fma.rn.f32x2: the even and the odd k of an output have a sum each), which leaves issue slots for
@@ -83,11 +83,18 @@ __global__ void __launch_bounds__(32 * FV_WARPS) f32_gemv_kernel(const __grid_co
       for (int c = 0; c < FV_COLS; ++c)
         wv[u][c] = f32_row4<VEC>(w + static_cast<long long>(n0 + c) * p.ldw, k + u * STEP, n0 + c < p.N ? p.K : 0);
   };
-  load(k0);                            // weights do not depend on the kernel before
-  pdl_wait();
   const int m0 = blockIdx.y * MR;
   F32Group g;
-  if (!f32_group(p, m0, g)) return;
+  const bool list = p.gr.groups > 0 && p.gr.counts;
+  if (list) {                          // the weights of a group without rows are not read: the list first
+    pdl_wait();
+    if (!f32_group(p, m0, g)) return;
+  }
+  load(k0);                            // weights do not depend on the kernel before
+  if (!list) {
+    pdl_wait();
+    if (!f32_group(p, m0, g)) return;
+  }
   const int rows = min(MR, g.M - m0);
   float2 acc[FV_COLS][MR];
 #pragma unroll

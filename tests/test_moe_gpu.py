@@ -151,3 +151,30 @@ def test_gathering_stops_at_the_bound_of_the_buffer(max_slots):
     for got in (xp, rows):
         assert torch.equal(got[:max_slots], xq[at]) and (got[max_slots:] == 111).all()
     assert torch.equal(sp[:max_slots], sx[at]) and (sp[max_slots:] == 7.0).all()
+
+
+def test_fp32_experts_without_rows_are_not_read():
+    """Four tokens, 24 experts of 32 MB: six chosen experts are a quarter of the bytes of all 24.  Reading what no token chose makes
+    both take the same time; the bound lies between."""
+    from mojo_linuxperiments_b200.ops import dense as D
+    from mojo_linuxperiments_b200.ops import moe as MO
+    E, n, k = 24, 4096, 2048
+    W = D.GroupedW(torch.randn((E * n, k), device="cuda"), E, n, k)
+    few = torch.arange(6).repeat(4, 1).to(torch.int32).cuda()
+    x = torch.randn((24, k), device="cuda")
+    ms = {}
+    for name, ids in (("few", few), ("all", torch.arange(24, dtype=torch.int32).view(4, 6).cuda())):
+        work = MO.moe_align(ids, 0, E)
+        for _ in range(3):
+            y = D.linear_experts(x, W, work)
+        t = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        t[0].record()
+        for _ in range(20):
+            D.linear_experts(x, W, work)
+        t[1].record()
+        torch.cuda.synchronize()
+        ms[name] = t[0].elapsed_time(t[1])
+        at = torch.repeat_interleave(torch.arange(E, device="cuda"), work.counts.long())
+        want = torch.stack([W.data.view(E, n, k)[e].double() @ x[i].double() for i, e in enumerate(at.tolist())])
+        assert (y[:, :n].double() - want).norm() <= 2e-6 * want.norm()
+    assert ms["few"] < 0.6 * ms["all"], ms
