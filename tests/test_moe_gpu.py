@@ -154,16 +154,17 @@ def test_gathering_stops_at_the_bound_of_the_buffer(max_slots):
 
 
 def test_fp32_experts_without_rows_are_not_read():
-    """Four tokens, 24 experts of 32 MB: six chosen experts are a quarter of the bytes of all 24.  Reading what no token chose makes
-    both take the same time; the bound lies between."""
+    """Four tokens, 24 experts of 32 MB, a row for each that is chosen: six are a quarter of the bytes of all 24 (the other choices lie
+    outside the local experts).  Reading what no token chose makes both take the same time; the bound lies between."""
     from mojo_linuxperiments_b200.ops import dense as D
     from mojo_linuxperiments_b200.ops import moe as MO
     E, n, k = 24, 4096, 2048
     W = D.GroupedW(torch.randn((E * n, k), device="cuda"), E, n, k)
-    few = torch.arange(6).repeat(4, 1).to(torch.int32).cuda()
+    every = torch.arange(24, dtype=torch.int32).view(4, 6).cuda()
+    few = torch.where(every % 4 == 0, every, every + E)
     x = torch.randn((24, k), device="cuda")
     ms = {}
-    for name, ids in (("few", few), ("all", torch.arange(24, dtype=torch.int32).view(4, 6).cuda())):
+    for name, ids in (("few", few), ("all", every)):
         work = MO.moe_align(ids, 0, E)
         for _ in range(3):
             y = D.linear_experts(x, W, work)
