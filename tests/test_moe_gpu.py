@@ -177,5 +177,5 @@ def test_fp32_experts_without_rows_are_not_read():
         ms[name] = t[0].elapsed_time(t[1])
         at = torch.repeat_interleave(torch.arange(E, device="cuda"), work.counts.long())
         want = torch.stack([W.data.view(E, n, k)[e].double() @ x[i].double() for i, e in enumerate(at.tolist())])
-        assert (y[:, :n].double() - want).norm() <= 2e-6 * want.norm()
+        assert (y[:at.numel(), :n].double() - want).norm() <= 2e-6 * want.norm()
     assert ms["few"] < 0.6 * ms["all"], ms
