@@ -21,6 +21,7 @@
 #include "launch.cuh"
 #include "hadamard.cuh"
 #include <cuda.h>
+#include <algorithm>
 #include <cstdlib>
 
 namespace b200 {
@@ -1161,8 +1162,51 @@ typedef CUresult (*EncodeTiledFn3)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
 // NB: 128-token blocks a CTA can hold.  4 with the merge zone (clusters of splits), 9 without it for a CTA that takes a
 // whole sequence of up to 1,152 tokens - both sized for two CTAs per SM.
 template <int G, bool FUSED, int NB>
-static int launch_adc(const CUtensorMap& tm, const DecodeTcParams& p, dim3 grid, cudaStream_t stream) {
+static int adc_resident_clusters(int size) {
+  static int known[ADC_ZONE_MAX_SPLITS + 1] = {};
+  if (size < 1 || size > ADC_ZONE_MAX_SPLITS) return 0;
+  if (!known[size]) {
+    constexpr int SMEM = AdcShared<G, NB>::BYTES;
+    cudaFuncSetAttribute(attn_decode_tc_kernel<G, FUSED, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    cudaFuncSetAttribute(attn_decode_tc_kernel<G, FUSED, NB>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(size, 64, 1);
+    cfg.blockDim = dim3(ADC_THREADS);
+    cfg.dynamicSmemBytes = SMEM;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = size; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, attn_decode_tc_kernel<G, FUSED, NB>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+    known[size] = n > 0 ? n : -1;
+  }
+  return known[size];
+}
+
+// Clusters of `size` CTAs that run at the same time.  Two CTAs share an SM, but the calculator counts one for a kernel with tensor
+// memory, and clusters are placed per GPC: an even cluster takes size / 2 whole SMs, as many as a cluster of half the size at
+// one CTA each; an odd one leaves half an SM that only another odd one can use.  Some room is left, because placing is not perfect
+// (on 148 SMs: 148, 83, 70, 48, 43, 28 and 32 of two to eight CTAs; measured to run in one round: 148 of two, 80 of three, 70 of four, 48
+// of five, 40 of six, 32 of eight, with more than two splits 30; in two rounds: 88 of three, 72 of four, 48 of six, 34 of eight).
+template <int G, bool FUSED, int NB>
+static int adc_room(int size, int splits) {
+  const int n = adc_resident_clusters<G, FUSED, NB>(size);
+  if (size % 2) return 2 * n - n / 6;
+  const int half = adc_resident_clusters<G, FUSED, NB>(size / 2), room = size == 2 ? half : half - half / 18;
+  return splits > 2 ? std::min(room, 2 * n) : room;
+}
+
+template <int G, bool FUSED, int NB>
+static int launch_adc(const CUtensorMap& tm, DecodeTcParams p, dim3 grid, cudaStream_t stream) {
   constexpr int SMEM = AdcShared<G, NB>::BYTES;
+  // Clusters that do not all run at once are worse than CTAs that meet through global memory, so they are counted as such, not
+  // as CTAs: all CTAs of a sequence first, then the splits of a KV head (a caller without scratch gets those in any case).
+  // Alone, counted as CTAs -> as clusters: 34 sequences of 8 KV heads 18.0 -> 11.3 us (250 tokens), 48.4 -> 28.0 (1,030 tokens), 24 of
+  // 4 heads in three splits 22.4 -> 17.6, 12 of 8 heads in three splits 20.9 -> 13.8.
+  const int sequences = static_cast<int>(grid.y), splits = static_cast<int>(grid.z), row = static_cast<int>(grid.x) * splits;
+  if (p.head_cluster && sequences > adc_room<G, FUSED, NB>(row, splits)) p.head_cluster = 0;
+  if (p.cluster_merge && !p.head_cluster && p.part_acc && p.counters && sequences * static_cast<int>(grid.x) > adc_room<G, FUSED, NB>(splits, splits)) p.cluster_merge = 0;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(attn_decode_tc_kernel<G, FUSED, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
@@ -1272,10 +1316,9 @@ static int attn_decode_tc_common(const void* q, const void* cache, int num_pages
   if (per_max > (long_form ? ADC_NB_LONG : ADC_NB)) return -1;
   p.cluster_merge = (!persistent && !long_form && cluster_env && G * splits <= ADC_ZONE_ROWS && splits >= 2 && splits <= ADC_ZONE_MAX_SPLITS &&
                      static_cast<long long>(B) * hkv * splits <= 2ll * sm_count) ? 1 : 0;
-  // All CTAs of a sequence as one cluster, in a grid that is resident in one go as above: a decode step of four layers 271.8 ->
+  // All CTAs of a sequence as one cluster, where these run at the same time (launch_adc): a decode step of four layers 271.8 ->
   // 268.3 us at one sequence and 327.5 -> 324.3 at 32; at 100 sequences (800 CTAs in three waves) 496 -> 514.
-  p.head_cluster = fuse && fuse->xq && hkv > 1 && hkv * splits <= 8 && (splits == 1 || p.cluster_merge) &&
-                   static_cast<long long>(B) * hkv * splits <= 2ll * sm_count;
+  p.head_cluster = fuse && fuse->xq && hkv > 1 && hkv * splits <= 8 && (splits == 1 || p.cluster_merge);
   if (splits > 1 && !p.cluster_merge && (!scratch || !counters)) return -1;
   if (persistent) {
     const int items = B * hkv * splits;

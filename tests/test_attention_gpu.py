@@ -287,3 +287,44 @@ def test_attn_decode_fused_with_one_cluster_per_sequence(hq, hkv, qk_norm, split
     """Up to eight CTAs of a sequence (KV heads x splits) as one cluster that merges and agrees on the row's scale, and the largest
     merge zones: the bounds of the test above."""
     test_attn_decode_fused_matches_the_three_kernels_it_replaces(hq, hkv, qk_norm, splits, longest)
+
+
+@pytest.mark.parametrize("fewer,more,hq,hkv,tokens,capacity", [(32, 34, 32, 8, 250, 256), (32, 34, 32, 8, 1030, 1152), (18, 24, 32, 4, 500, 640), (10, 12, 32, 8, 500, 640)])
+def test_attn_decode_fused_beyond_the_clusters_that_run_at_once(fewer, more, hq, hkv, tokens, capacity):
+    """A launch whose clusters no longer run all at once is two launches long (1.6 to 1.8 times); CTAs that meet through global memory
+    then take 1.03 to 1.25 times as long as the fewer sequences do.  The bound lies between."""
+    from mojo_linuxperiments_b200.ops import attention as A
+    from mojo_linuxperiments_b200.ops.workspace import default_workspace
+    us = {}
+    for B in (fewer, more):
+        pages = capacity // 16
+        cache = A.PagedKVCache(B * pages + 1, hkv, 16, "cuda")
+        cache.data.normal_()
+        table = torch.arange(B * pages, dtype=torch.int32, device="cuda").view(B, pages)
+        cos, sin = A.rope_tables(capacity + 1, 1e4, "cuda")
+        qkv = torch.randn((B, (hq + 2 * hkv) * 128), device="cuda").to(torch.bfloat16)
+        lens = torch.full((B,), tokens, dtype=torch.int32, device="cuda")
+        pos = lens - 1
+        splits = A.pick_decode_splits_tc(B, hkv, capacity, fused=True)
+        scratch = A.DecodeAttnScratch(B, hq, hkv, splits, "cuda")
+
+        def call():
+            return A.attn_decode_fused(qkv, pos, cos, sin, hq, hkv, cache, table, lens, scratch=scratch, splits=splits)
+
+        call()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(20):
+                call()
+        t = []
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            graph.replay()
+            b.record()
+            torch.cuda.synchronize()
+            t.append(a.elapsed_time(b))
+        us[B] = min(t) * 50
+    default_workspace(torch.device("cuda")).check_status()
+    assert us[more] < 1.45 * us[fewer], us
