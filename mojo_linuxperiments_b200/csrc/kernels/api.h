@@ -27,6 +27,7 @@ int b200_w8a8_gemm_decode(const void* xq, const float* sx, const void* wq, const
                           int num_sms, int force_splits, cudaStream_t stream);
 
 int b200_w8a8_gemm_decode_resident_clusters(int m, int splits);
+int b200_w8a8_gemm_decode_takes(int M, int N, int K, int num_sms);
 
 // Activation prologue carried inside a decode GEMM launch (quantiser CTAs of the same grid, see quant_row.cuh).
 // mode: 1 rotate + quantise x [M][K]; 2 RMSNorm(gamma, eps) first; 3 residual += x (bf16, in place) then RMSNorm of the

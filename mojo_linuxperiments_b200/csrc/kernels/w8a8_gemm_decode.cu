@@ -140,9 +140,8 @@ constexpr int decode_smem_bytes(int bn, int stages, bool xch = true) {
 
 // XCH = false: no split along K (S == 1) and no exchange buffer, whose 74 KB are what keeps two CTAs of the 128-token form
 // from sharing an SM.
-// 65 to 128 tokens: the persistent kernel's tiles of 128 tokens x 64 to 256 channels left most SMs idle or ran in two rounds.
-// 100 tokens x 28,672 x 4,096 36 -> 25 us, x 4,096 x 14,336 36 -> 20, x 32,000 x 4,096 29 -> 26, x 6,144 x 4,096 14 -> 16 (the
-// exchange of 64 KB per CTA): a decode step of four layers spends 319 us in its linears, 388 before.
+// 65 to 128 tokens: the persistent kernel's tiles of 128 tokens x 64 to 256 channels leave most SMs idle or run in two rounds;
+// which of the two kernels takes a call is decided in b200_w8a8_gemm_decode_takes.
 template <int BN, int STAGES, bool XCH = true>
 __global__ void __launch_bounds__(GEMM_THREADS, ((BN >= 64 && XCH) ? 1 : 2))
 w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
@@ -1083,6 +1082,27 @@ extern "C" int b200_w8a8_gemm_decode_p(const b200_quant_prolog* prolog, const vo
   const QuantProlog q = to_prolog(*prolog);
   return decode_gemm_impl(q.q, q.scale, wq, sw, y, residual, M, N, K, ldy, out_fp32, status, num_sms, 0, nullptr, stream, 0, nullptr,
                           nullptr, 0, &q);
+}
+
+// 1 if a plain call of 65 to 128 tokens and more than one channel tile is for this kernel, 0 if it is for the persistent one.  Above
+// that the persistent kernel's time is its main loop, 0.28 us per block of K.  This kernel's is that over S, and the exchange, which
+// grows with tokens and with the channels that a CTA finishes (128 / S).  In tenths of a microsecond it wins where
+//   2.8 (kb - kb / S) > 6 + M (0.2 + 1.4 / S).
+// Without a split (more than 74 tiles) nothing is gained until the persistent kernel needs a second round: one to two tiles per SM
+// (20,480 to 37,888 channels); above that both take several rounds and the persistent kernel's double-buffered ones are shorter.
+// Measured, this kernel | the persistent one, us at 65 and at 128 tokens (bf16 results):
+//   512 x 1,024 7.0, 9.2 | 5.8, 5.8       1,024 x 4,096 7.8, 9.6 | 13.0, 13.1     4,096 x 2,048 9.6, 12.0 | 8.8, 8.9
+//   4,096 x 4,096 10.9, 13.3 | 13.3, 13.3  4,096 x 14,336 18.0, 20.3 | 35.2, 35.5  6,144 x 4,096 14.2, 17.8 | 13.5, 13.7
+//   8,192 x 8,192 20.3, 23.8 | 22.5, 22.5  12,288 x 4,096 18.3, 19.8 | 14.9, 15.1  28,672 x 4,096 24.0, 24.8 | 25.8, 25.4
+//   57,344 x 4,096 48.0, 49.3 | 45.7, 45.4  128,256 x 4,096 98, 117 | 86, 94
+// Over 24 widths x 8 lengths x 3 numbers of tokens the choice is at most 4 % slower than the better one.  Where the persistent kernel
+// would write element by element (fp32 results, rows on odd addresses) it is this kernel's call in any case: 2,048 x 2,048 8.8, 11.3 |
+// 14.5, 17.1, 28,672 x 4,096 24.7, 26.8 | 52.7, 66.3.
+extern "C" int b200_w8a8_gemm_decode_takes(int M, int N, int K, int num_sms) {
+  const int tiles = (N + TILE_N - 1) / TILE_N, kb = (K + BLOCK_K - 1) / BLOCK_K;
+  const long long s = decode_pick_splits(tiles, kb, num_sms, 128, 1);
+  if (s == 1) return tiles > num_sms && tiles <= 2 * num_sms;
+  return 28ll * kb * (s - 1) > 60 * s + M * (2 * s + 14);
 }
 
 extern "C" int b200_w8a8_gemm_decode(const void* xq, const float* sx, const void* wq, const float* sw, void* y,

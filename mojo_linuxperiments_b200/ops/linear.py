@@ -40,17 +40,24 @@ DECODE_MAX_M = 64
 CLUSTER_MAX_M = 128     # the 128-token form of the cluster kernel: plain calls of more than one channel tile
 
 
+def _elementwise(out: torch.Tensor, residual: torch.Tensor | None) -> bool:
+    """The persistent kernel cannot write this result sixteen bytes at a time."""
+    return (out.dtype == torch.float32 or out.stride(0) % 8 != 0 or out.data_ptr() % 16 != 0
+            or (residual is not None and residual.data_ptr() % 16 != 0))
+
+
 def w8a8_gemm(xq: torch.Tensor, sx: torch.Tensor, wq: torch.Tensor, sw: torch.Tensor, *,
               residual: torch.Tensor | None = None, out: torch.Tensor | None = None,
               out_dtype: torch.dtype = torch.bfloat16, workspace: Workspace | None = None,
               force_mode: int = -1, force_splits: int = 0, narrow: bool = False) -> torch.Tensor:
     """y[m,n] = (sum_k xq[m,k] wq[n,k]) * sx[m] * sw[n] (+ residual); int8 operands, int32 accumulate in TMEM.
 
-    Up to 128 tokens the cluster split-K weight-streaming kernel runs (``force_mode`` -1) unless the problem has
-    enough tiles for the persistent kernel; ``force_mode`` 0 / 1 select the persistent kernel's whole-tile / stream-K
-    schedules, ``force_mode`` 2 the cluster kernel with ``force_splits`` CTAs per cluster, 128, 160, 192, 224 or 256 the two-CTA
-    kernel with that many channels per tile (its default above 128 tokens: what fills the rounds of the 74 pairs best).
-    Any other number is -1, and a width has no effect where the two-CTA kernel cannot take the call."""
+    Up to 64 tokens the cluster split-K weight-streaming kernel runs (``force_mode`` -1) unless the problem has
+    enough tiles for the persistent kernel, from 65 to 128 whichever of the two is faster; ``force_mode`` 0 / 1 select the
+    persistent kernel's whole-tile / stream-K schedules, ``force_mode`` 2 the cluster kernel with ``force_splits`` CTAs per
+    cluster, 128, 160, 192, 224 or 256 the two-CTA kernel with that many channels per tile (its default above 128 tokens: what
+    fills the rounds of the 74 pairs best).  Any other number keeps the cluster kernel out and leaves the rest to the rules; a width has no
+    effect where the two-CTA kernel cannot take the call."""
     assert xq.is_cuda and xq.dtype == torch.int8 and wq.dtype == torch.int8
     assert xq.is_contiguous() and wq.is_contiguous()
     M, K = xq.shape
@@ -63,20 +70,23 @@ def w8a8_gemm(xq: torch.Tensor, sx: torch.Tensor, wq: torch.Tensor, sw: torch.Te
         assert residual.dtype == torch.bfloat16 and residual.stride(0) == out.stride(0) and residual.stride(1) == 1
     w = workspace or default_workspace(xq.device)
     n_tiles = (N + 127) // 128
-    use_cluster = (M <= DECODE_MAX_M or (M <= CLUSTER_MAX_M and n_tiles > 1)) and (force_mode == 2 or (force_mode == -1 and n_tiles < _DECODE_TILE_WAVES * _lib.num_sms(xq.device.index)))
-    # a narrow output (a router: one channel tile) for up to 256 tokens is still a weight stream: the persistent
-    # kernel would walk its whole K loop on one or two CTAs, the cluster kernel splits K and takes 64 tokens per grid layer
-    # (one channel tile only: wider outputs stay on the persistent kernel, whose results the token-sharded paths are
-    # compared with bit for bit - the two kernels multiply the scales in a different order)
-    # The caller asks for it (``narrow=True``) because the two kernels multiply the scales in a different order and
-    # other callers compare this function's persistent-kernel results bit for bit with the token-sharded paths.
+    sms = _lib.num_sms(xq.device.index)
+    use_cluster = force_mode == 2 or (force_mode == -1 and n_tiles < _DECODE_TILE_WAVES * sms)
+    if M > DECODE_MAX_M:
+        # 65 to 128 tokens: the same bits from both kernels where the persistent one writes whole vectors; the rule and its
+        # figures stand at the C entry
+        use_cluster = use_cluster and M <= CLUSTER_MAX_M and n_tiles > 1 and (
+            force_mode == 2 or _elementwise(out, residual) or _lib.lib().b200_w8a8_gemm_decode_takes(M, N, K, sms) == 1)
+    # A narrow output (a router: one channel tile) for up to 256 tokens is still a weight stream: the persistent kernel would walk
+    # its whole K loop on one or two CTAs, the cluster kernel splits K and takes 64 tokens per grid layer.  The caller asks
+    # for it (``narrow=True``), because in that form the two multiply the scales in a different order, and others compare the
+    # persistent kernel's results bit for bit with the token-sharded paths.
     if not use_cluster and force_mode in (-1, 2) and M <= 4 * DECODE_MAX_M and (force_mode == 2 or (narrow and n_tiles == 1)):
         use_cluster = True
     if use_cluster:
         rc = _lib.lib().b200_w8a8_gemm_decode(
             xq.data_ptr(), sx.data_ptr(), wq.data_ptr(), sw.data_ptr(), out.data_ptr(), _lib.ptr(residual),
-            M, N, K, out.stride(0), 1 if out.dtype == torch.float32 else 0, w.status.data_ptr(),
-            _lib.num_sms(xq.device.index), force_splits, _lib.stream())
+            M, N, K, out.stride(0), 1 if out.dtype == torch.float32 else 0, w.status.data_ptr(), sms, force_splits, _lib.stream())
         _lib.check(rc, "w8a8_gemm_decode")
         return out
     if force_mode == 2:
@@ -84,8 +94,7 @@ def w8a8_gemm(xq: torch.Tensor, sx: torch.Tensor, wq: torch.Tensor, sw: torch.Te
     rc = _lib.lib().b200_w8a8_gemm(
         xq.data_ptr(), sx.data_ptr(), wq.data_ptr(), sw.data_ptr(), out.data_ptr(), _lib.ptr(residual),
         M, N, K, out.stride(0), 1 if out.dtype == torch.float32 else 0,
-        w.ws.data_ptr(), w.ws_bytes, w.counters.data_ptr(), w.counters.numel(), w.status.data_ptr(),
-        _lib.num_sms(xq.device.index), force_mode, _lib.stream())
+        w.ws.data_ptr(), w.ws_bytes, w.counters.data_ptr(), w.counters.numel(), w.status.data_ptr(), sms, force_mode, _lib.stream())
     _lib.check(rc, "w8a8_gemm")
     return out
 

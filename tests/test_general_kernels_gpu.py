@@ -195,6 +195,15 @@ def test_int8_linear_of_65_to_128_tokens(M, N, K, splits):
         assert torch.equal(L.w8a8_gemm(x, sx, w, sw), y)
 
 
+@pytest.mark.parametrize("M,N,K,cluster", [(65, 6144, 2048, 0), (100, 6144, 4096, 0), (128, 8192, 4096, 0), (100, 12288, 4096, 0), (65, 18944, 4096, 0),
+                                           (65, 57344, 4096, 0), (100, 128256, 4096, 0), (128, 512, 1024, 0), (100, 4096, 4096, 1), (128, 4096, 14336, 1),
+                                           (100, 1024, 4096, 1), (65, 8192, 8192, 1), (100, 28672, 4096, 1), (128, 32000, 4096, 1)])
+def test_int8_linear_of_65_to_128_tokens_goes_where_it_is_faster(M, N, K, cluster):
+    """Shapes that one of the two kernels takes at least 1.1 times as long for as the other (1.03 for one to two tiles per SM)."""
+    from mojo_linuxperiments_b200.ops import _lib
+    assert _lib.lib().b200_w8a8_gemm_decode_takes(M, N, K, 148) == cluster
+
+
 @pytest.mark.parametrize("residual", [False, True])
 @pytest.mark.parametrize("M,N,ld", [(20, 256, 258), (100, 256, 258), (100, 257, 259), (200, 256, 258), (100, 256, 257)])
 def test_int8_linear_writes_rows_that_start_anywhere(M, N, ld, residual):
