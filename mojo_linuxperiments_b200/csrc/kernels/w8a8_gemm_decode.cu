@@ -83,6 +83,7 @@ struct DecodeGemmParams {
   // as its own bytes are there), 0 = plain distributed-shared-memory stores followed by a barrier of the whole cluster
   int async_x;
   int l2_prefetch;     // this many weight tiles beyond the shared-memory ring are requested into L2 before the dependency wait
+  int elementwise;     // the persistent kernel could not write this result in vectors
   int narrow_epi;      // diagnostics: 1 = the unsplit epilogue stores 2 bytes per thread and token (the older form)
 };
 
@@ -116,10 +117,12 @@ __device__ __forceinline__ void emit2(const OutSink& k, int m, int n, float v0, 
   *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(k.y) + o) = __floats2bfloat162_rn(v0, v1);
 }
 
-// The 128-token form takes calls that the persistent kernel would also serve: it multiplies the scales in that kernel's order.
+// The 128-token form takes calls that the persistent kernel would also serve and multiplies the scales in the order which that one
+// would use for the result: token first where it writes element by element, the product of the scales where it writes vectors.
 template <int BN>
-__device__ __forceinline__ float scaled(int32_t acc, float w, float x) {
-  return BN > 64 ? static_cast<float>(acc) * (w * x) : static_cast<float>(acc) * w * x;
+__device__ __forceinline__ float scaled(int32_t acc, float w, float x, bool elementwise) {
+  if constexpr (BN > 64) return elementwise ? static_cast<float>(acc) * x * w : static_cast<float>(acc) * (w * x);
+  else return static_cast<float>(acc) * w * x;
 }
 
 // u / m for the handful of values the inline prologue meets (u < 8 unrolled, m = 1..4)
@@ -551,7 +554,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < CH; ++j)
-          tile_f[(c * CH + j) * TP + row] = scaled<BN>(static_cast<int32_t>(r[j]), swn, sx_s[c * CH + j]);
+          tile_f[(c * CH + j) * TP + row] = scaled<BN>(static_cast<int32_t>(r[j]), swn, sx_s[c * CH + j], p.elementwise);
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");
       const size_t col0 = static_cast<size_t>(n_tile) * TILE_N;
@@ -590,7 +593,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         if (!n_ok || jm <= 0) continue;
 #pragma unroll
         for (int j = 0; j < CH; ++j)
-          if (j < jm) emit1(sink, mc + j, n, scaled<BN>(static_cast<int32_t>(r[j]), swn, sx_s[c * CH + j]));
+          if (j < jm) emit1(sink, mc + j, n, scaled<BN>(static_cast<int32_t>(r[j]), swn, sx_s[c * CH + j], p.elementwise));
       }
     }
   } else {
@@ -678,8 +681,8 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
           if (!on[u]) continue;
           const int n = n_base + rr[u];
           const float sxj = sx_s[jj[u]];
-          const float v0 = scaled<BN>(a[u][0], sw_s[sw_off + rr[u]], sxj);
-          const float v1 = scaled<BN>(a[u][1], sw_s[sw_off + rr[u] + 1], sxj);
+          const float v0 = scaled<BN>(a[u][0], sw_s[sw_off + rr[u]], sxj, p.elementwise);
+          const float v1 = scaled<BN>(a[u][1], sw_s[sw_off + rr[u] + 1], sxj, p.elementwise);
           if (n + 1 < p.N) emit2(sink, m0 + jj[u], n, v0, v1);
           else if (n < p.N) emit1(sink, m0 + jj[u], n, v0);
         }
@@ -977,6 +980,7 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
   p.splits = s;
   p.sx = sx; p.sw = sw; p.y = y; p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.ldy = ldy; p.out_fp32 = out_fp32; p.status = status; p.limit_ns = 2000000000ull;
+  p.elementwise = out_fp32 || ldy % 8 || ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(residual)) & 15);
   if (ar) p.ar = *ar; else { p.ar = ArTail{}; p.ar.enabled = 0; }
   p.grp_offsets = groups > 0 ? grp_offsets : nullptr;
   p.grp_counts = groups > 0 ? grp_counts : nullptr;

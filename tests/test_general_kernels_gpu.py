@@ -204,6 +204,26 @@ def test_int8_linear_of_65_to_128_tokens_goes_where_it_is_faster(M, N, K, cluste
     assert _lib.lib().b200_w8a8_gemm_decode_takes(M, N, K, 148) == cluster
 
 
+@pytest.mark.parametrize("M,N,K,splits", [(65, 129, 1024, 0), (100, 1000, 1040, 1), (128, 640, 2048, 3), (96, 4096, 1152, 0), (100, 20480, 256, 0)])
+def test_int8_linear_of_65_to_128_tokens_has_the_bits_of_the_persistent_kernel(M, N, K, splits):
+    """fp32 results, bf16 results in vectors and element by element: whole sums, scaled in the same order."""
+    from mojo_linuxperiments_b200.ops import linear as L
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    x = torch.randint(-127, 128, (M, K), generator=g, device=DEV, dtype=torch.int8)
+    w = torch.randint(-127, 128, (N, K), generator=g, device=DEV, dtype=torch.int8)
+    sx, sw = torch.rand(M, generator=g, device=DEV) + 0.1, torch.rand(N, generator=g, device=DEV) + 0.1
+    odd = N | 1
+    for dtype, ld in ((torch.float32, N), (torch.bfloat16, (N + 7) // 8 * 8), (torch.bfloat16, odd)):
+        got = []
+        for force in (2, 0):
+            y = torch.zeros((M, ld), dtype=dtype, device=DEV)
+            L.w8a8_gemm(x, sx, w, sw, out=y[:, :N], force_mode=force, force_splits=splits if force == 2 else 0)
+            got.append(y)
+        _ok()
+        n = N // 32 * 32 if dtype == torch.bfloat16 and ld % 8 == 0 and N % 8 else N        # a last part of a vector row is written by elements
+        assert torch.equal(got[0][:, :n], got[1][:, :n]), (dtype, ld)
+
+
 @pytest.mark.parametrize("residual", [False, True])
 @pytest.mark.parametrize("M,N,ld", [(20, 256, 258), (100, 256, 258), (100, 257, 259), (200, 256, 258), (100, 256, 257)])
 def test_int8_linear_writes_rows_that_start_anywhere(M, N, ld, residual):
