@@ -17,6 +17,7 @@
 #include "api.h"
 #include "launch.cuh"
 #include "dense_epilogue.cuh"
+#include <algorithm>
 
 namespace b200 {
 
@@ -276,28 +277,33 @@ static int f32_resident_clusters(int size) {
 template <bool VEC>
 static int f32_gemm_any(const F32GemmParams& p, int groups, cudaStream_t stream) {
   // Up to 8 rows every weight is read once and used a few times: the streaming kernel (8 rows x 16,384 x 2,048: 47 us; the
-  // tile kernel takes 121 us for anything up to 64 rows).
-  if (p.M <= 2) f32_launch_gemv<2, VEC>(p, groups, stream);
-  else if (p.M <= 4) f32_launch_gemv<4, VEC>(p, groups, stream);
-  else if (p.M <= 8) f32_launch_gemv<8, VEC>(p, groups, stream);
-  else {
+  // tile kernel takes 121 us for anything up to 64 rows).  What it pays for a CTA of four columns whatever K (3 ns of the chip for
+  // up to two rows, 7 for eight) is too much for many columns and a short K: 16 heads of 512 x 128 with 8 rows 16.8 us
+  // (tiles, K split: 7.3), with one row 7.4 (7.1).
+  const int rows = p.M <= 2 ? 2 : p.M <= 4 ? 4 : 8;
+  const bool stream_weights = p.M <= 8 && !(static_cast<long long>((p.N + FV_COLS - 1) / FV_COLS) * groups >= 2048 && p.K <= 64 * std::min(rows, 4));
+  if (stream_weights) {
+    if (rows == 2) f32_launch_gemv<2, VEC>(p, groups, stream);
+    else if (rows == 4) f32_launch_gemv<4, VEC>(p, groups, stream);
+    else f32_launch_gemv<8, VEC>(p, groups, stream);
+  } else {
     static bool configured = false;
     if (!configured) {
       cudaError_t e = cudaFuncSetAttribute(f32_gemm_kernel<VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, FT_SMEM);
       if (e != cudaSuccess) return -1000 - static_cast<int>(e);
       configured = true;
     }
-    // K is split so that rounds of co-resident clusters times the length of a CTA are fewest, as long as a split keeps eight
-    // blocks of K (below that its prologue and the exchange of partial tiles weigh more).  Clusters are placed per GPC, so
-    // fewer of the odd sizes fit than 2 x 148 / size; a CTA that has its SM for itself takes 0.8 of the
-    // time (2.9 us per block of K, 3.6 us for two CTAs).
+    // K is split so that rounds of co-resident clusters times the length of a CTA, in blocks of K and one for its start and the
+    // exchange of partial tiles, are fewest.  Clusters are placed per GPC, so fewer of the odd sizes fit than 2 x 148 / size; a CTA
+    // that has its SM for itself takes 0.8 of the time (2.0 us per block of K, 3.6 us for two CTAs).  65 rows, 256 x 256: eight
+    // splits of a block 6.5 us, one CTA per tile 20.1; 380 x 2,048 x 2,048: eight splits 102, two 122.
     const int m_tiles = (p.M + FT_M - 1) / FT_M, n_tiles = (p.N + FT_N - 1) / FT_N, blocks = (p.K + FT_K - 1) / FT_K;
     const long long tiles = static_cast<long long>(m_tiles) * n_tiles * groups;
     int splits = 1;
     double best = 0.;
-    for (int s = 1; s <= 8 && (s == 1 || blocks >= 8 * s); ++s) {
+    for (int s = 1; s <= 8 && (s == 1 || blocks >= s); ++s) {
       const int room = f32_resident_clusters<VEC>(s);
-      const double cost = static_cast<double>((tiles + room - 1) / room) * (blocks / s + 2) * (tiles * s <= 148 ? 0.8 : 1.);
+      const double cost = static_cast<double>((tiles + room - 1) / room) * ((blocks + s - 1) / s + 1) * (tiles * s <= 148 ? 0.8 : 1.);
       if (s == 1 || cost < 0.95 * best) { best = cost; splits = s; }
     }
     launch_ex(f32_gemm_kernel<VEC>, dim3(n_tiles * splits, m_tiles, groups), dim3(FT_THREADS), FT_SMEM, stream, splits > 1 ? splits : 0, p, splits);

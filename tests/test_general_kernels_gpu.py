@@ -26,6 +26,61 @@ def test_f32_linear_at_tile_and_split_edges(M, N, K, aligned):
     assert (y.double() - want).abs().max() <= 2e-5 * want.abs().max().clamp_min(1.0)
 
 
+def _us(fn, n=10):
+    """Device time of a call in a captured run of ``n``, best of five."""
+    fn()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(n):
+            fn()
+    t = []
+    for _ in range(5):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        graph.replay()
+        b.record()
+        torch.cuda.synchronize()
+        t.append(a.elapsed_time(b) * 1e3 / n)
+    return min(t)
+
+
+@pytest.mark.parametrize("M,N,K", [(9, 64, 33), (16, 100, 300), (33, 256, 96), (64, 130, 160), (65, 256, 256), (130, 1030, 224), (380, 512, 192)])
+def test_f32_linear_with_fewer_than_eight_blocks_of_k_per_split(M, N, K):
+    """Splits of one and two blocks, a last one that is partly filled; the bound of the longer sums."""
+    from mojo_linuxperiments_b200.ops import dense as D
+    g = torch.Generator(device=DEV).manual_seed(M + K)
+    x = D.rows(M, K, torch.float32, DEV)
+    x.normal_(generator=g)
+    W = torch.randn((N, K), generator=g, device=DEV) * K ** -0.5
+    y = D.linear(x, D.DenseW.of(W, torch.float32, DEV))[:, :N]
+    want = x[:, :K].double() @ W.double().t()
+    assert (y.double() - want).norm() <= 2e-6 * want.norm()
+
+
+@pytest.mark.parametrize("M,heads,n,k", [(1, 16, 512, 128), (2, 16, 512, 132), (3, 16, 516, 256), (4, 17, 500, 260), (8, 16, 512, 128), (8, 16, 511, 256), (8, 4, 2048, 64)])
+def test_f32_heads_around_the_line_between_streaming_and_tiles(M, heads, n, k):
+    from mojo_linuxperiments_b200.ops import dense as D
+    g = torch.Generator(device=DEV).manual_seed(n + k)
+    W = torch.randn((heads, n, k), generator=g, device=DEV) * k ** -0.5
+    xk, yn = (k + 7) // 8 * 8, (n + 7) // 8 * 8
+    x = torch.randn((M, heads * xk), generator=g, device=DEV)
+    y = D.linear_heads(x, D.GroupedW.of(W, heads, torch.float32, DEV), xk, yn)
+    want = torch.einsum("mhk,hnk->mhn", x.view(M, heads, xk)[..., :k].double(), W.double())
+    assert (y.view(M, heads, yn)[..., :n].double() - want).norm() <= 2e-6 * want.norm()
+
+
+def test_f32_linear_of_a_short_sum_takes_a_short_time():
+    """K = 256 instead of 2,048 for few tiles: 6.3 us and 21 (20 and 21 where K was only split into eight blocks and more).  Eight rows over 16
+    heads of 512 x 128: 1.0 times the time of nine rows (1.4 with a CTA for every four columns).  The bounds lie between."""
+    from mojo_linuxperiments_b200.ops import dense as D
+    x = torch.randn((65, 2048), device=DEV)
+    short, long = D.DenseW.of(torch.randn((256, 256), device=DEV), torch.float32, DEV), D.DenseW.of(torch.randn((256, 2048), device=DEV), torch.float32, DEV)
+    assert _us(lambda: D.linear(x, short)) < 0.6 * _us(lambda: D.linear(x, long))
+    W, xh = D.GroupedW(torch.randn((16 * 512, 128), device=DEV), 16, 512, 128), torch.randn((9, 2048), device=DEV)
+    assert _us(lambda: D.linear_heads(xh[:8], W, 128, 512)) < 1.2 * _us(lambda: D.linear_heads(xh, W, 128, 512))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("repeat", [1, 4])
 @pytest.mark.parametrize("dk,dv,chunk", [(10, 6, None), (8, 8, 40), (130, 516, None), (36, 644, 100)])
