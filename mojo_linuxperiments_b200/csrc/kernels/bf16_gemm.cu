@@ -208,10 +208,11 @@ static int bf16_gemm_any(const void* x, long long ldx, const void* w, long long 
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w) & 15)) return -2;
   if (int rc = dense_epilogue_check(epi, N)) return rc;
   if (g && (g->groups <= 0 || !g->tiles || !g->num_tiles || g->max_tiles <= 0 || epi->mode != B200_EPI_STORE)) return -3;
-  if (!g && (force_bn < 0 || (force_bn == 0 && M > 128))) {
-    // -force_bn names the channels.  From 130 tokens on a
-    // pair beats the best tile of a CTA alone: 130 x 16,384 x 2,048 22 -> 19 us, 200 x 2,048 x 8,192 43 -> 34, 1,000 x 576 x 2,048
-    // 17.6 -> 16.3, 4,200 x 16,384 x 2,048 226 -> 198 (1,425 TFLOP/s), 4,200 x 2,048 x 8,192 146 -> 100, 4,000 x 64 x 2,048 15 -> 13.
+  if (!g && (force_bn < 0 || (force_bn == 0 && M > 128 && pair_pays(M, N, (K + BG_BK - 1) / BG_BK, epi->mode == B200_EPI_RESIDUAL ? 24 : 16, num_sms)))) {
+    // -force_bn names the channels.  A pair against the best tile of a CTA alone: 130 x 16,384 x 2,048 22 -> 19 us, 200 x 2,048 x 8,192
+    // 43 -> 34, 1,000 x 576 x 2,048 17.6 -> 16.3, 4,200 x 16,384 x 2,048 226 -> 198 (1,425 TFLOP/s), 4,200 x 2,048 x 8,192 146 -> 100,
+    // 4,000 x 64 x 2,048 15 -> 13.  From K = 1,024 on (1,536 where the residual rows go through its longer epilogue) it is at most 5 % slower;
+    // below, 257 x 1,024 x 256 5.5 (4.6), with residual rows 7.7 (5.8), 2,500 x 16,384 x 256 42 (38), but 2,500 x 1,024 x 256 6.6 (7.2).
     const int bn = pair_width(-force_bn) ? -force_bn : pair_pick_width(M, N, num_sms);
     return bf16_gemm_pair(x, ldx, w, ldw, M, N, K, epi, bn, status, num_sms, stream);
   }

@@ -28,7 +28,7 @@ inline int pair_count(long long tiles, int num_sms) {
   return static_cast<int>(tiles < pairs ? tiles : pairs);
 }
 // the width with the fewest rounds of the pairs times the cost of a tile (main loop ~ its channels, plus a fixed part)
-inline int pair_pick_width(int M, int N, int num_sms) {
+inline int pair_pick_width(int M, int N, int num_sms, long long* cost_out = nullptr) {
   long long best = -1;
   int bn = 0;
   for (int cand : {256, 224, 192, 160, 128}) {
@@ -36,7 +36,21 @@ inline int pair_pick_width(int M, int N, int num_sms) {
     const long long cost = (tiles + pairs - 1) / pairs * (cand + 32);
     if (best < 0 || cost < best) { best = cost; bn = cand; }
   }
+  if (cost_out) *cost_out = best;
   return bn;
+}
+// Above 128 tokens: is a pair on a tile faster than CTAs alone on 128 x 64 to 256?  Its start and its longer epilogue are paid back
+// from `enough` blocks of K on (each caller's figures), or at any length where the fuller rounds save a quarter.
+inline bool pair_pays(int M, int N, int kblocks, int enough, int num_sms) {
+  if (kblocks >= enough) return true;
+  long long pair, alone = -1;
+  pair_pick_width(M, N, num_sms, &pair);
+  for (int cand : {256, 128, 64}) {
+    const long long tiles = static_cast<long long>((M + 127) / 128) * ((N + cand - 1) / cand);
+    const long long cost = (tiles + num_sms - 1) / num_sms * (cand + 64);
+    if (alone < 0 || cost < alone) alone = cost;
+  }
+  return 4 * pair <= 3 * alone;
 }
 
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncols) {

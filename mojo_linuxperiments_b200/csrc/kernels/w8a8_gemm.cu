@@ -502,9 +502,10 @@ extern "C" int b200_w8a8_gemm(const void* xq, const float* sx, const void* wq, c
                        (reinterpret_cast<uintptr_t>(sw) & 15) == 0;
   // a number that names no tile width (0 and 1: the schedules of the one-CTA kernel) leaves the choice to the rule
   const bool width = pair_width(force_mode);
-  if (pair_ok && (width || (force_mode != 0 && force_mode != 1 && M > 128))) {
-    // Above 128 tokens a pair is never slower than a CTA alone: 200 x 28,672 x 4,096 30 us (40), 1,024 x 6,144 x 4,096 23 (37), 32,768 x 28,672 x
-    // 4,096 2,351 (2,989), 32,768 x 4,096 x 14,336 1,150 (1,341).
+  if (pair_ok && (width || (force_mode != 0 && force_mode != 1 && M > 128 && pair_pays(M, N, (K + BLOCK_K - 1) / BLOCK_K, 8, num_sms)))) {
+    // A pair against a CTA alone: 200 x 28,672 x 4,096 30 us (40), 1,024 x 6,144 x 4,096 23 (37), 32,768 x 28,672 x 4,096 2,351 (2,989),
+    // 32,768 x 4,096 x 14,336 1,150 (1,341).  From K = 1,024 on it is at most 5 % slower (2,500 x 16,384 x 1,024: 47.6, 45.3); below,
+    // 257 x 1,024 x 512 5.0 (4.9), 257 x 1,024 x 128 4.4 (4.0), 2,500 x 16,384 x 256 42 (36), but 2,500 x 1,024 x 256 6.0 (7.0).
     const int bn = width ? force_mode : pair_pick_width(M, N, num_sms);
     return w8a8_gemm_pair(xq, sx, wq, sw, y, M, N, K, ldy, bn, status, num_sms, stream);
   }

@@ -303,6 +303,21 @@ def test_int8_linear_writes_rows_that_start_anywhere(M, N, ld, residual):
     assert buf[0] == 7.0 and (buf[1:].view(M, ld)[:, N:] == 7.0).all()
 
 
+def test_linears_with_a_short_k_are_not_slower_than_a_cta_per_tile():
+    """More than 128 tokens, K too short for what a pair of CTAs costs at its start and end (1.16 to 1.33 times as long before the rule
+    looked at K): the call goes to the one-CTA tiles, which the right side forces."""
+    from mojo_linuxperiments_b200.ops import dense as D
+    from mojo_linuxperiments_b200.ops import linear as L
+    x, w, s = D.rows(257, 256, torch.bfloat16, DEV), D.DenseW.of(torch.randn((1024, 256), device=DEV), torch.bfloat16, DEV), D.rows(257, 1024, torch.float32, DEV)
+    x.normal_()
+    s.zero_()
+    for fn in (lambda force: D.linear(x, w, force=force), lambda force: D.linear_residual(x, w, s, 1e-6, None, None, force=force)):
+        assert _us(lambda: fn(0)) < 1.1 * _us(lambda: fn(1))
+    xq, sx = torch.randint(-127, 128, (2500, 256), device=DEV, dtype=torch.int8), torch.rand(2500, device=DEV)
+    wq, sw = torch.randint(-127, 128, (16384, 256), device=DEV, dtype=torch.int8), torch.rand(16384, device=DEV)
+    assert _us(lambda: L.w8a8_gemm(xq, sx, wq, sw)) < 1.1 * _us(lambda: L.w8a8_gemm(xq, sx, wq, sw, force_mode=0))
+
+
 @pytest.mark.parametrize("rows", [1, 127, 128, 129, 300])
 def test_end_of_a_decode_step(rows):
     """Whole numbers: exact."""
