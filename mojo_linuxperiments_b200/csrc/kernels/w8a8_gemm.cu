@@ -105,7 +105,9 @@ __device__ __forceinline__ void tile_coords(const GemmParams& p, int tile, int& 
 
 // tmap_a covers the operand whose 128-row tiles fill the MMA M dimension (weights when SWAP, tokens otherwise),
 // tmap_b the operand whose BN-row tiles fill the MMA N dimension.
-template <int BN, int STAGES, bool SWAP>
+// TURNED: results leave through shared memory (w8_tile.cuh); an instantiation of its own, because the other ways out need half the
+// registers and were 0.3 us slower beside it.
+template <int BN, int STAGES, bool SWAP, bool TURNED>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  const GemmParams p) {
@@ -121,7 +123,7 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* pieces = smem + STAGES * STAGE_BYTES;             // staging of the four epilogue warps (token rows on the M side only)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(pieces + (SWAP ? 0 : 4 * W8_PIECE));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(pieces + (TURNED ? 4 * W8_PIECE : 0));
   // bars: [0,STAGES) full, [STAGES,2*STAGES) empty, then tmem_full[2], tmem_empty[2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -259,17 +261,16 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const float sxm = m_ok ? p.sx[m] : 0.f;
         const int n0 = n_tile * BN;
         const size_t row_off = static_cast<size_t>(m_ok ? m : 0) * p.ldy;
-        const int m_first = p.grp_tiles ? p.grp_tiles[m_tile].y : m_tile * TILE_N, m_end = p.grp_tiles ? m_first + p.grp_tiles[m_tile].z : p.M;
         const bool vec_ok = !p.out_fp32 && (p.ldy % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.y) & 15) == 0) &&
                             (!p.residual || (reinterpret_cast<uintptr_t>(p.residual) & 15) == 0);
         // Row lists of 64,000 rows in 128 groups: 2,048 x 768 184 -> 154 us, 1,536 x 2,048 231 -> 205; of 2,400: 63 -> 52 and 79 -> 77.
-        const bool turned = vec_ok && !p.residual && p.N % 8 == 0 && (reinterpret_cast<uintptr_t>(swg) & 15) == 0;
-        if (turned) {
+        if constexpr (TURNED) {
+          const int m_first = p.grp_tiles ? p.grp_tiles[m_tile].y : m_tile * TILE_N, m_end = p.grp_tiles ? m_first + p.grp_tiles[m_tile].z : p.M;
           const W8TileRows rows{swg, reinterpret_cast<__nv_bfloat16*>(p.y), p.ldy, n0, p.N, m_first + q * 32, m_end, lane, sxm, pieces + (warp - 2) * W8_PIECE};
           rows.finish<BN>(t_addr);
         }
 #pragma unroll 1
-        for (int c = turned ? BN / 32 : 0; c < BN / 32; ++c) {
+        for (int c = 0; c < (TURNED ? 0 : BN / 32); ++c) {
           uint32_t r[32];
           tmem_ld_x32(t_addr + c * 32, r);
           tmem_ld_wait();
@@ -428,21 +429,31 @@ w8a8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 // ------------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------------
-template <int BN, int STAGES, bool SWAP>
-static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t stream) {
-  constexpr int SMEM = STAGES * (TILE_N * BLOCK_K + BN * BLOCK_K) + (SWAP ? 0 : 4 * W8_PIECE) + 1024 + 256;
+template <int BN, int STAGES, bool SWAP, bool TURNED>
+static int launch_gemm_as(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t stream) {
+  constexpr int SMEM = STAGES * (TILE_N * BLOCK_K + BN * BLOCK_K) + (TURNED ? 4 * W8_PIECE : 0) + 1024 + 256;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(w8a8_gemm_kernel<BN, STAGES, SWAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    cudaError_t e = cudaFuncSetAttribute(w8a8_gemm_kernel<BN, STAGES, SWAP, TURNED>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     // ask for the largest shared-memory carveout: with the default preference the occupancy calculator (and the
     // launch) may settle for a split of the L1 / shared array that holds fewer CTAs per SM than the kernel was sized for
-    cudaFuncSetAttribute(w8a8_gemm_kernel<BN, STAGES, SWAP>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute(w8a8_gemm_kernel<BN, STAGES, SWAP, TURNED>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return -1000 - static_cast<int>(e);
     configured = true;
   }
-  launch_ex(w8a8_gemm_kernel<BN, STAGES, SWAP>, dim3(grid), dim3(GEMM_THREADS), SMEM, stream, 0, ta, tb, p);
+  launch_ex(w8a8_gemm_kernel<BN, STAGES, SWAP, TURNED>, dim3(grid), dim3(GEMM_THREADS), SMEM, stream, 0, ta, tb, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
+}
+
+template <int BN, int STAGES, bool SWAP>
+static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t stream) {
+  if constexpr (!SWAP) {      // (the scales of a group start at a multiple of N)
+    if (!p.out_fp32 && !p.residual && p.N % 8 == 0 && p.ldy % 8 == 0 &&
+        ((reinterpret_cast<uintptr_t>(p.y) | reinterpret_cast<uintptr_t>(p.sw)) & 15) == 0)
+      return launch_gemm_as<BN, STAGES, SWAP, true>(ta, tb, p, grid, stream);
+  }
+  return launch_gemm_as<BN, STAGES, SWAP, false>(ta, tb, p, grid, stream);
 }
 
 
