@@ -54,6 +54,16 @@ __device__ __forceinline__ void rope_load8(const __nv_bfloat16* x, float (&v)[8]
   }
 }
 template <bool VEC>
+__device__ __forceinline__ void rope_table8(const float* x, float (&v)[8]) {
+  if constexpr (VEC) {
+    const float4 a = reinterpret_cast<const float4*>(x)[0], b = reinterpret_cast<const float4*>(x)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = x[i];
+  }
+}
+template <bool VEC>
 __device__ __forceinline__ void rope_store8(__nv_bfloat16* x, const __nv_bfloat162 (&v)[4]) {
   if constexpr (VEC) {
     *reinterpret_cast<uint4*>(x) = *reinterpret_cast<const uint4*>(v);
@@ -63,7 +73,8 @@ __device__ __forceinline__ void rope_store8(__nv_bfloat16* x, const __nv_bfloat1
   }
 }
 
-template <bool VEC>
+// ONCE: the grid has a half-warp for every head, whose row is asked for before the position is known
+template <bool VEC, bool ONCE>
 __global__ void __launch_bounds__(128) rope_kv_kernel(const __grid_constant__ RopeParams p) {
   pdl_launch_dependents();   // the next kernel may start its prologue now
   B200_TRACE_INIT();
@@ -74,6 +85,11 @@ __global__ void __launch_bounds__(128) rope_kv_kernel(const __grid_constant__ Ro
 
   const int tok = blockIdx.x;
   const int half = threadIdx.x >> 4, l = threadIdx.x & 15;
+  const int nheads = p.hq + 2 * p.hkv, stride = 8 * gridDim.y;
+  const __nv_bfloat16* row = p.qkv + static_cast<size_t>(tok) * p.ld_qkv + 8 * l;
+  float v[8];
+  auto load_head = [&](int h) { rope_load8<VEC>(row + static_cast<size_t>(h < nheads ? h : 0) * HEAD_DIM, v); };
+  if constexpr (ONCE) load_head(blockIdx.y * 8 + half);
   const int pos = p.positions[tok];
   const int seq = p.seq_ids ? p.seq_ids[tok] : tok;
   // A position beyond the tables or beyond the pages admitted for the sequence must not become a stray write: the
@@ -88,23 +104,19 @@ __global__ void __launch_bounds__(128) rope_kv_kernel(const __grid_constant__ Ro
     if (threadIdx.x == 0 && blockIdx.y == 0 && p.status) atomicCAS(p.status, 0, static_cast<int>(ST_BAD_ARGUMENT) | (7 << 8));
     return;
   }
-  const __nv_bfloat16* row = p.qkv + static_cast<size_t>(tok) * p.ld_qkv + 8 * l;
   float c[8], s[8];
+  rope_table8<VEC>(p.cos_tab + static_cast<size_t>(pos) * 64 + (l & 7) * 8, c);
+  rope_table8<VEC>(p.sin_tab + static_cast<size_t>(pos) * 64 + (l & 7) * 8, s);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    c[i] = p.cos_tab[static_cast<size_t>(pos) * 64 + (l & 7) * 8 + i];
-    s[i] = p.sin_tab[static_cast<size_t>(pos) * 64 + (l & 7) * 8 + i];
+  for (int i = 0; i < 8; ++i)
     if (l < 8) s[i] = -s[i];
-  }
   size_t cache_row = 0;
   if (p.cache) cache_row = static_cast<size_t>(page) * 2 * p.hkv * p.page_size + (pos % p.page_size);
-  const int nheads = p.hq + 2 * p.hkv, stride = 8 * gridDim.y;
-#pragma unroll 3
+#pragma unroll(ONCE ? 1 : 3)
   for (int h0 = blockIdx.y * 8; h0 < nheads; h0 += stride) {       // the same for the whole warp
     const int h = h0 + half;
     const bool there = h < nheads, is_q = h < p.hq, is_k = !is_q && h < p.hq + p.hkv;
-    float v[8];
-    rope_load8<VEC>(row + static_cast<size_t>(there ? h : 0) * HEAD_DIM, v);
+    if constexpr (!ONCE) load_head(h);
     const __nv_bfloat16* nw = is_q ? p.q_norm_w : is_k ? p.k_norm_w : nullptr;
     if (p.q_norm_w || p.k_norm_w) {
       float ss = 0.f;
@@ -143,6 +155,7 @@ __global__ void __launch_bounds__(128) rope_kv_kernel(const __grid_constant__ Ro
         rope_store8<VEC>(p.cache + off * HEAD_DIM + 8 * l, b);
       }
     }
+    if constexpr (ONCE) break;
   }
 }
 
@@ -274,11 +287,16 @@ extern "C" int b200_rope_kv_write(const void* qkv, long long ld_qkv, const int* 
   p.cache = static_cast<__nv_bfloat16*>(cache); p.page_table = page_table; p.max_pages = max_pages; p.page_size = page_size;
   p.hq = hq; p.hkv = hkv; p.M = M; p.max_pos = max_pos; p.num_pages = num_pages; p.status = status;
   auto al16 = [](const void* a) { return (reinterpret_cast<uintptr_t>(a) & 15) == 0; };
-  const bool vec = ld_qkv % 8 == 0 && al16(qkv) && al16(q_norm_w) && al16(k_norm_w) && al16(q_out) && al16(k_out) && al16(v_out) && al16(cache);
+  const bool vec = ld_qkv % 8 == 0 && al16(qkv) && al16(q_norm_w) && al16(k_norm_w) && al16(q_out) && al16(k_out) && al16(v_out) && al16(cache) &&
+                   al16(cos_tab) && al16(sin_tab);
   // few tokens: every half-warp takes one head; many: a CTA per token, so that the table rows are read once
-  const dim3 grid(M, M < 1024 ? (hq + 2 * hkv + 7) / 8 : 1);
-  if (vec) launch_ex(rope_kv_kernel<true>, grid, dim3(128), 0, stream, 0, p);
-  else launch_ex(rope_kv_kernel<false>, grid, dim3(128), 0, stream, 0, p);
+  const bool once = M < 1024;
+  const dim3 grid(M, once ? (hq + 2 * hkv + 7) / 8 : 1);
+  if (vec) {
+    if (once) launch_ex(rope_kv_kernel<true, true>, grid, dim3(128), 0, stream, 0, p);
+    else launch_ex(rope_kv_kernel<true, false>, grid, dim3(128), 0, stream, 0, p);
+  } else if (once) launch_ex(rope_kv_kernel<false, true>, grid, dim3(128), 0, stream, 0, p);
+  else launch_ex(rope_kv_kernel<false, false>, grid, dim3(128), 0, stream, 0, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }
