@@ -90,6 +90,7 @@ act_quant_kernel(const __nv_bfloat16* x, long long ldx, __nv_bfloat16* residual,
 
   const __nv_bfloat16* xr = x + row * ldx;
   float2 v[MAXC][8];
+  uint32_t gain[8];
   float2 ss = make_float2(0.f, 0.f);
   float amax = 0.f;
 #pragma unroll
@@ -101,6 +102,7 @@ act_quant_kernel(const __nv_bfloat16* x, long long ldx, __nv_bfloat16* residual,
     }
     uint32_t a[8], b[8];
     load16(xr + at(i), a);
+    if constexpr (NORM && MAXC == 1) load16(gamma + at(i), gain);      // asked for with the row, not behind the sum of its squares
     if constexpr (MODE == AQ_SWIGLU) load16(xr + K + at(i), b);
     if constexpr (MODE == AQ_ADD_NORM) load16(residual + row * ldr + at(i), b);
 #pragma unroll
@@ -131,10 +133,9 @@ act_quant_kernel(const __nv_bfloat16* x, long long ldx, __nv_bfloat16* residual,
 #pragma unroll
     for (int i = 0; i < MAXC; ++i) {
       if (!have(i)) continue;
-      uint32_t g[8];
-      load16(gamma + at(i), g);
+      if constexpr (MAXC > 1) load16(gamma + at(i), gain);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[i][j] = mul2(mul2(v[i][j], make_float2(rstd, rstd)), pair(g, j));
+      for (int j = 0; j < 8; ++j) v[i][j] = mul2(mul2(v[i][j], make_float2(rstd, rstd)), pair(gain, j));
       if (xn_out) store16(xn_out + row * ldn + at(i), v[i]);
     }
   }
