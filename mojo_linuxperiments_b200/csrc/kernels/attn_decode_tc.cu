@@ -45,7 +45,8 @@ constexpr int ADC_O_COL = 64;
 struct DecodeFuse {
   const __nv_bfloat16* qkv;        // [B][(hq + 2 hkv) * 128] (row pitch ld_qkv elements)
   long long ld_qkv;
-  const int* positions;            // [B] position of the new token (seq_lens[b] counts it: cached tokens = seq_lens[b] - 1)
+  const int* positions;            // [B] position of the new token (seq_lens[b] counts it: cached tokens = seq_lens[b] - 1); like lengths and
+                                   // page table settled before the kernel in front starts: read ahead of the dependency wait
   const float* cos_tab;            // [max_pos][64]
   const float* sin_tab;
   int max_pos;

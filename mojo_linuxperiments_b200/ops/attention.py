@@ -94,7 +94,7 @@ def attn_prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlens: 
 
     ``kv_chunk`` > 0 selects the split-KV form: every ``kv_chunk`` KV tiles of 128 tokens of a query tile are a CTA of
     their own and a merge kernel combines them - more parallelism when there are few (sequence, head) pairs.  Default
-    (``None``): B200RT_PREFILL_SPLIT if set, else split exactly when the un-split grid would not fill the GPU."""
+    (``None``): B200RT_PREFILL_SPLIT if set, else split where there are fewer (sequence, head, query tile) units than SMs."""
     T, hq, d = q.shape
     hkv = k.shape[1]
     assert d == HEAD_DIM and q.dtype == torch.bfloat16 and q.stride(2) == 1 and q.stride(1) == d
@@ -109,9 +109,12 @@ def attn_prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlens: 
         if env != "":
             kv_chunk = int(env)
         else:
-            # Few (sequence, head, query tile) CTAs leave most SMs idle while the last query tiles walk their KV tiles
-            # alone: split the KV range then (measured on B200: 1 x 1,024 tokens x 4 heads 33 -> 16 us, 1 x 4,096 x 4
-            # heads 143 -> 103 us; with >= 148 CTAs the un-split kernel is faster).
+            # Few (sequence, head, query tile) units leave most SMs idle while the last query tiles walk their KV tiles
+            # alone.  The line was drawn when the un-split kernel gave every unit a CTA of its own; now two units share one and it
+            # is two to three times as fast.  Measured with it: the split pays for few heads over a long range (1 x 1,024 tokens x
+            # 4 heads 15.9 us, un-split 23.8; 1 x 512 x 8 heads 14.3, 15.0; 1 x 2,048 x 4 heads 38.7, 41.4), and no longer does
+            # elsewhere below the line (1 x 300 x 32 heads 21.7, un-split 11.8; 1 x 512 x 32 heads 28.7, 15.4; 1 x 4,096 x 4 heads
+            # 100, 77).
             B_ = cu_seqlens.numel() - 1
             n_q = (int(max_len) + 127) // 128
             sms = _lib.num_sms(q.device.index)
@@ -258,7 +261,8 @@ def attn_decode_fused(qkv: torch.Tensor, positions: torch.Tensor, cos: torch.Ten
     """One launch for rope_kv_write + decode attention + the activation prologue of o_proj.
 
     qkv bf16 [B, (hq + 2 hkv) * 128]: the new token's raw projections; ``positions[b]`` is where it goes in the cache and
-    ``seq_lens[b]`` counts it.  Returns ``(xq int8 [B, hq*128], sx fp32 [B], out bf16 [B, hq, 128] or None)``; with
+    ``seq_lens[b]`` counts it (both, and the page table, are read ahead of the dependency wait: settled before the op in front of this
+    one starts).  Returns ``(xq int8 [B, hq*128], sx fp32 [B], out bf16 [B, hq, 128] or None)``; with
     ``quantize=False`` only ``out``.  Needs page size 16 and a group size of 1/2/4/8/16 (the tcgen05 kernel).
     ``next_weights``: a constant tensor the following kernel streams (the o-projection's int8 weights); the kernel's CTAs
     ask for it to be brought into L2 meanwhile."""

@@ -29,7 +29,8 @@ def rows(m: int, n: int, dtype: torch.dtype, device) -> torch.Tensor:
 
 @dataclass
 class DenseW:
-    """[n, k] weight stored with a padded row pitch (padding zero)."""
+    """[n, k] weight stored with a padded row pitch (padding zero).  Kernels for a few rows ask for weights before the op in front of
+    them has ended: they are settled before that op starts, as a model's weights are."""
     data: torch.Tensor
     n: int
     k: int

@@ -1,4 +1,5 @@
-"""The kernels of the 32-bit form and the general attention at the edges of their tiles, splits and load widths."""
+"""Linears (fp32, bf16, int8), attention (general, prefill), activation rows, rotary embedding and the end of a step: kernels one by one,
+at the edges of their tiles, splits, load widths and dispatch rules."""
 import pytest
 import torch
 
