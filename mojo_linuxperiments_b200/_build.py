@@ -26,7 +26,7 @@ NVCC_FLAGS = [
 ]
 # --use_fast_math is dropped for files whose numerics are compared bit-for-bit with an oracle
 # (act_quant) or that also carry the 32-bit form of a model
-NO_FAST_MATH = {"act_quant.cu", "bf16_gemm.cu", "bf16_gemm_decode.cu", "bf16_gemm_pair.cu", "f32_gemm.cu", "rotary_paged.cu", "attn_paged.cu", "latent.cu",
+NO_FAST_MATH = {"act_quant.cu", "bf16_gemm.cu", "bf16_gemm_decode.cu", "bf16_gemm_pair.cu", "f32_gemm.cu", "f32_gemm_tc.cu", "rotary_paged.cu", "attn_paged.cu", "latent.cu",
                 "mingru.cu", "moe_route.cu", "stream_rows.cu"}
 GXX_FLAGS = ["-O2", "-std=c++20", "-fPIC", "-Wall", "-Wextra", "-fno-stack-protector", "-pthread"]
 
@@ -39,7 +39,7 @@ KERNEL_LIB = "libb200_kernels.so"
 KERNEL_VARIANTS = {"": [], "trace": ["-DB200RT_TRACE"], "debug": ["-DB200RT_DEBUG"], "dense": []}
 KERNEL_SUBSETS = {"dense": ("attn_decode_paged.cu", "attn_latent.cu", "attn_paged.cu", "attn_prefill_latent.cu",
                             "attn_prefill_paged.cu", "bf16_gemm.cu", "bf16_gemm_decode.cu", "bf16_gemm_pair.cu",
-                            "f32_gemm.cu", "latent.cu", "mingru.cu", "moe.cu", "moe_route.cu", "rope_kv.cu", "rotary_paged.cu",
+                            "f32_gemm.cu", "f32_gemm_tc.cu", "latent.cu", "mingru.cu", "moe.cu", "moe_route.cu", "rope_kv.cu", "rotary_paged.cu",
                             "stream_rows.cu", "tmap.cu", "trace.cu")}
 
 

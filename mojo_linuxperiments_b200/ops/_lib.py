@@ -105,6 +105,8 @@ class _Sig:
     b200_bf16_gemm = (I, [P, LL, P, LL, I, I, I, P, P, I, I, P])
     b200_bf16_gemm_decode = (I, [P, LL, P, LL, I, I, I, P, P, I, I, P])
     b200_f32_gemm = (I, [P, LL, P, LL, I, I, I, P, P])
+    b200_f32_gemm_tc = (I, [P, LL, P, LL, I, I, I, P, P, I, P])
+    b200_f32_gemm_tc_takes = (I, [I, I, I])
     b200_bf16_gemm_grouped = (I, [P, LL, P, LL, I, I, I, P, P, P, I, I, P])
     b200_bf16_gemm_decode_grouped = (I, [P, LL, P, LL, I, I, I, I, P, P, P, I, I, P])
     b200_f32_gemm_grouped = (I, [P, LL, P, LL, I, I, I, P, P, P])

@@ -361,3 +361,49 @@ def test_bf16_linear_of_two_ctas_per_tile(M, N, K, bn):
     a, u = want[:, 0::2].clamp(max=7.0), want[:, 1::2].clamp(-7.0, 7.0)
     for got, ref in ((y16.double(), want), (glu, a * torch.sigmoid(1.702 * a) * (u + 1))):
         assert (got - ref).norm() <= 4e-3 * ref.norm()
+
+
+@pytest.mark.parametrize("splits", [0, 1, 2, 8])
+@pytest.mark.parametrize("M,N,K", [(1, 4, 32), (9, 128, 33), (16, 129, 511), (127, 5, 512), (128, 300, 1027), (129, 256, 2049), (400, 130, 4096)])
+def test_f32_linear_in_three_bf16_parts(M, N, K, splits):
+    """Edges of the 128 x 128 tiles, of blocks of 32 k, of the periods of 256 and 1,024 k, one block per split; what lies beyond K or M does
+    not matter.  Splitting is exact but for products below 2^-26, a sum of 32 k is cut off at 2^-23, sums of sums are rounded: no further from
+    64 bits than the sums of the CUDA cores from K = 512 on, shorter sums within 1e-7.  Where all products have one sign the cuts add up: two
+    per block, each at most 2^-23 and half of that on average, 1.2e-7."""
+    from mojo_linuxperiments_b200.ops import dense as D
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    for kind in ("signs", "positive", "sizes"):
+        X, W = torch.randn((M, K), generator=g, device=DEV), torch.randn((N, K), generator=g, device=DEV) * K ** -0.5
+        if kind == "positive":
+            X, W = X.abs(), W.abs()
+        if kind == "sizes":
+            X = X * torch.exp2(torch.randint(-20, 20, (M, K), generator=g, device=DEV).float())
+        x = torch.full((M + 1, (K + 3) // 4 * 4 + 4), float("nan"), device=DEV)[:M]
+        x[:, :K] = X
+        w = torch.full((N, (K + 3) // 4 * 4), float("nan"), device=DEV)
+        w[:, :K] = W
+        want = X.double() @ W.double().t()
+
+        def off(force):
+            y = D.linear(x, D.DenseW(w, N, K), force=force)[:, :N]
+            return ((y.double() - want).norm() / want.norm()).item()
+
+        assert off(splits if splits else 4) <= max(off(-1), 1.2e-7 if kind == "positive" else 1e-7 if K < 512 else 0.0), kind
+
+
+def test_f32_linear_in_three_parts_where_it_is_not_finite():
+    from mojo_linuxperiments_b200.ops import dense as D
+    g = torch.Generator(device=DEV).manual_seed(5)
+    x = D.rows(130, 640, torch.float32, DEV)
+    x.normal_(generator=g)
+    W = torch.randn((200, 640), generator=g, device=DEV)
+    inf = float("inf")
+    x[7] *= 1e30
+    x[:, 630], W[:, 0] = 1e-3, W[:, 0] * 1e-3
+    x[3, 7], x[5, 9], x[7, 3], x[8, 1], W[9, 1] = inf, float("nan"), -inf, 0.0, inf
+    x[129, 0], W[77, 630] = 3.4e38, -3.4e38                   # round to infinity in bf16; every sum of them is finite
+    a, b = (D.linear(x, D.DenseW.of(W, torch.float32, DEV), force=f)[:, :200] for f in (2, -1))
+    assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.isinf(a), torch.isinf(b)) and torch.equal(a[torch.isinf(a)], b[torch.isinf(b)])
+    fine = torch.isfinite(b)
+    assert ((a - b).abs() <= 1e-5 * x.abs().nan_to_num(0, 0, 0).amax(1, keepdim=True).clamp_min(1.0) * W.abs().nan_to_num(0, 0, 0).amax(1))[fine].all()
+    assert torch.isnan(a[8, 9]) and fine[129, 1] and fine[0, 77]
