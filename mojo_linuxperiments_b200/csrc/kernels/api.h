@@ -77,10 +77,9 @@ int b200_w8a8_gemm_decode_ar(const void* xq, const float* sx, const void* wq, co
                              size_t recv2_off1, size_t recv2_bytes, cudaStream_t stream);
 
 // Mixture-of-experts grouped forms (device-side offsets / tile tables, no host sync).
-int b200_w8a8_gemm_decode_grouped(const void* xq, const float* sx, const void* wq, const float* sw, void* y,
-                                  int max_tokens, int x_rows, int N, int K, int ldy, int groups,
-                                  const int* grp_offsets, const int* grp_counts, int* status, int num_sms,
-                                  cudaStream_t stream);
+// Decoding: at most 64 rows per expert, work list as for b200_w8a8_gemm_grouped; N % 128 == 0, ldy % 8 == 0, y on 16 bytes.
+int b200_w8a8_gemm_experts(const void* xq, const float* sx, const void* wq, const float* sw, void* y, int max_tokens, int x_rows, int N,
+                           int K, int ldy, int groups, const void* tiles, const int* num_tiles, int* status, int num_sms, cudaStream_t stream);
 int b200_w8a8_gemm_grouped(const void* xq, const float* sx, const void* wq, const float* sw, void* y, int x_rows,
                            int N, int K, int ldy, int groups, const void* tiles, const int* num_tiles,
                            int max_tiles, int* status, int num_sms, cudaStream_t stream);

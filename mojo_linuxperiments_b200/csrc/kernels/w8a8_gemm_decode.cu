@@ -71,10 +71,6 @@ struct DecodeGemmParams {
   int* status;
   unsigned long long limit_ns;
   ArTail ar;
-  // grouped (mixture-of-experts) form: blockIdx.z = local expert; its tokens are rows [grp_offsets[e], +grp_counts[e])
-  // of xq / y, its weights are rows [e*N, (e+1)*N) of wq / sw
-  const int* grp_offsets;
-  const int* grp_counts;
   // Activation prologue inside the launch: the first qp.rows grid rows are quantiser CTAs (one token row each) that turn
   // the bf16 input into the int8 operand and publish a flag per row; the GEMM CTAs prefetch their weights meanwhile
   // and wait for the flags instead of for an earlier kernel.
@@ -199,15 +195,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     return;
   }
   const int n_tile = blockIdx.y - (prolog ? p.qp.rows : 0);
-  int m0 = blockIdx.z * BN, rows_valid = min(BN, p.M - m0), w_base = 0;
-  const bool grouped = p.grp_counts != nullptr;
-  if (grouped) {
-    pdl_wait();                             // the work list comes from an earlier kernel of the stream
-    rows_valid = min(BN, p.grp_counts[blockIdx.z]);
-    if (rows_valid <= 0) return;            // same for every CTA of the cluster (they share blockIdx.z)
-    m0 = p.grp_offsets[blockIdx.z];
-    w_base = blockIdx.z * p.N;
-  }
+  const int m0 = blockIdx.z * BN, rows_valid = min(BN, p.M - m0);
   const int kb0 = static_cast<int>(static_cast<long long>(p.kblocks) * rank / S);
   const int kb1 = static_cast<int>(static_cast<long long>(p.kblocks) * (rank + 1) / S);
   const uint64_t limit = p.limit_ns;
@@ -226,7 +214,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   // channel scales never change: they are staged before the dependency wait
   if (threadIdx.x >= 64) {
     const int n = n_tile * TILE_N + (threadIdx.x - 64);
-    sw_s[threadIdx.x - 64] = n < p.N ? __ldg(p.sw + w_base + n) : 0.f;
+    sw_s[threadIdx.x - 64] = n < p.N ? __ldg(p.sw + n) : 0.f;
   }
   tc_fence_before();
   __syncthreads();
@@ -272,7 +260,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
       const int pre = min(STAGES, nkb);
       for (int i = 0; i < pre; ++i) {
         mbar_expect_tx(full_bar(i), A_BYTES);
-        tma_load_2d_hint(smem_base + i * STAGE_BYTES, &tmap_w, full_bar(i), (kb0 + i) * BLOCK_K, w_base + n_tile * TILE_N, pol);
+        tma_load_2d_hint(smem_base + i * STAGE_BYTES, &tmap_w, full_bar(i), (kb0 + i) * BLOCK_K, n_tile * TILE_N, pol);
       }
     }
     pdl_wait();
@@ -397,21 +385,21 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     bool ok = true;
     // Weights never change during inference, so the first ring-full of weight tiles is requested before waiting
     // for the previous kernel; the activation tiles (its output) are requested after the wait.
-    const int pre = grouped ? 0 : min(STAGES, kb1 - kb0);
+    const int pre = min(STAGES, kb1 - kb0);
     const uint32_t stage_tx = inl ? A_BYTES : STAGE_BYTES;     // inline prologue: the token rows are stored, not loaded
     if (lane == 0 && !inl) {
       prefetch_tmap(&tmap_w);
       prefetch_tmap(&tmap_x);
       for (int i = 0; i < pre; ++i) {
         mbar_expect_tx(full_bar(i), STAGE_BYTES);
-        tma_load_2d_hint(smem_base + i * STAGE_BYTES, &tmap_w, full_bar(i), (kb0 + i) * BLOCK_K, w_base + n_tile * TILE_N, pol_w);
+        tma_load_2d_hint(smem_base + i * STAGE_BYTES, &tmap_w, full_bar(i), (kb0 + i) * BLOCK_K, n_tile * TILE_N, pol_w);
       }
       // The ring holds the first STAGES tiles; the rest of this CTA's weights are pulled into L2 meanwhile, so that once
       // the input is there the stream runs from L2 for as far as HBM got ahead while the previous kernel finished.
       if (p.l2_prefetch > 0)
-        for (int kb = kb0 + pre; kb < min(kb1, kb0 + pre + p.l2_prefetch); ++kb) tma_prefetch_2d(&tmap_w, kb * BLOCK_K, w_base + n_tile * TILE_N);
+        for (int kb = kb0 + pre; kb < min(kb1, kb0 + pre + p.l2_prefetch); ++kb) tma_prefetch_2d(&tmap_w, kb * BLOCK_K, n_tile * TILE_N);
     }
-    if (!grouped && !inl) pdl_wait();
+    if (!inl) pdl_wait();
     if (prolog && !inl) {
       // the whole warp watches the row flags of this launch's quantiser CTAs (lane l: rows l and l + 32)
       const uint32_t ticket = quant_ticket(p.qp);
@@ -439,7 +427,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.status, (ST_TIMEOUT_SMEM_EMPTY | (2 << 8)), limit)) { ok = false; break; }
         mbar_expect_tx(full_bar(stage), stage_tx);
         const uint32_t a_dst = smem_base + stage * STAGE_BYTES;
-        tma_load_2d_hint(a_dst, &tmap_w, full_bar(stage), kb * BLOCK_K, w_base + n_tile * TILE_N, pol_w);
+        tma_load_2d_hint(a_dst, &tmap_w, full_bar(stage), kb * BLOCK_K, n_tile * TILE_N, pol_w);
         if (!inl) tma_load_2d(a_dst + A_BYTES, &tmap_x, full_bar(stage), kb * BLOCK_K, m0);
         if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
@@ -491,7 +479,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     }
   }
 
-  if (!grouped && warp != 0) pdl_wait();
+  if (warp != 0) pdl_wait();
   if (fuse_ar) {
     // Every thread is past its dependency wait here, so all earlier launches of the stream (which advance the epoch
     // word when they finish) have completed.  The word is bumped again only after every CTA of this grid has exited.
@@ -929,21 +917,18 @@ int decode_pick_splits(int tiles, int kblocks, int num_sms, int bn, int margin, 
 
 using namespace b200;
 
-// groups > 0: M is the bound on tokens per expert and on the rows of xq, wq holds groups*N rows
 static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, const float* sw, void* y,
                             const void* residual, int M, int N, int K, int ldy, int out_fp32, int* status,
-                            int num_sms, int force_splits, const ArTail* ar, cudaStream_t stream,
-                            int groups = 0, const int* grp_offsets = nullptr, const int* grp_counts = nullptr,
-                            int x_rows = 0, const QuantProlog* qp = nullptr) {
+                            int num_sms, int force_splits, const ArTail* ar, cudaStream_t stream, const QuantProlog* qp = nullptr) {
   // Plain calls may bring several token tiles (one grid layer each; every layer streams the weights again, so this
-  // is for narrow outputs such as a router, whose tiles stay at 64 tokens so that more CTAs share the work); the grouped,
+  // is for narrow outputs such as a router, whose tiles stay at 64 tokens so that more CTAs share the work); the
   // fused-prologue and all-reduce forms take one tile.
   constexpr int MULTI_TILE_MAX_M = 4 * SWAP_MAX_M;
   if (M <= 0 || N <= 0 || K <= 0 || (K % 16) != 0) return -1;
-  if (M > ((groups > 0 || qp || ar) ? SWAP_MAX_M : MULTI_TILE_MAX_M)) return -1;
+  if (M > ((qp || ar) ? SWAP_MAX_M : MULTI_TILE_MAX_M)) return -1;
   if (qp) {
     // the quantiser CTAs park a row as floats in the pipeline's stage memory and work in whole 128-blocks
-    if (groups > 0 || force_splits > 0 || (K % 128) || K * 4 > 80 * 1024 || qp->mode < QR_PLAIN || qp->mode > QR_SWIGLU) return -1;
+    if (force_splits > 0 || (K % 128) || K * 4 > 80 * 1024 || qp->mode < QR_PLAIN || qp->mode > QR_SWIGLU) return -1;
     if (!qp->x || !qp->q || !qp->scale || !qp->flags || !qp->step) return -1;
     if ((qp->mode == QR_NORM || qp->mode == QR_ADD_NORM) && !qp->gamma) return -1;
     if (qp->mode == QR_ADD_NORM && !qp->residual) return -1;
@@ -951,15 +936,14 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
     if ((qp->ldx % 4) || (qp->ldr % 4) || (reinterpret_cast<uintptr_t>(qp->x) & 7) || (reinterpret_cast<uintptr_t>(qp->residual) & 7) ||
         (reinterpret_cast<uintptr_t>(qp->gamma) & 7)) return -2;
   }
-  if (groups > 0 && ((N % TILE_N) || !grp_offsets || !grp_counts || ar)) return -1;
   if ((reinterpret_cast<uintptr_t>(xq) & 15) || (reinterpret_cast<uintptr_t>(wq) & 15)) return -2;
   const int bn = M <= 16 ? 16 : (M <= 32 ? 32 : ((M <= SWAP_MAX_M || N <= TILE_N) ? 64 : 128));
   DecodeGemmParams p;
   p.M = M; p.N = N; p.K = K;
   p.kblocks = (K + BLOCK_K - 1) / BLOCK_K;
-  const int n_tiles = (N + TILE_N - 1) / TILE_N, m_tiles = groups > 0 ? groups : (M + bn - 1) / bn;
+  const int n_tiles = (N + TILE_N - 1) / TILE_N, m_tiles = (M + bn - 1) / bn;
   // A split whose clusters do not all fit on the GPU at once runs as two waves: twice the latency for an op that is
-  // nothing but latency.  (Grouped launches have one grid row per expert and are multi-wave by nature.)
+  // nothing but latency.
   // Up to INL_MAX_ROWS tokens the GEMM CTAs quantise their own operand (inline prologue) when a warp's share of
   // (k-block, row) pairs fits its registers; otherwise the launch carries quantiser CTAs.
   bool inl = false;
@@ -974,7 +958,7 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
   // 32 tokens, K shard 512: 12.9 us against 15.0 us with two k-blocks per CTA; B200RT_AR_MIN_KBLOCKS=2 restores that).
   static int ar_min_kb = -1;
   if (ar_min_kb < 0) { const char* e = std::getenv("B200RT_AR_MIN_KBLOCKS"); ar_min_kb = e ? std::max(1, std::atoi(e)) : 1; }
-  if (!inl) s = force_splits > 0 ? force_splits : decode_pick_splits(n_tiles * m_tiles, p.kblocks, num_sms, bn, groups > 0 ? -100000 : 1, qp ? M : 0,
+  if (!inl) s = force_splits > 0 ? force_splits : decode_pick_splits(n_tiles * m_tiles, p.kblocks, num_sms, bn, 1, qp ? M : 0,
                                                                      ar ? ar_min_kb : 2);
   if (s < 1 || s > 8) return -1;
   p.splits = s;
@@ -982,10 +966,6 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
   p.ldy = ldy; p.out_fp32 = out_fp32; p.status = status; p.limit_ns = 2000000000ull;
   p.elementwise = out_fp32 || ldy % 8 || ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(residual)) & 15);
   if (ar) p.ar = *ar; else { p.ar = ArTail{}; p.ar.enabled = 0; }
-  p.grp_offsets = groups > 0 ? grp_offsets : nullptr;
-  p.grp_counts = groups > 0 ? grp_counts : nullptr;
-  const int w_rows = groups > 0 ? groups * N : N;
-  const int xr = groups > 0 ? x_rows : M;
   if (ar) {
     // Every CTA waits for the peers, so the whole grid has to be resident at once: ask the occupancy calculator how
     // many clusters of this size fit (clusters are placed per GPC, so this is less than SMs x CTAs-per-SM / size)
@@ -1006,7 +986,7 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
   p.async_x = async_env;
   static int l2_env = -1;
   if (l2_env < 0) { const char* e = std::getenv("B200RT_L2_PREFETCH_TILES"); l2_env = e ? std::atoi(e) : 0; }
-  p.l2_prefetch = (groups > 0) ? 0 : l2_env;
+  p.l2_prefetch = l2_env;
   static int narrow_env = -1;
   if (narrow_env < 0) { const char* e = std::getenv("B200RT_GEMM_NARROW_EPI"); narrow_env = (e && e[0] == '1') ? 1 : 0; }
   p.narrow_epi = narrow_env;
@@ -1022,8 +1002,8 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
     if (m_tiles != 1) return -1;
   }
   CUtensorMap tw, tx;
-  if (make_tmap_2d_u8(&tw, wq, static_cast<uint64_t>(K), static_cast<uint64_t>(w_rows), static_cast<uint64_t>(K), TILE_N)) return -11;
-  if (make_tmap_2d_u8(&tx, xq, static_cast<uint64_t>(K), static_cast<uint64_t>(xr), static_cast<uint64_t>(K), bn)) return -12;
+  if (make_tmap_2d_u8(&tw, wq, static_cast<uint64_t>(K), static_cast<uint64_t>(N), static_cast<uint64_t>(K), TILE_N)) return -11;
+  if (make_tmap_2d_u8(&tx, xq, static_cast<uint64_t>(K), static_cast<uint64_t>(M), static_cast<uint64_t>(K), bn)) return -12;
   dim3 grid(s, n_tiles + q_rows, m_tiles);
   switch (bn) {
     case 16: return launch_decode<16, 5>(tw, tx, p, grid, stream);
@@ -1084,8 +1064,7 @@ extern "C" int b200_w8a8_gemm_decode_p(const b200_quant_prolog* prolog, const vo
                                        int num_sms, cudaStream_t stream) {
   if (!prolog) return -1;
   const QuantProlog q = to_prolog(*prolog);
-  return decode_gemm_impl(q.q, q.scale, wq, sw, y, residual, M, N, K, ldy, out_fp32, status, num_sms, 0, nullptr, stream, 0, nullptr,
-                          nullptr, 0, &q);
+  return decode_gemm_impl(q.q, q.scale, wq, sw, y, residual, M, N, K, ldy, out_fp32, status, num_sms, 0, nullptr, stream, &q);
 }
 
 // 1 if a plain call of 65 to 128 tokens and more than one channel tile is for this kernel, 0 if it is for the persistent one.  Above
@@ -1113,17 +1092,6 @@ extern "C" int b200_w8a8_gemm_decode(const void* xq, const float* sx, const void
                                      const void* residual, int M, int N, int K, int ldy, int out_fp32, int* status,
                                      int num_sms, int force_splits, cudaStream_t stream) {
   return decode_gemm_impl(xq, sx, wq, sw, y, residual, M, N, K, ldy, out_fp32, status, num_sms, force_splits, nullptr, stream);
-}
-
-// Grouped form for mixture-of-experts decode: `groups` local experts, expert e multiplies rows
-// [grp_offsets[e], +grp_counts[e]) of xq (x_rows rows in total, at most max_tokens per expert, max_tokens <= 64) by
-// wq[e*N : (e+1)*N] and writes the same rows of y.  Offsets and counts are device arrays: nothing syncs the host.
-extern "C" int b200_w8a8_gemm_decode_grouped(const void* xq, const float* sx, const void* wq, const float* sw, void* y,
-                                             int max_tokens, int x_rows, int N, int K, int ldy, int groups,
-                                             const int* grp_offsets, const int* grp_counts, int* status, int num_sms,
-                                             cudaStream_t stream) {
-  return decode_gemm_impl(xq, sx, wq, sw, y, nullptr, max_tokens, N, K, ldy, 0, status, num_sms, 0, nullptr, stream, groups,
-                          grp_offsets, grp_counts, x_rows);
 }
 
 // Row-parallel linear fused with its all-reduce: y[m,n] = sum over ranks of (xq_r . wq_r^T * sx_r * sw) (+ residual).
@@ -1158,7 +1126,7 @@ static int decode_ar_impl(const void* xq, const float* sx, const void* wq, const
     if ((N + TILE_N - 1) / TILE_N < world) ar.two_hop = 0;
   }
   if ((part_off0 % 16) || (part_off1 % 16)) return -2;
-  return decode_gemm_impl(xq, sx, wq, sw, y, residual, M, N, K, ldy, 0, status, num_sms, 0, &ar, stream, 0, nullptr, nullptr, 0, qp);
+  return decode_gemm_impl(xq, sx, wq, sw, y, residual, M, N, K, ldy, 0, status, num_sms, 0, &ar, stream, qp);
 }
 
 extern "C" int b200_w8a8_gemm_decode_ar(const void* xq, const float* sx, const void* wq, const float* sw, void* y,

@@ -91,7 +91,7 @@ class _Sig:
     b200_trace_compiled = (I, [])
     b200_trace_set = (I, [P, ctypes.c_uint])
     b200_fill_uniform_reduce = (I, [P, c_uint64, c_uint64, c_uint64, P, I, P, P, P])
-    b200_w8a8_gemm_decode_grouped = (I, [P, P, P, P, P, I, I, I, I, I, I, P, P, P, I, P])
+    b200_w8a8_gemm_experts = (I, [P, P, P, P, P, I, I, I, I, I, I, P, P, P, I, P])
     b200_w8a8_gemm_grouped = (I, [P, P, P, P, P, I, I, I, I, I, P, P, I, P, I, P])
     b200_router_topk = (I, [P, LL, I, I, I, I, P, P, P])
     b200_moe_align = (I, [P, I, I, I, I, P, P, P, P, P, P, P])

@@ -82,10 +82,10 @@ def grouped_gemm(xp: torch.Tensor, sp: torch.Tensor, wq: torch.Tensor, sw: torch
     ws = default_workspace(xp.device)
     sms = _lib.num_sms(xp.device.index)
     if w.M <= L.DECODE_MAX_M:
-        rc = _lib.lib().b200_w8a8_gemm_decode_grouped(
+        rc = _lib.lib().b200_w8a8_gemm_experts(
             xp.data_ptr(), sp.data_ptr(), wq.data_ptr(), sw.data_ptr(), y.data_ptr(), w.M, w.max_slots, N, K,
-            y.stride(0), E, w.offsets.data_ptr(), w.counts.data_ptr(), ws.status.data_ptr(), sms, _lib.stream())
-        _lib.check(rc, "w8a8_gemm_decode_grouped")
+            y.stride(0), E, w.tiles.data_ptr(), w.meta[1:].data_ptr(), ws.status.data_ptr(), sms, _lib.stream())
+        _lib.check(rc, "w8a8_gemm_experts")
     else:
         rc = _lib.lib().b200_w8a8_gemm_grouped(
             xp.data_ptr(), sp.data_ptr(), wq.data_ptr(), sw.data_ptr(), y.data_ptr(), w.max_slots, N, K, y.stride(0), E,

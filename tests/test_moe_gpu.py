@@ -179,3 +179,28 @@ def test_fp32_experts_without_rows_are_not_read():
         want = torch.stack([W.data.view(E, n, k)[e].double() @ x[i].double() for i, e in enumerate(at.tolist())])
         assert (y[:at.numel(), :n].double() - want).norm() <= 2e-6 * want.norm()
     assert ms["few"] < 0.6 * ms["all"], ms
+
+
+@pytest.mark.parametrize("one", [False, True])
+@pytest.mark.parametrize("M,k,E,N,K", [(1, 1, 1, 128, 16), (1, 8, 128, 1152, 144), (16, 3, 5, 2176, 768), (17, 2, 40, 384, 1040), (33, 4, 6, 1280, 256),
+                                       (64, 8, 128, 640, 384), (64, 2, 3, 2048, 128)])
+def test_experts_linear_of_a_decoding_mixture(M, k, E, N, K, one):
+    """Token tiles of 16, 32 and 64, one to eight channel tiles per CTA with a shorter last CTA, experts without rows, all rows at few
+    experts.  Sums are whole numbers, so only the scales (two roundings of fp32) and the store round (bf16 has eight significant bits: at most
+    2^-8)."""
+    from mojo_linuxperiments_b200.ops import moe as MO
+    g = torch.Generator(device="cuda").manual_seed(M * 131 + N)
+    ids = torch.rand((M, E), device="cuda", generator=g).argsort(-1)[:, :k].to(torch.int32)
+    if one:
+        ids = torch.arange(k, dtype=torch.int32, device="cuda").expand(M, k)
+    w = MO.moe_align(ids.contiguous(), 0, E)
+    xp = torch.randint(-127, 128, (M * k, K), dtype=torch.int8, device="cuda", generator=g)
+    wq = torch.randint(-127, 128, (E, N, K), dtype=torch.int8, device="cuda", generator=g)
+    sp, sw = torch.rand(M * k, device="cuda", generator=g), torch.rand((E, N), device="cuda", generator=g)
+    y = MO.grouped_gemm(xp, sp, wq, sw, w).double()
+    seen = 0
+    for e, (at, n) in enumerate(zip(w.offsets.tolist(), w.counts.tolist())):
+        want = (xp[at:at + n].double() @ wq[e].double().t()) * sw[e].double() * sp[at:at + n, None].double()
+        assert ((y[at:at + n] - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -22)).all()
+        seen += n
+    assert seen == M * k
