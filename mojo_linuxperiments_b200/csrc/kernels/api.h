@@ -85,6 +85,10 @@ int b200_w8a8_gemm_grouped(const void* xq, const float* sx, const void* wq, cons
                            int max_tiles, int* status, int num_sms, cudaStream_t stream);
 int b200_router_topk(const float* logits, long long ld, int M, int E, int k, int renorm, int* ids, float* wts,
                      cudaStream_t stream);
+// router_topk, moe_align and moe_gather of up to 64 tokens and 512 pairs in one launch; -30: not for calls of this size
+int b200_router_place(const float* logits, long long ld, int M, int E, int k, int renorm, int* ids, float* wts, int e0, int n_local,
+                      int* counts, int* offsets, int* slot_token, int* inv, void* tiles, int* meta, const void* xq, const float* sx, int d,
+                      void* xq_perm, float* sx_perm, cudaStream_t stream);
 int b200_moe_align(const int* ids, int M, int k, int e0, int n_local, int* counts, int* offsets, int* slot_token,
                    int* inv, void* tiles, int* meta, cudaStream_t stream);
 int b200_moe_gather(const void* xq, const float* sx, int d, const int* slot_token, const int* meta, int max_slots,
@@ -302,6 +306,10 @@ int b200_stream_rows_launch(const b200_stream_rows* r, int M, int d, int num_sms
 // ---- routing with a correction, expert groups and identity experts (moe_route.cu) ------------------------------------------
 int b200_route_grouped(const float* logits, long long ld, const float* correction, int M, int E, int top, int groups, int keep,
                        float scale, int* ids, float* weights, cudaStream_t stream);
+// the same with moe_align (experts 0 .. n_local - 1) and moe_gather_rows in one launch, as b200_router_place
+int b200_route_grouped_place(const float* logits, long long ld, const float* correction, int M, int E, int top, int groups, int keep, float scale,
+                             int* ids, float* weights, int n_local, int* counts, int* offsets, int* slot_token, int* inv, void* tiles, int* meta,
+                             const void* x, long long row_bytes, void* out, cudaStream_t stream);
 int b200_moe_gather_rows(const void* x, long long row_bytes, const int* slot_token, const int* meta, int max_slots, void* out,
                          cudaStream_t stream);
 

@@ -21,17 +21,10 @@ __device__ __forceinline__ int rg_argmax(float v, int i) {
   return static_cast<int>(__reduce_min_sync(0xffffffffu, key == best ? static_cast<unsigned>(i) : 0x7fffffffu));
 }
 
-// one warp per token; lane <-> outputs lane, lane + 32, ...
+// a warp chooses for one token; lane <-> outputs lane, lane + 32, ...; ids and weights [top] of the token; lane j < top returns choice j
 template <int EPL>
-__global__ void __launch_bounds__(32 * RG_WARPS)
-route_grouped_kernel(const float* logits, long long ld, const float* correction, int M, int E, int top, int groups, int keep,
-                     float scale, int* ids, float* weights) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tok = blockIdx.x * RG_WARPS + warp;
-  if (tok >= M) return;
-  const float* x = logits + static_cast<size_t>(tok) * ld;
+__device__ __forceinline__ int route_token(const float* x, const float* correction, int E, int top, int groups, int keep, float scale, int lane, int* ids,
+                                           float* weights) {
   float s[EPL], c[EPL];
   float mx = -INFINITY;
 #pragma unroll
@@ -84,6 +77,7 @@ route_grouped_kernel(const float* logits, long long ld, const float* correction,
       if (!(in >> i & 1u)) c[i] = -INFINITY;
   }
   unsigned taken = 0;
+  int chosen = 0;
   for (int j = 0; j < top; ++j) {
     float best = -INFINITY;
     int bi = 0x7fffffff;
@@ -93,16 +87,48 @@ route_grouped_kernel(const float* logits, long long ld, const float* correction,
       if (e < E && !(taken >> i & 1u) && (c[i] > best || (c[i] == best && e < bi))) { best = c[i]; bi = e; }
     }
     bi = rg_argmax(best, bi);
-    const size_t at = static_cast<size_t>(tok) * top + j;
 #pragma unroll
     for (int i = 0; i < EPL; ++i)
       if (lane + 32 * i == bi) {                 // the winner's lane
         taken |= 1u << i;
-        ids[at] = bi;
-        weights[at] = s[i] * scale;
+        ids[j] = bi;
+        weights[j] = s[i] * scale;
       }
-    if (bi == 0x7fffffff && lane == 0) { ids[at] = E - 1; weights[at] = 0.f; }      // nothing eligible (no number among the scores)
+    if (bi == 0x7fffffff && lane == 0) { ids[j] = E - 1; weights[j] = 0.f; }      // nothing eligible (no number among the scores)
+    if (lane == j) chosen = bi == 0x7fffffff ? E - 1 : bi;
   }
+  return chosen;
+}
+
+template <int EPL>
+__global__ void __launch_bounds__(32 * RG_WARPS)
+route_grouped_kernel(const float* logits, long long ld, const float* correction, int M, int E, int top, int groups, int keep,
+                     float scale, int* ids, float* weights) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, tok = blockIdx.x * RG_WARPS + (threadIdx.x >> 5);
+  if (tok >= M) return;
+  const size_t at = static_cast<size_t>(tok) * top;
+  route_token<EPL>(logits + static_cast<size_t>(tok) * ld, correction, E, top, groups, keep, scale, lane, ids + at, weights + at);
+}
+
+// the same with the work list and the rows (moe_rows.cuh).  What it adds to a step of 8 tokens, 4 of 28 outputs: 4.3 us, the three launches 6.0
+template <int EPL>
+__global__ void __launch_bounds__(32 * MP_WARPS)
+route_grouped_place_kernel(const float* logits, long long ld, const float* correction, int E, int groups, int keep, float scale, int* ids, float* weights,
+                           const MoePlace p) {
+  __shared__ MoePlaceShared sh;
+  pdl_launch_dependents();
+  cluster_arrive_relaxed();            // "this CTA runs"
+  pdl_wait();
+  MoePlaceRow row;
+  mp_fetch(p, row);
+  cluster_wait_acquire();
+  for (int i = 0, t; (t = mp_token(i)) < p.M; ++i)
+    mp_tell(p, sh, t, route_token<EPL>(logits + static_cast<size_t>(t) * ld, correction, E, p.k, groups, keep, scale, threadIdx.x & 31, ids + t * p.k, weights + t * p.k));
+  __syncwarp();
+  cluster_sync_all();
+  mp_place(p, sh, row);
 }
 
 // grid = most slots; rows beyond meta[0] exit
@@ -153,6 +179,24 @@ extern "C" int b200_moe_gather_rows(const void* x, long long row_bytes, const in
     launch_ex(moe_gather_rows_walk_kernel, dim3(MOE_WALK_CTAS), dim3(32 * MOE_WALK_WARPS), 0, stream, 0, static_cast<const uint8_t*>(x), row_bytes, slot_token, meta,
               max_slots, static_cast<uint8_t*>(out));
   else launch_ex(moe_gather_rows_kernel, dim3(max_slots), dim3(128), 0, stream, 0, static_cast<const uint8_t*>(x), row_bytes, slot_token, meta, static_cast<uint8_t*>(out));
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
+}
+
+// route_grouped, moe_align (experts 0 .. n_local - 1) and the row gather in one launch; -30: not for calls of this size
+extern "C" int b200_route_grouped_place(const float* logits, long long ld, const float* correction, int M, int E, int top, int groups, int keep, float scale,
+                                        int* ids, float* weights, int n_local, int* counts, int* offsets, int* slot_token, int* inv, void* tiles, int* meta,
+                                        const void* x, long long row_bytes, void* out, cudaStream_t stream) {
+  const MoePlace p{M, top, 0, n_local, counts, offsets, slot_token, inv, static_cast<int4*>(tiles), meta, static_cast<const uint8_t*>(x), row_bytes,
+                   static_cast<uint8_t*>(out), nullptr, nullptr};
+  if (!logits || !correction || !ids || !weights || E <= 0 || E > 256 || groups <= 0 || E % groups || keep <= 0 || keep > groups || top > keep * (E / groups) ||
+      !moe_place_ok(p, E)) return -30;
+  const dim3 grid(MP_CTAS), block(32 * MP_WARPS);
+  if (E <= 32) launch_ex(route_grouped_place_kernel<1>, grid, block, 0, stream, MP_CTAS, logits, ld, correction, E, groups, keep, scale, ids, weights, p);
+  else if (E <= 64) launch_ex(route_grouped_place_kernel<2>, grid, block, 0, stream, MP_CTAS, logits, ld, correction, E, groups, keep, scale, ids, weights, p);
+  else if (E <= 96) launch_ex(route_grouped_place_kernel<3>, grid, block, 0, stream, MP_CTAS, logits, ld, correction, E, groups, keep, scale, ids, weights, p);
+  else if (E <= 128) launch_ex(route_grouped_place_kernel<4>, grid, block, 0, stream, MP_CTAS, logits, ld, correction, E, groups, keep, scale, ids, weights, p);
+  else launch_ex(route_grouped_place_kernel<8>, grid, block, 0, stream, MP_CTAS, logits, ld, correction, E, groups, keep, scale, ids, weights, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }

@@ -30,9 +30,7 @@ class MoEBlock:
         cfg = self.cfg
         M = xq.shape[0]
         logits = L.w8a8_gemm(xq, sx, W["router"].qweight, W["router"].scale, out_dtype=torch.float32, narrow=True)
-        ids, wts = MO.router_topk(logits, cfg.top_k, cfg.norm_topk_prob)
-        work = MO.moe_align(ids, self.e0, self.n_local)
-        xp, sp = MO.moe_gather(xq, sx, work)
+        _, wts, work, xp, sp = MO.route_rows(logits, cfg.top_k, cfg.norm_topk_prob, self.e0, self.n_local, xq, sx)
         gu = MO.grouped_gemm(xp, sp, W["experts_gate_up"].qweight, W["experts_gate_up"].scale, work)
         hq, sh = L.act_quant(gu, mode=L.AQ_SWIGLU)
         yd = MO.grouped_gemm(hq, sh, W["experts_down"].qweight, W["experts_down"].scale, work)
@@ -68,8 +66,7 @@ class GroupedExperts:
     def __call__(self, h: torch.Tensor, W: dict) -> RW.ExpertSum:
         m = self.m
         logits = D.linear(h, W["router"], out_dtype=torch.float32)
-        ids, wts = MO.route_grouped(logits, W["correction"], m.top, m.groups, m.keep, m.scale, m.outputs)
-        work = MO.moe_align(ids, 0, m.experts)
-        u = D.linear_experts(MO.gather_rows(h, work), W["experts_up"], work, act="relu2")
+        ids, wts, work, rows = MO.route_grouped_rows(logits, W["correction"], m.top, m.groups, m.keep, m.scale, m.outputs, m.experts, h)
+        u = D.linear_experts(rows, W["experts_up"], work, act="relu2")
         y = D.linear_experts(u, W["experts_down"], work)
         return RW.ExpertSum(y, work.inv, ids, wts, m.experts, h)

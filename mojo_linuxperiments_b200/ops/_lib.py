@@ -94,6 +94,7 @@ class _Sig:
     b200_w8a8_gemm_experts = (I, [P, P, P, P, P, I, I, I, I, I, I, P, P, P, I, P])
     b200_w8a8_gemm_grouped = (I, [P, P, P, P, P, I, I, I, I, I, P, P, I, P, I, P])
     b200_router_topk = (I, [P, LL, I, I, I, I, P, P, P])
+    b200_router_place = (I, [P, LL, I, I, I, I, P, P, I, I, P, P, P, P, P, P, P, P, I, P, P, P])
     b200_moe_align = (I, [P, I, I, I, I, P, P, P, P, P, P, P])
     b200_moe_gather = (I, [P, P, I, P, P, I, P, P, P])
     b200_moe_combine = (I, [P, LL, P, P, I, I, I, P, LL, P])
@@ -112,6 +113,7 @@ class _Sig:
     b200_f32_gemm_grouped = (I, [P, LL, P, LL, I, I, I, P, P, P])
     b200_stream_rows_launch = (I, [P, I, I, I, P])
     b200_route_grouped = (I, [P, LL, P, I, I, I, I, I, F, P, P, P])
+    b200_route_grouped_place = (I, [P, LL, P, I, I, I, I, I, F, P, P, I, P, P, P, P, P, P, P, LL, P, P])
     b200_moe_gather_rows = (I, [P, LL, P, P, I, P, P])
     b200_mingru_scratch_floats = (I, [I, I, I])
     b200_mingru = (I, [P, LL, P, P, I, I, P, LL, I, P, P, P, P, I, I, P, P, LL, I, P])

@@ -74,6 +74,54 @@ def gather_rows(x: torch.Tensor, w: MoEWorkList) -> torch.Tensor:
     return out
 
 
+_NOT_THIS_SIZE = -30
+
+
+def route_rows(logits: torch.Tensor, k: int, renorm: bool, e0: int, n_local: int, xq: torch.Tensor, sx: torch.Tensor):
+    """``router_topk``, ``moe_align`` and ``moe_gather`` -> (ids, weights, work list, rows, scales): one launch for a decoding batch, the
+    three of them above 64 tokens or 512 pairs."""
+    M, E = logits.shape
+    assert logits.dtype == torch.float32 and logits.stride(1) == 1 and xq.is_contiguous()
+    w = MoEWorkList(M, k, n_local, logits.device)
+    if M <= L.DECODE_MAX_M:
+        ids = torch.empty((M, k), dtype=torch.int32, device=logits.device)
+        wts = torch.empty((M, k), dtype=torch.float32, device=logits.device)
+        xp = torch.empty((w.max_slots, xq.shape[1]), dtype=torch.int8, device=xq.device)
+        sp = torch.empty((w.max_slots,), dtype=torch.float32, device=xq.device)
+        rc = _lib.lib().b200_router_place(logits.data_ptr(), logits.stride(0), M, E, k, 1 if renorm else 0, ids.data_ptr(), wts.data_ptr(), e0, n_local,
+                                          w.counts.data_ptr(), w.offsets.data_ptr(), w.slot_token.data_ptr(), w.inv.data_ptr(), w.tiles.data_ptr(),
+                                          w.meta.data_ptr(), xq.data_ptr(), sx.data_ptr(), xq.shape[1], xp.data_ptr(), sp.data_ptr(), _lib.stream())
+        if rc != _NOT_THIS_SIZE:
+            _lib.check(rc, "router_place")
+            return ids, wts, w, xp, sp
+    ids, wts = router_topk(logits, k, renorm)
+    moe_align(ids, e0, n_local, w)
+    return (ids, wts, w) + moe_gather(xq, sx, w)
+
+
+def route_grouped_rows(logits: torch.Tensor, correction: torch.Tensor, top: int, groups: int, keep: int, scale: float, outputs: int, n_local: int,
+                       x: torch.Tensor):
+    """``route_grouped``, ``moe_align`` (experts below ``n_local``) and ``gather_rows`` -> (ids, weights, work list, rows), likewise."""
+    M = logits.shape[0]
+    assert logits.dtype == torch.float32 and logits.stride(1) == 1 and correction.dtype == torch.float32 and correction.numel() >= outputs
+    assert x.is_contiguous()
+    w = MoEWorkList(M, top, n_local, logits.device)
+    if M <= L.DECODE_MAX_M:
+        ids = torch.empty((M, top), dtype=torch.int32, device=logits.device)
+        wts = torch.empty((M, top), dtype=torch.float32, device=logits.device)
+        out = torch.empty((w.max_slots, x.shape[1]), dtype=x.dtype, device=x.device)
+        rc = _lib.lib().b200_route_grouped_place(logits.data_ptr(), logits.stride(0), correction.data_ptr(), M, outputs, top, groups, keep, float(scale),
+                                                 ids.data_ptr(), wts.data_ptr(), n_local, w.counts.data_ptr(), w.offsets.data_ptr(),
+                                                 w.slot_token.data_ptr(), w.inv.data_ptr(), w.tiles.data_ptr(), w.meta.data_ptr(), x.data_ptr(),
+                                                 x.stride(0) * x.element_size(), out.data_ptr(), _lib.stream())
+        if rc != _NOT_THIS_SIZE:
+            _lib.check(rc, "route_grouped_place")
+            return ids, wts, w, out
+    ids, wts = route_grouped(logits, correction, top, groups, keep, scale, outputs)
+    moe_align(ids, 0, n_local, w)
+    return ids, wts, w, gather_rows(x, w)
+
+
 def grouped_gemm(xp: torch.Tensor, sp: torch.Tensor, wq: torch.Tensor, sw: torch.Tensor, w: MoEWorkList) -> torch.Tensor:
     """Per local expert e: y[slots of e] = xp[slots of e] . wq[e]^T * sp * sw[e].  wq int8 [E_local, N, K]."""
     E, N, K = wq.shape

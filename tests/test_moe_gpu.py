@@ -204,3 +204,36 @@ def test_experts_linear_of_a_decoding_mixture(M, k, E, N, K, one):
         assert ((y[at:at + n] - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -22)).all()
         seen += n
     assert seen == M * k
+
+
+@pytest.mark.parametrize("grouped", [False, True])
+@pytest.mark.parametrize("M,E,k,e0,n_local,units", [(1, 128, 8, 0, 128, 1), (16, 128, 8, 0, 128, 128), (17, 100, 3, 0, 90, 257), (64, 128, 8, 32, 64, 40), (64, 24, 6, 0, 20, 300),
+                                                    (64, 130, 8, 0, 130, 8), (33, 20, 1, 5, 1, 5), (64, 24, 9, 0, 24, 4), (65, 24, 4, 0, 24, 4)])
+def test_routing_work_list_and_rows_in_one_launch(M, E, k, e0, n_local, units, grouped):
+    """Against the three launches: the same choices and weights, and a work list that says the same (slots inside an expert may differ in
+    order).  Several pairs per warp, rows longer than what a warp holds, experts elsewhere, 576 pairs and 65 tokens (the three launches)."""
+    from mojo_linuxperiments_b200.ops import moe as MO
+    g = torch.Generator(device="cuda").manual_seed(M + E)
+    e0 = 0 if grouped else e0
+    logits = torch.randn((M, E + 3), generator=g, device="cuda")[:, :E]
+    logits[:, 1] = logits[:, 0]                                  # ties
+    x = torch.randint(-127, 128, (M, 16 * units), dtype=torch.int8, device="cuda", generator=g)
+    sx = torch.rand(M, device="cuda", generator=g)
+    if grouped:
+        groups = next(n for n in (4, 5, 2, 1) if E % n == 0 and k <= E // n * 2 and n >= 2 or n == 1)
+        args = (torch.rand(E, device="cuda", generator=g), k, groups, min(2, groups), 1.5, E)
+        ids, wts, w, rows = MO.route_grouped_rows(logits, *args, n_local, x)
+        ids0, wts0 = MO.route_grouped(logits, *args)
+    else:
+        ids, wts, w, rows, s = MO.route_rows(logits, k, True, e0, n_local, x, sx)
+        ids0, wts0 = MO.router_topk(logits, k, True)
+    w0 = MO.moe_align(ids0, e0, n_local)
+    assert torch.equal(ids, ids0) and torch.equal(wts, wts0) and torch.equal(w.counts, w0.counts) and torch.equal(w.offsets, w0.offsets) and torch.equal(w.meta, w0.meta)
+    slots, nt = int(w.meta[0]), int(w.meta[1])
+    assert torch.equal(w.tiles[:nt], w0.tiles[:nt]) and torch.equal(w.inv < 0, w0.inv < 0)
+    here = w.inv.reshape(-1) >= 0
+    at = w.inv.reshape(-1)[here].long()
+    assert torch.equal(at.sort().values, torch.arange(slots, device="cuda"))
+    pair_token, pair_expert = torch.arange(M * k, device="cuda")[here] // k, ids.reshape(-1)[here].long() - e0
+    assert torch.equal(w.slot_token[at].long(), pair_token) and ((w.offsets[pair_expert] <= at) & (at < w.offsets[pair_expert + 1])).all()
+    assert torch.equal(rows[at], x[pair_token]) and (grouped or torch.equal(s[at], sx[pair_token]))
