@@ -407,3 +407,39 @@ def test_f32_linear_in_three_parts_where_it_is_not_finite():
     fine = torch.isfinite(b)
     assert ((a - b).abs() <= 1e-5 * x.abs().nan_to_num(0, 0, 0).amax(1, keepdim=True).clamp_min(1.0) * W.abs().nan_to_num(0, 0, 0).amax(1))[fine].all()
     assert torch.isnan(a[8, 9]) and fine[129, 1] and fine[0, 77]
+
+
+@pytest.mark.parametrize("H,G,dk,dv,chunk,spans", [(8, 2, 128, 128, None, [(0, 127), (0, 128), (0, 129), (37, 300)]), (6, 2, 64, 96, 200, [(0, 257), (150, 260), (5, 1)]),
+                                                   (3, 3, 40, 16, 70, [(0, 513), (64, 130)]), (16, 4, 128, 128, 512, [(300 * (i % 2), 200 + 40 * i) for i in range(12)]),
+                                                   (5, 1, 8, 128, 128, [(100, 400), (0, 256)])])
+def test_paged_prefill_attention_pairs_heads_or_query_tiles(H, G, dk, dv, chunk, spans):
+    """(first position, tokens) of portions.  Two heads of a KV head share a CTA; an odd number of them: two query tiles, the second of which
+    may start in a later chunk.  Tile edges, portions that continue, more items than CTAs.  bf16 weights and outputs: 2^-8 of values up to 4."""
+    from mojo_linuxperiments_b200.ops import attention as A
+    ps, B = 16, len(spans)
+    g = torch.Generator(device=DEV).manual_seed(dk + B)
+    per = max((a + n + ps - 1) // ps for a, n in spans)
+    cache = A.PagedKVCache(B * per + 3, G, ps, DEV, dk=dk, dv=dv, dtype=torch.bfloat16)
+    cache.data.normal_(generator=g)
+    table = torch.randperm(B * per, generator=torch.Generator().manual_seed(1)).to(torch.int32).view(B, per).to(DEV)
+    lens = [n for _, n in spans]
+    pos = torch.cat([torch.arange(a, a + n, dtype=torch.int32) for a, n in spans]).to(DEV)
+    sid = torch.cat([torch.full((n,), b, dtype=torch.int32) for b, (_, n) in enumerate(spans)]).to(DEV)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32).to(DEV)
+    q = torch.randn((sum(lens), H * dk), generator=g, device=DEV).to(torch.bfloat16)
+    sink, gate = torch.randn(H, generator=g, device=DEV), torch.randn((sum(lens), 8 * ((H + 7) // 8)), generator=g, device=DEV).to(torch.bfloat16)
+    out = torch.full((sum(lens), H * dv), float("nan"), dtype=torch.bfloat16, device=DEV)
+    A.attn_prefill_paged(q, H, pos, sid, cu, max(lens), cache, table, A.attn_spec(dk ** -0.5, chunk=chunk, sink=sink, gate=gate), out)
+    _ok()
+    for b, (a, n) in enumerate(spans):
+        at, end = cu[b].item(), a + n
+        j = torch.arange(end, device=DEV)
+        k, v = (t[table[b].long()[j // ps], :, j % ps].double().repeat_interleave(H // G, 1) for t in (cache.keys(), cache.values()))
+        i = torch.arange(a, end, device=DEV)
+        seen = j[None] <= i[:, None]
+        if chunk:
+            seen &= j[None] // chunk == i[:, None] // chunk
+        s = torch.einsum("ihd,jhd->hij", q[at:at + n].double().view(n, H, dk), k) * dk ** -0.5
+        s = torch.cat([s.masked_fill(~seen, -float("inf")), sink.double()[:, None, None].expand(H, n, 1)], 2).softmax(-1)[..., :-1]
+        want = torch.einsum("hij,jhd->ihd", s, v) * torch.sigmoid(gate[at:at + n, :H].double())[..., None]
+        assert (out[at:at + n].double() - want.reshape(n, H * dv)).abs().max().item() < 1.6e-2, (b, a, n)
