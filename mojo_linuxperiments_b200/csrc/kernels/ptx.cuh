@@ -372,6 +372,13 @@ __device__ __forceinline__ void st_async_cluster_v4(uint32_t addr, uint32_t a, u
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
                ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d), "r"(mbar) : "memory");
 }
+__device__ __forceinline__ void st_async_cluster_u32(uint32_t addr, uint32_t v, uint32_t mbar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(mbar) : "memory");
+}
+// shared memory of this CTA -> of a CTA of the cluster, counted in bytes on a barrier there (all on 16 bytes)
+__device__ __forceinline__ void bulk_copy_cluster(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t mbar) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(src), "r"(bytes), "r"(mbar) : "memory");
+}
 // The two halves of the cluster barrier, for hiding its latency: every thread of every CTA arrives once and later
 // waits once per phase.  The relaxed arrive orders nothing (use it for "every CTA of the cluster has started").
 // The barrier instructions are the .aligned forms, defined only where all lanes of a warp execute them together: lanes that came

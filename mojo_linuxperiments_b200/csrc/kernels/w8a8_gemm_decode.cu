@@ -12,8 +12,8 @@
 //   * each CTA runs the usual TMA -> tcgen05.mma.kind::i8 -> TMEM pipeline (weights are the 128-row A operand, the
 //     token tile of BN in {16,32,64,128} rows is the B operand);
 //   * the S partial accumulators are combined through distributed shared memory: every CTA sends, for each of
-//     the S row slices of the tile, its int32 partial to the CTA that owns the slice (16-byte st.shared::cluster
-//     into an exchange buffer of its own, so nobody waits for a pipeline to drain), the cluster synchronises once,
+//     the S row slices of the tile, its int32 partial to the CTA that owns the slice (runs of 128 bytes, or one bulk copy, into
+//     an exchange buffer of its own, so nobody waits for a pipeline to drain), a CTA goes on when it has its bytes,
 //     and each CTA reduces and writes 128/S channels.  No global scratch, no atomics.  The "every CTA of the cluster
 //     runs" barrier that distributed shared memory needs is arrived at when the kernel starts and waited for just
 //     before the exchange, so its latency hides behind the weight stream.
@@ -150,9 +150,14 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   constexpr int TMEM_COLS = BN < 32 ? 32 : BN;
   constexpr uint32_t IDESC = umma_idesc_i8(TILE_N, BN);
-  constexpr int XS = BN + 4;                      // words per channel row of the exchange buffer (16-byte aligned rows)
+  // How partial sums travel to the CTA that finishes them.  Up to 16 tokens straight from the registers, a warp's 32 channels of a token as
+  // one run of 128 bytes; from 17 on staged in the idle pipeline and sent as one bulk copy per owner.  (16 bytes of a channel's
+  // tokens per lane, 32 runs per instruction | now, steps of four layers, us: one sequence 265 | 260, 7 x 600 305 | 298, 32 x 200 321 | 312,
+  // 60 x 100 433 | 424, 100 x 64 484 | 473; with runs of 128 bytes 32 x 200 takes 319 and 60 x 100 440, with bulk copies one sequence 264.)
+  constexpr bool BULK = BN >= 32;
+  constexpr int XS = BN + 4;                      // sizes the exchange buffer
   constexpr int EX_ROWS = TILE_N + 16;            // S senders x (slice of at most 2 * ceil(64 / S) channels) <= 128 + 2 S
-  constexpr int EX_BYTES = XCH ? EX_ROWS * XS * 4 : 0;      // [sender][channel of the slice][token]
+  constexpr int EX_BYTES = XCH ? EX_ROWS * XS * 4 : 0;      // [sender][token][channel of the slice]
   static_assert(STAGES * STAGE_BYTES >= BN * TILE_N * 4, "the staging buffer of the all-reduce tail aliases the pipeline stages");
 
   pdl_launch_dependents();     // the next kernel may be scheduled: it only reads our output after its own pdl_wait
@@ -222,11 +227,10 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   const uint32_t tmem_base = *tmem_slot;
   const bool async_x = S > 1 && p.async_x != 0;
   if (async_x && threadIdx.x == 0) {
-    // every CTA of the cluster (this one included) sends its partial of this CTA's slice: whole token chunks, 4 bytes
-    // each.  Expected before this CTA announces that it runs, so no sender's bytes can come first.
-    constexpr int CHX = (BN >= 32) ? 32 : 16;
+    // every CTA of the cluster (this one included) sends its partial of this CTA's slice, 4 bytes per token and channel.  Expected before
+    // this CTA announces that it runs, so no sender's bytes can come first.
     const int my_cw = 2 * ((64 * (rank + 1) + S - 1) / S) - 2 * ((64 * rank + S - 1) / S);
-    mbar_expect_tx(xch_bar, static_cast<uint32_t>(S * my_cw * ((rows_valid + CHX - 1) / CHX) * CHX * 4));
+    mbar_expect_tx(xch_bar, static_cast<uint32_t>(S * my_cw * (BULK ? (rows_valid + 1) & ~1 : rows_valid) * 4));
   }
   if (S > 1) cluster_arrive_relaxed();          // "this CTA runs": waited for just before the exchange
 
@@ -587,16 +591,50 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   } else {
     cluster_wait_acquire();                                 // every CTA of the cluster runs: its shared memory exists
     if (threadIdx.x == 64) B200_TRACE(TK_GEMM_DECODE, 5);
-    if (epi) {
-      // exchange buffer in the owner CTA: [sender][channel in the owner's slice][token] int32, XS words per channel row
+    if (BULK && async_x) {
+      // staged here as [owner][token][channel of the owner's slice], then one copy per owner
+      const int jp = (jmax + 1) & ~1;                       // copies of 16 bytes: slices are even
+      const uint32_t stage = smem_base + BN * TILE_N * 4;   // behind the staging of the all-reduce tail; the pipeline is idle
+      if (epi) {
+        const int owner = ((row >> 1) * S) >> 6, row_in = row - slice0(owner);
+        const int cw_owner = slice0(owner + 1) - slice0(owner);
+        const uint32_t mine = stage + 4u * static_cast<uint32_t>(jp * slice0(owner) + row_in);
+        const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+#pragma unroll 1
+        for (int c = 0; c < BN / CH; ++c) {
+          if (c * CH >= jmax) break;
+          uint32_t r[CH];
+          if (acc_ok) {
+            if constexpr (CH == 32) tmem_ld_x32(t_addr + c * CH, r); else tmem_ld_x16(t_addr + c * CH, r);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int j = 0; j < CH; ++j) r[j] = 0u;
+          }
+#pragma unroll
+          for (int j = 0; j < CH; ++j)
+            if (c * CH + j < jmax) asm volatile("st.shared.u32 [%0], %1;" ::"r"(mine + 4u * static_cast<uint32_t>((c * CH + j) * cw_owner)), "r"(r[j]) : "memory");
+        }
+        fence_proxy_async_smem();
+        named_bar_sync(1, 128);
+        if (et < S) {
+          const int cw_o = slice0(et + 1) - slice0(et);
+          const uint32_t bytes = 4u * static_cast<uint32_t>(jp * cw_o);
+          bulk_copy_cluster(mapa_shared(smem_u32(ex), static_cast<uint32_t>(et)) + rank * bytes, stage + 4u * static_cast<uint32_t>(jp * slice0(et)), bytes,
+                            mapa_shared(xch_bar, static_cast<uint32_t>(et)));
+        }
+      }
+    } else if (epi) {
+      // exchange buffer in the owner CTA: [sender][token][channel in the owner's slice] int32, so that a warp's 32 channels of a token
+      // travel as one run of 128 bytes (16 bytes of a channel's tokens per lane, 32 runs per instruction, before)
       const int owner = ((row >> 1) * S) >> 6, row_in = row - slice0(owner);
       const int cw_owner = slice0(owner + 1) - slice0(owner);
-      const uint32_t remote = mapa_shared(smem_u32(ex), static_cast<uint32_t>(owner)) +
-                              4u * static_cast<uint32_t>((rank * cw_owner + row_in) * XS);
+      const uint32_t remote = mapa_shared(smem_u32(ex), static_cast<uint32_t>(owner)) + 4u * static_cast<uint32_t>(rank * jmax * cw_owner + row_in);
       const uint32_t remote_bar = mapa_shared(xch_bar, static_cast<uint32_t>(owner));
       const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
 #pragma unroll 1
       for (int c = 0; c < BN / CH; ++c) {
+        if (c * CH >= jmax) break;                          // token rows beyond the batch are never read back
         uint32_t r[CH];
         if (acc_ok) {
           if constexpr (CH == 32) tmem_ld_x32(t_addr + c * CH, r); else tmem_ld_x16(t_addr + c * CH, r);
@@ -605,11 +643,11 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
 #pragma unroll
           for (int j = 0; j < CH; ++j) r[j] = 0u;           // empty K range (or aborted): contributes nothing
         }
-        if (c * CH < jmax) {                                // token rows beyond the batch are never read back
 #pragma unroll
-          for (int j = 0; j < CH; j += 4) {
-            if (async_x) st_async_cluster_v4(remote + 4u * (c * CH + j), r[j], r[j + 1], r[j + 2], r[j + 3], remote_bar);
-            else st_shared_cluster_v4(remote + 4u * (c * CH + j), r[j], r[j + 1], r[j + 2], r[j + 3]);
+        for (int j = 0; j < CH; ++j) {
+          if (c * CH + j < jmax) {
+            const uint32_t at = remote + 4u * static_cast<uint32_t>((c * CH + j) * cw_owner);
+            if (async_x) st_async_cluster_u32(at, r[j], remote_bar); else st_shared_cluster_u32(at, r[j]);
           }
         }
       }
@@ -618,61 +656,42 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     tc_fence_before();
     bool x_ok = true;
     if (async_x) {
-      cluster_arrive_relaxed();      // "my stores are issued": waited for just before this CTA leaves (below), so that no
-                                     // CTA exits while a peer may still write into it
+      // "my stores are issued" (copies: "what I was sent has arrived"): waited for just before this CTA leaves (below), so that no CTA exits
+      // while a peer may still write into it (or read from it)
+      if (!BULK) cluster_arrive_relaxed();
       x_ok = mbar_wait(xch_bar, 0, abort_flag, p.status, (ST_TIMEOUT_SMEM_FULL | (2 << 8)), limit);
+      if (BULK) { __syncwarp(); cluster_arrive_relaxed(); }
     } else {
       cluster_sync_all();
     }
     if (threadIdx.x == 64) B200_TRACE(TK_GEMM_DECODE, 6);
     if (x_ok) {
-      // All six warps finish blocks of 4 tokens x 8 channel pairs: shared-memory reads spread over the banks (2-way
-      // conflicts at worst) and every token row gets 32 contiguous bytes, i.e. whole sectors.  With one warp per
-      // scheduler every instruction's latency is exposed, so the loop avoids integer division and works on two
-      // independent blocks at a time (all loads first, then the arithmetic and the stores).
-      const int pairs = cw >> 1, jt_n = (jmax + 3) >> 2, blocks = jt_n * ((pairs + 7) >> 3);
-      const int sw_off = n_base - n_tile * TILE_N;
-      const uint32_t inv_jt = (65536u + jt_n - 1) / jt_n;            // blk / jt_n == (blk * inv_jt) >> 16 for blk < 4096
-      const int lj = lane & 3, lp = lane >> 2;
-      constexpr int NWARP = GEMM_THREADS / 32;
-      constexpr int UB = 3;                       // blocks per round: with the sender loop unrolled, all their loads fly together
-      for (int blk0 = warp; blk0 < blocks; blk0 += UB * NWARP) {
-        int32_t a[UB][2];
-        int jj[UB], rr[UB];
-        bool on[UB];
-#pragma unroll
-        for (int u = 0; u < UB; ++u) {
-          const int blk = blk0 + u * NWARP;
-          const int pt = static_cast<int>((static_cast<uint32_t>(blk) * inv_jt) >> 16), jt = blk - pt * jt_n;
-          jj[u] = 4 * jt + lj;
-          rr[u] = 2 * (8 * pt + lp);
-          on[u] = blk < blocks && jj[u] < jmax && rr[u] < cw;
-          a[u][0] = 0; a[u][1] = 0;
-        }
-        int32_t ld[UB][8][2];
+      // All six warps finish channel pairs, neighbouring lanes neighbouring pairs of a token.  With one warp per scheduler every
+      // instruction's latency is exposed, so the loop avoids integer division and works on three independent pairs at a time (all loads
+      // first, then the arithmetic and the stores).
+      const int pairs = cw >> 1, todo = pairs * jmax, per_sender = pairs * (BULK && async_x ? (jmax + 1) & ~1 : jmax), sw_off = n_base - n_tile * TILE_N;
+      const uint32_t inv_pairs = ((1u << 20) + pairs - 1) / pairs;     // i / pairs == (i * inv_pairs) >> 20 for i < 8,192 and up to 64 pairs
+      constexpr int UB = 3;                       // pairs per round: with the sender loop unrolled, all their loads fly together
+      for (int i0 = threadIdx.x; i0 < todo; i0 += UB * GEMM_THREADS) {
+        int2 ld[UB][8];
 #pragma unroll
         for (int u = 0; u < UB; ++u)
 #pragma unroll
           for (int sdr = 0; sdr < 8; ++sdr) {
-            ld[u][sdr][0] = 0; ld[u][sdr][1] = 0;
-            if (on[u] && sdr < S) {
-              ld[u][sdr][0] = ex[(sdr * cw + rr[u]) * XS + jj[u]];
-              ld[u][sdr][1] = ex[(sdr * cw + rr[u] + 1) * XS + jj[u]];
-            }
+            const int i = i0 + u * GEMM_THREADS;
+            ld[u][sdr] = i < todo && sdr < S ? *reinterpret_cast<const int2*>(ex + 2 * (sdr * per_sender + i)) : make_int2(0, 0);
           }
 #pragma unroll
-        for (int u = 0; u < UB; ++u)
-#pragma unroll
-          for (int sdr = 0; sdr < 8; ++sdr) { a[u][0] += ld[u][sdr][0]; a[u][1] += ld[u][sdr][1]; }
-#pragma unroll
         for (int u = 0; u < UB; ++u) {
-          if (!on[u]) continue;
-          const int n = n_base + rr[u];
-          const float sxj = sx_s[jj[u]];
-          const float v0 = scaled<BN>(a[u][0], sw_s[sw_off + rr[u]], sxj, p.elementwise);
-          const float v1 = scaled<BN>(a[u][1], sw_s[sw_off + rr[u] + 1], sxj, p.elementwise);
-          if (n + 1 < p.N) emit2(sink, m0 + jj[u], n, v0, v1);
-          else if (n < p.N) emit1(sink, m0 + jj[u], n, v0);
+          const int i = i0 + u * GEMM_THREADS;
+          if (i >= todo) break;
+          const int j = static_cast<int>((static_cast<uint32_t>(i) * inv_pairs) >> 20), r = 2 * (i - j * pairs), n = n_base + r;
+          int a0 = 0, a1 = 0;
+#pragma unroll
+          for (int sdr = 0; sdr < 8; ++sdr) { a0 += ld[u][sdr].x; a1 += ld[u][sdr].y; }
+          const float v0 = scaled<BN>(a0, sw_s[sw_off + r], sx_s[j], p.elementwise), v1 = scaled<BN>(a1, sw_s[sw_off + r + 1], sx_s[j], p.elementwise);
+          if (n + 1 < p.N) emit2(sink, m0 + j, n, v0, v1);
+          else if (n < p.N) emit1(sink, m0 + j, n, v0);
         }
       }
       if (threadIdx.x == 64) B200_TRACE(TK_GEMM_DECODE, 11);
@@ -1075,7 +1094,7 @@ extern "C" int b200_w8a8_gemm_decode_p(const b200_quant_prolog* prolog, const vo
 // (20,480 to 37,888 channels); above that both take several rounds and the persistent kernel's double-buffered ones are shorter.
 // Measured, this kernel | the persistent one, us at 65 and at 128 tokens (bf16 results):
 //   512 x 1,024 7.0, 9.2 | 5.8, 5.8       1,024 x 4,096 7.8, 9.6 | 13.0, 13.1     4,096 x 2,048 9.6, 12.0 | 8.8, 8.9
-//   4,096 x 4,096 10.9, 13.3 | 13.3, 13.3  4,096 x 14,336 18.0, 20.3 | 35.2, 35.5  6,144 x 4,096 14.2, 17.8 | 13.5, 13.7
+//   4,096 x 4,096 9.7, 13.3 | 13.3, 13.3   4,096 x 14,336 16.6, 19.8 | 35.2, 35.5  6,144 x 4,096 13.0, 17.0 | 13.5, 13.7
 //   8,192 x 8,192 20.3, 23.8 | 22.5, 22.5  12,288 x 4,096 18.3, 19.8 | 14.9, 15.1  28,672 x 4,096 24.0, 24.8 | 25.8, 25.4
 //   57,344 x 4,096 48.0, 49.3 | 45.7, 45.4  128,256 x 4,096 98, 117 | 86, 94
 // Over 24 widths x 8 lengths x 3 numbers of tokens the choice is at most 4 % slower than the better one.  Where the persistent kernel

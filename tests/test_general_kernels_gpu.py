@@ -443,3 +443,20 @@ def test_paged_prefill_attention_pairs_heads_or_query_tiles(H, G, dk, dv, chunk,
         s = torch.cat([s.masked_fill(~seen, -float("inf")), sink.double()[:, None, None].expand(H, n, 1)], 2).softmax(-1)[..., :-1]
         want = torch.einsum("hij,jhd->ihd", s, v) * torch.sigmoid(gate[at:at + n, :H].double())[..., None]
         assert (out[at:at + n].double() - want.reshape(n, H * dv)).abs().max().item() < 1.6e-2, (b, a, n)
+
+
+@pytest.mark.parametrize("splits", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 31, 33, 63, 64, 65, 99, 128])
+def test_w8a8_decode_exchange(M, splits):
+    """Partial sums of every split, odd and even numbers of tokens, slices that are no multiple of four channels, a last tile that is partly
+    filled: whole numbers until the scales (two fp32 roundings) and the store (bf16, 2^-8)."""
+    from mojo_linuxperiments_b200.ops import linear as L
+    g = torch.Generator(device=DEV).manual_seed(M * 8 + splits)
+    N, K = 328, 1168
+    x = torch.randint(-127, 128, (M, K), dtype=torch.int8, device=DEV, generator=g)
+    w = torch.randint(-127, 128, (N, K), dtype=torch.int8, device=DEV, generator=g)
+    sx, sw = torch.rand(M, device=DEV, generator=g), torch.rand(N, device=DEV, generator=g)
+    want = (x.double() @ w.double().t()) * sx.double()[:, None] * sw.double()
+    y = L.w8a8_gemm(x, sx, w, sw, force_mode=2, force_splits=splits)
+    _ok()
+    assert ((y.double() - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -22)).all()
