@@ -34,14 +34,16 @@ struct BfDecodeParams {
 
 // first channel (of 128) that cluster rank r finishes: slices are multiples of four channels
 __host__ __device__ __forceinline__ int bd_slice0(int r, int S) { return 4 * ((32 * r + S - 1) / S); }
-// exchange rows: S senders x padded slice, at most 168 floats per token (S = 7: 24 x 7)
-constexpr int BD_XROW = 168;
+// exchange rows: S senders x padded slice, at most 144 floats per token (S = 6: 24 x 6)
+constexpr int BD_XROW = 144;
 
+// Two CTAs per SM for every number of tokens: with one CTA and six stages of the 64-token form a step of eight layers took 585 us at 40 x 300, with two
+// and three stages 545.
 template <int BN, int STAGES>
 constexpr int bd_smem_bytes() { return STAGES * (128 + BN) * 128 + BN * BD_XROW * 4 + 1024 + 256; }
 
 template <int BN, int STAGES>
-__global__ void __launch_bounds__(GEMM_THREADS, BN == 64 ? 1 : 2)
+__global__ void __launch_bounds__(GEMM_THREADS, 2)
 bf16_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                         const __grid_constant__ BfDecodeParams p) {
   constexpr int A_BYTES = 128 * 128, B_BYTES = BN * 128, STAGE_BYTES = A_BYTES + B_BYTES;
@@ -52,7 +54,7 @@ bf16_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  float* ex = reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES);                 // [S][BN][cw + 4]
+  float* ex = reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES);                 // [S][BN][cw]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES + BN * BD_XROW * 4);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -136,7 +138,7 @@ bf16_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     }
     __syncwarp();
   }
-  const int s0 = bd_slice0(rank, S), cw = bd_slice0(rank + 1, S) - s0, cwp = cw + 4, quads = cw >> 2;
+  const int s0 = bd_slice0(rank, S), cw = bd_slice0(rank + 1, S) - s0, cwp = cw, quads = cw >> 2;
   // Residual form: the norm's columns and the old residual of a thread's first four channels are asked for ahead of the exchange, not
   // behind it (2,048 channels of 12 tokens end 0.4 us earlier: a decode step of eight layers 376 -> 369 us).  The
   // epilogue warps come first in that order: warps 0 and 1 arrive when their loops have ended.
@@ -159,7 +161,7 @@ bf16_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   if (S > 1) cluster_wait_acquire();            // every CTA of the cluster runs: its shared memory exists
   if (warp >= 2) {
     const int owner = (row >> 2) * S / 32;      // the rank whose slice holds this channel
-    const int cwp = bd_slice0(owner + 1, S) - bd_slice0(owner, S) + 4;
+    const int cwp = bd_slice0(owner + 1, S) - bd_slice0(owner, S);
     const uint32_t local = smem_u32(ex) + 4u * static_cast<uint32_t>(rank * BN * cwp + row - bd_slice0(owner, S));
     const uint32_t remote = mapa_shared(local, static_cast<uint32_t>(owner));
     const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
@@ -257,7 +259,7 @@ static int bf16_decode_any(const void* x, long long ldx, const void* w, long lon
     double best = 0;
     const int busy = lists && g->expected > 0 && g->expected < g->groups ? g->expected : (lists ? g->groups : z);
     for (int s = 1; s <= 8 && s <= p.kblocks; ++s) {
-      const int clusters = n_tiles * busy, res = bd_resident(s, num_sms, bn == 64 ? 1 : 2);
+      const int clusters = n_tiles * busy, res = bd_resident(s, num_sms, 2);
       const double cost = static_cast<double>((clusters + res - 1) / res) * ((p.kblocks + s - 1) / s + 6 + (s > 1 ? 1 : 0));
       if (splits == 0 || cost < best) { best = cost; splits = s; }
     }
@@ -272,7 +274,7 @@ static int bf16_decode_any(const void* x, long long ldx, const void* w, long lon
   switch (bn) {
     case 16: return launch_bf16_decode<16, 5>(tw, tx, p, grid, stream);
     case 32: return launch_bf16_decode<32, 4>(tw, tx, p, grid, stream);
-    default: return launch_bf16_decode<64, 6>(tw, tx, p, grid, stream);
+    default: return launch_bf16_decode<64, 3>(tw, tx, p, grid, stream);
   }
 }
 

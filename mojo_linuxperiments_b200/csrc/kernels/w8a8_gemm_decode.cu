@@ -4,8 +4,8 @@
 //
 // The op is bound by the bytes of Wq, so the grid is shaped for bandwidth, not for the tensor core:
 //   * one CTA = 128 output channels x (K / S) of the reduction; the S CTAs of a cluster share one output tile;
-//   * shared memory is sized for two co-resident CTAs per SM (up to 32 tokens; the 64-token form takes the SM alone
-//     with a deeper pipeline), which keeps > 150 KB of TMA loads in flight per SM and lets CTAs of different tiles
+//   * shared memory is sized for two co-resident CTAs per SM (up to 64 tokens: with one CTA and seven stages the 64-token form took 29 us for
+//     28,672 x 4,096 at 40 tokens, with two and three stages each 22), which keeps 140 KB of TMA loads and more in flight per SM and lets CTAs of different tiles
 //     overlap head and tail.  The occupancy calculator answers "1 CTA per SM" for every kernel that allocates tensor
 //     memory (tcgen05.alloc), whatever its other resources; in-kernel time stamps show two CTAs per SM running, so
 //     the host doubles the calculator's cluster counts for the two-CTA forms;
@@ -129,6 +129,7 @@ __device__ __forceinline__ int inl_div(int u, int m) {
 // inline prologue: [4 warps][4 rows][2] partial statistics of this CTA + [8 senders][4 rows][4] of the cluster
 constexpr int STAT_BYTES = (32 + 128) * 4;
 constexpr int INL_MAX_ROWS = 4;       // token rows the inline prologue handles
+constexpr int QUANT_ROW_BYTES = 80 * 1024;
 constexpr int INL_UNITS = 8;          // (k-block, row) pairs per quantising warp: their rotated values stay in registers
 
 // dynamic shared memory: pipeline stages, split-K exchange buffer, channel / token scales, barriers, alignment slack
@@ -142,7 +143,7 @@ constexpr int decode_smem_bytes(int bn, int stages, bool xch = true) {
 // 65 to 128 tokens: the persistent kernel's tiles of 128 tokens x 64 to 256 channels leave most SMs idle or run in two rounds;
 // which of the two kernels takes a call is decided in b200_w8a8_gemm_decode_takes.
 template <int BN, int STAGES, bool XCH = true>
-__global__ void __launch_bounds__(GEMM_THREADS, ((BN >= 64 && XCH) ? 1 : 2))
+__global__ void __launch_bounds__(GEMM_THREADS, ((BN > 64 && XCH) ? 1 : 2))
 w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                         const DecodeGemmParams p) {
   constexpr int A_BYTES = TILE_N * BLOCK_K;
@@ -158,7 +159,10 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   constexpr int XS = BN + 4;                      // sizes the exchange buffer
   constexpr int EX_ROWS = TILE_N + 16;            // S senders x (slice of at most 2 * ceil(64 / S) channels) <= 128 + 2 S
   constexpr int EX_BYTES = XCH ? EX_ROWS * XS * 4 : 0;      // [sender][token][channel of the slice]
-  static_assert(STAGES * STAGE_BYTES >= BN * TILE_N * 4, "the staging buffer of the all-reduce tail aliases the pipeline stages");
+  static_assert(STAGES * STAGE_BYTES >= BN * TILE_N * (XCH ? 8 : 4), "the staging of the all-reduce tail, and behind it that of the exchange, alias the pipeline stages");
+  // a quantiser CTA parks a row of up to QUANT_ROW_BYTES from the first stage on, if need be into the exchange buffer, and needs a few words behind it
+  constexpr int QUANT_WORDS_AT = STAGES * STAGE_BYTES > QUANT_ROW_BYTES ? STAGES * STAGE_BYTES : QUANT_ROW_BYTES;
+  static_assert(!XCH || QUANT_WORDS_AT + 1024 <= STAGES * STAGE_BYTES + EX_BYTES, "the quantiser's row and words fit");
 
   pdl_launch_dependents();     // the next kernel may be scheduled: it only reads our output after its own pdl_wait
   extern __shared__ uint8_t smem_raw[];
@@ -192,7 +196,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     const int qrow = blockIdx.y * p.splits + static_cast<int>(cluster_ctarank());
     if (qrow < p.M) {
       const uint32_t ticket = quant_ticket(p.qp);
-      quant_row_cta<GEMM_THREADS / 32>(p.qp, qrow, p.K, reinterpret_cast<float*>(smem), reinterpret_cast<float*>(smem + STAGES * STAGE_BYTES));
+      quant_row_cta<GEMM_THREADS / 32>(p.qp, qrow, p.K, reinterpret_cast<float*>(smem), reinterpret_cast<float*>(smem + QUANT_WORDS_AT));
       __syncthreads();                            // the release below is cumulative over what this barrier orders
       if (threadIdx.x == 0) { st_release_gpu(p.qp.flags + qrow, ticket); B200_TRACE(TK_GEMM_DECODE, 22); }
     }
@@ -897,7 +901,7 @@ static int max_resident_clusters(int s) {
 
 // CTAs of the decode GEMM one SM really holds: two when twice the shared memory (plus the per-CTA reservation) fits
 static int ctas_per_sm(int bn) {
-  const int smem = bn <= 16 ? decode_smem_bytes(16, 5) : (bn <= 32 ? decode_smem_bytes(32, 4) : (bn <= 64 ? decode_smem_bytes(64, 7) : decode_smem_bytes(128, 4)));
+  const int smem = bn <= 16 ? decode_smem_bytes(16, 5) : (bn <= 32 ? decode_smem_bytes(32, 4) : (bn <= 64 ? decode_smem_bytes(64, 3) : decode_smem_bytes(128, 4)));
   return 2 * (smem + 1024) <= 228 * 1024 ? 2 : 1;
 }
 
@@ -905,17 +909,21 @@ static int resident_clusters(int bn, int s) {
   return resident_clusters_reported(bn, s) * ctas_per_sm(bn);
 }
 
+// Clusters that a launch whose CTAs wait for one another may count on: the 64-token form's two CTAs fill an SM's shared memory to the last
+// 256 bytes, so there the calculator's answer stands.
+static int waiting_clusters(int bn, int s) { return bn == 64 ? resident_clusters_reported(bn, s) : resident_clusters(bn, s); }
+
 static int resident_clusters_reported(int bn, int s) {
   switch (bn) {
     case 16: return max_resident_clusters<16, 5>(s);
     case 32: return max_resident_clusters<32, 4>(s);
-    case 64: return max_resident_clusters<64, 7>(s);
+    case 64: return max_resident_clusters<64, 3>(s);
     default: return max_resident_clusters<128, 4>(s);
   }
 }
 
 // Split along K: the largest cluster size (1..8, any value: slices need not divide the tile evenly) whose grid of
-// tiles x S CTAs (a) fits the SMs (two CTAs each for up to 32 tokens), (b) leaves every CTA at least two k-blocks, and (c) is resident at
+// tiles x S CTAs (a) fits the SMs (two CTAs each for up to 64 tokens), (b) leaves every CTA at least two k-blocks, and (c) is resident at
 // once according to the occupancy query, with `margin` spare clusters.
 // quant_rows > 0: the launch also carries ceil(quant_rows / S) clusters of quantiser CTAs.
 // min_kb: fewest k-blocks a CTA should keep.
@@ -947,7 +955,7 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
   if (M > ((qp || ar) ? SWAP_MAX_M : MULTI_TILE_MAX_M)) return -1;
   if (qp) {
     // the quantiser CTAs park a row as floats in the pipeline's stage memory and work in whole 128-blocks
-    if (force_splits > 0 || (K % 128) || K * 4 > 80 * 1024 || qp->mode < QR_PLAIN || qp->mode > QR_SWIGLU) return -1;
+    if (force_splits > 0 || (K % 128) || K * 4 > QUANT_ROW_BYTES || qp->mode < QR_PLAIN || qp->mode > QR_SWIGLU) return -1;
     if (!qp->x || !qp->q || !qp->scale || !qp->flags || !qp->step) return -1;
     if ((qp->mode == QR_NORM || qp->mode == QR_ADD_NORM) && !qp->gamma) return -1;
     if (qp->mode == QR_ADD_NORM && !qp->residual) return -1;
@@ -969,7 +977,7 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
   int s = 0;
   if (qp && M <= INL_MAX_ROWS && qp->allow_inline && !(qp->mode == QR_ADD_NORM && (!qp->residual_out || qp->residual_out == qp->residual))) {
     s = decode_pick_splits(n_tiles * m_tiles, p.kblocks, num_sms, bn, 1, 0);
-    if (ar) while (s >= 1 && n_tiles * m_tiles + 1 > resident_clusters(bn, s)) --s;
+    if (ar) while (s >= 1 && n_tiles * m_tiles + 1 > waiting_clusters(bn, s)) --s;
     if (s >= 1 && (((p.kblocks + s - 1) / s + 3) / 4) * M <= INL_UNITS) inl = true;
   }
   // With the all-reduce tail every CTA also pushes, polls and sums its slice of the output: a launch of few CTAs (the
@@ -990,7 +998,7 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
     // many clusters of this size fit (clusters are placed per GPC, so this is less than SMs x CTAs-per-SM / size)
     // and narrow the split until the grid fits, keeping a margin of one cluster.
     if ((N % 8) || (ldy % 8) || out_fp32) return -2;
-    while (s >= 1 && n_tiles * m_tiles + ((qp && !inl) ? (M + s - 1) / s : 0) + 1 > resident_clusters(bn, s)) --s;
+    while (s >= 1 && n_tiles * m_tiles + ((qp && !inl) ? (M + s - 1) / s : 0) + 1 > waiting_clusters(bn, s)) --s;
     if (s < 1) return -20;
     p.splits = s;
     // The two-hop tail pays for its second NVLink trip by spreading the owner's work over many CTAs; a launch split
@@ -1027,7 +1035,7 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
   switch (bn) {
     case 16: return launch_decode<16, 5>(tw, tx, p, grid, stream);
     case 32: return launch_decode<32, 4>(tw, tx, p, grid, stream);
-    case 64: return launch_decode<64, 7>(tw, tx, p, grid, stream);
+    case 64: return launch_decode<64, 3>(tw, tx, p, grid, stream);
     default: return s > 1 ? launch_decode<128, 4>(tw, tx, p, grid, stream) : launch_decode<128, 3, false>(tw, tx, p, grid, stream);
   }
 }
@@ -1048,7 +1056,7 @@ static void occupancy_facts(int* out) {
 // Occupancy facts of the decode GEMM for `m` tokens: {CTAs per SM without clusters, static shared bytes, registers per
 // thread, dynamic shared bytes}.
 extern "C" void b200_w8a8_gemm_decode_occupancy(int m, int* out4) {
-  if (m <= 16) occupancy_facts<16, 5>(out4); else if (m <= 32) occupancy_facts<32, 4>(out4); else occupancy_facts<64, 7>(out4);
+  if (m <= 16) occupancy_facts<16, 5>(out4); else if (m <= 32) occupancy_facts<32, 4>(out4); else occupancy_facts<64, 3>(out4);
 }
 
 // Occupancy calculator's answer for the 32-token decode GEMM at an arbitrary dynamic shared-memory size (diagnostics).

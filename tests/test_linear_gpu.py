@@ -316,3 +316,18 @@ def test_swiglu_rows_either_way(M, F, K):
     here = off(*L.swiglu_rows(xq, sx, wq, sw))
     before = off(*L.act_quant(L.w8a8_gemm(xq, sx, wq, sw), mode=L.AQ_SWIGLU))
     assert here <= before * 1.001        # no further from 64 bits than with gate and up rounded to bf16 in between
+
+
+@pytest.mark.parametrize("M,K", [(33, 18560), (64, 20480), (17, 20480), (64, 2048)])
+def test_rows_quantised_inside_the_launch_up_to_the_longest(M, K):
+    """A parked row may reach into the exchange buffer of the 64-token form.  Rounding may take a number to the other side of an int8 edge: as in
+    the tests of the fused prologue."""
+    from mojo_linuxperiments_b200.ops import linear as L
+    from mojo_linuxperiments_b200.ops.workspace import default_workspace
+    x = _mk_x(M, K, M)
+    wq, sw = _mk_w(384, K)
+    q, s = Q.rotate_quantize(x)
+    want = (q.double() @ wq.double().t()) * s.double().view(-1, 1) * sw.double()
+    y = L.fused_linear(x, wq, sw)
+    default_workspace(x.device).check_status()
+    assert torch.allclose(y.double(), want, rtol=2e-2, atol=2e-2 * want.abs().max().item())
