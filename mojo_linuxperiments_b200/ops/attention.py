@@ -94,7 +94,7 @@ def attn_prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlens: 
 
     ``kv_chunk`` > 0 selects the split-KV form: every ``kv_chunk`` KV tiles of 128 tokens of a query tile are a CTA of
     their own and a merge kernel combines them - more parallelism when there are few (sequence, head) pairs.  Default
-    (``None``): B200RT_PREFILL_SPLIT if set, else split where there are fewer (sequence, head, query tile) units than SMs."""
+    (``None``): B200RT_PREFILL_SPLIT if set, else ``pick_prefill_kv_chunk``."""
     T, hq, d = q.shape
     hkv = k.shape[1]
     assert d == HEAD_DIM and q.dtype == torch.bfloat16 and q.stride(2) == 1 and q.stride(1) == d
@@ -109,18 +109,7 @@ def attn_prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlens: 
         if env != "":
             kv_chunk = int(env)
         else:
-            # Few (sequence, head, query tile) units leave most SMs idle while the last query tiles walk their KV tiles
-            # alone.  The line was drawn when the un-split kernel gave every unit a CTA of its own; now two units share one and it
-            # is two to three times as fast.  Measured with it: the split pays for few heads over a long range (1 x 1,024 tokens x
-            # 4 heads 15.9 us, un-split 23.8; 1 x 512 x 8 heads 14.3, 15.0; 1 x 2,048 x 4 heads 38.7, 41.4), and no longer does
-            # elsewhere below the line (1 x 300 x 32 heads 21.7, un-split 11.8; 1 x 512 x 32 heads 28.7, 15.4; 1 x 4,096 x 4 heads
-            # 100, 77).
-            B_ = cu_seqlens.numel() - 1
-            n_q = (int(max_len) + 127) // 128
-            sms = _lib.num_sms(q.device.index)
-            kv_chunk = 0
-            if B_ * hq * n_q < sms and n_q > 1:
-                kv_chunk = max(1, min(8, B_ * hq * n_q * (n_q + 1) // 2 // sms))
+            kv_chunk = pick_prefill_kv_chunk(cu_seqlens.numel() - 1, hq, int(max_len), _lib.num_sms(q.device.index))
     if kv_chunk > 0:
         B = cu_seqlens.numel() - 1
         n = _lib.lib().b200_attn_prefill_split_scratch_floats(B, hq, int(max_len), kv_chunk)
@@ -141,6 +130,23 @@ def attn_prefill(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlens: 
         float(scale if scale is not None else 1.0 / math.sqrt(d)), ws.status.data_ptr(), _lib.stream())
     _lib.check(rc, "attn_prefill")
     return out
+
+
+def pick_prefill_kv_chunk(B: int, hq: int, max_len: int, sms: int = 148) -> int:
+    """KV tiles per CTA of the split form, 0 for the plain kernel.
+
+    A few heads leave most SMs idle while the last query tiles walk their KV tiles alone.  The plain kernel then takes as long as
+    its longest walk, 5.5 + 2.2 us per query tile; the split form and its merge 13 us and a fiftieth per KV tile of the whole call while those
+    fit one round of the SMs, 18 and a twenty-fifth above.  Split, plain, us: 1 x 1,024 tokens x 4 heads 15.9, 23.7; 1 x 512 x 2 12.5, 14.7;
+    1 x 3,000 x 2 41, 57; 1 x 2,048 x 4 39.3, 41.5; but 1 x 3,000 x 4 69, 58; 1 x 1,024 x 8 26.5, 24.0; 1 x 2,048 x 8 66, 42; 1 x 512 x 16 22, 15;
+    1 x 512 x 32 29, 15.5; 1 x 256 x 4 12.0, 10.3."""
+    n_q = (max_len + 127) // 128
+    units = B * hq * n_q
+    work = units * (n_q + 1) // 2
+    if units >= sms or n_q < 4:
+        return 0
+    pays = 650 + work < 275 + 110 * n_q if work <= sms else 450 + work < 137 + 55 * n_q
+    return max(1, min(8, work // sms)) if pays else 0
 
 
 class DecodeAttnScratch:
