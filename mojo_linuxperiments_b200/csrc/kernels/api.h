@@ -100,6 +100,9 @@ int b200_moe_combine(const void* y, long long ldy, const int* inv, const float* 
 int b200_act_quant(const void* x, long long ldx, void* residual, long long ldr, const void* gamma, float eps,
                    void* q, long long ldq, float* scale, void* xn_out, long long ldn, int M, int K, int mode,
                    cudaStream_t stream);
+// the same with mode 2, where what is added is the weighted sum of rows of y [slots][K]: slots, weights [M][k] (slot -1: none), k <= 32
+int b200_act_quant_sum(const void* y, long long ldy, const int* slots, const float* weights, int k, void* residual, long long ldr, const void* gamma,
+                       float eps, void* q, long long ldq, float* scale, int M, int K, cudaStream_t stream);
 
 // ---- attention and token-wise glue ---------------------------------------------------------------------
 // max_pos: rows of cos_tab / sin_tab; num_pages: pages of the cache.  A token whose position is outside the tables,

@@ -13,6 +13,7 @@ import torch
 
 from ..ops import attention as A
 from ..ops import linear as L
+from ..ops.moe import ExpertSum
 from ..parallel.comm import Comm
 from ..utils.trace import op_range
 from .config import ModelConfig, RuntimeConfig, kv_heads_per_rank
@@ -68,6 +69,8 @@ class Decoder:
     def _norm_quant(self, h, delta, gamma, want_normed=False):
         if delta is None:
             return L.act_quant(h, mode=L.AQ_NORM, gamma=gamma, eps=self.cfg.eps, want_normed=want_normed)
+        if isinstance(delta, ExpertSum):
+            return delta.act_quant(h, gamma, self.cfg.eps)
         return L.act_quant(delta, mode=L.AQ_ADD_NORM, gamma=gamma, eps=self.cfg.eps, residual=h, want_normed=want_normed)
 
     def _row_parallel(self, xq, sx, lw):
@@ -133,10 +136,10 @@ class Decoder:
             return self._row_parallel(hq, sh, lw)
         return L.fused_linear(gu, lw.qweight, lw.scale, mode=L.QR_SWIGLU, inline=self.inline_quant)
 
-    def _mlp(self, l, xq, sx, xn):
+    def _mlp(self, l, xq, sx, xn, pending=False):
         W = self.w["layers"][l]
         if self.moe is not None:
-            return self.moe.forward(W, xq, sx, xn)
+            return self.moe.forward(W, xq, sx, xn, pending)
         if self.comm.world == 1:
             hq, sh = L.swiglu_rows(xq, sx, W["gate_up"].qweight, W["gate_up"].scale)
         else:       # as in the token-sharded prefill, whose rows this path has to repeat bit by bit
@@ -186,7 +189,7 @@ class Decoder:
                 continue
             xq, sx = self._norm_quant(h, delta, W["mlp_norm"])      # the router, too, consumes the quantised rows
             with op_range(f"layer{l}.mlp"):
-                delta = self._mlp(l, xq, sx, None)
+                delta = self._mlp(l, xq, sx, None, pending=not fq)
         if last_idx is not None:
             h = h.index_select(0, last_idx)
             delta = delta.index_select(0, last_idx)

@@ -26,7 +26,8 @@ class MoEBlock:
         self.n_local = cfg.n_experts // max(rt.ep, 1)
         self.e0 = comm.rank * self.n_local if rt.ep > 1 else 0
 
-    def forward(self, W: dict, xq: torch.Tensor, sx: torch.Tensor, xn=None) -> torch.Tensor:
+    def forward(self, W: dict, xq: torch.Tensor, sx: torch.Tensor, xn=None, pending: bool = False):
+        """``pending``: on one rank, leave the weighted sum to the norm that reads it (``ops.moe.ExpertSum``)."""
         cfg = self.cfg
         M = xq.shape[0]
         logits = L.w8a8_gemm(xq, sx, W["router"].qweight, W["router"].scale, out_dtype=torch.float32, narrow=True)
@@ -36,8 +37,9 @@ class MoEBlock:
         yd = MO.grouped_gemm(hq, sh, W["experts_down"].qweight, W["experts_down"].scale, work)
         if self.tp_ctx is not None:
             return self.tp_ctx.reduce_partial(lambda out: MO.moe_combine(yd, work, wts, out=out), M, cfg.d_model)
-        out = MO.moe_combine(yd, work, wts)
-        return self.comm.all_reduce(out)
+        if pending and self.comm.world == 1 and cfg.top_k <= 32:
+            return MO.ExpertSum(yd, work.inv, wts)
+        return self.comm.all_reduce(MO.moe_combine(yd, work, wts))
 
     def forward_sharded(self, W: dict, xq_loc: torch.Tensor, sx_loc: torch.Tensor, M: int) -> torch.Tensor:
         """xq_loc / sx_loc: the normalised, quantised rows this rank owns of an M-token call; returns the MoE output of

@@ -99,6 +99,7 @@ class _Sig:
     b200_moe_gather = (I, [P, P, I, P, P, I, P, P, P])
     b200_moe_combine = (I, [P, LL, P, P, I, I, I, P, LL, P])
     b200_act_quant = (I, [P, LL, P, LL, P, F, P, LL, P, P, LL, I, I, I, P])
+    b200_act_quant_sum = (I, [P, LL, P, P, I, P, LL, P, F, P, LL, P, I, I, P])
     b200_rope_kv_write = (I, [P, LL, P, P, P, P, P, P, F, P, P, P, P, P, I, I, I, I, I, I, I, P, P])
     b200_embed_gather = (I, [P, P, P, I, I, I, P])
     b200_argmax_rows = (I, [P, LL, I, I, I, I, P, P, P])

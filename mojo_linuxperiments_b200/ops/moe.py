@@ -150,3 +150,27 @@ def moe_combine(y: torch.Tensor, w: MoEWorkList, wts: torch.Tensor, out: torch.T
     _lib.check(_lib.lib().b200_moe_combine(y.data_ptr(), y.stride(0), w.inv.data_ptr(), wts.data_ptr(), w.M, w.k, d,
                                            out.data_ptr(), out.stride(0), _lib.stream()), "moe_combine")
     return out
+
+
+class ExpertSum:
+    """The output of a mixture before its weighted sum (``moe_combine``), for a norm that adds it: ``act_quant``."""
+
+    def __init__(self, y: torch.Tensor, inv: torch.Tensor, wts: torch.Tensor):
+        self.y, self.inv, self.wts = y, inv, wts
+
+    def index_select(self, dim: int, rows: torch.Tensor) -> "ExpertSum":
+        assert dim == 0
+        return ExpertSum(self.y, self.inv.index_select(0, rows), self.wts.index_select(0, rows))
+
+    def act_quant(self, residual: torch.Tensor, gamma: torch.Tensor, eps: float):
+        """``residual`` += the sum, in place, and (int8 rows, scales) of its RMS norm, rotated: the bits of ``moe_combine`` and
+        ``linear.act_quant`` with AQ_ADD_NORM, in one launch."""
+        M, k = self.inv.shape
+        K = self.y.shape[1]
+        assert residual.dtype == torch.bfloat16 and residual.stride(1) == 1 and residual.shape == (M, K) and self.y.stride(1) == 1
+        q = torch.empty((M, K), dtype=torch.int8, device=residual.device)
+        s = torch.empty((M,), dtype=torch.float32, device=residual.device)
+        _lib.check(_lib.lib().b200_act_quant_sum(self.y.data_ptr(), self.y.stride(0), self.inv.data_ptr(), self.wts.data_ptr(), k, residual.data_ptr(),
+                                                 residual.stride(0), gamma.data_ptr(), float(eps), q.data_ptr(), q.stride(0), s.data_ptr(), M, K, _lib.stream()),
+                   "act_quant_sum")
+        return q, s

@@ -237,3 +237,23 @@ def test_routing_work_list_and_rows_in_one_launch(M, E, k, e0, n_local, units, g
     pair_token, pair_expert = torch.arange(M * k, device="cuda")[here] // k, ids.reshape(-1)[here].long() - e0
     assert torch.equal(w.slot_token[at].long(), pair_token) and ((w.offsets[pair_expert] <= at) & (at < w.offsets[pair_expert + 1])).all()
     assert torch.equal(rows[at], x[pair_token]) and (grouped or torch.equal(s[at], sx[pair_token]))
+
+
+@pytest.mark.parametrize("M,k,d,pitch", [(1, 8, 2048, 2048), (16, 8, 2048, 2048), (3, 9, 384, 388), (64, 1, 128, 128), (65, 8, 2048, 2048), (300, 5, 640, 644), (70, 12, 8320, 8320)])
+def test_weighted_sum_inside_the_norm(M, k, d, pitch):
+    """The bits of the weighted sum and of the activation kernel: rows of a cluster and of one CTA, more experts than a batch of loads, slots
+    without a row, pitches off sixteen bytes, two chunks per warp."""
+    from mojo_linuxperiments_b200.ops import linear as L
+    from mojo_linuxperiments_b200.ops import moe as MO
+    g = torch.Generator(device="cuda").manual_seed(M + d)
+    y = torch.randn((M * k, pitch), device="cuda", generator=g).to(torch.bfloat16)[:, :d]
+    w = MO.MoEWorkList(M, k, 4, "cuda")
+    w.inv.copy_(torch.randperm(M * k, device="cuda", generator=g).view(M, k))
+    w.inv[torch.rand((M, k), device="cuda", generator=g) < 0.2] = -1
+    wts = torch.rand((M, k), device="cuda", generator=g)
+    h = torch.randn((M, d), device="cuda", generator=g).to(torch.bfloat16)
+    gain = (1 + 0.1 * torch.randn(d, device="cuda", generator=g)).to(torch.bfloat16)
+    h0 = h.clone()
+    q0, s0 = L.act_quant(MO.moe_combine(y.contiguous(), w, wts), mode=L.AQ_ADD_NORM, gamma=gain, eps=1e-5, residual=h0)
+    q, s = MO.ExpertSum(y, w.inv, wts).act_quant(h, gain, 1e-5)
+    assert torch.equal(h, h0) and torch.equal(q, q0) and torch.equal(s, s0)
