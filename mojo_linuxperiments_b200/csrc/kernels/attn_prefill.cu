@@ -2,7 +2,9 @@
 //
 // A work item is two blocks ("units") of 128 query rows that walk the same KV tiles of 128 tokens: two heads of one KV head, or,
 // where a KV head has an odd number of heads, two neighbouring query tiles of one head.  One CTA per SM takes items, long ones
-// first.
+// first.  Where every item has an SM to itself, the call takes as long as its longest walk, and a unit alone walks faster than
+// two: 1.9 instead of 2.2 us per KV tile.  There an item is the last query tile of a head and the first, the last but one and
+// the second, ..., so that the longest walk is alone for most of its way.
 //   warp 0       TMA producer: the Q block of each unit, K and V tiles into two-stage rings (128-byte swizzle)
 //   warp 1       MMA issuer: S = Q.K^T (both from shared memory) and O += P.V (P from TMEM, V MN-major from shared memory),
 //                tcgen05.mma.kind::f16; the whole warp walks the loop so that descriptors stay in uniform registers
@@ -16,7 +18,7 @@
 // Sequences are concatenated along the token axis (cu_seqlens); a tile may read rows of the next sequence, which the causal /
 // length mask removes.  All waits are bounded.
 // 32 x 1,024 tokens, 32 heads over 8: 388 us = 709 TFLOP/s (1,425 us with one unit per CTA, O in registers and S read twice);
-// 3 x 3,001: 271 us (996); 1 x 1,024: 26 us (66); 32 x 200: 51 us (166); 100 x 64: 55 us (174).
+// 3 x 3,001: 271 us (996); 1 x 1,024: 21 us (66); 32 x 200: 51 us (166); 100 x 64: 55 us (174).
 #include "ptx.cuh"
 #include "api.h"
 #include "launch.cuh"
@@ -28,6 +30,7 @@ constexpr int AP_THREADS = 384;
 // registers: 384 x 168 at launch, 128 x (72 + 216 + 216) afterwards, which is as many
 constexpr int AP_REGS_FEW = 72, AP_REGS_MANY = 216;
 constexpr int AP_BM = 128, AP_BN = 128, AP_D = 128;
+constexpr int AP_SMS = 148;
 constexpr int AP_CHUNK_BYTES = 128 * 128;            // 128 rows x 64 bf16
 constexpr int AP_TILE_BYTES = 2 * AP_CHUNK_BYTES;    // 128 x 128 bf16
 
@@ -45,7 +48,8 @@ struct PrefillParams {
 
 int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t pitch_bytes);
 
-// the items of a CTA, in the same order for every warp
+// the items of a CTA, in the same order for every warp; FAR: the units are the last query tile and the first, the last but one and the second, ...
+template <bool FAR>
 struct PrefillItem {
   int row0, len, kvh;         // first token row of the sequence, its length, KV head
   int first_head, head_step;  // of the units
@@ -60,6 +64,16 @@ struct PrefillItem {
       next += gridDim.x;
       row0 = p.cu_seqlens[b];
       len = p.cu_seqlens[b + 1] - row0;
+      if constexpr (FAR) {
+        const int last = (len + AP_BM - 1) / AP_BM - 1 - step;
+        if (last < step) continue;
+        first_head = col;
+        head_step = 0;
+        first_q = last * AP_BM;
+        q_step = last > step ? (step - last) * AP_BM : len;      // the middle tile is alone
+        kvh = col / (p.hq / p.hkv);
+        return true;
+      }
       head_step = p.pair_heads ? 1 : 0;
       first_head = p.pair_heads ? 2 * col : col;
       q_step = p.pair_heads ? 0 : AP_BM;
@@ -75,6 +89,7 @@ struct PrefillItem {
   __device__ int tiles() const { return max(n(0), n(1)); }
 };
 
+template <bool FAR>
 __global__ void __launch_bounds__(AP_THREADS, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ PrefillParams p) {
@@ -106,7 +121,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   const uint32_t tmem_base = *tmem_slot;       // columns: S of unit u at 128 u, O at 256 + 128 u
   pdl_wait();                                  // everything before this kernel in the stream has completed
   auto wait = [&](int i, uint32_t par, int code) { return mbar_wait(bar(i), par, abort_flag, p.status, code | (3 << 8), limit); };
-  PrefillItem it;
+  PrefillItem<FAR> it;
 
   if (warp < 4) {
     warpgroup_regs_dec<AP_REGS_FEW>();
@@ -350,19 +365,27 @@ extern "C" int b200_attn_prefill(const void* q, long long ld_q, const void* k, l
   PrefillParams p;
   p.cu_seqlens = cu_seqlens; p.out = static_cast<__nv_bfloat16*>(out); p.hq = hq; p.hkv = hkv; p.B = B;
   const int q_tiles = (max_len + AP_BM - 1) / AP_BM;
-  p.pair_heads = (hq / hkv) % 2 == 0;
+  // far pairs only where each has an SM to itself.  Heads paired, far pairs, us, 32 heads over 8: 1 x 128 8.7, 7.1; 1 x 256 10.9, 9.1;
+  // 1 x 512 15.4, 13.1; 1 x 1,024 24.6, 21.1; 2 x 512 15.8, 13.4; 16 over 4: 1 x 2,048 42.5, 36.4.  Beyond that the work of all SMs is
+  // what counts, a pair of heads loads each KV tile once for both, and with both rules in one instance two registers were
+  // spilled: 1 x 3,000 x 32 112 -> 118
+  const bool far = static_cast<long long>(B) * hq * ((q_tiles + 1) / 2) <= AP_SMS;
+  p.pair_heads = !far && (hq / hkv) % 2 == 0;
   p.q_steps = p.pair_heads ? q_tiles : (q_tiles + 1) / 2;
   p.columns = p.pair_heads ? hq / 2 : hq;
   p.scale_log2 = scale * 1.4426950408889634f; p.status = status; p.limit_ns = 2000000000ull;
   constexpr int SMEM = 6 * AP_TILE_BYTES + 1024 + 256;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_prefill_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return -1000 - static_cast<int>(e);
     configured = true;
   }
   const long long items = static_cast<long long>(p.q_steps) * p.columns * B;
-  launch_ex(attn_prefill_kernel, dim3(static_cast<unsigned>(items < 148 ? items : 148)), dim3(AP_THREADS), SMEM, stream, 0, tq, tk, tv, p);
+  const dim3 grid(static_cast<unsigned>(items < AP_SMS ? items : AP_SMS));
+  if (far) launch_ex(attn_prefill_kernel<true>, grid, dim3(AP_THREADS), SMEM, stream, 0, tq, tk, tv, p);
+  else launch_ex(attn_prefill_kernel<false>, grid, dim3(AP_THREADS), SMEM, stream, 0, tq, tk, tv, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }

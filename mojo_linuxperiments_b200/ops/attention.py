@@ -136,16 +136,16 @@ def pick_prefill_kv_chunk(B: int, hq: int, max_len: int, sms: int = 148) -> int:
     """KV tiles per CTA of the split form, 0 for the plain kernel.
 
     A few heads leave most SMs idle while the last query tiles walk their KV tiles alone.  The plain kernel then takes as long as
-    its longest walk, 5.5 + 2.2 us per query tile; the split form and its merge 13 us and a fiftieth per KV tile of the whole call while those
-    fit one round of the SMs, 18 and a twenty-fifth above.  Split, plain, us: 1 x 1,024 tokens x 4 heads 15.9, 23.7; 1 x 512 x 2 12.5, 14.7;
-    1 x 3,000 x 2 41, 57; 1 x 2,048 x 4 39.3, 41.5; but 1 x 3,000 x 4 69, 58; 1 x 1,024 x 8 26.5, 24.0; 1 x 2,048 x 8 66, 42; 1 x 512 x 16 22, 15;
-    1 x 512 x 32 29, 15.5; 1 x 256 x 4 12.0, 10.3."""
+    its longest walk, 4.7 + 1.93 us per query tile; the split form and its merge 13 us and a fiftieth per KV tile of the whole call while those
+    fit one round of the SMs, 18 and a twenty-fifth above.  Split, plain, us: 1 x 1,024 tokens x 4 heads 15.9, 20.2; 1 x 700 x 2 13.6, 15.5;
+    1 x 3,000 x 2 41, 49; 1 x 1,500 x 2 24.3, 27.2; but 1 x 512 x 2 12.8, 12.4; 1 x 2,048 x 4 38.7, 35.4; 1 x 3,000 x 4 68, 49; 1 x 1,024 x 8 26.3, 20.4;
+    1 x 2,048 x 8 66, 36; 1 x 512 x 16 22, 13; 1 x 512 x 32 29, 13; 1 x 256 x 4 12.1, 8.7."""
     n_q = (max_len + 127) // 128
     units = B * hq * n_q
     work = units * (n_q + 1) // 2
     if units >= sms or n_q < 4:
         return 0
-    pays = 650 + work < 275 + 110 * n_q if work <= sms else 450 + work < 137 + 55 * n_q
+    pays = 650 + work < 235 + 96 * n_q if work <= sms else 450 + work < 117 + 48 * n_q
     return max(1, min(8, work // sms)) if pays else 0
 
 

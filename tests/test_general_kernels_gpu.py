@@ -135,6 +135,21 @@ def test_prefill_attention_pairs_heads_or_query_tiles(lens, hq, hkv):
         assert (o.double() - torch.einsum("hij,jhd->ihd", s, v)).abs().max().item() < 1.6e-2
 
 
+@pytest.mark.parametrize("lens,hq,hkv", [([1], 2, 1), ([128], 4, 2), ([129, 256], 8, 2), ([1024], 32, 8), ([1025], 32, 8), ([128, 640, 641, 5], 8, 8), ([2049], 16, 4),
+                                         ([300, 1, 129, 900] * 20, 3, 3)])
+def test_prefill_attention_pairs_far_query_tiles(lens, hq, hkv):
+    """A head's last query tile and its first share a CTA where all pairs fit one wave: one tile, a middle tile alone, sequences
+    shorter than the longest, the sizes on both sides of a wave.  The weights of a row sum to 1, each is rounded
+    to bf16 by at most 2^-9 of itself and the output by 2^-9 of values up to 4: 2^-8 * 4.  An empty sequence changes nothing."""
+    test_prefill_attention_pairs_heads_or_query_tiles(lens, hq, hkv)
+    from mojo_linuxperiments_b200.ops import attention as A
+    x = torch.randn((sum(lens), hq + 2 * hkv, 128), device=DEV).to(torch.bfloat16)
+    cu = [torch.tensor([0] + ls).cumsum(0).to(torch.int32).to(DEV) for ls in (lens, [0] + lens[:1] + [0] + lens[1:])]
+    a, b = (A.attn_prefill(x[:, :hq].contiguous(), x[:, hq:hq + hkv], x[:, hq + hkv:], c, max(lens), kv_chunk=0) for c in cu)
+    _ok()
+    assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("shift", [0, 4])
 @pytest.mark.parametrize("K", [128, 384, 512, 640, 2048, 4096, 8192, 8320, 14336, 16384])
 @pytest.mark.parametrize("mode", [0, 1, 2, 3])
