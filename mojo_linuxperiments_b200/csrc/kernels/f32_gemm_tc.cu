@@ -125,13 +125,14 @@ __global__ void __launch_bounds__(FC_THREADS, 1) f32_gemm_tc_kernel(const __grid
     const long long ld = is_w ? p.ldw : p.ldx;
     const int first = is_w ? n0 : m0, rows = (is_w ? p.N : p.M) - first;
     const float* src = (is_w ? p.w : p.x) + static_cast<long long>(first + r0) * ld + c;
+    // past L1: X is what the launch in front has written, often over rows that an older one has read (ptx.cuh), and nothing is read twice
     auto fetch = [&](int i, float4 (&v)[4]) {
       const int k = (kb0 + i) * FC_K;
       if (i >= blocks) return;
       if (k + FC_K <= p.K) {
 #pragma unroll
         for (int it = 0; it < 4; ++it)
-          v[it] = r0 + it < rows ? __ldg(reinterpret_cast<const float4*>(src + it * ld + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          v[it] = r0 + it < rows ? __ldcg(reinterpret_cast<const float4*>(src + it * ld + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
       } else {                                    // what lies beyond K counts as zero, whatever it is
 #pragma unroll
         for (int it = 0; it < 4; ++it) {

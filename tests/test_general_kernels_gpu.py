@@ -475,3 +475,43 @@ def test_w8a8_decode_exchange(M, splits):
     y = L.w8a8_gemm(x, sx, w, sw, force_mode=2, force_splits=splits)
     _ok()
     assert ((y.double() - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -22)).all()
+
+
+@pytest.mark.parametrize("M", [9, 16, 64, 380])
+def test_f32_linears_that_hand_one_buffer_on(M):
+    """Read, rewritten in place, read again, launch after launch, as the stream of a model's layers: captured and replayed, with kernels that
+    start before their input is there, the bits of the same launches one at a time.  A row that L1 still holds from the launch
+    before would show."""
+    from mojo_linuxperiments_b200.ops import dense as D
+    g, d, layers = torch.Generator(device=DEV).manual_seed(M), 2048, 4
+    w = [[D.DenseW.of(torch.randn((d, d), generator=g, device=DEV) * d ** -0.5, torch.float32, DEV) for _ in range(2)] for _ in range(layers)]
+    norm = D.DynamicTanh.of(0.5, torch.randn(d, generator=g, device=DEV), torch.randn(d, generator=g, device=DEV), DEV)
+    x0 = torch.empty((M, d), device=DEV)
+    x, h = torch.empty_like(x0), torch.empty_like(x0)
+
+    def run(after=lambda: None):
+        x.copy_(x0)
+        h.copy_(x0)
+        for a, b in w:
+            y = D.linear(h, a)
+            after()
+            D.linear_residual(y, b, x, 0.7, norm, h)
+            after()
+        return D.linear(h, w[0][0])
+
+    side = torch.cuda.Stream()
+    x0.normal_(generator=g)
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        run()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = run()
+    for _ in range(20):
+        x0.normal_(generator=g)
+        graph.replay()
+        got = x.clone(), h.clone(), y.clone()
+        want_y = run(torch.cuda.synchronize)
+        assert torch.equal(got[0], x) and torch.equal(got[1], h) and torch.equal(got[2], want_y)
+    _ok()

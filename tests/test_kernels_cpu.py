@@ -1,5 +1,6 @@
 """What the kernel library's host side decides, and rules its sources keep: no GPU needed."""
 import os
+import re
 import subprocess
 import sys
 
@@ -43,6 +44,33 @@ def test_cluster_barriers_are_reached_by_whole_warps():
                 found += 1
                 assert "__syncwarp();" in lines[i - 1], f"{path.name}:{i + 1}"
     assert found >= 3
+
+
+# tensors that never change while a model runs: scales of weights, norm gains and shifts, gate biases, routing corrections, tables of
+# embeddings, vectors of a step
+SETTLED = {"gamma", "q_gain", "c_gain", "zb", "xb", "correction", "table", "add", "shift", "swp", "swg", "sw", "norm_w", "norm_b"}
+
+
+def _arguments(text: str, call: str):
+    for m in re.finditer(re.escape(call), text):
+        depth, at = 1, m.end()
+        while depth:
+            depth += {"(": 1, ")": -1}.get(text[at], 0)
+            at += 1
+        yield text.count("\n", 0, m.start()) + 1, text[m.end():at - 1]
+
+
+def test_only_settled_tensors_are_read_through_the_non_coherent_path():
+    """A kernel may be resident before its input is written, so a line that an older kernel left in L1 may be stale: activations are
+    read with plain loads or past L1."""
+    found = 0
+    for path in sorted((_build.CSRC / "kernels").glob("*.cu*")):
+        text = re.sub(r"//.*", "", path.read_text())
+        for line, arg in _arguments(text, "__ldg("):
+            found += 1
+            assert SETTLED & set(re.findall(r"\w+", arg)), f"{path.name}:{line}: {arg}"
+        assert "ld.global.nc" not in text, path.name
+    assert found >= 20
 
 
 def test_the_kernels_that_open_a_step_wait_for_all_of_the_step_before():
