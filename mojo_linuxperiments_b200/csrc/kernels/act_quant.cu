@@ -358,7 +358,7 @@ act_quant_cluster_kernel(const __nv_bfloat16* x, long long ldx, __nv_bfloat16* r
 // 32,768 x 14,336 in 277 us = 5.1 TB/s, 3,200 x 14,336 in 30 (gate, rotation and int8 from bf16 gate and up: 753 and 77)
 constexpr int QB_STEPS = 4, QB_SPAN = QB_STEPS * 512;
 __global__ void __launch_bounds__(256)
-quant_blocks_kernel(const int16_t* __restrict__ blocks, const float* __restrict__ tops, int8_t* __restrict__ q, float* __restrict__ scale, int M, int K, int spans) {
+quant_blocks_kernel(const int16_t* blocks, const float* tops, int8_t* q, float* scale, int M, int K, int spans) {
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31, nb = K >> 7;

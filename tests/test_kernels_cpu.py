@@ -69,7 +69,7 @@ def test_only_settled_tensors_are_read_through_the_non_coherent_path():
         for line, arg in _arguments(text, "__ldg("):
             found += 1
             assert SETTLED & set(re.findall(r"\w+", arg)), f"{path.name}:{line}: {arg}"
-        assert "ld.global.nc" not in text, path.name
+        assert "ld.global.nc" not in text and "__restrict" not in text, path.name      # a restricted parameter lets the compiler choose that path
     assert found >= 20
 
 
