@@ -102,9 +102,27 @@ print("rc", rc)
 
 
 def test_prefill_split_only_where_a_few_heads_walk_far():
-    """Measured on both sides of the line (132 to 148 multiprocessors change nothing here)."""
+    """Measured on both sides of the line, with 148 multiprocessors."""
     from mojo_linuxperiments_b200.ops.attention import pick_prefill_kv_chunk as pick
     assert all(pick(*c) > 0 for c in ((1, 2, 700), (1, 2, 1024), (1, 2, 3000), (1, 4, 700), (1, 4, 1024), (2, 2, 1024)))
     assert all(pick(*c) == 0 for c in ((1, 2, 256), (1, 2, 512), (1, 4, 256), (1, 4, 512), (1, 4, 2048), (1, 4, 3000), (2, 4, 1024), (1, 8, 700), (1, 8, 2048), (1, 16, 512), (1, 32, 129), (1, 32, 512),
                                        (1, 32, 4096), (32, 32, 1024), (1, 1, 64)))
     assert pick(1, 2, 3000) == 4 and pick(1, 4, 1024) == 1
+
+
+def test_every_kernel_that_reports_a_status_has_a_name():
+    import torch
+
+    from mojo_linuxperiments_b200.ops.workspace import Workspace, _KERNEL_NAMES
+    w = Workspace(torch.device("cpu"), ws_bytes=64, counters=16)
+    numbers = set()
+    for path in sorted((_build.CSRC / "kernels").glob("*.cu*")):
+        text = re.sub(r"//.*", "", path.read_text())
+        numbers |= {int(n) for n in re.findall(r"\((?:\w+(?:<\w+>)?\(?\w*\)? \| \()?(\d+) << 8\)", text)} | {int(n) for n in re.findall(r"\| \((\d+) << 8\)", text)}
+        numbers |= {int(n) for n in re.findall(r"loop\.open\(\w+, [\w.]+, (\d+),", text)}
+    assert {1, 2, 3, 20, 21, 22, 23} <= numbers and numbers <= set(_KERNEL_NAMES), numbers - set(_KERNEL_NAMES)
+    for n in numbers:
+        w.status[0] = 1 | n << 8
+        with pytest.raises(RuntimeError, match=_KERNEL_NAMES[n]):
+            w.check_status()
+        assert int(w.status[0]) == 0
