@@ -108,6 +108,8 @@ def test_prefill_split_only_where_a_few_heads_walk_far():
     assert all(pick(*c) == 0 for c in ((1, 2, 256), (1, 2, 512), (1, 4, 256), (1, 4, 512), (1, 4, 2048), (1, 4, 3000), (2, 4, 1024), (1, 8, 700), (1, 8, 2048), (1, 16, 512), (1, 32, 129), (1, 32, 512),
                                        (1, 32, 4096), (32, 32, 1024), (1, 1, 64)))
     assert pick(1, 2, 3000) == 4 and pick(1, 4, 1024) == 1
+    # 144 KV tiles in all: one round of 148 or 144 multiprocessors, more than one of 140
+    assert pick(1, 4, 1024, 144) == 1 and pick(1, 4, 1024, 140) == 0 and pick(2, 2, 1024, 144) == 1 and pick(2, 2, 1024, 132) == 0
 
 
 def test_every_kernel_that_reports_a_status_has_a_name():
