@@ -159,6 +159,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   constexpr int XS = BN + 4;                      // sizes the exchange buffer
   constexpr int EX_ROWS = TILE_N + 16;            // S senders x (slice of at most 2 * ceil(64 / S) channels) <= 128 + 2 S
   constexpr int EX_BYTES = XCH ? EX_ROWS * XS * 4 : 0;      // [sender][token][channel of the slice]
+  constexpr int SX_WARPS = BN < 32 ? 1 : BN / 32;           // warps (from warp 2 on) that store the token scales
   static_assert(STAGES * STAGE_BYTES >= BN * TILE_N * (XCH ? 8 : 4), "the staging of the all-reduce tail, and behind it that of the exchange, alias the pipeline stages");
   // a quantiser CTA parks a row of up to QUANT_ROW_BYTES from the first stage on, if need be into the exchange buffer, and needs a few words behind it
   constexpr int QUANT_WORDS_AT = STAGES * STAGE_BYTES > QUANT_ROW_BYTES ? STAGES * STAGE_BYTES : QUANT_ROW_BYTES;
@@ -181,7 +182,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
   const uint32_t tfull_bar = bar_base + 8u * (2 * STAGES);
-  const uint32_t xch_bar = bar_base + 8u * (2 * STAGES + 1);     // split-K exchange: bytes the other CTAs send to this one
+  const uint32_t xch_bar = bar_base + 8u * (2 * STAGES + 1);     // split-K exchange: bytes the CTAs of the cluster send to this one, and its token scales
 
   const int S = XCH ? p.splits : 1;
   const int rank = static_cast<int>(cluster_ctarank());          // == blockIdx.x: position along K
@@ -213,7 +214,7 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     // inline prologue: a stage is full when the weight tile has landed and a quantising warp has stored the rows
     for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), inl ? 2 : 1); mbar_init(empty_bar(s), 1); }
     mbar_init(tfull_bar, 1);
-    mbar_init(xch_bar, 1);
+    mbar_init(xch_bar, 1 + SX_WARPS);
     *abort_flag = 0;
     mbar_fence_init();
     B200_TRACE_INIT();
@@ -511,6 +512,11 @@ w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
     // fused prologue: the scales are written by this launch's quantiser CTAs; the accumulator can only be complete
     // after the producer warp saw every row's flag, so they are there now (read past L1)
     if (prolog && !inl && et < BN) sx_s[et] = et < jmax ? __ldcg(p.sx + m0 + et) : 0.f;
+    if (async_x && et < 32 * SX_WARPS) {
+      // the token scales of this warp are stored: the reduction reads them behind the same barrier as the partial sums
+      __syncwarp();
+      if (lane == 0) mbar_arrive(xch_bar);
+    }
     if (et == 0) B200_TRACE(TK_GEMM_DECODE, 4);
   }
 

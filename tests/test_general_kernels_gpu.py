@@ -515,3 +515,41 @@ def test_f32_linears_that_hand_one_buffer_on(M):
         want_y = run(torch.cuda.synchronize)
         assert torch.equal(got[0], x) and torch.equal(got[1], h) and torch.equal(got[2], want_y)
     _ok()
+
+
+@pytest.mark.parametrize("prologue", [False, True])
+@pytest.mark.parametrize("M", [1, 5, 16, 17, 40, 64])
+def test_token_scales_of_launch_after_launch(M, prologue):
+    """Every split, launches that follow each other with other scales: a finished value takes those of its own launch."""
+    from mojo_linuxperiments_b200.ops import linear as L
+    from mojo_linuxperiments_b200.ops.workspace import default_workspace
+    g = torch.Generator(device=DEV).manual_seed(M)
+    N, K, n = 1152, 2048, 7
+    w = torch.randint(-127, 128, (N, K), dtype=torch.int8, device=DEV, generator=g)
+    sw = torch.rand(N, device=DEV, generator=g)
+    x = torch.randint(-127, 128, (M, K), dtype=torch.int8, device=DEV, generator=g)
+    xb = torch.randn((M, K), device=DEV, generator=g).to(torch.bfloat16)
+    scales = [torch.rand(M, device=DEV, generator=g) * 10.0 ** i for i in range(n)]
+    rows_ = [xb * 4.0 ** i for i in range(n)]
+    acc = x.double() @ w.double().t() * sw.double()
+
+    def run():
+        if prologue:                                     # the launch's own quantiser CTAs publish the scales; powers of four: the same int8 rows
+            default_workspace(torch.device(DEV)).next_step()
+            return [L.fused_linear(r, w, sw) for r in rows_]
+        return [L.w8a8_gemm(x, s, w, sw, force_mode=2, force_splits=2 + i) for i, s in enumerate(scales)]
+
+    run()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = run()
+    for _ in range(30):
+        graph.replay()
+        for i, y in enumerate(out):
+            if prologue:
+                assert torch.equal(y, out[0] * 4.0 ** i)
+            else:
+                want = acc * scales[i].double()[:, None]
+                assert ((y.double() - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -22)).all()
+    _ok()

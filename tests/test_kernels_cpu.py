@@ -128,3 +128,13 @@ def test_every_kernel_that_reports_a_status_has_a_name():
         with pytest.raises(RuntimeError, match=_KERNEL_NAMES[n]):
             w.check_status()
         assert int(w.status[0]) == 0
+
+
+def test_token_scales_are_stored_before_the_sums_count_as_complete():
+    """Split along K, the int8 decode linear's reduction runs on all six warps, its token scales are stored by the first of the epilogue's: the
+    barrier that counts the partial sums counts the warps that store scales, and each arrives behind its stores."""
+    text = (_build.CSRC / "kernels" / "w8a8_gemm_decode.cu").read_text()
+    assert "mbar_init(xch_bar, 1 + SX_WARPS);" in text
+    stores = [m.start() for m in re.finditer(r"sx_s\[\w+\] = ", text)]
+    arrives = [m.start() for m in re.finditer(r"mbar_arrive\(xch_bar\)", text)]
+    assert len(stores) == 3 and len(arrives) == 1 and max(stores) < arrives[0] < text.index("mbar_wait(xch_bar")
