@@ -298,6 +298,13 @@ template <int N> __device__ __forceinline__ void warpgroup_regs_inc() { asm vola
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
+// the same, and true for all threads if it was for one: what decides whether they meet at a barrier again
+__device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool mine) {
+  uint32_t any;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, %2, %3, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(any) : "r"(static_cast<uint32_t>(mine)), "r"(id), "r"(nthreads) : "memory");
+  return any != 0;
+}
 
 // ---------------------------------------------------------------------------------------------
 // system-scope signalling (flags another GPU or another CTA writes)

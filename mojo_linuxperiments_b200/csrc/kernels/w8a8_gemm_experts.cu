@@ -53,7 +53,6 @@ w8a8_gemm_experts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
   uint64_t* bars = reinterpret_cast<uint64_t*>(sx_s + BN);
   uint32_t* slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + EX_TILES);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(slot + 1);
-  volatile int* verdict = abort_flag + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t base = smem_u32(smem), bar0 = smem_u32(bars);
   auto full = [&](int s) { return bar0 + 8u * s; };
@@ -128,9 +127,7 @@ w8a8_gemm_experts_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gri
         const float sw = __ldg(p.sw + static_cast<size_t>(e) * p.N + n0 + row);
         const bool ok = mbar_wait(done(t), 0, abort_flag, p.status, (ST_TIMEOUT_TMEM_FULL | (23 << 8)), p.limit_ns);
         tc_fence_after();
-        if (et == 0) *verdict = *abort_flag;
-        named_bar_sync(1, 128);                        // scales; the last tile has been stored; one verdict for all four warps
-        if (!__all_sync(0xffffffffu, ok) || *verdict) break;
+        if (named_bar_or(1, 128, !ok)) break;              // scales; the last tile has been stored; one verdict for all four warps
         const uint32_t at = tmem + t * BN + (static_cast<uint32_t>(q * 32) << 16);
 #pragma unroll 1
         for (int c = 0; c < BN; c += 16) {

@@ -138,3 +138,11 @@ def test_token_scales_are_stored_before_the_sums_count_as_complete():
     stores = [m.start() for m in re.finditer(r"sx_s\[\w+\] = ", text)]
     arrives = [m.start() for m in re.finditer(r"mbar_arrive\(xch_bar\)", text)]
     assert len(stores) == 3 and len(arrives) == 1 and max(stores) < arrives[0] < text.index("mbar_wait(xch_bar")
+
+
+def test_the_experts_kernel_leaves_its_loop_with_all_epilogue_warps_or_none():
+    """They meet at barriers: a warp whose bounded wait ran out takes the others along through the barrier that joins the verdicts, not through a
+    flag that one thread may have read before."""
+    text = (_build.CSRC / "kernels" / "w8a8_gemm_experts.cu").read_text()
+    loop = text[text.index("tmem_ld_x16") - 1500:text.index("tmem_ld_x16")]
+    assert "if (named_bar_or(1, 128, !ok)) break;" in loop and "verdict =" not in text
