@@ -71,10 +71,11 @@ struct PagedItem {
       if (first_q >= len) continue;
       start = p.positions[row0];
       seq = p.seq_ids ? p.seq_ids[row0] : b;
-      if (start < 0 || seq < 0 || seq >= p.num_seqs || last_pos(q0(1) < len ? 1 : 0) / PP_PS >= p.max_pages) {
-        if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, static_cast<int>(ST_BAD_ARGUMENT) | (11 << 8));
-        continue;
-      }
+      const bool bad = start < 0 || seq < 0 || seq >= p.num_seqs || last_pos(0) / PP_PS >= p.max_pages;
+      const bool bad_second = q0(1) < len && last_pos(1) / PP_PS >= p.max_pages;
+      if ((bad || bad_second) && threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, static_cast<int>(ST_BAD_ARGUMENT) | (11 << 8));
+      if (bad) continue;
+      if (bad_second) q_step = len - first_q;        // the first query tile of the pair has its pages: the second one has no rows
       kvh = first_head / (p.hq / p.hkv);
       kv_start = p.chunk > 0 ? (start + first_q) - (start + first_q) % p.chunk : 0;
       kv_start -= kv_start % PP_PS;

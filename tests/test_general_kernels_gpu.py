@@ -553,3 +553,27 @@ def test_token_scales_of_launch_after_launch(M, prologue):
                 want = acc * scales[i].double()[:, None]
                 assert ((y.double() - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -22)).all()
     _ok()
+
+
+@pytest.mark.parametrize("H,G", [(3, 3), (4, 2)])
+def test_paged_prefill_attention_drops_the_query_tile_without_pages(H, G):
+    """A table that ends inside the second query tile of a portion: that tile is reported and left out, the first one is computed, with pairs
+    of heads and with pairs of query tiles."""
+    from mojo_linuxperiments_b200.ops import attention as A
+    g = torch.Generator(device=DEV).manual_seed(H)
+    n, dk, ps, pages = 250, 64, 16, 10
+    cache = A.PagedKVCache(16, G, ps, DEV, dk=dk, dv=dk, dtype=torch.bfloat16)
+    cache.data.normal_(generator=g)
+    table = torch.arange(pages, dtype=torch.int32, device=DEV).view(1, pages)
+    q = torch.randn((n, H * dk), generator=g, device=DEV).to(torch.bfloat16)
+    pos, sid, out = torch.arange(n, dtype=torch.int32, device=DEV), torch.zeros(n, dtype=torch.int32, device=DEV), {}
+    for rows in (128, n):
+        cu = torch.tensor([0, rows], dtype=torch.int32, device=DEV)
+        out[rows] = torch.full((n, H * dk), 7.0, dtype=torch.bfloat16, device=DEV)
+        A.attn_prefill_paged(q, H, pos, sid, cu, rows, cache, table, A.attn_spec(dk ** -0.5), out[rows])
+        if rows == n:
+            with pytest.raises(RuntimeError, match="attn_prefill_paged"):
+                _ok()
+        else:
+            _ok()
+    assert torch.equal(out[n][:128], out[128][:128]) and (out[n][128:] == 7.0).all() and not (out[n][:128] == 7.0).all()
