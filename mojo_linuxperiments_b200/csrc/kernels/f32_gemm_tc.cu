@@ -46,6 +46,7 @@ constexpr int FC_PERIOD = 32;                                    // blocks after
 constexpr int FC_OPERAND = FC_TILE * 128;                        // bytes of one operand tile
 constexpr int FC_BUFFER = 3 * FC_OPERAND;
 constexpr int FC_OUT_PITCH = FC_TILE + 4;                        // floats
+constexpr int FC_MAX_N = 65535 * FC_TILE;                        // column tiles are the grid's second dimension
 constexpr int FC_SMEM = 2 * FC_BUFFER + FC_TILE * FC_OUT_PITCH * 4 + 1024 + 64;
 
 // columns of tensor memory: two accumulators of x1 w1 blocks, two of the small products
@@ -279,13 +280,13 @@ using namespace b200;
 
 // Up to 8 rows the streaming kernel of f32_gemm.cu.  Shorter sums take as long there (9 x 256 x 256 5.8 us | 5.6, 380 x 256 x 256 8.2 | 8.0) and
 // lose least; at K = 512 it is 9 x 16 x 512 7.3 | 6.2, 130 x 256 x 512 8.8 | 8.9, 380 x 4,096 x 512 53 | 22.
-extern "C" int b200_f32_gemm_tc_takes(int M, int N, int K) { return M > 8 && K >= 512; }
+extern "C" int b200_f32_gemm_tc_takes(int M, int N, int K) { return M > 8 && K >= 512 && N <= FC_MAX_N; }
 
 // x, w, ldx and ldw on 16 bytes; splits: 0 or 1..8 CTAs along K
 extern "C" int b200_f32_gemm_tc(const float* x, long long ldx, const float* w, long long ldw, int M, int N, int K, const b200_dense_epilogue* epi,
                                 int* status, int splits, cudaStream_t stream) {
   if (M <= 0) return 0;
-  if (N <= 0 || K <= 0 || ldx < K || ldw < K || (ldx % 4) || (ldw % 4) || splits < 0 || splits > 8 || (N + FC_TILE - 1) / FC_TILE > 65535) return -1;
+  if (N <= 0 || K <= 0 || ldx < K || ldw < K || (ldx % 4) || (ldw % 4) || splits < 0 || splits > 8 || N > FC_MAX_N) return -1;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) return -2;
   if (int rc = dense_epilogue_check(epi, N)) return rc;
   static bool configured = false;

@@ -85,16 +85,18 @@ ACTIVATIONS = {None: 0, "relu2": 1}
 
 
 def _run(x: torch.Tensor, w: DenseW, epi, force: int = 0) -> None:
-    """fp32: ``force`` -1 keeps to the CUDA cores, above 0 is the number of CTAs along K of the tensor-core kernel."""
+    """``force``, bf16: CTAs along K up to 64 tokens, columns per tile above (see the C entries).  fp32: -1 keeps to the CUDA cores, 1 to 8 is
+    the number of CTAs along K of the tensor-core kernel where it can take the operands, any other value the rule."""
     M = x.shape[0]
     if M == 0:
         return
     assert x.dtype == w.data.dtype and x.stride(1) == 1 and x.shape[1] >= w.k
     if x.dtype == torch.float32:
         aligned = (x.data_ptr() | w.data.data_ptr()) % 16 == 0 and x.stride(0) % 4 == 0 and w.data.stride(0) % 4 == 0
-        if force >= 0 and aligned and (force > 0 or _lib.lib().b200_f32_gemm_tc_takes(M, w.n, w.k) == 1):
+        splits = force if 0 < force <= 8 else 0
+        if force != -1 and aligned and (splits or _lib.lib().b200_f32_gemm_tc_takes(M, w.n, w.k) == 1):
             rc = _lib.lib().b200_f32_gemm_tc(x.data_ptr(), x.stride(0), w.data.data_ptr(), w.data.stride(0), M, w.n, w.k, ctypes.byref(epi),
-                                             default_workspace(x.device).status.data_ptr(), force, _lib.stream())
+                                             default_workspace(x.device).status.data_ptr(), splits, _lib.stream())
             _lib.check(rc, "f32_gemm_tc")
             return
         rc = _lib.lib().b200_f32_gemm(x.data_ptr(), x.stride(0), w.data.data_ptr(), w.data.stride(0), M, w.n, w.k,

@@ -577,3 +577,11 @@ def test_paged_prefill_attention_drops_the_query_tile_without_pages(H, G):
         else:
             _ok()
     assert torch.equal(out[n][:128], out[128][:128]) and (out[n][128:] == 7.0).all() and not (out[n][:128] == 7.0).all()
+
+
+def test_f32_linear_takes_the_values_of_force_that_choose_a_bf16_tile():
+    from mojo_linuxperiments_b200.ops import dense as D
+    x, w = torch.randn((16, 1024), device=DEV), D.DenseW.of(torch.randn((200, 1024), device=DEV), torch.float32, DEV)
+    want = D.linear(x, w)[:, :200]
+    for force in (9, 64, 256, -64, -256):
+        assert torch.equal(D.linear(x, w, force=force)[:, :200], want), force

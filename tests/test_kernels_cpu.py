@@ -146,3 +146,7 @@ def test_the_experts_kernel_leaves_its_loop_with_all_epilogue_warps_or_none():
     text = (_build.CSRC / "kernels" / "w8a8_gemm_experts.cu").read_text()
     loop = text[text.index("tmem_ld_x16") - 1500:text.index("tmem_ld_x16")]
     assert "if (named_bar_or(1, 128, !ok)) break;" in loop and "verdict =" not in text
+
+
+def test_f32_tensor_core_linear_takes_no_more_columns_than_its_grid_has(lib):
+    assert lib.b200_f32_gemm_tc_takes(16, 65535 * 128, 2048) == 1 and lib.b200_f32_gemm_tc_takes(16, 65535 * 128 + 1, 2048) == 0
