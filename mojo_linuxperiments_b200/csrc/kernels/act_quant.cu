@@ -353,55 +353,6 @@ act_quant_cluster_kernel(const __nv_bfloat16* x, long long ldx, __nv_bfloat16* r
   B200_TRACE_FLUSH(TK_ACT_QUANT);
 }
 
-// 16-bit blocks (hadamard.cuh) -> int8 rows.  A warp takes 2,048 elements of a row and finds the row's scale itself, from a float per
-// 128 elements; everything is asked for at once and no warp waits for another.  Bound by its bytes:
-// 32,768 x 14,336 in 277 us = 5.1 TB/s, 3,200 x 14,336 in 30 (gate, rotation and int8 from bf16 gate and up: 753 and 77)
-constexpr int QB_STEPS = 4, QB_SPAN = QB_STEPS * 512;
-__global__ void __launch_bounds__(256)
-quant_blocks_kernel(const int16_t* blocks, const float* tops, int8_t* q, float* scale, int M, int K, int spans) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int lane = threadIdx.x & 31, nb = K >> 7;
-  const long long item = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-  const long long row = item / spans;
-  if (row >= M) return;
-  const int span = static_cast<int>(item - row * spans), e0 = span * QB_SPAN + lane * 16;
-  const int16_t* src = blocks + row * K;
-  const float* top = tops + row * nb;
-  uint4 raw[QB_STEPS][2];
-  float mine[QB_STEPS];
-#pragma unroll
-  for (int i = 0; i < QB_STEPS; ++i) {
-    const int e = e0 + i * 512;
-    const bool have = e < K;
-    raw[i][0] = have ? __ldcs(reinterpret_cast<const uint4*>(src + e)) : make_uint4(0u, 0u, 0u, 0u);
-    raw[i][1] = have ? __ldcs(reinterpret_cast<const uint4*>(src + e) + 1) : make_uint4(0u, 0u, 0u, 0u);
-    mine[i] = have ? top[e >> 7] : 0.f;
-  }
-  float amax = 0.f;
-  for (int b = lane; b < nb; b += 32) amax = fmaxf(amax, top[b]);
-  amax = warp_max(amax);
-  const float s = quant_scale_from_amax(amax), inv = quant_inv_scale(s);
-  if (span == 0 && lane == 0) scale[row] = s;
-#pragma unroll
-  for (int i = 0; i < QB_STEPS; ++i) {
-    const int e = e0 + i * 512;
-    if (e >= K) break;
-    const float f = __fmul_rn(__fmul_rn(mine[i], inv), 1.f / 32767.f);
-    uint32_t out[4];
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-      const uint4 x = raw[i][g >> 1];
-      const uint32_t a = g & 1 ? x.z : x.x, b = g & 1 ? x.w : x.y;
-      out[g] = quant_bytes4(__float2int_rn(__fmul_rn(static_cast<float>(static_cast<int16_t>(a & 0xffffu)), f)),
-                            __float2int_rn(__fmul_rn(static_cast<float>(static_cast<int32_t>(a) >> 16), f)),
-                            __float2int_rn(__fmul_rn(static_cast<float>(static_cast<int16_t>(b & 0xffffu)), f)),
-                            __float2int_rn(__fmul_rn(static_cast<float>(static_cast<int32_t>(b) >> 16), f)));
-    }
-    *reinterpret_cast<uint4*>(q + row * K + e) = make_uint4(out[0], out[1], out[2], out[3]);
-  }
-}
-
 template <int MAXB>
 static void launch_aq_cluster(int mode, const __nv_bfloat16* x, long long ldx, __nv_bfloat16* residual, long long ldr,
                               const __nv_bfloat16* gamma, float eps, int8_t* q, long long ldq, float* scale,
@@ -500,17 +451,4 @@ extern "C" int b200_act_quant_sum(const void* y, long long ldy, const int* slots
                                   float eps, void* q, long long ldq, float* scale, int M, int K, cudaStream_t stream) {
   if (M > 0 && (!slots || !weights || k <= 0 || k > AQ_MAX_K)) return -1;
   return act_quant_any(y, ldy, residual, ldr, gamma, eps, q, ldq, scale, nullptr, 0, M, K, AQ_SUM_NORM, ExpertRows{slots, weights, k}, stream);
-}
-
-extern "C" int b200_quant_blocks(const void* blocks, const float* tops, void* q, float* scale, int M, int K, cudaStream_t stream) {
-  if (M <= 0) return 0;
-  if (K <= 0 || (K % 128) != 0) return -1;
-  if ((reinterpret_cast<uintptr_t>(blocks) | reinterpret_cast<uintptr_t>(q)) & 15) return -2;
-  const int spans = (K + QB_SPAN - 1) / QB_SPAN;
-  const long long ctas = (static_cast<long long>(M) * spans + 7) / 8;
-  if (ctas > 2147483647ll) return -1;
-  launch_ex(quant_blocks_kernel, dim3(static_cast<unsigned>(ctas)), dim3(256), 0, stream, 0, static_cast<const int16_t*>(blocks), tops, static_cast<int8_t*>(q),
-            scale, M, K, spans);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
 }

@@ -20,15 +20,6 @@ int b200_w8a8_gemm(const void* xq, const float* sx, const void* wq, const float*
                    void* ws, size_t ws_bytes, void* counters, int counters_len, int* status,
                    int num_sms, int force_mode, cudaStream_t stream);
 
-// Rotated rows of silu(g) u, g and u the products of rows n and N / 2 + n of wq, as 16-bit blocks: blocks [M][N / 2] whole numbers, tops
-// [M][N / 256] the largest magnitude of each block of 128; element = number * top / 32767.  N % 256 == 0, everything on 16 bytes.
-int b200_w8a8_gemm_swiglu(const void* xq, const float* sx, const void* wq, const float* sw, void* blocks, float* tops, int M, int N, int K,
-                          int* status, int num_sms, cudaStream_t stream);
-// 1 where that is the faster way to the gated rows: the rule and its figures stand at the function
-int b200_w8a8_gemm_swiglu_takes(int M, int N, int K);
-// 16-bit blocks -> int8 rows and a scale per row (K % 128 == 0; blocks and q on 16 bytes, rows contiguous)
-int b200_quant_blocks(const void* blocks, const float* tops, void* q, float* scale, int M, int K, cudaStream_t stream);
-
 // Decode form (M <= 64): split-K thread-block clusters reduced through distributed shared memory; no scratch.
 // force_splits: 0 auto, else 1/2/4/8 CTAs per cluster along K.
 int b200_w8a8_gemm_decode(const void* xq, const float* sx, const void* wq, const float* sw, void* y,

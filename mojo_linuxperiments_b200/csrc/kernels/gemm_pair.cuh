@@ -148,8 +148,8 @@ struct PairLoop {
     tmem = *slot;
   }
 
-  // warp 0.  The weight rows of a tile: BN / 2 from n_tile * step on in CTA 0, as many from `second` rows further on in CTA 1
-  __device__ void produce(const CUtensorMap* tmap_x, const CUtensorMap* tmap_w, PairTiles tiles, int kblocks, int step = BN, int second = BN / 2) const {
+  // warp 0
+  __device__ void produce(const CUtensorMap* tmap_x, const CUtensorMap* tmap_w, PairTiles tiles, int kblocks) const {
     if ((threadIdx.x & 31) != 0) return;
     prefetch_tmap(tmap_x);
     prefetch_tmap(tmap_w);
@@ -158,7 +158,7 @@ struct PairLoop {
     uint32_t phase = 0;
     bool ok = true;
     while (ok && tiles.take(m_tile, n_tile)) {
-      const int row = m_tile * PAIR_M + static_cast<int>(rank) * 128, wrow = n_tile * step + static_cast<int>(rank) * second;
+      const int row = m_tile * PAIR_M + static_cast<int>(rank) * 128, wrow = n_tile * BN + static_cast<int>(rank) * (BN / 2);
       for (int kb = 0; kb < kblocks; ++kb) {
         ok = wait(empty(stage), phase ^ 1u, ST_TIMEOUT_SMEM_EMPTY);
         if (!ok) break;

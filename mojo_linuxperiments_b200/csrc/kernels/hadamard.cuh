@@ -89,51 +89,6 @@ __device__ __forceinline__ void fwht128_lane16(float2 (&v)[8], int lane) {
   for (int i = 0; i < 8; ++i) v[i] = mul2(v[i], s);
 }
 
-// The same rotation, before its scale, by one thread that holds a block as pairs v[i] = (element i, element i + 64): no lane is crossed.
-__device__ __forceinline__ void fwht128_thread(float2 (&v)[64]) {
-  const float2 minus = make_float2(-1.f, -1.f);
-#pragma unroll
-  for (int h = 1; h < 64; h *= 2)
-#pragma unroll
-    for (int i = 0; i < 64; ++i)
-      if (!(i & h)) {
-        const float2 a = v[i], b = v[i + h];
-        v[i] = add2(a, b);
-        v[i + h] = fma2(b, minus, a);
-      }
-#pragma unroll
-  for (int i = 0; i < 64; ++i) v[i] = make_float2(__fadd_rn(v[i].x, v[i].y), __fsub_rn(v[i].x, v[i].y));
-}
-
-// Rotated blocks on their way to the kernel that knows the row's scale: 128 whole numbers of 16 bits and the block's largest magnitude
-// `top` (after the rotation's 1/sqrt(128)); an element is number * top / 32767.  The step is a 65,534th of the block's range, the int8
-// step that follows a 254th of the row's, so at most one value in 250 rounds to the other side of an int8 edge and nothing moves by
-// more than that step.  A block with an infinity has top = infinity, one of NaN top = 0: both become zeros under the row's scale, as
-// they do when rows are quantised directly.
-// v: as fwht128_thread leaves it; element e of the block is put into word e / 2
-__device__ __forceinline__ float block16_pack(float2 (&v)[64], uint32_t (&w)[64]) {
-  float top = 0.f;
-#pragma unroll
-  for (int i = 0; i < 64; ++i) top = fmaxf(top, fmaxf(fabsf(v[i].x), fabsf(v[i].y)));
-  float scaled = top;
-  if (top < 0x1p-60f) {                        // 32,767 / top would leave the range of fp32
-    scaled = top * 0x1p64f;
-#pragma unroll
-    for (int i = 0; i < 64; ++i) v[i] = mul2(v[i], make_float2(0x1p64f, 0x1p64f));
-  }
-  const float r = scaled > 0.f ? __fdiv_rn(32767.f, scaled) : 0.f;
-  // 1.5 x 2^23 makes the sum's unit 1: rounded to nearest, the low half of the word is the number
-  const float2 rr = make_float2(r, r), magic = make_float2(12582912.f, 12582912.f);
-#pragma unroll
-  for (int i = 0; i < 64; ++i) v[i] = fma2(v[i], rr, magic);
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    w[i] = __byte_perm(__float_as_uint(v[2 * i].x), __float_as_uint(v[2 * i + 1].x), 0x5410);
-    w[32 + i] = __byte_perm(__float_as_uint(v[2 * i].y), __float_as_uint(v[2 * i + 1].y), 0x5410);
-  }
-  return __fmul_rn(top, 0.08838834764831845f);
-}
-
 // per-token scale from the row's largest rotated magnitude (a row of zeros quantises with scale 1)
 __device__ __forceinline__ float quant_scale_from_amax(float amax) {
   return (amax > 0.f) ? __fdiv_rn(amax, 127.f) : 1.f;

@@ -3,33 +3,23 @@
 // The epilogue turns 32 rows x 64 channels through shared memory, so that eight lanes write one row's 128 bytes: a thread owns
 // a token row in TMEM, and storing from there touches 32 rows per instruction with half a sector each.
 // The products and scales are those of the one-CTA kernel (w8a8_gemm.cu) in the same order: the results have the same bits.
-//
-// Gated form (GLU): Wq is gate rows above as many up rows, the result the rotated rows of silu(gate) up as 16-bit blocks (hadamard.cuh).
-// CTA 0 of a pair loads 128 gate rows and CTA 1 the up rows of the same channels, so a thread finds 128 gates and their ups in its
-// accumulator row: one rotation block, which it multiplies, rotates and packs in fp32 without crossing a lane.  What is left for the
-// next kernel is a stream of two bytes in, one out per element, instead of four in and a rotation that its shuffles bound.  The epilogue
-// (about 2,700 instructions per row and tile) hides under the main loop of the next tile from K = 2,048 on.  Linear and rows together, bf16 gate and up in
-// between | this way: 32,768 x 28,672 x 4,096 2,969 us | 2,794, 3,200 x 28,672 x 4,096 299 | 265, 1,024 x 28,672 x 4,096 96.6 | 91.3,
-// 8,000 x 11,264 x 2,048 184 | 163.
 #include "ptx.cuh"
 #include "api.h"
 #include "launch.cuh"
 #include "gemm_pair.cuh"
-#include "hadamard.cuh"
 #include <type_traits>
 
 namespace b200 {
 
 struct W8PairParams {
-  int M, N, m_tiles, n_tiles, kblocks;      // N: channels of the result
+  int M, N, m_tiles, n_tiles, kblocks;
   const float* sx; const float* sw;
   __nv_bfloat16* y; long long ldy;
-  int16_t* blocks; float* tops;         // GLU: [M][N] and [M][N / 128]
   int* status;
   unsigned long long limit_ns;
 };
 
-template <int BN, int STAGES, bool GLU>
+template <int BN, int STAGES>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 w8a8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ W8PairParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -40,63 +30,19 @@ w8a8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   PairTiles tiles(p.m_tiles, p.n_tiles);
   if (warp == 0) {
-    if constexpr (GLU) loop.produce(&tmap_x, &tmap_w, tiles, p.kblocks, BN / 2, p.N);
-    else loop.produce(&tmap_x, &tmap_w, tiles, p.kblocks);
+    loop.produce(&tmap_x, &tmap_w, tiles, p.kblocks);
     __syncwarp();
   } else if (warp == 1) {
     loop.issue(tiles, p.kblocks);
   } else {
-    constexpr int WIDTH = GLU ? BN / 2 : BN;      // channels of the result in a tile
     const int q = warp & 3;                 // TMEM lane quarter this warp may read
     uint8_t* piece = loop.pieces + (warp - 2) * PAIR_PIECE;
     int m_tile, n_tile;
     for (int idx = 0; tiles.take(m_tile, n_tile); ++idx) {
-      const int m0 = m_tile * PAIR_M + static_cast<int>(loop.rank) * 128 + q * 32, n0 = n_tile * WIDTH;
+      const int m0 = m_tile * PAIR_M + static_cast<int>(loop.rank) * 128 + q * 32, n0 = n_tile * BN;
       const float sxm = m0 + lane < p.M ? p.sx[m0 + lane] : 0.f;
       if (!loop.take_accumulator(idx)) break;
       const uint32_t t = loop.accumulator(idx) + (static_cast<uint32_t>(q * 32) << 16);
-      if constexpr (GLU) {
-        float2 v[64];
-#pragma unroll
-        for (int c = 0; c < 128; c += 16) {
-          uint32_t g[16], up[16];
-          tmem_ld_x16(t + c, g);
-          tmem_ld_x16(t + 128 + c, up);
-          tmem_ld_wait();
-          if (c == 112) loop.give_accumulator(idx);
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const float4 a = __ldg(reinterpret_cast<const float4*>(p.sw + n0 + c) + u), b = __ldg(reinterpret_cast<const float4*>(p.sw + p.N + n0 + c) + u);
-            const float s[4] = {a.x, a.y, a.z, a.w}, r[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float x = static_cast<float>(static_cast<int32_t>(g[4 * u + j])) * (s[j] * sxm);
-              const float h = __fdividef(x, 1.f + __expf(-x)) * (static_cast<float>(static_cast<int32_t>(up[4 * u + j])) * (r[j] * sxm));
-              if (c < 64) v[(c & 63) + 4 * u + j].x = h; else v[(c & 63) + 4 * u + j].y = h;
-            }
-          }
-        }
-        fwht128_thread(v);
-        uint32_t w[64];
-        const float top = block16_pack(v, w);
-        if (m0 + lane < p.M) p.tops[static_cast<long long>(m0 + lane) * (p.N >> 7) + n_tile] = top;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {                           // 64 channels of a row at a time: 128 bytes
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            *reinterpret_cast<uint4*>(piece + lane * 128 + ((u ^ (lane & 7)) << 4)) =
-                make_uint4(w[32 * half + 4 * u], w[32 * half + 4 * u + 1], w[32 * half + 4 * u + 2], w[32 * half + 4 * u + 3]);
-          __syncwarp();
-#pragma unroll
-          for (int it = 0; it < 8; ++it) {
-            const int row = it * 4 + (lane >> 3), u = lane & 7;
-            const uint4 x = *reinterpret_cast<const uint4*>(piece + row * 128 + ((u ^ (row & 7)) << 4));
-            if (m0 + row < p.M) *reinterpret_cast<uint4*>(p.blocks + static_cast<long long>(m0 + row) * p.N + n0 + 64 * half + 8 * u) = x;
-          }
-          __syncwarp();
-        }
-        continue;
-      }
       // CH channels (64, or 32 at the end of a tile): 16-byte unit u of row r sits at unit u ^ (r & 7)
       auto emit = [&](int c, auto width) {
         constexpr int CH = decltype(width)::value;
@@ -140,37 +86,29 @@ w8a8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
   loop.close();
 }
 
-template <int BN, int STAGES, bool GLU = false>
+template <int BN, int STAGES>
 static int launch_w8_pair(const CUtensorMap& tx, const CUtensorMap& tw, const W8PairParams& p, int pairs, cudaStream_t stream) {
   constexpr int SMEM = PairLoop<BN, STAGES, true>::SMEM;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(w8a8_gemm_pair_kernel<BN, STAGES, GLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    cudaError_t e = cudaFuncSetAttribute(w8a8_gemm_pair_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return -1000 - static_cast<int>(e);
     configured = true;
   }
-  launch_ex(w8a8_gemm_pair_kernel<BN, STAGES, GLU>, dim3(2 * pairs), dim3(GEMM_THREADS), SMEM, stream, 2, tx, tw, p);
+  launch_ex(w8a8_gemm_pair_kernel<BN, STAGES>, dim3(2 * pairs), dim3(GEMM_THREADS), SMEM, stream, 2, tx, tw, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -2000 - static_cast<int>(e);
-}
-
-static int pair_setup(W8PairParams& p, CUtensorMap& tx, CUtensorMap& tw, const void* xq, const float* sx, const void* wq, const float* sw, int M,
-                      int N, int K, int bn, int* status) {
-  p = W8PairParams{};
-  p.M = M; p.N = N; p.m_tiles = (M + PAIR_M - 1) / PAIR_M; p.n_tiles = (N + bn - 1) / bn; p.kblocks = (K + BLOCK_K - 1) / BLOCK_K;
-  p.sx = sx; p.sw = sw; p.status = status; p.limit_ns = 2000000000ull;
-  if (make_tmap_2d_u8(&tw, wq, static_cast<uint64_t>(K), static_cast<uint64_t>(N), static_cast<uint64_t>(K), bn / 2)) return -11;
-  if (make_tmap_2d_u8(&tx, xq, static_cast<uint64_t>(K), static_cast<uint64_t>(M), static_cast<uint64_t>(K), 128)) return -12;
-  return 0;
 }
 
 // bf16 output, N and ldy multiples of eight, y on 16 bytes; bn: channels per tile
 int w8a8_gemm_pair(const void* xq, const float* sx, const void* wq, const float* sw, void* y, int M, int N, int K, int ldy, int bn,
                    int* status, int num_sms, cudaStream_t stream) {
   W8PairParams p;
+  p.M = M; p.N = N; p.m_tiles = (M + PAIR_M - 1) / PAIR_M; p.n_tiles = (N + bn - 1) / bn; p.kblocks = (K + BLOCK_K - 1) / BLOCK_K;
+  p.sx = sx; p.sw = sw; p.y = static_cast<__nv_bfloat16*>(y); p.ldy = ldy; p.status = status; p.limit_ns = 2000000000ull;
   CUtensorMap tw, tx;
-  if (int rc = pair_setup(p, tx, tw, xq, sx, wq, sw, M, N, K, bn, status)) return rc;
-  p.y = static_cast<__nv_bfloat16*>(y); p.ldy = ldy;
+  if (make_tmap_2d_u8(&tw, wq, static_cast<uint64_t>(K), static_cast<uint64_t>(N), static_cast<uint64_t>(K), bn / 2)) return -11;
+  if (make_tmap_2d_u8(&tx, xq, static_cast<uint64_t>(K), static_cast<uint64_t>(M), static_cast<uint64_t>(K), 128)) return -12;
   const int pairs = pair_count(static_cast<long long>(p.m_tiles) * p.n_tiles, num_sms);
   switch (bn) {
     case 256: return launch_w8_pair<256, 6>(tx, tw, p, pairs, stream);
@@ -182,23 +120,3 @@ int w8a8_gemm_pair(const void* xq, const float* sx, const void* wq, const float*
 }
 
 }  // namespace b200
-
-using namespace b200;
-
-// The rows kernel saves 0.7 us per million gated elements; the longer epilogue of the last tile and the fixed width cost 2 to 5 us a
-// call: 200 x 28,672 x 4,096 (2.9 million) 38.2 us against 36.4, 1,000 x 11,264 x 2,048 (5.6 million) 31.4 against 29.8.  Below K = 2,048 the
-// epilogue no longer hides: 8,000 x 4,096 x 1,024 95.5 against 89.5.
-extern "C" int b200_w8a8_gemm_swiglu_takes(int M, int N, int K) {
-  return N % 256 == 0 && K >= 2048 && K % 16 == 0 && static_cast<long long>(M) * (N / 2) >= 8000000;
-}
-
-extern "C" int b200_w8a8_gemm_swiglu(const void* xq, const float* sx, const void* wq, const float* sw, void* blocks, float* tops, int M, int N, int K,
-                                     int* status, int num_sms, cudaStream_t stream) {
-  if (M <= 0 || N <= 0 || (N % 256) || K <= 0 || (K % 16)) return -1;
-  if ((reinterpret_cast<uintptr_t>(xq) | reinterpret_cast<uintptr_t>(wq) | reinterpret_cast<uintptr_t>(blocks) | reinterpret_cast<uintptr_t>(sw)) & 15) return -2;
-  W8PairParams p;
-  CUtensorMap tw, tx;
-  if (int rc = pair_setup(p, tx, tw, xq, sx, wq, sw, M, N, K, 256, status)) return rc;
-  p.N = N / 2; p.blocks = static_cast<int16_t*>(blocks); p.tops = tops;
-  return launch_w8_pair<256, 6, true>(tx, tw, p, pair_count(static_cast<long long>(p.m_tiles) * p.n_tiles, num_sms), stream);
-}

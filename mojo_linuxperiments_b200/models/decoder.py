@@ -140,10 +140,8 @@ class Decoder:
         W = self.w["layers"][l]
         if self.moe is not None:
             return self.moe.forward(W, xq, sx, xn, pending)
-        if self.comm.world == 1:
-            hq, sh = L.swiglu_rows(xq, sx, W["gate_up"].qweight, W["gate_up"].scale)
-        else:       # as in the token-sharded prefill, whose rows this path has to repeat bit by bit
-            hq, sh = L.act_quant(L.w8a8_gemm(xq, sx, W["gate_up"].qweight, W["gate_up"].scale), mode=L.AQ_SWIGLU)
+        gu = L.w8a8_gemm(xq, sx, W["gate_up"].qweight, W["gate_up"].scale)
+        hq, sh = L.act_quant(gu, mode=L.AQ_SWIGLU)
         return self._row_parallel(hq, sh, W["down"])
 
     # -- full forward ------------------------------------------------------------------------------------------

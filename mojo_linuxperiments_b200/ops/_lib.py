@@ -66,9 +66,6 @@ F = c_float
 class _Sig:
     b200_w8a8_gemm_ws_bytes = (c_size_t, [I, I, I, I])
     b200_w8a8_gemm = (I, [P, P, P, P, P, P, I, I, I, I, I, P, c_size_t, P, I, P, I, I, P])
-    b200_w8a8_gemm_swiglu = (I, [P, P, P, P, P, P, I, I, I, P, I, P])
-    b200_quant_blocks = (I, [P, P, P, P, I, I, P])
-    b200_w8a8_gemm_swiglu_takes = (I, [I, I, I])
     b200_w8a8_gemm_decode = (I, [P, P, P, P, P, P, I, I, I, I, I, P, I, I, P])
     b200_w8a8_gemm_decode_resident_clusters = (I, [I, I])
     b200_w8a8_gemm_decode_takes = (I, [I, I, I, I])

@@ -99,40 +99,6 @@ def w8a8_gemm(xq: torch.Tensor, sx: torch.Tensor, wq: torch.Tensor, sw: torch.Te
     return out
 
 
-def w8a8_gemm_swiglu(xq: torch.Tensor, sx: torch.Tensor, wq: torch.Tensor, sw: torch.Tensor):
-    """Rotated rows of silu(g) * u with g | u = the int8 linear of ``w8a8_gemm`` (gate rows of ``wq`` above up rows), as 16-bit blocks:
-    (int16 [M, F], largest magnitude of each block of 128, fp32 [M, F / 128]); an element is number * magnitude / 32767."""
-    assert xq.is_cuda and xq.dtype == torch.int8 and wq.dtype == torch.int8 and xq.is_contiguous() and wq.is_contiguous()
-    M, K = xq.shape
-    N = wq.shape[0]
-    assert wq.shape[1] == K
-    blocks = torch.empty((M, N // 2), dtype=torch.int16, device=xq.device)
-    tops = torch.empty((M, N // 256), dtype=torch.float32, device=xq.device)
-    rc = _lib.lib().b200_w8a8_gemm_swiglu(xq.data_ptr(), sx.data_ptr(), wq.data_ptr(), sw.data_ptr(), blocks.data_ptr(), tops.data_ptr(), M, N, K,
-                                          default_workspace(xq.device).status.data_ptr(), _lib.num_sms(xq.device.index), _lib.stream())
-    _lib.check(rc, "w8a8_gemm_swiglu")
-    return blocks, tops
-
-
-def quant_blocks(blocks: torch.Tensor, tops: torch.Tensor):
-    """16-bit blocks -> (int8 rows, fp32 scale per row)."""
-    M, K = blocks.shape
-    assert blocks.dtype == torch.int16 and blocks.is_contiguous() and tops.is_contiguous() and tops.shape == (M, K // 128) and K % 128 == 0
-    q = torch.empty((M, K), dtype=torch.int8, device=blocks.device)
-    s = torch.empty((M,), dtype=torch.float32, device=blocks.device)
-    _lib.check(_lib.lib().b200_quant_blocks(blocks.data_ptr(), tops.data_ptr(), q.data_ptr(), s.data_ptr(), M, K, _lib.stream()), "quant_blocks")
-    return q, s
-
-
-def swiglu_rows(xq: torch.Tensor, sx: torch.Tensor, wq: torch.Tensor, sw: torch.Tensor):
-    """(int8 rows, scales) of silu(gate) * up, rotated: the operand of a down projection.  Gate and rotation are applied inside the
-    linear where the two-CTA kernel runs, by the activation kernel where another one does."""
-    if _lib.lib().b200_w8a8_gemm_swiglu_takes(xq.shape[0], wq.shape[0], xq.shape[1]) == 1 and not (
-            wq.data_ptr() | xq.data_ptr() | sw.data_ptr()) & 15:
-        return quant_blocks(*w8a8_gemm_swiglu(xq, sx, wq, sw))
-    return act_quant(w8a8_gemm(xq, sx, wq, sw), mode=AQ_SWIGLU)
-
-
 # up to this many 128-channel tiles per SM a small-M GEMM goes to the weight-streaming cluster kernel
 _DECODE_TILE_WAVES = int(os.environ.get("B200RT_DECODE_TILE_WAVES", "4"))
 

@@ -252,72 +252,6 @@ def test_fused_linear_inline_prologue_for_a_few_tokens(mode, m, n, k):
     assert torch.equal(yg, y1)
 
 
-def _hadamard():
-    h = torch.ones((1, 1), dtype=torch.float64, device="cuda")
-    while h.shape[0] < 128:
-        h = torch.cat([torch.cat([h, h], 1), torch.cat([h, -h], 1)])
-    return h * 128 ** -0.5
-
-
-@pytest.mark.parametrize("M,F,K", [(1, 128, 16), (129, 128, 128), (256, 256, 1040), (257, 384, 256), (700, 1152, 1024), (511, 640, 2048)])
-def test_swiglu_linear_blocks(M, F, K):
-    from mojo_linuxperiments_b200.ops import linear as L
-    g = torch.Generator(device="cuda").manual_seed(M + F + K)
-    xq = torch.randint(-127, 128, (M, K), dtype=torch.int8, device="cuda", generator=g)
-    wq = torch.randint(-127, 128, (2 * F, K), dtype=torch.int8, device="cuda", generator=g)
-    sx = torch.rand(M, device="cuda", generator=g) * 1e-2 + 1e-4
-    sw = torch.rand(2 * F, device="cuda", generator=g) * (6e-2 * K ** -0.5)
-    if M > 4:
-        sx[0], sx[1], sx[2], sx[3] = 50.0, 0.0, 1e-16, 1e-18       # gates far out on both sides, nothing, products near 1e-34 and 1e-38
-    blocks, tops = L.w8a8_gemm_swiglu(xq, sx, wq, sw)
-    v = (xq.double() @ wq.double().t()) * (sw.double() * sx.double()[:, None])
-    gate, up = v[:, :F], v[:, F:]
-    h = (gate * torch.sigmoid(gate) * up).view(M, F // 128, 128)
-    want = h @ _hadamard()
-    top = tops.double()[:, :, None]
-    # gate, up and their product: about ten roundings, and the exponential's argument is |gate| wide; seven butterfly stages, each off by
-    # half a unit of a sum of magnitudes; half a step of the whole number.  1e-37: what flushes to zero
-    size = h.abs().sum(-1, keepdim=True) * 128 ** -0.5
-    wide = (gate.abs().view(M, F // 128, 128) * h.abs()).sum(-1, keepdim=True) * 128 ** -0.5
-    bound = (20 * size + 4 * wide) * 2.0 ** -23 + top / 65534 + 1e-37
-    assert ((blocks.double().view(M, F // 128, 128) * top / 32767 - want).abs() <= bound).all()
-    assert ((top[:, :, 0] - want.abs().amax(-1)).abs() <= bound[:, :, 0]).all()
-    q, s = L.quant_blocks(blocks, tops)
-    amax = tops.amax(-1)
-    assert torch.equal(s, torch.where(amax > 0, amax / torch.full_like(amax, 127), torch.ones_like(amax)))
-    exact = (blocks.double().view(M, F // 128, 128) * top / 32767).view(M, F) / s.double()[:, None]
-    assert ((q.double() - exact).abs() <= 0.5 + 127 * 2.0 ** -21)[s > 1e-37].all()      # half a step, and three roundings of up to 127 steps
-    if M > 4:
-        assert q[0].abs().max() == 127 and not q[1].any()
-
-
-def test_quant_blocks_without_a_finite_scale():
-    from mojo_linuxperiments_b200.ops import linear as L
-    blocks = torch.randint(-32767, 32768, (3, 384), dtype=torch.int16, device="cuda")
-    tops = torch.tensor([[1.0, 2.0, 3.0], [1.0, float("inf"), 3.0], [0.0, 2.0, 0.0]], device="cuda")
-    q, s = L.quant_blocks(blocks, tops)
-    assert q[0].any() and s[0] == 3.0 / 127 and not q[1].any() and torch.isinf(s[1])
-    assert not q[2, :128].any() and q[2, 128:256].any() and not q[2, 256:].any()
-
-
-@pytest.mark.parametrize("M,F,K", [(100, 256, 1024), (600, 768, 2048), (4000, 1920, 2048), (4001, 2048, 2048), (4096, 2048, 1024)])
-def test_swiglu_rows_either_way(M, F, K):
-    from mojo_linuxperiments_b200.ops import linear as L
-    g = torch.Generator(device="cuda").manual_seed(M)
-    xq = torch.randint(-127, 128, (M, K), dtype=torch.int8, device="cuda", generator=g)
-    wq = torch.randint(-127, 128, (2 * F, K), dtype=torch.int8, device="cuda", generator=g)
-    sx, sw = torch.rand(M, device="cuda", generator=g) * 1e-2, torch.rand(2 * F, device="cuda", generator=g) * (3e-2 * K ** -0.5)
-    v = (xq.double() @ wq.double().t()) * (sw.double() * sx.double()[:, None])
-    want = ((v[:, :F] * torch.sigmoid(v[:, :F]) * v[:, F:]).view(M, F // 128, 128) @ _hadamard()).view(M, F)
-
-    def off(q, s):
-        return ((q.double() * s.double()[:, None] - want).norm() / want.norm()).item()
-
-    here = off(*L.swiglu_rows(xq, sx, wq, sw))
-    before = off(*L.act_quant(L.w8a8_gemm(xq, sx, wq, sw), mode=L.AQ_SWIGLU))
-    assert here <= before * 1.001        # no further from 64 bits than with gate and up rounded to bf16 in between
-
-
 @pytest.mark.parametrize("M,K", [(33, 18560), (64, 20480), (17, 20480), (64, 2048)])
 def test_rows_quantised_inside_the_launch_up_to_the_longest(M, K):
     """A parked row may reach into the exchange buffer of the 64-token form.  Rounding may take a number to the other side of an int8 edge: as in
@@ -331,3 +265,22 @@ def test_rows_quantised_inside_the_launch_up_to_the_longest(M, K):
     y = L.fused_linear(x, wq, sw)
     default_workspace(x.device).check_status()
     assert torch.allclose(y.double(), want, rtol=2e-2, atol=2e-2 * want.abs().max().item())
+
+
+@pytest.mark.parametrize("F,K", [(2048, 2048), (14336, 1024)])
+def test_mlp_rows_do_not_depend_on_the_rows_beside_them(F, K):
+    """The rotated int8 rows behind gate and up have the same bits in a prompt of a hundred rows and in the largest call: the linears are whole
+    numbers until their scales, and a row is gated, rotated and rounded by itself."""
+    from types import SimpleNamespace as NS
+
+    from mojo_linuxperiments_b200.models.decoder import Decoder
+    g = torch.Generator(device="cuda").manual_seed(F)
+    M = 8000000 // F + 2
+    xq = torch.randint(-127, 128, (M, K), dtype=torch.int8, device="cuda", generator=g)
+    wq = torch.randint(-127, 128, (2 * F, K), dtype=torch.int8, device="cuda", generator=g)
+    sx, sw = torch.rand(M, device="cuda", generator=g) * 1e-2, torch.rand(2 * F, device="cuda", generator=g) * (3e-2 * K ** -0.5)
+    d = NS(w={"layers": [{"gate_up": NS(qweight=wq, scale=sw), "down": None}]}, moe=None, comm=NS(world=1), _row_parallel=lambda hq, sh, w: (hq, sh))
+    q, s = Decoder._mlp(d, 0, xq, sx, None)
+    for n in (100, 300):
+        qn, sn = Decoder._mlp(d, 0, xq[:n], sx[:n], None)
+        assert torch.equal(qn, q[:n]) and torch.equal(sn, s[:n]), n
