@@ -269,7 +269,7 @@ int b200_f32_gemm(const float* x, long long ldx, const float* w, long long ldw, 
 // the same on the tensor cores, in three bf16 parts per operand (x, w, ldx and ldw on 16 bytes; splits: 0 or CTAs along K)
 int b200_f32_gemm_tc(const float* x, long long ldx, const float* w, long long ldw, int M, int N, int K,
                      const b200_dense_epilogue* epi, int* status, int splits, cudaStream_t stream);
-int b200_f32_gemm_tc_takes(int M, int N, int K);      // 1 where that is faster; the rule and its figures stand at the function
+int b200_f32_gemm_tc_takes(int M, int N, int K);      // 1 where that is faster and no further from exact; the rule and its figures stand at the function
 
 // Grouped forms.  decode: M = most rows of a group, rows_total = rows of x.  prefill: row lists only.
 int b200_bf16_gemm_grouped(const void* x, long long ldx, const void* w, long long ldw, int rows_total, int N, int K,

@@ -6,7 +6,7 @@
 //     16 bytes of each column's row at a time, and the first block of weights is on its way before the kernel waits for
 //     its input (row lists: once the group is known to have rows).  Bound by HBM: 2 rows x 16,384 x 2,048 in 25 us = 5.4 TB/s (260 us with the 64 x 64 tiles of one
 //     CTA per tile that served all sizes before), 2 rows x 2,048 x 8,192 in 18 us (594 us).
-//   * above that, where the tensor cores do not take the call (f32_gemm_tc.cu: K below 512, grouped calls, addresses or pitches off 16
+//   * above that, where the tensor cores do not take the call (f32_gemm_tc.cu: K below 2,048, grouped calls, addresses or pitches off 16
 //     bytes), 64 x 128 tiles through a three-stage cp.async ring, 4 x 8 outputs per thread.  Two fused multiply-adds
 //     are one instruction (fma.rn.f32x2: the even and the odd k of an output have a sum each), which leaves issue slots for
 //     the shared-memory reads.  Where the tiles do not fill the chip, a cluster of CTAs shares out K and adds its partial tiles

@@ -1,10 +1,11 @@
-// fp32 linear above a few rows on the tensor cores, without giving up a bit of its operands: v[m,n] = sum_k X[m,k] W[n,k].
+// fp32 linear above a few rows on the tensor cores, from the same operands bit for bit: v[m,n] = sum_k X[m,k] W[n,k].
 //
-// An fp32 number is the sum of three bf16 numbers, x = x1 + x2 + x3 (eight bits each; the remainders are exact), so a product is a sum
-// of nine bf16 products.  Six of them are multiplied (tcgen05.mma kind::f16, fp32 accumulators): x1 w1, x1 w2, x2 w1, x2 w2, x1 w3,
-// x3 w1; the other three are below 2^-26 of the product.  The tensor core cuts its sums off where fp32 ends instead of rounding them, so
-// no sum is left there for long: x1 w1 of 32 k (two MMAs) is added to fp32 registers, rounded, before the next 32 start, the sum of 256 k to
-// that of all before in shared memory; the five small products have an accumulator of their own, 2^-8 of the size, that is added every 1,024 k.
+// An fp32 number is the sum of three bf16 numbers, x = x1 + x2 + x3 (eight bits each; the remainders are exact from magnitudes of 2^-110 on,
+// below that the last bits are smaller than bf16's smallest number), so a product is a sum of nine bf16 products.  Eight of them are multiplied
+// (tcgen05.mma kind::f16, fp32 accumulators); x3 w3 is at most 2^-34 of the product.  The tensor core cuts its sums off where fp32 ends instead of
+// rounding them, so no sum is left there for long: x1 w1 of 32 k (two MMAs) is added to fp32 registers, rounded, before the next 32 start, the sum
+// of 256 k to that of all before in shared memory; the seven small products have an accumulator of their own, 2^-8 of the size, that is added every
+// 1,024 k.
 //
 // What comes out is not finite if an operand is not (the remainder of an infinity is NaN), or if the sum overflows: such an output is
 // computed again with fused multiply-adds, which is what decides between infinity and NaN.
@@ -14,11 +15,12 @@
 // between they take the finished sums out of tensor memory.  The last issues the MMAs.  Where the tiles do not fill the chip a cluster shares
 // out K and adds its partial tiles through distributed shared memory in rank order.
 //
-// Bound by issue slots (65 % of them; splitting is 9 instructions per two elements, and every 32 k of a tile 64 KB of operands change
-// their form), tensor cores at 40 %.  On the CUDA cores | here, us: 380 rows x 16,384 x 2,048 690 | 204 (125 TFLOP/s, the fp32 pipe ends at 74),
-// 380 x 2,048 x 8,192 370 | 116, 380 x 2,048 x 2,048 106 | 38, 65 x 16,384 x 2,048 237 | 68, 9 x 2,048 x 2,048 33 | 16.
-// Against 64 bits, operands of random signs, K = 512, 2,048, 8,192: 1.5e-7, 2.6e-7, 4.1e-7 | 0.8e-7, 0.9e-7, 1.0e-7; all of one sign: 0.55e-7,
-// 0.80e-7, 0.90e-7 | 0.58e-7, 0.58e-7, 0.58e-7.
+// Bound by issue slots (splitting is 9 instructions per two elements, and every 32 k of a tile 64 KB of operands change
+// their form), tensor cores at a half.  On the CUDA cores | here, us: 380 rows x 16,384 x 2,048 691 | 211 (121 TFLOP/s, the fp32 pipe ends at 74; 204
+// without x2 w3 and x3 w2, which are up to 2^-24 of a product), 380 x 2,048 x 8,192 371 | 118, 380 x 2,048 x 2,048 106 | 41, 65 x 16,384 x 2,048 239 | 70,
+// 9 x 2,048 x 2,048 33 | 16.
+// Error against 64 bits (2-norms), CUDA cores | here, 1e-7: operands of random signs, K = 2,048, 8,192 2.1 | 0.9, 4.1 | 1.0; all of one sign 0.60 | 0.58, 0.90 | 0.58;
+// near 1 0.67 | 0.47, 1.0 | 0.5; all operands 1.00388 with random signs 0.93 | 0.50, 1.10 | 0.53.
 #include "ptx.cuh"
 #include "api.h"
 #include "launch.cuh"
@@ -109,7 +111,9 @@ __global__ void __launch_bounds__(FC_THREADS, 1) f32_gemm_tc_kernel(const __grid
 #pragma unroll
         for (int k = 0; k < 2; ++k) {             // 16 k of a part: 32 bytes; parts are 64 bytes apart
           umma_f16_ss(main, x12 + 2 * k, w12 + 2 * k, IDESC, k);
-          umma_f16_ss(small, x12 + 2 * k, xw3 + 4 + 2 * k, IDESC, i % FC_PERIOD > 0 || k > 0);
+          umma_f16_ss(small, x12 + 4 + 2 * k, xw3 + 4 + 2 * k, IDESC, i % FC_PERIOD > 0 || k > 0);
+          umma_f16_ss(small, xw3 + 2 * k, w12 + 4 + 2 * k, IDESC, 1);
+          umma_f16_ss(small, x12 + 2 * k, xw3 + 4 + 2 * k, IDESC, 1);
           umma_f16_ss(small, xw3 + 2 * k, w12 + 2 * k, IDESC, 1);
           umma_f16_ss(small, x12 + 4 + 2 * k, w12 + 4 + 2 * k, IDESC, 1);
           umma_f16_ss(small, x12 + 2 * k, w12 + 4 + 2 * k, IDESC, 1);
@@ -278,9 +282,11 @@ static int f32_tc_clusters(int size) {
 
 using namespace b200;
 
-// Up to 8 rows the streaming kernel of f32_gemm.cu.  Shorter sums take as long there (9 x 256 x 256 5.8 us | 5.6, 380 x 256 x 256 8.2 | 8.0) and
-// lose least; at K = 512 it is 9 x 16 x 512 7.3 | 6.2, 130 x 256 x 512 8.8 | 8.9, 380 x 4,096 x 512 53 | 22.
-extern "C" int b200_f32_gemm_tc_takes(int M, int N, int K) { return M > 8 && K >= 512 && N <= FC_MAX_N; }
+// Up to 8 rows the streaming kernel of f32_gemm.cu.  Shorter sums lose to the CUDA cores where all products have one sign, since cuts add up and
+// rounding does not: the error is 0.6e-7 at any length here, there 0.50e-7 at K = 512, 0.60 at 1,024 to 2,048, 0.72 at 3,072 (the other way round for
+// mixed signs: 1.2, 1.6, 2.1, 2.6 against 0.8 to 0.9).  6 widths x 6 numbers of rows: further from 64 bits than the CUDA cores at 1,536 and
+// 1,792, not from 2,048 on.  Time is not the reason: 380 x 4,096 x 512 53 us there, 23 here.
+extern "C" int b200_f32_gemm_tc_takes(int M, int N, int K) { return M > 8 && K >= 2048 && N <= FC_MAX_N; }
 
 // x, w, ldx and ldw on 16 bytes; splits: 0 or 1..8 CTAs along K
 extern "C" int b200_f32_gemm_tc(const float* x, long long ldx, const float* w, long long ldw, int M, int N, int K, const b200_dense_epilogue* epi,

@@ -378,21 +378,24 @@ def test_bf16_linear_of_two_ctas_per_tile(M, N, K, bn):
         assert (got - ref).norm() <= 4e-3 * ref.norm()
 
 
-@pytest.mark.parametrize("splits", [0, 1, 2, 8])
-@pytest.mark.parametrize("M,N,K", [(1, 4, 32), (9, 128, 33), (16, 129, 511), (127, 5, 512), (128, 300, 1027), (129, 256, 2049), (400, 130, 4096)])
+@pytest.mark.parametrize("splits", range(9))
+@pytest.mark.parametrize("M,N,K", [(1, 4, 32), (9, 128, 33), (16, 129, 511), (127, 5, 512), (128, 300, 1027), (129, 256, 2049), (400, 130, 4096), (40, 66, 2048)])
 def test_f32_linear_in_three_bf16_parts(M, N, K, splits):
-    """Edges of the 128 x 128 tiles, of blocks of 32 k, of the periods of 256 and 1,024 k, one block per split; what lies beyond K or M does
-    not matter.  Splitting is exact but for products below 2^-26, a sum of 32 k is cut off at 2^-23, sums of sums are rounded: no further from
-    64 bits than the sums of the CUDA cores from K = 512 on, shorter sums within 1e-7.  Where all products have one sign the cuts add up: two
-    per block, each at most 2^-23 and half of that on average, 1.2e-7."""
+    """Every split (0: as the rule has it), edges of the 128 x 128 tiles, of blocks of 32 k, of the periods of 256 and 1,024 k, one block per split;
+    what lies beyond K or M does not matter.  Splitting is exact but for products of 2^-34, a sum of 32 k is cut off at 2^-23, sums of sums are
+    rounded: no further from 64 bits than the sums of the CUDA cores for the calls that go there.  Forced: two cuts per block, each at most 2^-23
+    and half of that on average, 1.2e-7 of the blocks' sums, which add up where all products have one sign; a dozen roundings of the sum so far,
+    0.3e-7 each and half of it large on average, as a root of squares 0.6e-7: 1.5e-7 together for the lengths that the rule leaves out."""
     from mojo_linuxperiments_b200.ops import dense as D
     g = torch.Generator(device=DEV).manual_seed(M + N + K)
-    for kind in ("signs", "positive", "sizes"):
+    for kind in ("signs", "positive", "sizes", "last bits"):
         X, W = torch.randn((M, K), generator=g, device=DEV), torch.randn((N, K), generator=g, device=DEV) * K ** -0.5
         if kind == "positive":
             X, W = X.abs(), W.abs()
         if kind == "sizes":
             X = X * torch.exp2(torch.randint(-20, 20, (M, K), generator=g, device=DEV).float())
+        if kind == "last bits":                            # the second and third parts are as large as they can be: x2 w3 + x3 w2 is 2^-24 of x w
+            X, W = 1.0038833618164062 * X.sign(), 1.0038833618164062 * W.sign()
         x = torch.full((M + 1, (K + 3) // 4 * 4 + 4), float("nan"), device=DEV)[:M]
         x[:, :K] = X
         w = torch.full((N, (K + 3) // 4 * 4), float("nan"), device=DEV)
@@ -403,7 +406,35 @@ def test_f32_linear_in_three_bf16_parts(M, N, K, splits):
             y = D.linear(x, D.DenseW(w, N, K), force=force)[:, :N]
             return ((y.double() - want).norm() / want.norm()).item()
 
-        assert off(splits if splits else 4) <= max(off(-1), 1.2e-7 if kind == "positive" else 1e-7 if K < 512 else 0.0), kind
+        most = 0.0 if splits == 0 else 1.5e-7 if K < 2048 else 1.2e-7 if kind == "positive" else 0.0
+        assert off(splits) <= max(off(-1), most), kind
+
+
+@pytest.mark.parametrize("M,N,K", [(9, 256, 2048), (70, 2050, 2048), (300, 520, 2500)])
+def test_f32_linears_with_their_epilogues_on_the_tensor_cores(M, N, K):
+    """The calls that the rule sends there, with a gate and up (interleaved columns) and with a residual, against 64 bits and the CUDA cores: 2e-7 of
+    the sum, tanh and the exponential two units more."""
+    from mojo_linuxperiments_b200.ops import _lib
+    from mojo_linuxperiments_b200.ops import dense as D
+    assert _lib.lib().b200_f32_gemm_tc_takes(M, N, K) == 1
+    g = torch.Generator(device=DEV).manual_seed(M)
+    x = D.rows(M, K, torch.float32, DEV)
+    x.normal_(generator=g)
+    W = torch.randn((N, K), generator=g, device=DEV) * K ** -0.5
+    w = D.DenseW.of(W, torch.float32, DEV)
+    v = x[:, :K].double() @ W.double().t()
+    gate, up = v[:, 0::2].clamp(max=1.0), v[:, 1::2].clamp(-1.0, 1.0)
+    glu = gate * torch.sigmoid(1.702 * gate) * (up + 1)
+    s0 = torch.randn((M, D.padded(N)), generator=g, device=DEV)
+    norm = D.DynamicTanh.of(0.7, torch.randn(N, generator=g, device=DEV), torch.randn(N, generator=g, device=DEV), DEV)
+    new = s0[:, :N].double() + 0.5 * v
+    for force in (0, -1):
+        assert (D.linear_glu(x, w, 1.0, force=force)[:, :N // 2].double() - glu).norm() <= 5e-7 * glu.norm()
+        s, out = s0.clone(), D.rows(M, N, torch.float32, DEV)
+        D.linear_residual(x, w, s, 0.5, norm, out, force=force)
+        want = torch.tanh(norm.alpha * new) * norm.w[:N].double() + norm.b[:N].double()
+        assert (s[:, :N].double() - new).norm() <= 3e-7 * new.norm() and (out[:, :N].double() - want).norm() <= 5e-7 * want.norm()
+    _ok()
 
 
 def test_f32_linear_in_three_parts_where_it_is_not_finite():
@@ -581,7 +612,7 @@ def test_paged_prefill_attention_drops_the_query_tile_without_pages(H, G):
 
 def test_f32_linear_takes_the_values_of_force_that_choose_a_bf16_tile():
     from mojo_linuxperiments_b200.ops import dense as D
-    x, w = torch.randn((16, 1024), device=DEV), D.DenseW.of(torch.randn((200, 1024), device=DEV), torch.float32, DEV)
+    x, w = torch.randn((16, 2048), device=DEV), D.DenseW.of(torch.randn((200, 2048), device=DEV), torch.float32, DEV)
     want = D.linear(x, w)[:, :200]
     for force in (9, 64, 256, -64, -256):
         assert torch.equal(D.linear(x, w, force=force)[:, :200], want), force
