@@ -28,6 +28,8 @@ int b200_w8a8_gemm_decode(const void* xq, const float* sx, const void* wq, const
 
 int b200_w8a8_gemm_decode_resident_clusters(int m, int splits);
 int b200_w8a8_gemm_decode_takes(int M, int N, int K, int num_sms);
+// which form of the 64-token kernel a launch is: 2 * CTAs along K + (seven stages); one [9]: clusters of s CTAs that run at once, one CTA per SM
+int b200_w8a8_gemm_decode_ring(int tiles, int kblocks, int tokens, int splits, int fixed, const int* one);
 
 // Activation prologue carried inside a decode GEMM launch (quantiser CTAs of the same grid, see quant_row.cuh).
 // mode: 1 rotate + quantise x [M][K]; 2 RMSNorm(gamma, eps) first; 3 residual += x (bf16, in place) then RMSNorm of the
@@ -275,6 +277,7 @@ int b200_f32_gemm_tc_takes(int M, int N, int K);      // 1 where that is faster 
 int b200_bf16_gemm_grouped(const void* x, long long ldx, const void* w, long long ldw, int rows_total, int N, int K,
                            const b200_dense_epilogue* epi, const b200_gemm_groups* g, int* status, int num_sms, int force_bn,
                            cudaStream_t stream);
+int b200_bf16_gemm_decode_ring(int clusters, int kblocks, int tokens, int splits, int num_sms);      // 1: six stages, 0: three
 int b200_bf16_gemm_decode_grouped(const void* x, long long ldx, const void* w, long long ldw, int M, int rows_total, int N, int K,
                                   const b200_dense_epilogue* epi, const b200_gemm_groups* g, int* status, int num_sms, int splits,
                                   cudaStream_t stream);

@@ -38,12 +38,12 @@ __host__ __device__ __forceinline__ int bd_slice0(int r, int S) { return 4 * ((3
 constexpr int BD_XROW = 144;
 
 // Two CTAs per SM for every number of tokens: with one CTA and six stages of the 64-token form a step of eight layers took 585 us at 40 x 300, with two
-// and three stages 545.
+// and three stages 545.  A 64-token grid of no more than a CTA per SM has six stages (bd_deep).
 template <int BN, int STAGES>
 constexpr int bd_smem_bytes() { return STAGES * (128 + BN) * 128 + BN * BD_XROW * 4 + 1024 + 256; }
 
 template <int BN, int STAGES>
-__global__ void __launch_bounds__(GEMM_THREADS, 2)
+__global__ void __launch_bounds__(GEMM_THREADS, BN * STAGES > 3 * 64 ? 1 : 2)
 bf16_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                         const __grid_constant__ BfDecodeParams p) {
   constexpr int A_BYTES = 128 * 128, B_BYTES = BN * 128, STAGE_BYTES = A_BYTES + B_BYTES;
@@ -227,6 +227,13 @@ static int bd_resident(int S, int num_sms, int per_sm) {
   }
 }
 
+// 33 tokens and more: six stages where the grid is no more than a CTA per SM, unless a CTA has too few blocks to fill them.  us, three | six stages, same split, at
+// 33 and 64 tokens: 512 x 14,336 13.5, 14.1 | 11.0, 11.9; 1,536 x 4,096 6.9, 8.0 | 6.6, 7.3; 4,096 x 8,192 17.2, 18.2 | 14.7, 15.3; 1,536 x 1,024 at 64 5.4 |
+// 4.9; the other way round 4,096 x 1,024 at 33 5.4 | 5.8, 1,024 x 2,048 4.5 | 4.6.
+static bool bd_deep(int clusters, int kblocks, int tokens, int S, int num_sms) {
+  return clusters <= bd_resident(S, num_sms, 1) && ((kblocks + S - 1) / S >= 8 || tokens > 48);
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -274,8 +281,14 @@ static int bf16_decode_any(const void* x, long long ldx, const void* w, long lon
   switch (bn) {
     case 16: return launch_bf16_decode<16, 5>(tw, tx, p, grid, stream);
     case 32: return launch_bf16_decode<32, 4>(tw, tx, p, grid, stream);
-    default: return launch_bf16_decode<64, 3>(tw, tx, p, grid, stream);
+    default: return bd_deep(n_tiles * z, p.kblocks, M, splits, num_sms) ? launch_bf16_decode<64, 6>(tw, tx, p, grid, stream)
+                                                                        : launch_bf16_decode<64, 3>(tw, tx, p, grid, stream);
   }
+}
+
+// 1 if a launch of 64-token tiles has six stages, 0 if it has three
+extern "C" int b200_bf16_gemm_decode_ring(int clusters, int kblocks, int tokens, int splits, int num_sms) {
+  return splits >= 1 && splits <= 8 && bd_deep(clusters, kblocks, tokens, splits, num_sms);
 }
 
 // At most 128 tokens.

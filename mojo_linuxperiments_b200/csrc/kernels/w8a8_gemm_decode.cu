@@ -4,9 +4,10 @@
 //
 // The op is bound by the bytes of Wq, so the grid is shaped for bandwidth, not for the tensor core:
 //   * one CTA = 128 output channels x (K / S) of the reduction; the S CTAs of a cluster share one output tile;
-//   * shared memory is sized for two co-resident CTAs per SM (up to 64 tokens: with one CTA and seven stages the 64-token form took 29 us for
-//     28,672 x 4,096 at 40 tokens, with two and three stages each 22), which keeps 140 KB of TMA loads and more in flight per SM and lets CTAs of different tiles
-//     overlap head and tail.  The occupancy calculator answers "1 CTA per SM" for every kernel that allocates tensor
+//   * shared memory is sized for two co-resident CTAs per SM (33 to 64 tokens: with one CTA and seven stages 28,672 x 4,096 took 29 us
+//     at 40 tokens, with two and three stages each 22), which keeps 140 KB of TMA loads and more in flight per SM and lets CTAs of different tiles
+//     overlap head and tail.  Where a grid of 64-token tiles is no more than a CTA per SM, or may count on no more (all-reduce tail), the CTA has seven
+//     stages (b200_w8a8_gemm_decode_ring).  The occupancy calculator answers "1 CTA per SM" for every kernel that allocates tensor
 //     memory (tcgen05.alloc), whatever its other resources; in-kernel time stamps show two CTAs per SM running, so
 //     the host doubles the calculator's cluster counts for the two-CTA forms;
 //   * each CTA runs the usual TMA -> tcgen05.mma.kind::i8 -> TMEM pipeline (weights are the 128-row A operand, the
@@ -143,7 +144,7 @@ constexpr int decode_smem_bytes(int bn, int stages, bool xch = true) {
 // 65 to 128 tokens: the persistent kernel's tiles of 128 tokens x 64 to 256 channels leave most SMs idle or run in two rounds;
 // which of the two kernels takes a call is decided in b200_w8a8_gemm_decode_takes.
 template <int BN, int STAGES, bool XCH = true>
-__global__ void __launch_bounds__(GEMM_THREADS, ((BN > 64 && XCH) ? 1 : 2))
+__global__ void __launch_bounds__(GEMM_THREADS, ((BN * STAGES > 3 * 64 && XCH) ? 1 : 2))
 w8a8_gemm_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                         const DecodeGemmParams p) {
   constexpr int A_BYTES = TILE_N * BLOCK_K;
@@ -915,9 +916,9 @@ static int resident_clusters(int bn, int s) {
   return resident_clusters_reported(bn, s) * ctas_per_sm(bn);
 }
 
-// Clusters that a launch whose CTAs wait for one another may count on: the 64-token form's two CTAs fill an SM's shared memory to the last
-// 256 bytes, so there the calculator's answer stands.
-static int waiting_clusters(int bn, int s) { return bn == 64 ? resident_clusters_reported(bn, s) : resident_clusters(bn, s); }
+// Clusters that a launch whose CTAs wait for one another may count on: the 64-token form's two CTAs would fill an SM's shared memory to the
+// last 256 bytes, so there the calculator's answer stands, and the CTA that an SM holds has seven stages.
+static int waiting_clusters(int bn, int s) { return bn == 64 ? max_resident_clusters<64, 7>(s) : resident_clusters(bn, s); }
 
 static int resident_clusters_reported(int bn, int s) {
   switch (bn) {
@@ -949,6 +950,24 @@ int decode_pick_splits(int tiles, int kblocks, int num_sms, int bn, int margin, 
 }  // namespace b200
 
 using namespace b200;
+
+// 33 to 64 tokens (and narrow outputs of more): which of the two forms, two CTAs per SM with three stages or one with seven.  tiles: clusters
+// of the launch; one[s]: clusters of s CTAs that run at once with one per SM; fixed: the split is not to be changed.  Returns 2 * splits + (seven stages).
+//   A grid that is no more than a CTA per SM has only three stages in flight there: seven, unless a CTA has too few blocks to fill them.  us, three |
+//   seven stages, same split, at 33 and 64 tokens: 512 x 14,336 8.9, 9.7 | 7.7, 8.7; 1,024 x 28,672 14.6, 15.3 | 12.4, 13.2; 1,536 x 8,192 8.2, 9.1 |
+//   8.2, 8.3; 18,944 x 4,096 18.1, 18.5 | 16.2, 16.4; the other way round 1,024 x 2,048 at 33 4.6 | 4.9, 18,944 x 1,024 at 64 7.9 | 8.5, and fifteen
+//   clusters of eight (all that there are) 1,920 x 8,192 at 33 7.7 | 8.2.
+//   75 to 148 tiles: whole tiles with seven stages instead of two or three CTAs for each with three, for as long as the exchange is not paid back by
+//   the SMs that whole tiles leave idle.  12,800 x 1,024 7.7, 10.1 | 7.1, 7.3; 16,384 x 4,096 15.7, 17.5 | 14.9, 15.2; 14,336 x 8,192 23.2, 25.6 | 23.7, 24.0;
+//   12,800 x 14,336 34.4, 36.5 | 36.5, 36.9; three CTAs each: 10,240 x 1,024 7.0, 8.5 | 6.5, 6.9, x 2,048 8.7, 10.0 | 9.7, 9.9, x 4,096 11.4, 12.8 | 13.9, 14.3.
+extern "C" int b200_w8a8_gemm_decode_ring(int tiles, int kblocks, int tokens, int splits, int fixed, const int* one) {
+  const bool many = tokens > 48;
+  if (!fixed && (splits == 2 || splits == 3) && tiles > one[2] && tiles <= one[1] &&
+      (splits == 2 ? many || kblocks <= 32 : kblocks <= (many ? 16 : 8))) return 2 * 1 + 1;
+  const int blocks = (kblocks + splits - 1) / splits;
+  const bool fits = tiles + (splits > 1 ? 1 : 0) <= one[splits];
+  return 2 * splits + (fits && (splits == 1 ? blocks >= 16 : blocks > 3 || many) ? 1 : 0);
+}
 
 static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, const float* sw, void* y,
                             const void* residual, int M, int N, int K, int ldy, int out_fp32, int* status,
@@ -994,6 +1013,14 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
   if (!inl) s = force_splits > 0 ? force_splits : decode_pick_splits(n_tiles * m_tiles, p.kblocks, num_sms, bn, 1, qp ? M : 0,
                                                                      ar ? ar_min_kb : 2);
   if (s < 1 || s > 8) return -1;
+  bool deep = false;
+  if (bn == 64) {
+    int one[9] = {};
+    for (int c = 1; c <= 8; ++c) one[c] = max_resident_clusters<64, 7>(c);
+    const int r = b200_w8a8_gemm_decode_ring(n_tiles * m_tiles + (qp && !inl ? (M + s - 1) / s : 0), p.kblocks, M, s, force_splits > 0 || qp, one);
+    deep = ar || (r & 1);
+    if (!ar) s = r >> 1;
+  }
   p.splits = s;
   p.sx = sx; p.sw = sw; p.y = y; p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.ldy = ldy; p.out_fp32 = out_fp32; p.status = status; p.limit_ns = 2000000000ull;
@@ -1041,7 +1068,7 @@ static int decode_gemm_impl(const void* xq, const float* sx, const void* wq, con
   switch (bn) {
     case 16: return launch_decode<16, 5>(tw, tx, p, grid, stream);
     case 32: return launch_decode<32, 4>(tw, tx, p, grid, stream);
-    case 64: return launch_decode<64, 3>(tw, tx, p, grid, stream);
+    case 64: return deep ? launch_decode<64, 7>(tw, tx, p, grid, stream) : launch_decode<64, 3>(tw, tx, p, grid, stream);
     default: return s > 1 ? launch_decode<128, 4>(tw, tx, p, grid, stream) : launch_decode<128, 3, false>(tw, tx, p, grid, stream);
   }
 }

@@ -69,6 +69,8 @@ class _Sig:
     b200_w8a8_gemm_decode = (I, [P, P, P, P, P, P, I, I, I, I, I, P, I, I, P])
     b200_w8a8_gemm_decode_resident_clusters = (I, [I, I])
     b200_w8a8_gemm_decode_takes = (I, [I, I, I, I])
+    b200_w8a8_gemm_decode_ring = (I, [I, I, I, I, I, P])
+    b200_bf16_gemm_decode_ring = (I, [I, I, I, I, I])
     b200_w8a8_gemm_decode_p = (I, [P, P, P, P, P, I, I, I, I, I, P, I, P])
     b200_w8a8_gemm_decode_ar_p = (I, [P, P, P, P, P, I, I, I, I, P, I, P, P, P, I, I, c_size_t, c_size_t, P, I, I, c_size_t, c_size_t, c_size_t, I, c_size_t, c_size_t, c_size_t, P])
     b200_peer_allreduce = (I, [P, P, P, I, I, c_size_t, c_size_t, P, P, c_size_t, I, I, P, P, I, I, I, P])

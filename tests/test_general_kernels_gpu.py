@@ -616,3 +616,25 @@ def test_f32_linear_takes_the_values_of_force_that_choose_a_bf16_tile():
     want = D.linear(x, w)[:, :200]
     for force in (9, 64, 256, -64, -256):
         assert torch.equal(D.linear(x, w, force=force)[:, :200], want), force
+
+
+@pytest.mark.parametrize("M", [33, 48, 49, 64])
+@pytest.mark.parametrize("N,K", [(512, 4096), (1920, 1024), (4352, 1040), (12928, 1024), (18944, 2048), (19072, 512)])
+def test_decode_linears_with_either_ring(M, N, K):
+    """Grids on both sides of a CTA per multiprocessor, whole tiles and split ones.  int8: whole numbers until the scales (two fp32 roundings) and the
+    store (bf16, 2^-8).  bf16: products are exact, fp32 sums of K terms of random signs are off by less than 1e-5 of the largest, the store 2^-8."""
+    from mojo_linuxperiments_b200.ops import dense as D
+    from mojo_linuxperiments_b200.ops import linear as L
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    x = torch.randint(-127, 128, (M, K), dtype=torch.int8, device=DEV, generator=g)
+    w = torch.randint(-127, 128, (N, K), dtype=torch.int8, device=DEV, generator=g)
+    sx, sw = torch.rand(M, device=DEV, generator=g), torch.rand(N, device=DEV, generator=g)
+    want = (x.double() @ w.double().t()) * sx.double()[:, None] * sw.double()
+    y = L.w8a8_gemm(x, sx, w, sw)
+    assert ((y.double() - want).abs() <= want.abs() * (2.0 ** -8 + 2.0 ** -22)).all()
+    xb = torch.randn((M, K), device=DEV, generator=g).to(torch.bfloat16)
+    wb = (torch.randn((N, K), device=DEV, generator=g) * K ** -0.5).to(torch.bfloat16)
+    want = xb.double() @ wb.double().t()
+    y = D.linear(xb, D.DenseW.of(wb, torch.bfloat16, DEV))[:, :N].double()
+    assert ((y - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5 * want.abs().max()).all()
+    _ok()

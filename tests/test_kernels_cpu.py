@@ -150,3 +150,25 @@ def test_the_experts_kernel_leaves_its_loop_with_all_epilogue_warps_or_none():
 
 def test_f32_tensor_core_linear_takes_no_more_columns_than_its_grid_has(lib):
     assert lib.b200_f32_gemm_tc_takes(16, 65535 * 128, 2048) == 1 and lib.b200_f32_gemm_tc_takes(16, 65535 * 128 + 1, 2048) == 0
+
+
+def test_decode_linears_of_up_to_64_tokens_fill_the_shared_memory_they_have(lib):
+    """A grid of no more than a CTA per multiprocessor has the deep ring; a fuller one two CTAs with three stages.  Measured on both sides; clusters of
+    1 .. 8 CTAs that 148 multiprocessors hold with one CTA each."""
+    import ctypes
+    one = (ctypes.c_int * 9)(0, 148, 74, 45, 33, 26, 22, 15, 15)
+
+    def ring(n, k, tokens, splits, fixed=0):
+        r = lib.b200_w8a8_gemm_decode_ring((n + 127) // 128, k // 128, tokens, splits, fixed, one)
+        return r >> 1, r & 1
+    assert ring(512, 14336, 33, 8) == (8, 1) and ring(1536, 2048, 64, 8) == (8, 1) and ring(18944, 4096, 40, 1) == (1, 1)
+    assert ring(1024, 2048, 33, 8) == (8, 0) and ring(1920, 8192, 64, 8) == (8, 0) and ring(2048, 4096, 64, 8) == (8, 0)
+    assert ring(18944, 1024, 64, 1) == (1, 0) and ring(28672, 4096, 64, 1) == (1, 0) and ring(8192, 4096, 64, 4) == (4, 0)
+    assert ring(16384, 4096, 33, 2) == (1, 1) and ring(16384, 8192, 33, 2) == (2, 0) and ring(16384, 8192, 64, 2) == (1, 1)
+    assert ring(10240, 1024, 33, 3) == (1, 1) and ring(10240, 2048, 33, 3) == (3, 0) and ring(10240, 4096, 64, 3) == (3, 0)
+    assert ring(16384, 4096, 64, 2, fixed=1) == (2, 0)
+
+    def bf(n, k, tokens, splits):
+        return lib.b200_bf16_gemm_decode_ring((n + 127) // 128, k // 64, tokens, splits, 148)
+    assert bf(512, 14336, 33, 8) == 1 and bf(1536, 1024, 64, 8) == 1 and bf(4096, 4096, 33, 4) == 1
+    assert bf(4096, 1024, 33, 4) == 0 and bf(2048, 4096, 64, 8) == 0 and bf(6144, 4096, 64, 4) == 0 and bf(512, 4096, 64, 9) == 0
