@@ -457,10 +457,11 @@ def test_f32_linear_in_three_parts_where_it_is_not_finite():
 
 @pytest.mark.parametrize("H,G,dk,dv,chunk,spans", [(8, 2, 128, 128, None, [(0, 127), (0, 128), (0, 129), (37, 300)]), (6, 2, 64, 96, 200, [(0, 257), (150, 260), (5, 1)]),
                                                    (3, 3, 40, 16, 70, [(0, 513), (64, 130)]), (16, 4, 128, 128, 512, [(300 * (i % 2), 200 + 40 * i) for i in range(12)]),
-                                                   (5, 1, 8, 128, 128, [(100, 400), (0, 256)])])
+                                                   (5, 1, 8, 128, 128, [(100, 400), (0, 256)]), (16, 4, 128, 128, None, [(0, 128), (300, 100)]),
+                                                   (16, 4, 64, 64, 200, [(100 * i, 128 - 9 * i) for i in range(10)])])
 def test_paged_prefill_attention_pairs_heads_or_query_tiles(H, G, dk, dv, chunk, spans):
     """(first position, tokens) of portions.  Two heads of a KV head share a CTA; an odd number of them: two query tiles, the second of which
-    may start in a later chunk.  Tile edges, portions that continue, more items than CTAs.  bf16 weights and outputs: 2^-8 of values up to 4."""
+    may start in a later chunk; one query tile each of a few portions: a head alone.  Tile edges, portions that continue, more items than CTAs.  bf16 weights and outputs: 2^-8 of values up to 4."""
     from mojo_linuxperiments_b200.ops import attention as A
     ps, B = 16, len(spans)
     g = torch.Generator(device=DEV).manual_seed(dk + B)
