@@ -381,7 +381,7 @@ extern "C" int b200_attn_prefill_paged(const void* q, long long ldq, void* out, 
   const int q_tiles = (max_len + PP_BM - 1) / PP_BM;
   p.B = B;
   // One query tile per portion, and an SM for every head: a unit alone ends sooner than two that take turns.  us, 16 heads over 8, heads of a pair together |
-  // alone: 1 x 128 9.9 | 7.8 (9.2 with a head per CTA before), 1 x 20 8.5 | 7.2, 100 behind 8,000 152 | 127
+  // alone: 1 x 128 9.9 | 8.3 (9.2 with a head per CTA before), 1 x 20 8.5 | 7.7, 100 behind 8,000 152 | 128
   p.pair_heads = (hq / c->kv_heads) % 2 == 0 && !(q_tiles == 1 && static_cast<long long>(hq) * B <= 148);
   p.q_steps = p.pair_heads ? q_tiles : (q_tiles + 1) / 2;
   p.columns = p.pair_heads ? hq / 2 : hq;

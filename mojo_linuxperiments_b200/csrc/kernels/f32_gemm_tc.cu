@@ -54,13 +54,42 @@ constexpr int FC_SMEM = 2 * FC_BUFFER + FC_TILE * FC_OUT_PITCH * 4 + 1024 + 64;
 // columns of tensor memory: two accumulators of x1 w1 blocks, two of the small products
 constexpr uint32_t FC_MAIN = 0, FC_SMALL = 256;
 
-// the general way for one output, in case the fast one is not finite
-__device__ __noinline__ float f32_tc_dot(const float* x, const float* w, int K) {
-  float s = 0.f;
-  for (int k = 0; k < K; ++k) s = fmaf(x[k], w[k], s);
-  return s;
-}
 __device__ __forceinline__ bool not_finite(float v) { return !(fabsf(v) <= 3.4028234663852886e38f); }
+// The general way, by a whole warp, for the outputs of row x of which the fast one is not finite: lane l has columns 4 l .. of the `columns`
+// that begin at w.  A row with a NaN is all NaN; else a fused multiply-add chain per lane and the sum of those.  (One column after the other:
+// serial sums by the lanes that own them took 71 ms for 1,000 x 4,096 x 4,096 all NaN, which take 0.9 on the CUDA cores.)
+__device__ __noinline__ float4 f32_tc_again(const float* x, const float* w, long long ldw, int columns, int K, float4 was) {
+  float o[4] = {was.x, was.y, was.z, was.w};
+  const int lane = threadIdx.x & 31;
+  bool nan = false;
+  for (int k = 4 * lane; k < K; k += 128)
+    for (int i = k; i < min(k + 4, K); ++i) nan = nan || isnan(x[i]);
+  if (__any_sync(0xffffffffu, nan)) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) if (not_finite(o[j])) o[j] = __uint_as_float(0x7fffffffu);
+    return make_float4(o[0], o[1], o[2], o[3]);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    for (uint32_t left = __ballot_sync(0xffffffffu, 4 * lane + j < columns && not_finite(o[j])); left; left &= left - 1) {
+      const int owner = __ffs(left) - 1;
+      const float* y = w + (4 * owner + j) * ldw;
+      float s = 0.f;
+#pragma unroll 4
+      for (int k = 4 * lane; k < K; k += 128) {
+        if (k + 4 <= K) {
+          const float4 a = *reinterpret_cast<const float4*>(x + k), b = *reinterpret_cast<const float4*>(y + k);
+          s = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
+        } else {
+          for (int i = k; i < K; ++i) s = fmaf(x[i], y[i], s);
+        }
+      }
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+      if (lane == owner) o[j] = s;
+    }
+  return make_float4(o[0], o[1], o[2], o[3]);
+}
 
 // two numbers -> their leading bf16 parts (first in the low half); what is left of them replaces them
 __device__ __forceinline__ uint32_t take_bf16(float2& v) {
@@ -237,8 +266,8 @@ __global__ void __launch_bounds__(FC_THREADS, 1) f32_gemm_tc_kernel(const __grid
   tc_fence_before();
   if (S > 1) cluster_sync_all(); else __syncthreads();
   // this CTA finishes every S-th row of the tile, adding the cluster's partial tiles in rank order
-  const int col = lane * 4;
-  if (warp < FC_WORKERS && n0 + col < p.N && !*abort_flag)
+  const int col = lane * 4, columns = min(FC_TILE, p.N - n0);
+  if (warp < FC_WORKERS && !*abort_flag)
     for (int r = warp * S + rank; r < min(FC_TILE, p.M - m0); r += FC_WORKERS * S) {
       const uint32_t at = smem_u32(tile + r * FC_OUT_PITCH + col);
       float o[4] = {0.f, 0.f, 0.f, 0.f};
@@ -248,10 +277,10 @@ __global__ void __launch_bounds__(FC_THREADS, 1) f32_gemm_tc_kernel(const __grid
                      : "=f"(part.x), "=f"(part.y), "=f"(part.z), "=f"(part.w) : "r"(S > 1 ? mapa_shared(at, s) : at) : "memory");
         o[0] += part.x; o[1] += part.y; o[2] += part.z; o[3] += part.w;
       }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (not_finite(o[j]) && n0 + col + j < p.N) o[j] = f32_tc_dot(p.x + (m0 + r) * p.ldx, p.w + (n0 + col + j) * p.ldw, p.K);
-      epi_apply4(p.epi, m0 + r, n0 + col, make_float4(o[0], o[1], o[2], o[3]));
+      float4 v = make_float4(o[0], o[1], o[2], o[3]);
+      const bool bad = col < columns && (not_finite(o[0]) || not_finite(o[1]) || not_finite(o[2]) || not_finite(o[3]));
+      if (__any_sync(0xffffffffu, bad)) v = f32_tc_again(p.x + (m0 + r) * p.ldx, p.w + n0 * p.ldw, p.ldw, columns, p.K, v);
+      if (col < columns) epi_apply4(p.epi, m0 + r, n0 + col, v);
     }
   if (S > 1) cluster_sync_all(); else __syncthreads();           // nobody leaves while its tile is being read
   if (warp == FC_WORKERS) { tc_fence_after(); tmem_dealloc(tmem, 512); }
