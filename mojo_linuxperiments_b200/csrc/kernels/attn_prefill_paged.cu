@@ -5,7 +5,8 @@
 // run from the start of the first row's chunk (rounded down to a page) to the last row's position, in tiles of 128 tokens = 8 pages.
 //
 // As in attn_prefill.cu a work item is two blocks ("units") of 128 query rows that walk the same KV tiles: two heads of one KV head, or,
-// where a KV head has an odd number of heads, two neighbouring query tiles of one head; one CTA per SM takes items, long ones first.
+// where a KV head has an odd number of heads, two neighbouring query tiles of one head (a few portions of one tile: a head alone); one CTA per
+// SM takes items, long ones first.
 //   warp 0       TMA producer: the Q block of each unit, K and V pages (16 x 64-column boxes straight into the swizzled operand
 //                layout) into two-stage rings; lane <-> page.  Pages past the last key are requested at an out-of-range
 //                coordinate, which fills with zeros.
